@@ -15,7 +15,7 @@ __device__ __forceinline__ double vx_sp(const double a[2], const double b[2]) {
     return a[0] * b[0] + a[1] * b[1];
 }
 
-VX_DEVK void k_panel_influence_body(VxBlkB<0, 0> vb, const vx_panel *pan, int P, double *L) {
+VX_DEVK void k_panel_influence_body(VxBlkB<0, 0> vb, const vx_panel *pan, int P, double *L, long long ld) {
     const long long S = P + 1;
     for (long long e = vb.x * (long long)blockDim.x + threadIdx.x; e < S * S;
          e += (long long)vb.n * blockDim.x) {
@@ -73,12 +73,12 @@ VX_DEVK void k_panel_influence_body(VxBlkB<0, 0> vb, const vx_panel *pan, int P,
                              - (q21 * c1[0] + q22 * c2[0] + q23 * c3[0]));
             val = v0 * pi.tang[0] + v1 * pi.tang[1];
         }
-        L[e] = val;
+        L[i * ld + j] = val;
     }
 }
-__global__ void k_panel_influence(const vx_panel *pan, int P, double *L) {
+__global__ void k_panel_influence(const vx_panel *pan, int P, double *L, long long ld) {
     VX_PDL_WAIT();
-    k_panel_influence_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, pan, P, L);
+    k_panel_influence_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, pan, P, L, ld);
 }
 
 VX_DEVK void k_identity_body(VxBlkB<0, 0> vb, double *A, long long S) {
@@ -232,19 +232,32 @@ __global__ void k_gj_scale(const double *A, double *Inv, long long S, const int 
     k_gj_scale_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, A, Inv, S, flag);
 }
 
-// d_work must hold 2 (P+1)^2 + (P+1) doubles.  *d_flag is set when a pivot
-// falls below 1e-12 (the reference returns NULL then).
+// Doubles of scratch vx_build_matrix needs.
+long long vx_matrix_work(int P) {
+    const long long S = P + 1;
+    return std::max(2 * S * S + S, vx_gj_fits(S) ? vx_gj_work(S) : 0LL);
+}
+
+// *d_flag is set when a pivot falls below 1e-12 (the reference returns NULL
+// then).  The elimination goes in blocks of columns (vx_gj.cu) for the
+// systems whose rows fit the threads of a cluster, 4095 panels; a larger
+// one column by column, two launches each.
 cudaError_t vx_build_matrix(const VxLaunch &L, const vx_panel *d_pan, int P, double *d_minv,
                             double *d_work, int *d_flag, double *d_L_out, int robust) {
     const long long S = P + 1;
     double *A = d_work;
     double *c = d_work + S * S;
     const int grid = L.num_sms * 4;
+    const bool blocked = robust != 3 && vx_gj_fits(S);
+    const long long ld = blocked ? vx_gj_stride(S) : S;
     cudaMemsetAsync(d_flag, 0, sizeof(int), L.stream);
-    vx_launch<k_panel_influence, k_panel_influence_body>(L, grid, 256, 0, d_pan, P, A);
-    if (d_L_out) cudaMemcpyAsync(d_L_out, A, sizeof(double) * S * S, cudaMemcpyDeviceToDevice, L.stream);
+    vx_launch<k_panel_influence, k_panel_influence_body>(L, grid, 256, 0, d_pan, P, A, ld);
+    if (d_L_out)
+        cudaMemcpy2DAsync(d_L_out, sizeof(double) * S, A, sizeof(double) * ld, sizeof(double) * S, S,
+                          cudaMemcpyDeviceToDevice, L.stream);
     if (robust == 3)   // blocked LU with partial pivoting (vx_lu.cu)
         return vx_invert_lu(L, A, d_minv, S, reinterpret_cast<int *>(c), d_flag);
+    if (blocked) return vx_invert_gj(L, A, d_minv, S, d_flag, robust);
     vx_launch<k_identity, k_identity_body>(L, grid, 256, 0, d_minv, S);
     for (long long k = 0; k < S - 1; ++k) {
         vx_launch<k_gj_pivot, k_gj_pivot_body>(L, 1, 1024, 0, A, d_minv, S, k, c, d_flag, robust);

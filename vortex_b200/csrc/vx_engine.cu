@@ -556,7 +556,7 @@ extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t
     if (cudaMalloc(&s->d_minv, sizeof(double) * S1 * S1) != cudaSuccess) return fail(VX_ERR_NOMEM);
     double *work = nullptr;
     int *flag = nullptr;
-    if (cudaMalloc(&work, sizeof(double) * (2 * S1 * S1 + S1)) != cudaSuccess) return fail(VX_ERR_NOMEM);
+    if (cudaMalloc(&work, sizeof(double) * vx_matrix_work((int)P)) != cudaSuccess) return fail(VX_ERR_NOMEM);
     if (cudaMalloc(&flag, sizeof(int)) != cudaSuccess) { cudaFree(work); return fail(VX_ERR_NOMEM); }
     VxLaunch L = launch_of(s);
     const int mode = conf->gj_pivot == 1 ? 1 : (conf->gj_pivot == 3 ? 3 : 0);

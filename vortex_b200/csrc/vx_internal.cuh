@@ -711,7 +711,16 @@ cudaError_t vx_build_matrix(const VxLaunch &L, const vx_panel *d_pan, int P, dou
                             double *d_work, int *d_flag, double *d_L_out,
                             int robust = 0);
 // robust: 0 the reference's pivot rule, 1 Gauss-Jordan with partial
-// pivoting, 3 blocked LU with partial pivoting (vx_invert_lu).
+// pivoting, 3 blocked LU with partial pivoting (vx_invert_lu).  d_work:
+// vx_matrix_work(P) doubles.
+long long vx_matrix_work(int P);
+// The Gauss-Jordan inverse in blocks of columns (vx_gj.cu): systems it takes,
+// the row stride and the scratch (doubles, the matrix first) of a system of
+// S rows.
+bool vx_gj_fits(long long S);
+long long vx_gj_stride(long long S);
+long long vx_gj_work(long long S);
+cudaError_t vx_invert_gj(const VxLaunch &L, double *A, double *Inv, long long S, int *flag, int robust);
 // A (n x n) -> Inv = A^-1 by blocked LU with partial pivoting; A is
 // overwritten, piv holds n ints; *flag set on a pivot below 1e-12.
 cudaError_t vx_invert_lu(const VxLaunch &L, double *A, double *Inv, long long n, int *piv, int *flag);

@@ -202,7 +202,7 @@ double *matr_creation(vx_panel *panels, size_t s, size_t birth) {
     bool ok = cudaMalloc(&d_pan, sizeof(vx_panel) * s) == cudaSuccess &&
               cudaMalloc(&d_minv, sizeof(double) * S1 * S1) == cudaSuccess &&
               cudaMalloc(&d_L, sizeof(double) * S1 * S1) == cudaSuccess &&
-              cudaMalloc(&d_work, sizeof(double) * (2 * S1 * S1 + S1)) == cudaSuccess &&
+              cudaMalloc(&d_work, sizeof(double) * vx_matrix_work((int)s)) == cudaSuccess &&
               cudaMalloc(&d_flag, sizeof(int)) == cudaSuccess &&
               cudaMemcpy(d_pan, panels, sizeof(vx_panel) * s, cudaMemcpyHostToDevice) == cudaSuccess;
     if (ok) {
