@@ -261,168 +261,220 @@ __device__ __forceinline__ void fmm_shift_table(cplx (*se)[P]) {
     }
 }
 
-// P2M of leaf c (level L, m leaves a side), by one warp: each lane expands
-// its own vortices (FP64 positions), then a fixed butterfly sums the lanes.
-// An empty leaf is not written (nothing reads its expansion).
-template <int P>
-__device__ __forceinline__ void fmm_p2m_leaf(const VxView &v, const VxScalars *S, const int *start,
-                                             const int *sorted, cplx *ML, long long c, long long m, int lane) {
-    const int j0 = start[c], j1 = start[c + 1];
-    if (j0 == j1) return;
-    const long long n = S->n;
-    const double h = S->fside / (double)m;
-    cplx b[P];
-#pragma unroll
-    for (int k = 0; k < P; ++k) b[k] = {0.0, 0.0};
-    const double cx = S->fx0 + ((double)(c % m) + 0.5) * h, cy = S->fy0 + ((double)(c / m) + 0.5) * h;
-    for (int q = j0 + lane; q < j1; q += 32) {
-        const long long j = sorted[q];
-        if (j >= n) continue;
-        const double gj = v.g[j * v.ps];
-        const cplx w = {(v.x[j * v.ps] - cx) / h, (v.y[j * v.ps] - cy) / h};
-        cplx pw = {gj, 0.0};   // G w^k / k!
-#pragma unroll
-        for (int k = 0; k < P; ++k) {
-            b[k] = cadd(b[k], pw);
-            pw = cscale(cmul(pw, w), c_fmm_inv[k + 1]);
-        }
-    }
-    // reduce-scatter over the warp: at each halving the lane keeps the half
-    // of its values selected by its lane bit and adds the partner's copy of
-    // it (31 shuffles instead of 160 for an all-reduce of 32 values);
-    // afterwards lane q holds value q = coefficient q/2, part q&1
-    // (in groups of 16 coefficients, the last one padded with zeros)
-#pragma unroll
-    for (int g0 = 0; g0 < P; g0 += 16) {
-        double vv[32];
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            const int kk = min(g0 + k, P - 1);
-            vv[2 * k] = g0 + k < P ? b[kk].r : 0.0;
-            vv[2 * k + 1] = g0 + k < P ? b[kk].i : 0.0;
-        }
-#pragma unroll
-        for (int half = 16; half > 0; half >>= 1) {
-            const bool up = (lane & half) != 0;
-#pragma unroll
-            for (int i = 0; i < half; ++i) {
-                const double send = up ? vv[i] : vv[i + half];
-                const double keep = up ? vv[i + half] : vv[i];
-                vv[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
-            }
-        }
-        if (g0 + (lane >> 1) < P) reinterpret_cast<double *>(ML + c * P)[2 * g0 + lane] = vv[0];
-    }
+// The upward pass.  A warp takes a cell of level L - 1: P2M of its four
+// leaves (8 lanes each, a lane every eighth vortex of the leaf, FP64
+// positions), then M2M of the cell from the coefficients just summed, in
+// shared memory; a block's four warps are the children of a cell of level
+// L - 2, which its first warp sums last.  Eight lanes a leaf keep the sum over
+// the lanes short (28 shuffles for four leaves; a warp a leaf, 31 each, spent
+// most of its time on them) and a block's chain is two levels whatever the
+// depth: 4^(L-2) blocks instead of 4^(L-3), with one leaf after another a
+// quarter as long.  Upward pass (this kernel and k_fmm_up_top, event times) at
+// 2e4 vortices 87 -> 26 us, at 1e6 131 -> 68, at 3e6 370 -> 192; bound by the
+// gathers of the positions and the levels' latency.
+//
+// Expansions of empty cells are not written: nothing reads them (the counts
+// of all levels start at zero).  Levels 1 and 0 have no interactions and are
+// not summed beyond what a block of a shallow tree writes on its way.
+constexpr int FMM_TOP = 3;  // levels below this one are left to the last block of the upward pass
+constexpr int UP_W = 4;     // warps of a block of k_fmm_up
+
+__device__ __forceinline__ double fmm_pow2n(int k) {   // 2^-k
+    return __longlong_as_double((long long)(1023 - k) << 52);
 }
 
-// M2M of coefficient k of cell c of level l from its 4 children at level
-// l+1; the thread of coefficient 0 also writes the cell's vortex count (the
-// sum of its children's).  Children are read through L2: in the fused
-// upward kernels another block of the same launch may have written them.
+// M2M of one cell by one warp, coefficients of the children q = 0..3 in
+// src[q][m], already scaled by 2^-m: lane (k, q) sums the terms of
+// coefficient k from child q, four lanes add up (all get the sum).
 template <int P>
-__device__ __forceinline__ void fmm_m2m_cell(const cplx (*se)[P], int *cnt, cplx *M, int l, long long c, int k) {
-    const long long m = 1LL << l, m2 = 2 * m;
-    cplx *Mp = M + fmm_level_off(l) * P;
-    const cplx *Mc = M + fmm_level_off(l + 1) * P;
-    int *cp = cnt + fmm_level_off(l);
-    const int *cc = cnt + fmm_level_off(l + 1);
-    const long long ix = c % m, iy = c / m;
-    int nq[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) nq[q] = __ldcg(&cc[(2 * iy + (q >> 1)) * m2 + 2 * ix + (q & 1)]);
-    const int np = nq[0] + nq[1] + nq[2] + nq[3];
-    if (k == 0) cp[c] = np;
+__device__ __forceinline__ cplx fmm_m2m_terms(const cplx (*se)[P], const cplx (*src)[P], int k, int q) {
     cplx b = {0.0, 0.0};
-    if (np > 0) {
-        for (int q = 0; q < 4; ++q) {
-            const long long child = (2 * iy + (q >> 1)) * m2 + 2 * ix + (q & 1);
-            if (nq[q] == 0) continue;
-            // unrolled over the P terms (those above k predicated off), so
-            // the child's coefficients are loaded together, not one L2
-            // round trip per term
 #pragma unroll
-            for (int mm = 0; mm < P; ++mm) {
-                if (mm <= k) {
-                    const double2 t = __ldcg(reinterpret_cast<const double2 *>(&Mc[child * P + mm]));
-                    b = cadd(b, cscale(cmul(se[q][k - mm], cplx{t.x, t.y}), ldexp(1.0, -mm)));
+    for (int m = 0; m < P; ++m)
+        if (m <= k) {
+            const cplx e = se[q][k - m], t = src[q][m];
+            b.r = fma(e.r, t.r, fma(-e.i, t.i, b.r));
+            b.i = fma(e.r, t.i, fma(e.i, t.r, b.i));
+        }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+        b.r += __shfl_xor_sync(0xffffffffu, b.r, o);
+        b.i += __shfl_xor_sync(0xffffffffu, b.i, o);
+    }
+    return b;
+}
+
+template <int P>
+VX_DEVK void k_fmm_up_body(VxBlkB<32 * UP_W, 4> vb, const VxView &v, const VxScalars *S, const int *start,
+                           const int *sorted, int *cnt, cplx *M) {
+    constexpr int V = 2 * P / 8;   // values a lane keeps of its leaf's 2 P
+    __shared__ cplx se[4][P];
+    __shared__ double sf[P];                // 1 / k!
+    __shared__ cplx sb[UP_W][4][P];         // the leaves' coefficients times 2^-k
+    __shared__ cplx sp[4][P];               // and those of level L - 1
+    __shared__ int sn[UP_W];
+    const int L = S->fL;
+    if (L < 2) return;   // no expansions
+    const long long m = 1LL << L, n = S->n;
+    const double h = S->fside / (double)m, ih = 1.0 / h, fx0 = S->fx0, fy0 = S->fy0;
+    cplx *ML = M + fmm_level_off(L) * P, *M1 = M + fmm_level_off(L - 1) * P, *M2 = M + fmm_level_off(L - 2) * P;
+    int *cnt1 = cnt + fmm_level_off(L - 1), *cnt2 = cnt + fmm_level_off(L - 2);
+    fmm_shift_table<P>(se);
+    if (threadIdx.x == 0) {
+        double f = 1.0;
+        for (int k = 0; k < P; ++k) { sf[k] = f; f *= c_fmm_inv[k + 1]; }
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane >> 3, l8 = lane & 7;
+    const long long m2 = m >> 2;
+    for (long long r = vb.x; r < m2 * m2; r += vb.n) {
+        const long long px = 2 * (r % m2) + (warp & 1), py = 2 * (r / m2) + (warp >> 1);   // level L - 1
+        const long long ix = 2 * px + (q & 1), iy = 2 * py + (q >> 1), c = iy * m + ix;
+        const int j0 = start[c], j1 = start[c + 1];
+        const int np = __reduce_add_sync(0xffffffffu, l8 == 0 ? j1 - j0 : 0);
+        if (np > 0) {
+            double acc[2 * P];
+#pragma unroll
+            for (int k = 0; k < 2 * P; ++k) acc[k] = 0.0;
+            const double cx = fx0 + ((double)ix + 0.5) * h, cy = fy0 + ((double)iy + 0.5) * h;
+            long long jn = j0 + l8 < j1 ? sorted[j0 + l8] : n;
+            for (int t = j0 + l8; t < j1; t += 8) {
+                const long long j = jn;   // the next vortex's index is loaded before this one is expanded
+                jn = t + 8 < j1 ? sorted[t + 8] : n;
+                if (j >= n) continue;
+                const double wr = (v.x[j * v.ps] - cx) * ih, wi = (v.y[j * v.ps] - cy) * ih;
+                double pr = v.g[j * v.ps], pi = 0.0;   // G w^k
+#pragma unroll
+                for (int k = 0; k < P; ++k) {
+                    acc[2 * k] += pr;
+                    acc[2 * k + 1] += pi;
+                    const double nr = fma(pr, wr, -(pi * wi));
+                    pi = fma(pr, wi, pi * wr);
+                    pr = nr;
                 }
             }
+            __syncwarp();
+            // reduce-scatter over the leaf's eight lanes: at each halving a
+            // lane keeps the half its lane bit selects and adds the partner's
+            // copy of it; lane l8 ends with values V l8 ..
+#pragma unroll
+            for (int half = P, o = 4; o > 0; half >>= 1, o >>= 1) {
+                const bool up = (l8 & o) != 0;
+#pragma unroll
+                for (int i = 0; i < half; ++i) {
+                    const double send = up ? acc[i] : acc[i + half];
+                    const double keep = up ? acc[i + half] : acc[i];
+                    acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                const int e = V * l8 + i, k = e >> 1;
+                const double b = acc[i] * sf[k];
+                if (j1 > j0) reinterpret_cast<double *>(ML + c * P)[e] = b;
+                reinterpret_cast<double *>(sb[warp][q])[e] = b * fmm_pow2n(k);
+            }
+            __syncwarp();
         }
-    }
-    Mp[c * P + k] = b;
-}
-
-// M2M of levels hi-1 down to lo inside the subtree of cell r of level lo (one
-// block; a barrier between levels).
-template <int P>
-__device__ __forceinline__ void fmm_m2m_subtree(const cplx (*se)[P], int *cnt, cplx *M, int lo, int hi, long long r) {
-    const long long mlo = 1LL << lo, rx = r % mlo, ry = r / mlo;
-    for (int l = hi - 1; l >= lo; --l) {
-        const long long sl = 1LL << (l - lo), m = 1LL << l;
-        for (long long e = threadIdx.x; e < sl * sl * P; e += blockDim.x) {
-            const long long q = e / P;
-            const long long c = (ry * sl + q / sl) * m + rx * sl + q % sl;
-            fmm_m2m_cell<P>(se, cnt, M, l, c, (int)(e % P));
+        if (np > 0) {
+            const long long c1 = py * (m >> 1) + px;
+            if (lane == 0) cnt1[c1] = np;
+#pragma unroll
+            for (int k0 = 0; k0 < P; k0 += 8) {
+                const int k = k0 + (lane >> 2);
+                const cplx b = fmm_m2m_terms<P>(se, sb[warp], k < P ? k : P - 1, lane & 3);
+                if ((lane & 3) == 0 && k < P) {
+                    M1[c1 * P + k] = b;
+                    sp[warp][k] = cscale(b, fmm_pow2n(k));
+                }
+            }
+        } else {
+            for (int k = lane; k < P; k += 32) sp[warp][k] = cplx{0.0, 0.0};
+        }
+        if (lane == 0) sn[warp] = np;
+        __syncthreads();
+        const int np2 = sn[0] + sn[1] + sn[2] + sn[3];
+        if (warp == 0 && np2 > 0) {
+            if (lane == 0) cnt2[r] = np2;
+#pragma unroll
+            for (int k0 = 0; k0 < P; k0 += 8) {
+                const int k = k0 + (lane >> 2);
+                const cplx b = fmm_m2m_terms<P>(se, sp, k < P ? k : P - 1, lane & 3);
+                if ((lane & 3) == 0 && k < P) M2[r * P + k] = b;
+            }
         }
         __syncthreads();
     }
 }
-
-constexpr int FMM_UP = 3;   // levels of the upward pass per fused launch
-constexpr int FMM_TOP = 3;  // levels below this one are left to the last block of the upward pass
-
-// Upward pass, first part: a block takes a cell r of level lo = max(L - 3, 0),
-// computes P2M at the leaves of its subtree (one warp per leaf), then M2M of
-// the 3 levels above them.
 template <int P>
-VX_DEVK void k_fmm_up_body(VxBlkB<128, 4> vb, const VxView &v, const VxScalars *S, const int *start, const int *sorted,
-                           int *cnt, cplx *M) {
+__global__ void __launch_bounds__(32 * UP_W, 4) k_fmm_up(VxView v, const VxScalars *S, const int *start,
+                                                         const int *sorted, int *cnt, cplx *M) {
+    VX_PDL_WAIT();
+    k_fmm_up_body<P>(VxBlkB<32 * UP_W, 4>{blockIdx.x, gridDim.x}, v, S, start, sorted, cnt, M);
+}
+
+// M2M of the cells of level l below cell r of level lo, a warp per cell.
+// Children are read through L2: another block of the same launch may have
+// written them.
+template <int P>
+__device__ __forceinline__ void fmm_m2m_level(const cplx (*se)[P], cplx (*src)[P], int *cnt, cplx *M, int lo, int l,
+                                              long long r) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const long long m = 1LL << l, m2 = 2 * m, mlo = 1LL << lo, sl = 1LL << (l - lo);
+    const int *cc = cnt + fmm_level_off(l + 1);
+    const cplx *Mc = M + fmm_level_off(l + 1) * P;
+    for (long long e = threadIdx.x >> 5; e < sl * sl; e += nw) {
+        const long long ix = (r % mlo) * sl + e % sl, iy = (r / mlo) * sl + e / sl;
+        // a child's count and coefficients are loaded side by side (an empty
+        // child's are whatever was there, and dropped)
+        int np = 0;
+#pragma unroll
+        for (int w0 = 0; w0 < 4 * P; w0 += 32) {
+            const int w = w0 + lane, q = min(w / P, 3), k = w % P;
+            const long long child = (2 * iy + (q >> 1)) * m2 + 2 * ix + (q & 1);
+            const int nq = __ldcg(&cc[child]);
+            const double2 t = __ldcg(reinterpret_cast<const double2 *>(&Mc[child * P + k]));
+            np += __reduce_add_sync(0xffffffffu, w < 4 * P && k == 0 ? nq : 0);
+            if (w < 4 * P) src[q][k] = nq > 0 ? cscale(cplx{t.x, t.y}, fmm_pow2n(k)) : cplx{0.0, 0.0};
+        }
+        __syncwarp();
+        if (np == 0) continue;
+        const long long c = iy * m + ix;
+        if (lane == 0) (cnt + fmm_level_off(l))[c] = np;
+#pragma unroll
+        for (int k0 = 0; k0 < P; k0 += 8) {
+            const int k = k0 + (lane >> 2);
+            const cplx b = fmm_m2m_terms<P>(se, src, k < P ? k : P - 1, lane & 3);
+            if ((lane & 3) == 0 && k < P) M[(fmm_level_off(l) + c) * P + k] = b;
+        }
+        __syncwarp();
+    }
+}
+
+// The rest of the upward pass: levels L - 3 up to 3, a block per cell of
+// level 3, then level 2 by the block that finishes last.
+constexpr int TOP_W = 16;
+template <int P>
+VX_DEVK void k_fmm_up_top_body(VxBlkB<32 * TOP_W, 0> vb, VxScalars *S, int *cnt, cplx *M) {
     __shared__ cplx se[4][P];
-    const int L = S->fL;
-    const int lo = max(L - FMM_UP, 0);
-    const long long m = 1LL << L, mlo = 1LL << lo, sl = 1LL << (L - lo);
-    cplx *ML = M + fmm_level_off(L) * P;
+    __shared__ cplx src[TOP_W][4][P];
+    const int hi = S->fL - 2;
+    if (hi < FMM_TOP) return;
     fmm_shift_table<P>(se);
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (long long r = vb.x; r < mlo * mlo; r += vb.n) {
-        const long long rx = r % mlo, ry = r / mlo;
-        for (long long q = warp; q < sl * sl; q += nw)
-            fmm_p2m_leaf<P>(v, S, start, sorted, ML, (ry * sl + q / sl) * m + rx * sl + q % sl, m, lane);
-        __syncthreads();
-        fmm_m2m_subtree<P>(se, cnt, M, lo, L, r);
-    }
+    const int warp = threadIdx.x >> 5;
+    for (long long r = vb.x; r < (1LL << (2 * FMM_TOP)); r += vb.n)
+        for (int l = hi - 1; l >= FMM_TOP; --l) {
+            fmm_m2m_level<P>(se, src[warp], cnt, M, FMM_TOP, l, r);
+            __syncthreads();
+        }
+    if (!vx_last_block(&S->sync_ctr, vb.n)) return;
+    fmm_m2m_level<P>(se, src[warp], cnt, M, 0, FMM_TOP - 1, 0);
 }
 template <int P>
-__global__ void __launch_bounds__(128) k_fmm_up(VxView v, const VxScalars *S, const int *start, const int *sorted,
-                                                int *cnt, cplx *M) {
+__global__ void __launch_bounds__(32 * TOP_W) k_fmm_up_top(VxScalars *S, int *cnt, cplx *M) {
     VX_PDL_WAIT();
-    k_fmm_up_body<P>(VxBlkB<128, 4>{blockIdx.x, gridDim.x}, v, S, start, sorted, cnt, M);
-}
-
-// Upward pass, the rest: M2M of the levels from L - 4 up to 3 by subtrees
-// as above (a block per cell of level 3), then the block that finishes last
-// runs levels 2, 1 and 0.
-template <int P>
-VX_DEVK void k_fmm_up_top_body(VxBlkB<128, 0> vb, VxScalars *S, int *cnt, cplx *M) {
-    __shared__ cplx se[4][P];
-    const int hi = max(S->fL - FMM_UP, 0);
-    const int lo = min(FMM_TOP, hi);
-    if (hi == 0) return;
-    fmm_shift_table<P>(se);
-    __syncthreads();
-    for (long long r = vb.x; r < (1LL << (2 * lo)); r += vb.n) fmm_m2m_subtree<P>(se, cnt, M, lo, hi, r);
-    if (lo == 0 || !vx_last_block(&S->sync_ctr, vb.n)) return;
-    for (int l = lo - 1; l >= 0; --l) {
-        for (long long e = threadIdx.x; e < (1LL << (2 * l)) * P; e += blockDim.x)
-            fmm_m2m_cell<P>(se, cnt, M, l, e / P, (int)(e % P));
-        __syncthreads();
-    }
-}
-template <int P>
-__global__ void __launch_bounds__(128) k_fmm_up_top(VxScalars *S, int *cnt, cplx *M) {
-    VX_PDL_WAIT();
-    k_fmm_up_top_body<P>(VxBlkB<128, 0>{blockIdx.x, gridDim.x}, S, cnt, M);
+    k_fmm_up_top_body<P>(VxBlkB<32 * TOP_W, 0>{blockIdx.x, gridDim.x}, S, cnt, M);
 }
 
 // M2L at level l (2 <= l <= L) plus L2L from level l-1.  A block takes a
@@ -1111,11 +1163,11 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
                     w.bk_mid, w.bk_big, w.val0, gt);
     const unsigned *skey = w.key1;
     const int *sorted = w.val1;
-    // upward pass: P2M + M2M of the 3 levels above the leaves by subtrees,
-    // then the levels above those (two launches whatever the depth)
-    const int gup = (int)std::min<long long>(grid * 4, 1LL << (2 * std::max(Lmax - FMM_UP, 0)));
-    vx_launch<k_fmm_up<P>, k_fmm_up_body<P>>(L, gup, 128, 0, v, S, w.fmm_start, sorted, w.fmm_cnt, (cplx *)w.fmm_M);
-    vx_launch<k_fmm_up_top<P>, k_fmm_up_top_body<P>>(L, 1 << (2 * FMM_TOP), 128, 0, S, w.fmm_cnt, (cplx *)w.fmm_M);
+    // upward pass: P2M + M2M of the 2 levels above the leaves, then the
+    // levels above those (two launches whatever the depth)
+    const int gup = (int)std::min<long long>(grid * 4, 1LL << (2 * std::max(Lmax - 2, 0)));
+    vx_launch<k_fmm_up<P>, k_fmm_up_body<P>>(L, gup, 32 * UP_W, 0, v, S, w.fmm_start, sorted, w.fmm_cnt, (cplx *)w.fmm_M);
+    vx_launch<k_fmm_up_top<P>, k_fmm_up_top_body<P>>(L, Lmax - 2 > FMM_TOP ? 1 << (2 * FMM_TOP) : 1, 32 * TOP_W, 0, S, w.fmm_cnt, (cplx *)w.fmm_M);
     {
         long long tiles = 0;
         for (int l = 2; l <= std::min(Lmax, M2L_SMALL); ++l) tiles += vx_ceil_div(1LL << (2 * l), 16LL);
