@@ -1141,7 +1141,7 @@ extern "C" vx_status vx_estimate_bytes(const vx_conf *c, int64_t P, int64_t n_ma
     const long long need = vx_round32(n_max + P) + 64;
     const long long cap = cap_after_growth(need, c->inc_step);
     const long long S1 = P + 1;
-    const long long transient = (2 * S1 * S1 + S1) * 8;     // Gauss-Jordan work area at creation
+    const long long transient = vx_matrix_work((int)P) * 8;     // Gauss-Jordan work area at creation
     const long long wall = 4LL * (9 * P + 4096);              // wall panel lists (bound)
     const int fp = vx_fmm_order_ok(c->fmm_p) ? c->fmm_p : VX_FMM_P;
     *out = 6 * 8 * cap + vx_work_bytes(cap, (int)vx_round32(P), sms, fp) + fixed_bytes(P) + transient + wall;
@@ -1264,9 +1264,7 @@ extern "C" vx_status vx_probe(vx_sim *s, const double *px, const double *py, int
     double *dpx = s->d_probe, *dpy = dpx + np, *dvx = dpy + np, *dvy = dvx + np;
     CU(cudaMemcpyAsync(dpx, px, sizeof(double) * np, cudaMemcpyHostToDevice, s->stream));
     CU(cudaMemcpyAsync(dpy, py, sizeof(double) * np, cudaMemcpyHostToDevice, s->stream));
-    const int tile = s->prm.prec == VX_PREC_FP32 ? 1024 : 512;
-    const int K = vx_ksplit(np, tile, s->num_sms);
-    CU(vx_launch_probe(launch_of(s), s->prm, view_of(s), s->d_S, s->w, dpx, dpy, 1, np, dvx, dvy, 1, K));
+    CU(vx_launch_probe(launch_of(s), s->prm, view_of(s), s->d_S, s->w, dpx, dpy, 1, np, dvx, dvy, 1));
     CU(cudaMemcpyAsync(ovx, dvx, sizeof(double) * np, cudaMemcpyDeviceToHost, s->stream));
     CU(cudaMemcpyAsync(ovy, dvy, sizeof(double) * np, cudaMemcpyDeviceToHost, s->stream));
     CU(cudaStreamSynchronize(s->stream));

@@ -208,12 +208,23 @@ __host__ __device__ inline int vx_body_parts(long long n, int sms, int cap) {
     const int q = 4 * vx_body_sms(n, sms);
     return q < cap ? q : cap;
 }
-// Source chunks of the pair kernels: about 8 work items per SM over tiles
-// of `tile` targets, 1 to 64.
-__host__ __device__ inline int vx_ksplit(long long n, int tile, int sms) {
-    const long long tiles = vx_ceil_div(n > 0 ? n : 1, tile);
-    long long k = vx_ceil_div(8LL * sms, tiles);
-    return (int)(k < 1 ? 1 : (k > 64 ? 64 : k));
+// Source chunks of the pair kernels for nt targets in tiles of `tile` and ns
+// sources: the (tile, chunk) items are to fill the `slots` resident blocks a
+// whole number of times, up to `rounds`, with as few idle slots in the last
+// one as possible; at least 64 sources a chunk, at most 256 chunks.
+__host__ __device__ inline int vx_pair_split(long long nt, long long ns, int tile, int slots, int rounds) {
+    const long long tiles = vx_ceil_div(nt > 0 ? nt : 1, tile);
+    const long long kmax = ns < 128 ? 1 : (ns < 64 * 256 ? ns / 64 : 256);
+    long long best = 1, num = 0, den = 1;   // the best share of filled slots so far, num / den
+    for (int w = 1; w <= rounds; ++w) {
+        long long k = (long long)slots * w / tiles;
+        if (k < 1) continue;
+        if (k > kmax) k = kmax;
+        const long long items = tiles * k, room = vx_ceil_div(items, slots) * slots;
+        if (items * den > num * room) { best = k; num = items; den = room; }
+        if (items * 20 >= room * 17) break;   // more, shorter chunks cost more than they fill
+    }
+    return (int)best;
 }
 // Source chunks of the birth right-hand side for P panels and n0 sources:
 // enough (panel tile, chunk) items for every SM to hold several blocks,
@@ -608,7 +619,7 @@ struct VxLaunch {
     // small bodies on concurrent streams overlap); full_sms (0: num_sms)
     // stays the device's count: the all-pairs sums' grid, and the SM count
     // the result-defining partitions are derived from on the device
-    // (vx_body_parts, vx_ksplit, vx_rhs_chunks), so a body gets the same
+    // (vx_body_parts, vx_pair_split, vx_rhs_chunks), so a body gets the same
     // results whatever share of the GPU it runs on.
     int num_sms;
     int full_sms = 0;
@@ -703,8 +714,7 @@ cudaError_t vx_launch_collapse(const VxLaunch &L, const VxParams &p, const VxVie
                                VxWork &w, int pass, int n_col);
 cudaError_t vx_launch_probe(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                             VxWork &w, const double *px, const double *py, long long pstride,
-                            long long np, double *out_vx, double *out_vy, long long ostride,
-                            int ksplit);
+                            long long np, double *out_vx, double *out_vy, long long ostride);
 // Panel system on the device: L (P+1)^2 then Gauss-Jordan inverse.
 // d_L_out (nullable) receives a copy of the influence matrix before elimination.
 cudaError_t vx_build_matrix(const VxLaunch &L, const vx_panel *d_pan, int P, double *d_minv,

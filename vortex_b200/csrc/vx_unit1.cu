@@ -386,10 +386,8 @@ int velocity_control(vxu_vortex *pos, double (*V_inf)[2], size_t n, vxu_vortex *
     ++U.launches;
     const double *px = (const double *)Contr_points;
     double *ov = (double *)V;
-    const int tile = U.prm.prec == VX_PREC_FP32 ? 1024 : 512;
-    const int K = vx_ksplit((long long)n_contr, tile, U.num_sms);
     CK(vx_launch_probe(launch0(), U.prm, aos_view(pos, nullptr, nullptr), U.d_S, U.w, px, px + 1, 3,
-                       (long long)n_contr, ov, ov + 1, 2, K));
+                       (long long)n_contr, ov, ov + 1, 2));
     CK(cudaDeviceSynchronize());
     return 0;
 }
@@ -500,7 +498,7 @@ int64_t vxu_launch_count(void) { return U.launches; }
 //     array and must be serialised by the caller.
 namespace {
 constexpr long long NA_MAX_POINTS = 4096;   // control points per call
-constexpr int NA_MAX_SPLIT = 64;            // source splits (vx_ksplit's cap)
+constexpr int NA_MAX_SPLIT = 64;            // source splits a point takes of the scratch at that many points
 constexpr long long NA_HEAD = ((long long)sizeof(VxScalars) + 255) / 256 * 256 / (long long)sizeof(double);
 constexpr long long NA_PART = 2LL * NA_MAX_SPLIT * NA_MAX_POINTS;
 constexpr long long NA_WORDS = NA_HEAD + NA_PART;   // 4 MiB + the scalars
@@ -573,9 +571,8 @@ extern "C" int velocity_control_noalloc(vxu_vortex *pos, double (*V_inf)[2], siz
     ++U.launches;
     const double *px = (const double *)Contr_points;
     double *ov = (double *)V;
-    const int K = vx_ksplit((long long)n_contr, 512, d->num_sms);
     CK(vx_launch_probe(L, prm, aos_view(pos, nullptr, nullptr), S, w, px, px + 1, 3, (long long)n_contr, ov,
-                       ov + 1, 2, K));
+                       ov + 1, 2));
     CK(cudaDeviceSynchronize());
     return 0;
 }
