@@ -316,19 +316,22 @@ struct RhsMath<float> {
 };
 
 template <typename T>
-VX_DEVK void k_rhs_partial_body(VxBlkB<RHS_T, 0> vb, const VxView &v, const VxScalars *S,
+__host__ __device__ constexpr int rhs_t() { return sizeof(T) == 8 ? 64 : RHS_T; }   // threads and panels of a tile
+template <typename T>
+VX_DEVK void k_rhs_partial_body(VxBlkB<rhs_t<T>(), 0> vb, const VxView &v, const VxScalars *S,
                                 const vx_panel *pan, int P, int P32,
                                 double *part, int sms) {
-    const int nchunks = vx_rhs_chunks(S->n0, P, sms);   // from the body's own count
-    __shared__ T sx[RHS_T], sy[RHS_T], sg[RHS_T];
+    constexpr int RT = rhs_t<T>();
+    const int nchunks = vx_rhs_chunks(S->n0, P, sms, sizeof(T) == 8);   // from the body's own count
+    __shared__ T sx[RT], sy[RT], sg[RT];
     const long long n0 = S->n0;
-    const long long cs = vx_ceil_div(vx_ceil_div(n0, nchunks), RHS_T) * RHS_T;
-    const int tiles = (P + RHS_T - 1) / RHS_T;
+    const long long cs = vx_ceil_div(vx_ceil_div(n0, nchunks), RT) * RT;
+    const int tiles = (P + RT - 1) / RT;
     const long long items = (long long)tiles * nchunks;
     for (long long it = vb.x; it < items; it += vb.n) {
         const int pt = (int)(it % tiles);
         const long long sc = it / tiles;
-        const int i = pt * RHS_T + threadIdx.x;
+        const int i = pt * RT + threadIdx.x;
         const bool valid = i < P;
         T al0 = 0, al1 = 0, d0 = 1, d1 = 0;
         if (valid) {
@@ -339,7 +342,7 @@ VX_DEVK void k_rhs_partial_body(VxBlkB<RHS_T, 0> vb, const VxView &v, const VxSc
         const T dd2 = fma(d0, d0, d1 * d1);
         T y0 = 0, y1 = 0;
         const long long j0 = sc * cs, j1 = min(n0, j0 + cs);
-        for (long long jt = j0; jt < j1; jt += RHS_T) {
+        for (long long jt = j0; jt < j1; jt += RT) {
             __syncthreads();
             long long j = jt + threadIdx.x;
             if (j < j1) {
@@ -348,7 +351,7 @@ VX_DEVK void k_rhs_partial_body(VxBlkB<RHS_T, 0> vb, const VxView &v, const VxSc
                 sg[threadIdx.x] = (T)v.g[j * v.ps];
             }
             __syncthreads();
-            const int cnt = (int)min((long long)RHS_T, j1 - jt);
+            const int cnt = (int)min((long long)RT, j1 - jt);
             for (int q = 0; q < cnt; ++q) {
                 T s00 = al0 - sx[q], s01 = al1 - sy[q];
                 T s10 = s00 + d0, s11 = s01 + d1;
@@ -369,11 +372,11 @@ VX_DEVK void k_rhs_partial_body(VxBlkB<RHS_T, 0> vb, const VxView &v, const VxSc
     }
 }
 template <typename T>
-__global__ void __launch_bounds__(RHS_T) k_rhs_partial(VxView v, const VxScalars *S,
+__global__ void __launch_bounds__(rhs_t<T>()) k_rhs_partial(VxView v, const VxScalars *S,
                                                        const vx_panel *pan, int P, int P32,
                                                        double *part, int sms) {
     VX_PDL_WAIT();
-    k_rhs_partial_body<T>(VxBlkB<RHS_T, 0>{blockIdx.x, gridDim.x}, v, S, pan, P, P32, part, sms);
+    k_rhs_partial_body<T>(VxBlkB<rhs_t<T>(), 0>{blockIdx.x, gridDim.x}, v, S, pan, P, P32, part, sms);
 }
 
 // ---------------------------------------------------------------------------
@@ -452,11 +455,11 @@ __device__ __forceinline__ void bf_far_part(unsigned q, unsigned nparts, const V
                 double pr = wr, pi = wi;
 #pragma unroll
                 for (int s2 = 0; s2 < 4; ++s2) {
-                    const double nr = pr * pr - pi * pi, ni = 2.0 * pr * pi;
+                    const double nr = fma(pr, pr, -(pi * pi)), ni = 2.0 * pr * pi;
                     pr = nr; pi = ni;
                 }
                 for (int k = 0; k < pass; ++k) {
-                    const double nr = tr * pr - ti * pi, ni = tr * pi + ti * pr;
+                    const double nr = fma(tr, pr, -(ti * pi)), ni = fma(tr, pi, ti * pr);
                     tr = nr; ti = ni;
                 }
             }
@@ -464,7 +467,7 @@ __device__ __forceinline__ void bf_far_part(unsigned q, unsigned nparts, const V
             for (int l = 0; l < 16; ++l) {
                 acc[2 * l] += tr;
                 acc[2 * l + 1] += ti;
-                const double nr = tr * wr - ti * wi, ni = tr * wi + ti * wr;
+                const double nr = fma(tr, wr, -(ti * wi)), ni = fma(tr, wi, ti * wr);
                 tr = nr; ti = ni;
             }
         }
@@ -674,7 +677,7 @@ __device__ __forceinline__ float vx_half_log_ratio(float r0, float r1, float num
 // Direct FP32 panel terms over the near list (chunked like k_rhs_partial).
 VX_DEVK void k_rhs_near_body(VxBlkB<RHS_T, 8> vb, const VxScalars *S, const vx_panel *pan, int P, int P32,
                              const float4 *near, double *part, int sms) {
-    const int nchunks = vx_rhs_chunks(S->n0, P, sms);   // from the body's own count
+    const int nchunks = vx_rhs_chunks(S->n0, P, sms, false);   // from the body's own count
     __shared__ float4 sq4[RHS_T];   // (x, y, G, unused)
     const long long nn = S->bf_nnear;
     const long long cs = vx_ceil_div(vx_ceil_div(nn, nchunks), RHS_T) * RHS_T;
@@ -728,187 +731,124 @@ __global__ void __launch_bounds__(RHS_T) k_rhs_near(const VxScalars *S, const vx
 
 // R_i = -(mean velocity along panel i + V_inf) . tau_i; the far field (if
 // coef) adds Re[I_far (tau_x + i tau_y) / (2 pi i dz)] with dz = zb - za.
-// WARP: one warp per panel, its lanes summing the chunk partials (bulk form,
-// fixed butterfly); otherwise one thread per panel in chunk order.
-template <bool WARP>
-VX_DEVK void k_rhs_final_body(VxBlkB<0, 0> vb, const VxScalars *S, const vx_panel *pan, int P, int P32,
-                              const double *part, int sms, double *R, const VxParams &p, const double *coef) {
-    const int nchunks = vx_rhs_chunks(S->n0, P, sms);   // from the body's own count
-    const int i = WARP ? (int)((vb.x * blockDim.x + threadIdx.x) >> 5) : vb.x * blockDim.x + threadIdx.x;
+// One warp per panel: its lanes sum the chunk partials, and two terms each of
+// the far field's series, (z - c)^(l + 1) by squaring, by fixed butterflies (one
+// lane's chain of 48 products and divisions: 1000 panels 22 -> 12 us).  The panel's new
+// vortex gets its place here (src/kernel.cu:862-872); its strength follows
+// from the gamma solve.
+VX_DEVK void k_rhs_final_body(VxBlkB<128, 0> vb, const VxView &v, const VxScalars *S, const vx_panel *pan, int P,
+                              int P32, const double *part, int sms, double *R, const VxParams &p,
+                              const double *coef) {
+    const int nchunks = vx_rhs_chunks(S->n0, P, sms, p.prec == VX_PREC_FP64);   // from the body's own count
+    const int i = (int)((vb.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (i >= P) return;
     double y0 = 0.0, y1 = 0.0;
-    if (WARP) {
-        const int lane = threadIdx.x & 31;
-        for (int sc = lane; sc < nchunks; sc += 32) {
-            y0 += part[((long long)sc * P32 + i) * 2 + 0];
-            y1 += part[((long long)sc * P32 + i) * 2 + 1];
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            y0 += __shfl_xor_sync(0xffffffffu, y0, o);
-            y1 += __shfl_xor_sync(0xffffffffu, y1, o);
-        }
-        if (lane != 0) return;
-    } else {
-        for (int sc = 0; sc < nchunks; ++sc) {
-            y0 += part[((long long)sc * P32 + i) * 2 + 0];
-            y1 += part[((long long)sc * P32 + i) * 2 + 1];
+    for (int sc = lane; sc < nchunks; sc += 32) {
+        y0 += part[((long long)sc * P32 + i) * 2 + 0];
+        y1 += part[((long long)sc * P32 + i) * 2 + 1];
+    }
+    const double l0 = pan[i].left[0], l1 = pan[i].left[1], r0 = pan[i].right[0], r1 = pan[i].right[1];
+    const double d0 = r0 - l0, d1 = r1 - l1;
+    double Ir = 0.0, Ii = 0.0;
+    if (coef) {
+        bcplx za = {l0 - p.bc_x, l1 - p.bc_y}, zb = {r0 - p.bc_x, r1 - p.bc_y};
+        bcplx pa = {1.0, 0.0}, pb = {1.0, 0.0};   // (z - c)^(lane + 1)
+        const auto mul = [](bcplx a, bcplx b) {
+            return bcplx{fma(a.r, b.r, -(a.i * b.i)), fma(a.r, b.i, a.i * b.r)};
+        };
+#pragma unroll
+        for (int e = 1; e <= 32; e <<= 1) {
+            if ((lane + 1) & e) { pa = mul(pa, za); pb = mul(pb, zb); }
+            if (e < 32) { za = mul(za, za); zb = mul(zb, zb); }
+        }   // za, zb: to the 32nd power
+#pragma unroll
+        for (int l = lane; l < BF_P; l += 32) {
+            const double q = 1.0 / (double)(l + 1);
+            const double dr = (pb.r - pa.r) * q, di = (pb.i - pa.i) * q;
+            const double cr = coef[2 * l], ci = coef[2 * l + 1];
+            Ir = fma(cr, dr, fma(-ci, di, Ir));
+            Ii = fma(cr, di, fma(ci, dr, Ii));
+            pa = mul(pa, za);
+            pb = mul(pb, zb);
         }
     }
-    double d0 = pan[i].right[0] - pan[i].left[0], d1 = pan[i].right[1] - pan[i].left[1];
+    for (int o = 16; o > 0; o >>= 1) {
+        y0 += __shfl_xor_sync(0xffffffffu, y0, o);
+        y1 += __shfl_xor_sync(0xffffffffu, y1, o);
+        Ir += __shfl_xor_sync(0xffffffffu, Ir, o);
+        Ii += __shfl_xor_sync(0xffffffffu, Ii, o);
+    }
+    if (lane != 0) return;
     double mnog = 1.0 / (VX_TWO_PI * (d0 * d0 + d1 * d1));
     double u = mnog * y0, w = mnog * y1;
     if (coef) {
-        const double ar = pan[i].left[0] - p.bc_x, ai = pan[i].left[1] - p.bc_y;
-        const double br = pan[i].right[0] - p.bc_x, bi = pan[i].right[1] - p.bc_y;
-        double pa_r = ar, pa_i = ai, pb_r = br, pb_i = bi;   // (z - c)^(l+1)
-        double Ir = 0.0, Ii = 0.0;
-        for (int l = 0; l < BF_P; ++l) {
-            const double dr = (pb_r - pa_r) / (double)(l + 1), di = (pb_i - pa_i) / (double)(l + 1);
-            const double cr = coef[2 * l], ci = coef[2 * l + 1];
-            Ir += cr * dr - ci * di;
-            Ii += cr * di + ci * dr;
-            double t = pa_r * ar - pa_i * ai; pa_i = pa_r * ai + pa_i * ar; pa_r = t;
-            t = pb_r * br - pb_i * bi; pb_i = pb_r * bi + pb_i * br; pb_r = t;
-        }
         // mean conjugate velocity W = I / (2 pi i dz): u = Re W, v = -Im W
         const double qr = -VX_TWO_PI * d1, qi = VX_TWO_PI * d0;   // 2 pi i dz
         const double qq = qr * qr + qi * qi;
-        const double Wr = (Ir * qr + Ii * qi) / qq, Wi = (Ii * qr - Ir * qi) / qq;
-        u += Wr;
-        w += -Wi;
+        u += (Ir * qr + Ii * qi) / qq;
+        w -= (Ii * qr - Ir * qi) / qq;
     }
     R[i] = -((u + S->vinf[0]) * pan[i].tang[0] + (w + S->vinf[1]) * pan[i].tang[1]);
-}
-template <bool WARP>
-__global__ void k_rhs_final(const VxScalars *S, const vx_panel *pan, int P, int P32,
-                            const double *part, int sms, double *R, VxParams p, const double *coef) {
-    VX_PDL_WAIT();
-    k_rhs_final_body<WARP>(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, S, pan, P, P32, part, sms, R, p, coef);
-}
-
-// One new vortex per panel at [n0, n0+P) (src/kernel.cu:862-872), written
-// by the block that finishes the gamma solve last (a vortex takes the gamma
-// of its panel's right neighbour too, so every gamma must be final).
-__device__ void birth_place(const VxParams &p, const VxView &v, VxScalars *S, const vx_panel *pan, int P,
-                            const double *gamma) {
-    const long long n0 = S->n0;
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
-        const int in = (int)pan[i].n_of_rpanel;
-        const double mx = (pan[i].left[0] + pan[i].right[0]) / 2;
-        const double my = (pan[i].left[1] + pan[i].right[1]) / 2;
-        double bx, by;
-        if (p.birth_mode == VX_BIRTH_FILE) {
-            bx = pan[i].birth[0]; by = pan[i].birth[1];
-        } else if (p.birth_mode == VX_BIRTH_HALF_PANEL) {
-            const double h = 0.5 * pan[i].length;
-            bx = mx + h * pan[i].norm[0]; by = my + h * pan[i].norm[1];
-        } else {
-            bx = mx + 1e-6 * pan[i].norm[0]; by = my + 1e-6 * pan[i].norm[1];
-        }
-        const long long k = (n0 + i) * v.ps;
-        v.x[k] = bx;
-        v.y[k] = by;
-        v.g[k] = 0.5 * (__ldcg(&gamma[i]) * pan[i].length + __ldcg(&gamma[in]) * pan[in].length);
+    const double mx = (l0 + r0) / 2, my = (l1 + r1) / 2;
+    double bx, by;
+    if (p.birth_mode == VX_BIRTH_FILE) {
+        bx = pan[i].birth[0]; by = pan[i].birth[1];
+    } else if (p.birth_mode == VX_BIRTH_HALF_PANEL) {
+        const double h = 0.5 * pan[i].length;
+        bx = mx + h * pan[i].norm[0]; by = my + h * pan[i].norm[1];
+    } else {
+        bx = mx + 1e-6 * pan[i].norm[0]; by = my + 1e-6 * pan[i].norm[1];
     }
-    if (threadIdx.x == 0) S->n = n0 + P;
+    const long long k = (S->n0 + i) * v.ps;
+    v.x[k] = bx;
+    v.y[k] = by;
+}
+__global__ void __launch_bounds__(128) k_rhs_final(VxView v, const VxScalars *S, const vx_panel *pan, int P, int P32,
+                                                   const double *part, int sms, double *R, VxParams p,
+                                                   const double *coef) {
+    VX_PDL_WAIT();
+    k_rhs_final_body(VxBlkB<128, 0>{blockIdx.x, gridDim.x}, v, S, pan, P, P32, part, sms, R, p, coef);
 }
 
-// gamma_i = sum_j M_ij R_j + M_iP dg, sequential in j with fma (as the
-// oracle), one thread per row; ld is the matrix row stride.  Then the
-// vortices are placed (birth_place).
-VX_DEVK void k_gamma_body(VxBlkB<0, 0> vb, const VxParams &p, const VxView &v, VxScalars *S, const vx_panel *pan, const double *M,
+// gamma_i = sum_j M_ij R_j + M_iP dg: a warp per row (row stride ld), lanes
+// striding the row, eight loads on their way at a time, FP64 partial sums
+// combined by a fixed butterfly.  The block that finishes last then sets the
+// new vortices' strengths (a vortex takes the gamma of its panel's right
+// neighbour too, so every gamma must be final).
+constexpr int GAM_T = 256;
+VX_DEVK void k_gamma_body(VxBlkB<GAM_T, 0> vb, const VxView &v, VxScalars *S, const vx_panel *pan, const double *M,
                           long long ld, int P, const double *R, double *gamma) {
-    const int i = vb.x * blockDim.x + threadIdx.x;
-    if (i < P) {
-        const double *row = M + (long long)i * ld;
-        double acc = 0.0;
-        for (int j = 0; j < P; ++j) acc = fma(row[j], R[j], acc);
-        gamma[i] = fma(row[P], S->dg, acc);
-    }
-    if (vx_last_block(&S->sync_ctr, vb.n)) birth_place(p, v, S, pan, P, gamma);
-}
-__global__ void k_gamma(VxParams p, VxView v, VxScalars *S, const vx_panel *pan, const double *M, long long ld, int P,
-                        const double *R, double *gamma) {
-    VX_PDL_WAIT();
-    k_gamma_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, p, v, S, pan, M, ld, P, R, gamma);
-}
-
-// The same sums from the transposed inverse Mt (Mt[j ld + i] = M[i ld + j]):
-// the same order and fma per row, but a warp's 32 rows read 32 consecutive
-// doubles per step instead of 32 rows' worth of cache lines.
-VX_DEVK void k_gamma_t_body(VxBlkB<0, 0> vb, const VxParams &p, const VxView &v, VxScalars *S, const vx_panel *pan,
-                            const double *Mt, long long ld, int P, const double *R, double *gamma) {
-    const int i = vb.x * blockDim.x + threadIdx.x;
-    if (i < P) {
-        double acc = 0.0;
-        for (int j = 0; j < P; ++j) acc = fma(Mt[(long long)j * ld + i], R[j], acc);
-        gamma[i] = fma(Mt[(long long)P * ld + i], S->dg, acc);
-    }
-    if (vx_last_block(&S->sync_ctr, vb.n)) birth_place(p, v, S, pan, P, gamma);
-}
-__global__ void k_gamma_t(VxParams p, VxView v, VxScalars *S, const vx_panel *pan, const double *Mt, long long ld,
-                          int P, const double *R, double *gamma) {
-    VX_PDL_WAIT();
-    k_gamma_t_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, p, v, S, pan, Mt, ld, P, R, gamma);
-}
-
-// Bulk form: one warp per row, lanes striding the row (coalesced), FP64
-// partial sums combined by a fixed butterfly.
-VX_DEVK void k_gamma_w_body(VxBlkB<0, 0> vb, const VxParams &p, const VxView &v, VxScalars *S, const vx_panel *pan,
-                            const double *M, long long ld, int P, const double *R, double *gamma) {
     const int lane = threadIdx.x & 31;
     const int i = (vb.x * blockDim.x + threadIdx.x) >> 5;
     if (i < P) {
         const double *row = M + (long long)i * ld;
         double acc = 0.0;
+#pragma unroll 8
         for (int j = lane; j < P; j += 32) acc = fma(row[j], R[j], acc);
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (lane == 0) gamma[i] = fma(row[P], S->dg, acc);
     }
-    if (vx_last_block(&S->sync_ctr, vb.n)) birth_place(p, v, S, pan, P, gamma);
+    if (!vx_last_block(&S->sync_ctr, vb.n)) return;
+    const long long n0 = S->n0;
+#pragma unroll 4
+    for (int q = threadIdx.x; q < P; q += GAM_T) {
+        const int in = (int)pan[q].n_of_rpanel;
+        v.g[(n0 + q) * v.ps] = 0.5 * (__ldcg(&gamma[q]) * pan[q].length + __ldcg(&gamma[in]) * pan[in].length);
+    }
+    if (threadIdx.x == 0) S->n = n0 + P;
 }
-__global__ void k_gamma_w(VxParams p, VxView v, VxScalars *S, const vx_panel *pan, const double *M, long long ld,
-                          int P, const double *R, double *gamma) {
+__global__ void __launch_bounds__(GAM_T) k_gamma(VxView v, VxScalars *S, const vx_panel *pan, const double *M,
+                                                 long long ld, int P, const double *R, double *gamma) {
     VX_PDL_WAIT();
-    k_gamma_w_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, p, v, S, pan, M, ld, P, R, gamma);
+    k_gamma_body(VxBlkB<GAM_T, 0>{blockIdx.x, gridDim.x}, v, S, pan, M, ld, P, R, gamma);
 }
 
-VX_DEVK void k_transpose_body(VxBlkB<0, 0> vb, const double *A, double *At, long long nr) {
-    __shared__ double t[32][33];
-    for (long long by = blockIdx.y; by * 32 < nr; by += gridDim.y)
-        for (long long bx = vb.x; bx * 32 < nr; bx += vb.n) {
-            for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-                const long long i = by * 32 + r, j = bx * 32 + threadIdx.x;
-                if (i < nr && j < nr) t[r][threadIdx.x] = A[i * nr + j];
-            }
-            __syncthreads();
-            for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-                const long long i = bx * 32 + r, j = by * 32 + threadIdx.x;
-                if (i < nr && j < nr) At[i * nr + j] = t[threadIdx.x][r];
-            }
-            __syncthreads();
-        }
-}
-__global__ void k_transpose(const double *A, double *At, long long nr) {
-    VX_PDL_WAIT();
-    k_transpose_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, A, At, nr);
-}
-
-cudaError_t vx_transpose_square(const VxLaunch &L, const double *A, double *At, long long nr) {
-    const long long nb = vx_ceil_div(nr, 32LL);
-    const dim3 grid((unsigned)std::min(nb, 64LL), (unsigned)std::min(nb, 64LL)), block(32, 8);
-    vx_launch<k_transpose, k_transpose_body>(L, grid, block, 0, A, At, nr);
-    return cudaGetLastError();
-}
-
-// rhs_chunks: the source chunks the host expects, for the grid only (the
-// kernels take the chunk count from the body's own count, vx_rhs_chunks).
-static cudaError_t birth_impl(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
-                              const vx_panel *pan, const double *minv, long long ld, const double *minv_t,
-                              int rhs_chunks) {
+cudaError_t vx_launch_birth(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
+                            const vx_panel *pan, const double *minv, long long ld, int rhs_chunks) {
     const int P = p.P, P32 = (int)vx_round32(P);
-    const int tiles = (P + RHS_T - 1) / RHS_T;
-    const int grid = (int)min((long long)tiles * rhs_chunks, (long long)L.num_sms * 16);
+    const int T = p.prec == VX_PREC_FP64 ? rhs_t<double>() : RHS_T;
+    const int grid = (int)std::min((long long)((P + T - 1) / T) * rhs_chunks,
+                                   16LL * (p.prec == VX_PREC_FP64 ? vx_full_sms(L) : L.num_sms));
     const int sms = vx_full_sms(L);   // the device's SMs: partitions follow the body, not the launch
     const bool far = p.prec == VX_PREC_FP32 && p.birth_far;
     if (far) {
@@ -919,38 +859,11 @@ static cudaError_t birth_impl(const VxLaunch &L, const VxParams &p, const VxView
     } else if (p.prec == VX_PREC_FP32) {
         vx_launch<k_rhs_partial<float>, k_rhs_partial_body<float>>(L, grid, RHS_T, 0, v, S, pan, P, P32, w.rhs_part, sms);
     } else {
-        vx_launch<k_rhs_partial<double>, k_rhs_partial_body<double>>(L, grid, RHS_T, 0, v, S, pan, P, P32, w.rhs_part, sms);
+        vx_launch<k_rhs_partial<double>, k_rhs_partial_body<double>>(L, grid, T, 0, v, S, pan, P, P32, w.rhs_part, sms);
     }
-
-    const int b = (P + 127) / 128;
-    if (far)
-        vx_launch<k_rhs_final<true>, k_rhs_final_body<true>>(L, (P + 3) / 4, 128, 0, S, pan, P, P32, w.rhs_part, sms, w.R, p, w.bf_coef);
-    else
-        vx_launch<k_rhs_final<false>, k_rhs_final_body<false>>(L, b, 128, 0, S, pan, P, P32, w.rhs_part, sms, w.R, p, nullptr);
-
-    if (minv_t && p.prec == VX_PREC_FP32)
-        vx_launch<k_gamma_w, k_gamma_w_body>(L, (P + 3) / 4, 128, 0, p, v, S, pan, minv, ld, P, w.R, w.gamma);
-    else if (minv_t)
-        vx_launch<k_gamma_t, k_gamma_t_body>(L, b, 128, 0, p, v, S, pan, minv_t, ld, P, w.R, w.gamma);
-    else
-        vx_launch<k_gamma, k_gamma_body>(L, b, 128, 0, p, v, S, pan, minv, ld, P, w.R, w.gamma);
+    vx_launch<k_rhs_final, k_rhs_final_body>(L, (P + 3) / 4, 128, 0, v, S, pan, P, P32, w.rhs_part, sms, w.R, p, far ? w.bf_coef : nullptr);
+    vx_launch<k_gamma, k_gamma_body>(L, (int)vx_ceil_div(P, GAM_T / 32), GAM_T, 0, v, S, pan, minv, ld, P, w.R, w.gamma);
     return cudaGetLastError();
-}
-
-// Row-major inverse with row stride ld (the reference's padded matrix).
-cudaError_t vx_launch_birth_ld(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
-                               VxWork &w, const vx_panel *pan, const double *minv, long long ld,
-                               int rhs_chunks) {
-    return birth_impl(L, p, v, S, w, pan, minv, ld, nullptr, rhs_chunks);
-}
-
-// Native engine: the inverse and its transpose, unpadded, stride P+1.  The
-// plain form solves in the reference's row order from the transpose; the
-// bulk form a warp per row.
-cudaError_t vx_launch_birth(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
-                            VxWork &w, const vx_panel *pan, const double *minv, const double *minv_t,
-                            int rhs_chunks) {
-    return birth_impl(L, p, v, S, w, pan, minv, (long long)p.P + 1, minv_t, rhs_chunks);
 }
 
 cudaError_t vx_launch_step_end(const VxLaunch &L, VxScalars *S) {

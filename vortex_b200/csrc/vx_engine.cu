@@ -393,7 +393,7 @@ static vx_status ensure_capacity(vx_sim *s) {
 // them) change only when that bound crosses one, not every few steps.  They
 // are grids only: the partitions that fix summation orders are derived on
 // the device from the body's own count.
-static int rhs_chunks_for(vx_sim *s) { return vx_rhs_chunks(s->n_upper, s->P, s->num_sms); }
+static int rhs_chunks_for(vx_sim *s) { return vx_rhs_chunks(s->n_upper, s->P, s->num_sms, s->prm.prec == VX_PREC_FP64); }
 
 // SMs a step's grid-stride launches are sized for: one per 2048 sources of
 // the rounded bound, at least 4, at most the device's.
@@ -569,10 +569,6 @@ extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t
         if (e == cudaSuccess) e = cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     }
-    if (e == cudaSuccess && cudaMalloc(&s->d_minvT, sizeof(double) * S1 * S1) != cudaSuccess)
-        e = cudaErrorMemoryAllocation;
-    if (e == cudaSuccess) e = vx_transpose_square(L, s->d_minv, s->d_minvT, S1);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     cudaFree(work);
     cudaFree(flag);
     if (e != cudaSuccess) { vx_set_error("panel system: %s", cudaGetErrorString(e)); return fail(VX_ERR_CUDA); }
@@ -594,7 +590,6 @@ extern "C" vx_status vx_destroy(vx_sim *s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->d_pan) cudaFree(s->d_pan);
     if (s->d_minv) cudaFree(s->d_minv);
-    if (s->d_minvT) cudaFree(s->d_minvT);
     if (s->d_wstart) cudaFree(s->d_wstart);
     if (s->d_widx) cudaFree(s->d_widx);
     if (s->d_hstart) cudaFree(s->d_hstart);
@@ -770,13 +765,12 @@ extern "C" vx_status vx_set_step_index(vx_sim *s, int64_t step) {
 }
 
 // Replace the inverted panel system (row-major (P+1)^2, e.g. a matrix file
-// the caller loaded) and its transposed copy.
+// the caller loaded).
 extern "C" vx_status vx_set_matrix(vx_sim *s, const double *minv) {
     if (!s || !minv) return VX_ERR_ARG;
     CU(cudaSetDevice(s->device));
     const long long S1 = s->P + 1;
-    CU(cudaMemcpy(s->d_minv, minv, sizeof(double) * S1 * S1, cudaMemcpyHostToDevice));
-    CU(vx_transpose_square(launch_of(s), s->d_minv, s->d_minvT, S1));
+    CU(cudaMemcpyAsync(s->d_minv, minv, sizeof(double) * S1 * S1, cudaMemcpyHostToDevice, s->stream));
     CU(cudaStreamSynchronize(s->stream));
     return VX_OK;
 }
@@ -926,7 +920,7 @@ static cudaError_t launch_stages(vx_sim *s, unsigned mask, bool whole_step, VxRe
     ev(0);
     if (mask & VX_STAGE_BIRTH) {
         if ((e = vx_launch_step_begin(L, s->d_S)) != cudaSuccess) return e;
-        if ((e = vx_launch_birth(L, p, v, s->d_S, s->w, s->d_pan, s->d_minv, s->d_minvT, rhs_chunks_for(s))) != cudaSuccess) return e;
+        if ((e = vx_launch_birth(L, p, v, s->d_S, s->w, s->d_pan, s->d_minv, (long long)s->P + 1, rhs_chunks_for(s))) != cudaSuccess) return e;
     }
     ev(1);
     if (mask & VX_STAGE_VELOCITY) {
@@ -1126,7 +1120,7 @@ extern "C" vx_status vx_get_launch_count(vx_sim *s, int64_t *count) {
 // is transient and counted by the estimate only).
 static long long fixed_bytes(long long P) {
     const long long P32 = vx_round32(P), S1 = P + 1;
-    return P32 * (long long)sizeof(vx_panel) + 2 * S1 * S1 * 8 + (long long)sizeof(VxScalars) + 4096;
+    return P32 * (long long)sizeof(vx_panel) + S1 * S1 * 8 + (long long)sizeof(VxScalars) + 4096;
 }
 
 static long long cap_after_growth(long long need, long long inc_step) {

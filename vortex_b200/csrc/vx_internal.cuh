@@ -229,13 +229,15 @@ __host__ __device__ inline int vx_pair_split(long long nt, long long ns, int til
 // Source chunks of the birth right-hand side for P panels and n0 sources:
 // enough (panel tile, chunk) items for every SM to hold several blocks,
 // within the partial-sum buffer (sms * 4 chunks), one per 1024 sources (n0
-// rounded up to a power of two) at most.
-__host__ __device__ inline int vx_rhs_chunks(long long n0, int P, int sms) {
-    const long long tiles = (P + 127) / 128;
-    long long want = (long long)sms * 16 / tiles;
+// rounded up to a power of two) at most in FP32, where a chunk is a sum in
+// 32 bits.  The plain form's FP64 terms are some 150 instructions each: one
+// per 64 sources (16 chunks of 1024 kept 32 blocks busy at 16 000 vortices).
+__host__ __device__ inline int vx_rhs_chunks(long long n0, int P, int sms, bool fp64) {
+    const long long tiles = fp64 ? (P + 63) / 64 : (P + 127) / 128;
+    long long want = (long long)sms * (fp64 ? 32 : 16) / tiles;
     if (want < 1) want = 1;
     if (want > (long long)sms * 4) want = (long long)sms * 4;
-    long long bysrc = vx_ceil_div(vx_pow2_ceil(n0), 1024);
+    long long bysrc = vx_ceil_div(vx_pow2_ceil(n0), fp64 ? 64 : 1024);
     if (bysrc < 1) bysrc = 1;
     return (int)(want < bysrc ? want : bysrc);
 }
@@ -691,11 +693,11 @@ inline cudaError_t vx_launch(const VxLaunch &L, dim3 grid, dim3 block, size_t sm
 
 // Stage launchers (each returns the first CUDA error it saw).
 cudaError_t vx_launch_step_begin(const VxLaunch &L, VxScalars *S);
-// minv / minv_t: the inverted panel system and its transpose, stride P+1
+// minv: the inverted panel system, row stride ld; rhs_chunks: the source
+// chunks the host expects, for the grid only
 cudaError_t vx_launch_birth(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
-                            VxWork &w, const vx_panel *pan, const double *minv, const double *minv_t,
+                            VxWork &w, const vx_panel *pan, const double *minv, long long ld,
                             int rhs_chunks);
-cudaError_t vx_transpose_square(const VxLaunch &L, const double *A, double *At, long long nr);
 cudaError_t vx_launch_velocity(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                                VxWork &w);
 cudaError_t vx_launch_diffusion(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
@@ -734,9 +736,6 @@ cudaError_t vx_invert_gj(const VxLaunch &L, double *A, double *Inv, long long S,
 // A (n x n) -> Inv = A^-1 by blocked LU with partial pivoting; A is
 // overwritten, piv holds n ints; *flag set on a pivot below 1e-12.
 cudaError_t vx_invert_lu(const VxLaunch &L, double *A, double *Inv, long long n, int *piv, int *flag);
-cudaError_t vx_launch_birth_ld(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
-                               VxWork &w, const vx_panel *pan, const double *minv, long long ld,
-                               int rhs_chunks);
 cudaError_t vx_launch_step_end(const VxLaunch &L, VxScalars *S);
 cudaError_t vx_launch_compact_skip(const VxLaunch &L, const VxParams &p, const VxView &v,
                                    VxScalars *S, VxWork &w, const int *skip, bool count_step = false);

@@ -13,7 +13,6 @@ struct vx_sim {
     VxParams prm;
     vx_panel *d_pan = nullptr;
     double *d_minv = nullptr;
-    double *d_minvT = nullptr;   // transposed copy read by the birth solve
     int *d_wstart = nullptr, *d_widx = nullptr;   // wall panel lists per wall cell
     int *d_hstart = nullptr, *d_hidx = nullptr;   // hitting-test panel lists per cell
     long long wall_bytes = 0;

@@ -307,9 +307,8 @@ int vort_creation(vxu_vortex *pos, double (*V_infDev)[2], size_t n_of_birth, siz
     if (ensure_work((long long)n + (long long)n_of_birth_BLOCK_S)) return 1;
     k_u_set<<<1, 1>>>(U.d_S, (long long)n, (long long)n, (const double *)V_infDev, d_g);
     ++U.launches;
-    const int tiles = (int)vx_ceil_div(n_of_birth, 128);
-    const int chunks = (int)std::max(1LL, std::min((long long)U.num_sms * 4 / tiles, vx_ceil_div((long long)n, 2048)));
-    CK(vx_launch_birth_ld(launch0(), U.prm, aos_view(pos, nullptr, nullptr), U.d_S, U.w, panels, M_Dev,
+    const int chunks = vx_rhs_chunks((long long)n, (int)n_of_birth, U.num_sms, U.prm.prec == VX_PREC_FP64);
+    CK(vx_launch_birth(launch0(), U.prm, aos_view(pos, nullptr, nullptr), U.d_S, U.w, panels, M_Dev,
                           (long long)n_of_birth_BLOCK_S + 1, chunks));
     CK(cudaDeviceSynchronize());
     return 0;
