@@ -14,18 +14,22 @@
 // Segment (x2,y2)->(x1,y1) against one panel: on a crossing, sets hit and
 // keeps the crossing nearest to (x2,y2) (the lower panel index on a tie,
 // which is the reference's choice when it scans panels in index order).
-__device__ __forceinline__ void vx_hit_panel(const vx_panel &q, int i, double A, double B, double D, double x1,
+struct VxEnds {
+    double l0, l1, r0, r1;   // a panel's end points
+};
+__device__ __forceinline__ VxEnds vx_ends(const vx_panel &q) { return {q.left[0], q.left[1], q.right[0], q.right[1]}; }
+__device__ __forceinline__ void vx_hit_panel(const VxEnds &q, int i, double A, double B, double D, double x1,
                                              double y1, double x2, double y2, bool &hit, double &minDist,
                                              int &minN) {
     const double thr = 1e-12;
-    double r0 = A * q.left[0] + B * q.left[1] + D;
-    double r1 = A * q.right[0] + B * q.right[1] + D;
+    double r0 = A * q.l0 + B * q.l1 + D;
+    double r1 = A * q.r0 + B * q.r1 + D;
     if (fabs(r0) < thr) r0 = 0.0;
     if (fabs(r1) < thr) r1 = 0.0;
     if (r0 * r1 <= 0) {
-        double A1 = q.right[1] - q.left[1];
-        double B1 = q.left[0] - q.right[0];
-        double D1 = q.left[1] * q.right[0] - q.left[0] * q.right[1];
+        double A1 = q.r1 - q.l1;
+        double B1 = q.l0 - q.r0;
+        double D1 = q.l1 * q.r0 - q.l0 * q.r1;
         double r2 = A1 * x1 + B1 * y1 + D1;
         double r3 = A1 * x2 + B1 * y2 + D1;
         if (fabs(r2) < thr) r2 = 0.0;
@@ -68,9 +72,20 @@ __device__ bool vx_hitting(const VxParams &p, const vx_panel *pan, double x1, do
                     for (int cy = cy0; cy <= cy1; ++cy)
                         for (int cx = cx0; cx <= cx1; ++cx) {
                             const int c = cy * p.hit_nx + cx;
-                            for (int q = hstart[c]; q < hstart[c + 1]; ++q) {
-                                const int i = hidx[q];
-                                vx_hit_panel(pan[i], i, A, B, D, x1, y1, x2, y2, hit, minDist, minN);
+                            // four panels' loads at a time (the order of the
+                            // tests does not matter: the nearest crossing,
+                            // the lowest index on a tie)
+                            const int qe = hstart[c + 1];
+                            for (int q = hstart[c]; q < qe; q += 4) {
+                                int id[4];
+                                VxEnds en[4];
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) id[u] = hidx[min(q + u, qe - 1)];
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) en[u] = vx_ends(pan[id[u]]);
+#pragma unroll
+                                for (int u = 0; u < 4; ++u)
+                                    vx_hit_panel(en[u], id[u], A, B, D, x1, y1, x2, y2, hit, minDist, minN);
                             }
                         }
                     done = true;
@@ -78,7 +93,7 @@ __device__ bool vx_hitting(const VxParams &p, const vx_panel *pan, double x1, do
             }
         }
         if (!done)
-            for (int i = 0; i < p.P; ++i) vx_hit_panel(pan[i], i, A, B, D, x1, y1, x2, y2, hit, minDist, minN);
+            for (int i = 0; i < p.P; ++i) vx_hit_panel(vx_ends(pan[i]), i, A, B, D, x1, y1, x2, y2, hit, minDist, minN);
     }
     *hitpan = minN;
     return hit;
@@ -156,7 +171,7 @@ __device__ __forceinline__ void advect_part(unsigned part, unsigned nparts, cons
             bool h = false;
             double md = 25.0;
             int mn = -1;
-            for (int q = lane; q < p.P; q += 32) vx_hit_panel(pan[q], q, A, B, D, x1, y1, x2, y2, h, md, mn);
+            for (int q = lane; q < p.P; q += 32) vx_hit_panel(vx_ends(pan[q]), q, A, B, D, x1, y1, x2, y2, h, md, mn);
             h = __any_sync(0xffffffffu, h);
             for (int o = 16; o > 0; o >>= 1) {
                 const double od = __shfl_xor_sync(0xffffffffu, md, o);
@@ -194,6 +209,12 @@ __device__ __forceinline__ void advect_part(unsigned part, unsigned nparts, cons
     t = vx_block_sum(sfy, sh); if (threadIdx.x == 0) red[part * 4 + 2] = t;
     t = vx_block_sum(sm, sh);  if (threadIdx.x == 0) red[part * 4 + 3] = t;
 }
+// Partitions of the force sums: one particle a thread up to VX_RED_BLOCKS
+// partitions (a function of the body's count alone).
+__device__ __forceinline__ int advect_parts(long long n) {
+    const long long q = (n + VX_THREADS - 1) / VX_THREADS;
+    return (int)(q < 1 ? 1 : (q > VX_RED_BLOCKS ? VX_RED_BLOCKS : q));
+}
 // The particles are split into nparts fixed partitions (block-strided, as a
 // grid of nparts blocks would take them) whatever the grid: each block takes
 // partitions blockIdx, blockIdx + grid, ...; a partition past the last
@@ -202,9 +223,9 @@ __device__ __forceinline__ void advect_part(unsigned part, unsigned nparts, cons
 // partition sums: thread t adds partitions t, t + 256, ... in order, then a
 // fixed shared-memory tree, so the result is run-to-run identical.
 VX_DEVK void k_advect_body(VxBlkB<VX_THREADS, 0> vb, const VxParams &p, const VxView &v, VxScalars *S, const vx_panel *pan,
-                           double *red, const int *hstart, const int *hidx, int sms) {
+                           double *red, const int *hstart, const int *hidx) {
     const long long n = S->n;
-    const int nparts = vx_body_parts(n, sms, VX_RED_BLOCKS);
+    const int nparts = advect_parts(n);
     for (unsigned q = vb.x; q < (unsigned)nparts; q += vb.n) {
         if ((long long)q * blockDim.x >= n) {
             if (threadIdx.x < 4) red[q * 4 + threadIdx.x] = 0.0;
@@ -226,17 +247,17 @@ VX_DEVK void k_advect_body(VxBlkB<VX_THREADS, 0> vb, const VxParams &p, const Vx
     S->m = a[3] * (p.rho / (2 * p.dt));
 }
 __global__ void __launch_bounds__(VX_THREADS) k_advect(VxParams p, VxView v, VxScalars *S, const vx_panel *pan,
-                                                       double *red, const int *hstart, const int *hidx, int sms) {
+                                                       double *red, const int *hstart, const int *hidx) {
     VX_PDL_WAIT();
-    k_advect_body(VxBlkB<VX_THREADS, 0>{blockIdx.x, gridDim.x}, p, v, S, pan, red, hstart, hidx, sms);
+    k_advect_body(VxBlkB<VX_THREADS, 0>{blockIdx.x, gridDim.x}, p, v, S, pan, red, hstart, hidx);
 }
 
 cudaError_t vx_launch_advect(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                              VxWork &w, const vx_panel *pan, const int *hstart, const int *hidx) {
     if (p.hit_nx <= 0 || p.hit_ny <= 0) hstart = hidx = nullptr;
     // partitions of the force sums follow the body's count on the device
-    // (vx_body_parts), the grid the SMs this launch is given
-    const int grid = std::min(VX_RED_BLOCKS, L.num_sms * 4);
-    vx_launch<k_advect, k_advect_body>(L, grid, VX_THREADS, 0, p, v, S, pan, w.red, hstart, hidx, vx_full_sms(L));
+    // (advect_parts), the grid the SMs this launch is given
+    const int grid = std::min(VX_RED_BLOCKS, L.num_sms * 8);
+    vx_launch<k_advect, k_advect_body>(L, grid, VX_THREADS, 0, p, v, S, pan, w.red, hstart, hidx);
     return cudaGetLastError();
 }
