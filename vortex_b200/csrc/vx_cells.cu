@@ -34,6 +34,8 @@
 // digits (an error of order |offset| 6e-8 / d), its own cell's frame does
 // not.  Each target is owned by one warp, so the velocity is updated in place
 // with no partial sums.
+#include <algorithm>
+
 #include "vx_internal.cuh"
 
 constexpr int CG_T = 256;
@@ -352,27 +354,56 @@ struct DiffRow {
     float oy;        // row offset * cell height
 };
 constexpr int DIFF_ROWS = 2 * CG_KMAX + 2;   // rows of the widest window, and the total
-VX_DEVK void k_diff_cells_body(VxBlkB<CG_T, VX_DIFF_MINB> vb, const VxParams &p, const VxView &v, VxScalars *S,
-                               const float4 *srt, const unsigned *skey,
-                               const int *sorted, const int *start,
-                               const int2 *items, int *wide) {
+static_assert(DIFF_ROWS <= 32, "a lane per row");
+
+// Warps an item's sources are split over: a body of few items would leave
+// most of the GPU idle behind the longest of them, one warp's chain of 32
+// sources after 32 (an item of the 20 000-vortex wake has about 40 of them,
+// one at the edge of a Gaussian cloud hundreds).  Each warp takes a run of the
+// window's chunks; every chunk is summed as before, only the FP64 sums over
+// the chunks are added in W parts; the window's rows are listed by the warps
+// together.  A function of the body's item count, so its results do not
+// depend on the launch.  1000 / 5000 / 20 000 vortices of the wake: 43 / 50 /
+// 53 us in one part, 15 / 17 / 35 split (event times), a Gaussian cloud of 20
+// 000 76 -> 46; at 60 000 (2000 items) two parts are still 90 -> 83, at 250 000
+// nothing is gained.
+__device__ __forceinline__ int diff_split(long long nitems) {
+    return nitems > 2048 ? 1 : (nitems > 1024 ? 2 : (nitems > 512 ? 4 : 8));
+}
+struct DiffShared {
     // per warp 32 staged sources as x[32], y[32], G[32]: one 16-byte shared
     // load brings four sources' x (or y, or G)
-    __shared__ float4 sx[CG_T / 4], sy[CG_T / 4], sg[CG_T / 4];
-    __shared__ DiffRow srow[CG_T / 32][DIFF_ROWS];
+    float4 sx[CG_T / 4], sy[CG_T / 4], sg[CG_T / 4];
+    DiffRow row[CG_T / 32][DIFF_ROWS];
+    // the split's partial sums, by warp: two sets, so that one barrier an item is enough
+    double sum[2][CG_T / 32][3][32];
+};
+// SPLIT: W = diff_split warps an item; else W = 1.
+template <bool SPLIT>
+__device__ __forceinline__ void diff_items(const VxBlkB<CG_T, VX_DIFF_MINB> &vb, const VxParams &p, const VxView &v,
+                                           VxScalars *S, const float4 *srt, const unsigned *skey, const int *sorted,
+                                           const int *start, const int2 *items, int *wide, DiffShared &sh, int W) {
+    if (!SPLIT) W = 1;
     const int lane = threadIdx.x & 31;
-    float4 *wx = sx + ((threadIdx.x & ~31) >> 2), *wy = sy + ((threadIdx.x & ~31) >> 2),
-           *wg = sg + ((threadIdx.x & ~31) >> 2);
-    DiffRow *wrow = srow[threadIdx.x >> 5];
+    float4 *wx = sh.sx + ((threadIdx.x & ~31) >> 2), *wy = sh.sy + ((threadIdx.x & ~31) >> 2),
+           *wg = sh.sg + ((threadIdx.x & ~31) >> 2);
     const long long nitems = S->cnitems, nx = S->cnx, ny = S->cny;
+    const int warp = threadIdx.x >> 5, part = SPLIT ? warp % W : 0;   // this warp's part of its item
+    DiffRow *wrow = sh.row[warp - part];   // the item's row list
+    // the item's W warps only: other items of the block run on their own
+    const auto barrier = [&]() {
+        if (SPLIT) asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / W), "r"(32 * W) : "memory");
+        else __syncwarp();
+    };
+    int flip = 0;
     const double hyd = S->chy;
     const float hx = (float)S->ch, hy = (float)hyd;
     const float cut = (float)p.diff_cutoff;
     const float thr2 = (float)(0.001 * p.eps) * (float)(0.001 * p.eps);
     const float log2e = 1.4426950408889634f;
-    const long long wpb = CG_T / 32;
+    const long long wpb = CG_T / 32 / W;   // items of a block at a time
     unsigned long long pairs = 0;
-    for (long long it = vb.x * wpb + (threadIdx.x >> 5); it < nitems; it += vb.n * wpb) {
+    for (long long it = vb.x * wpb + warp / W; it < nitems; it += vb.n * wpb) {
         const int2 item = items[it];
         const long long row = item.x;
         const long long row_end = start[(row + 1) * nx];
@@ -402,7 +433,7 @@ VX_DEVK void k_diff_cells_body(VxBlkB<CG_T, VX_DIFF_MINB> vb, const VxParams &p,
         const float rmean = rsum / (float)max(rcnt, 1);
         const bool too_wide = R > (float)CG_KMAX * hy || (R > (float)CG_KCAP * hy && R > 2.0f * rmean);
         const bool is_wide = valid && (too_wide || far_frame);
-        if (is_wide) wide[atomicAdd(&S->cnwide, 1)] = (int)t;
+        if (is_wide && part == 0) wide[atomicAdd(&S->cnwide, 1)] = (int)t;
         const bool act = valid && !is_wide;
         float rmax = act ? R : 0.0f;
         for (int o = 16; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
@@ -411,71 +442,82 @@ VX_DEVK void k_diff_cells_body(VxBlkB<CG_T, VX_DIFF_MINB> vb, const VxParams &p,
         const f2 TX = f2_pack(me.x, me.x), TY = f2_pack(me.y, me.y);
         const float nd = -log2e / me.w;
         const f2 NDD = f2_pack(nd, nd);
-        // rows -kk..kk (kk <= CG_KMAX: a non-wide target's radius is at most CG_KMAX cells)
+        // rows -kk..kk (kk <= CG_KMAX: a non-wide target's radius is at most
+        // CG_KMAX cells), every W-th of them listed by this warp
         const int kk = min((int)ceilf(rmax / hy), CG_KMAX);
         const int nrows = 2 * kk + 1;
-        int total = 0;
-        for (int r0 = 0; r0 < nrows; r0 += 32) {
-            // columns of row r0 + lane: the union of the active targets' own
-            // ranges in that row, each within sqrt(R^2 - gy^2) of the
-            // target's x (gy its vertical gap to the row, less a margin over
-            // FP32 rounding), column offsets from the item's first column
-            int mc0 = 0, mc1 = -1;
-            const int rn = min(32, nrows - r0);
-            for (int q = 0; q < rn; ++q) {
-                const float fy = (float)(r0 + q - kk) * hy;
-                int lo = 0x7fffffff, hi = -0x7fffffff;
-                if (act) {
-                    const float gy = fmaxf(fmaxf(fy - 0.5f * hy - me.y, me.y - fy - 0.5f * hy) - 1e-3f * hy, 0.0f);
-                    const float w2 = R * R - gy * gy;
-                    if (w2 >= 0.0f) {
-                        const float hw = sqrtf(w2) * 1.0001f + 1e-3f * hx;
-                        lo = (int)floorf((me.x - hw) / hx + 0.5f);
-                        hi = (int)floorf((me.x + hw) / hx + 0.5f);
-                    }
-                }
-                lo = __reduce_min_sync(0xffffffffu, lo);
-                hi = __reduce_max_sync(0xffffffffu, hi);
-                if (lane == q) { mc0 = lo; mc1 = hi; }
-            }
-            const int r = r0 + lane;
-            DiffRow e = {0, 0, 0u, 0.0f};
-            int len = 0;
-            if (r < nrows && mc0 <= mc1) {
-                const int dy = r - kk;
-                const long long rr = row + dy;
-                const long long c0 = max(ocol + mc0, 0LL), c1 = min(ocol + (long long)mc1, nx - 1);
-                if (rr >= 0 && rr < ny && c0 <= c1) {
-                    e.j0 = start[rr * nx + c0];
-                    len = start[rr * nx + c1 + 1] - e.j0;
-                    e.base = (unsigned)(rr * nx + ocol);
-                    e.oy = (float)((double)dy * hyd);
+        // columns of a row: the union of the active targets' own ranges in
+        // that row, each within sqrt(R^2 - gy^2) of the target's x (gy its
+        // vertical gap to the row, less a margin over FP32 rounding), column
+        // offsets from the item's first column; lane q keeps row q's
+        int mc0 = 0, mc1 = -1;
+        for (int q = part; q < nrows; q += W) {
+            const float fy = (float)(q - kk) * hy;
+            int lo = 0x7fffffff, hi = -0x7fffffff;
+            if (act) {
+                const float gy = fmaxf(fmaxf(fy - 0.5f * hy - me.y, me.y - fy - 0.5f * hy) - 1e-3f * hy, 0.0f);
+                const float w2 = R * R - gy * gy;
+                if (w2 >= 0.0f) {
+                    const float hw = sqrtf(w2) * 1.0001f + 1e-3f * hx;
+                    lo = (int)floorf((me.x - hw) / hx + 0.5f);
+                    hi = (int)floorf((me.x + hw) / hx + 0.5f);
                 }
             }
-            int inc = len;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += u;
-            }
-            e.pre = total + inc - len;
-            if (r < nrows) wrow[r] = e;
-            total += __shfl_sync(0xffffffffu, inc, 31);
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            if (lane == q) { mc0 = lo; mc1 = hi; }
         }
-        if (lane == 0) wrow[nrows].pre = total;
-        __syncwarp();
+        DiffRow e = {0, 0, 0u, 0.0f};
+        int len = 0;
+        if (lane < nrows && (!SPLIT || lane % W == part)) {
+            const int dy = lane - kk;
+            const long long rr = row + dy;
+            const long long c0 = max(ocol + mc0, 0LL), c1 = min(ocol + (long long)mc1, nx - 1);
+            if (mc0 <= mc1 && rr >= 0 && rr < ny && c0 <= c1) {
+                e.j0 = start[rr * nx + c0];
+                len = start[rr * nx + c1 + 1] - e.j0;
+                e.base = (unsigned)(rr * nx + ocol);
+                e.oy = (float)((double)dy * hyd);
+            }
+            if (SPLIT) {
+                e.pre = len;   // until all rows are listed
+                wrow[lane] = e;
+            }
+        }
+        if (SPLIT) {
+            barrier();
+            len = lane < nrows ? wrow[lane].pre : 0;
+        }
+        int inc = len;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        const int total = __shfl_sync(0xffffffffu, inc, 31);
+        if (SPLIT) {
+            barrier();
+            if (part == 0 && lane <= nrows) wrow[lane].pre = inc - len;   // the entry after the last row: the total
+            barrier();
+        } else {
+            e.pre = inc - len;
+            if (lane <= nrows) wrow[lane] = e;
+            __syncwarp();
+        }
         double I2x = 0.0, I2y = 0.0, I1 = 0.0;
         int rc = 0;   // this lane's row cursor (rows only advance as the chunks do)
+        const int nch = (total + 31) / 32;
+        const int jt0 = part * nch / W * 32, jt1 = min(total, (part + 1) * nch / W * 32);
         // the next chunk's source is loaded before the current chunk's pairs
         // run, so its L2 latency overlaps them
         float4 qn = make_float4(0.f, 0.f, 0.f, 0.f);
         unsigned kn = 0u;
-        if (lane < total) {
-            while (rc < nrows - 1 && wrow[rc + 1].pre <= lane) ++rc;
-            const int j = wrow[rc].j0 + (lane - wrow[rc].pre);
+        if (jt0 + lane < total) {
+            while (rc < nrows - 1 && wrow[rc + 1].pre <= jt0 + lane) ++rc;
+            const int j = wrow[rc].j0 + (jt0 + lane - wrow[rc].pre);
             qn = srt[j];
             kn = skey[j];
         }
-        for (int jt = 0; jt < total; jt += 32) {
+        for (int jt = jt0; jt < jt1; jt += 32) {
             const int f = jt + lane;
             float x = 0.f, y = 0.f, gq = 0.f;
             if (f < total) {
@@ -520,6 +562,19 @@ VX_DEVK void k_diff_cells_body(VxBlkB<CG_T, VX_DIFF_MINB> vb, const VxParams &p,
             f2_unpack(S1, a, b); I1 += (double)(a + b);
         }
         __syncwarp();   // the row list is rewritten by the next item
+        if (SPLIT) {
+            double (*o)[32] = sh.sum[flip][warp];
+            o[0][lane] = I2x; o[1][lane] = I2y; o[2][lane] = I1;
+            barrier();
+            if (part == 0)
+                for (int w = 1; w < W; ++w) {
+                    I2x += sh.sum[flip][warp + w][0][lane];
+                    I2y += sh.sum[flip][warp + w][1][lane];
+                    I1 += sh.sum[flip][warp + w][2][lane];
+                }
+            flip ^= 1;
+            if (part != 0) continue;
+        }
         pairs += (unsigned long long)total * (unsigned long long)nact;
         if (act && fabs(I1) > 1e-5) {
             const long long i = sorted[t];
@@ -529,6 +584,15 @@ VX_DEVK void k_diff_cells_body(VxBlkB<CG_T, VX_DIFF_MINB> vb, const VxParams &p,
         }
     }
     if (lane == 0 && pairs) atomicAdd(&S->pairs_diff, pairs);
+}
+VX_DEVK void k_diff_cells_body(VxBlkB<CG_T, VX_DIFF_MINB> vb, const VxParams &p, const VxView &v, VxScalars *S,
+                               const float4 *srt, const unsigned *skey,
+                               const int *sorted, const int *start,
+                               const int2 *items, int *wide) {
+    __shared__ DiffShared sh;
+    const int W = diff_split(S->cnitems);
+    if (W > 1) diff_items<true>(vb, p, v, S, srt, skey, sorted, start, items, wide, sh, W);
+    else diff_items<false>(vb, p, v, S, srt, skey, sorted, start, items, wide, sh, 1);
 }
 __global__ void __launch_bounds__(CG_T, VX_DIFF_MINB) k_diff_cells(VxParams p, VxView v, VxScalars *S,
                                                                    const float4 *srt, const unsigned *skey,
@@ -540,9 +604,9 @@ __global__ void __launch_bounds__(CG_T, VX_DIFF_MINB) k_diff_cells(VxParams p, V
 
 // Targets left out of the work items (radius beyond CG_KCAP rows).  Most
 // have windows of about a thousand sources inside their circles (the sparse
-// edge of a Gaussian cloud: about 1 % of its vortices): one warp each
-// (k_diff_wide), the lanes taking the concatenated sources of 32 rows at a
-// time.  A vortex whose window spans more than WIDE_ROWS rows each side (up
+// edge of a Gaussian cloud: about 1 % of its vortices): one warp each, or a few
+// (k_diff_wide), the lanes taking the concatenated sources of 32 rows.  A
+// vortex whose window spans more than WIDE_ROWS rows each side (up
 // to the whole grid: a vortex flung far from the cloud) is passed on to
 // k_diff_huge: one block of WIDE_T threads each, its warps taking the rows in
 // batches of equal height.  FP32 pair sums per lane over at most 16 sources,
@@ -550,19 +614,13 @@ __global__ void __launch_bounds__(CG_T, VX_DIFF_MINB) k_diff_cells(VxParams p, V
 constexpr int WIDE_ROWS = 16 * CG_DIV_Y;   // sixteen mean cut-off radii
 constexpr int WIDE_T = 512;
 
-// Rows dy0 .. dy0 + nr - 1 (nr <= 32) of one target's window: lane l lists
-// row dy0 + l (its column range clipped to the target's own circle) in the
-// warp's row table (first source, offset in the concatenation, cell-key base,
-// y offset; entry 32 holds the total), and the lanes take the concatenated
-// sources 32 at a time, so rows of a few sources (the window of an isolated
-// vortex is mostly empty rows and short ranges) do not idle the warp.  FP32
-// sums per lane, carried into FP64 every 16 sources.
+// Rows dy0 .. dy0 + nr - 1 (nr <= 32) of one target's window, listed by a
+// warp: lane l lists row dy0 + l (its column range clipped to the target's own
+// circle) in the row table (first source, offset in the concatenation,
+// cell-key base, y offset; entry 32 holds the total, which is returned).
 constexpr int WIDE_TABLE = 33;
-__device__ __forceinline__ void wide_rows32(const VxScalars *S, const float4 *srt, const unsigned *skey,
-                                            const int *start, const float4 me, long long row, long long ocol,
-                                            float R, float R2, float ndd, float thr2, long long dy0, int nr,
-                                            int lane, DiffRow *wrow, double &I2x, double &I2y, double &I1,
-                                            unsigned long long &pairs) {
+__device__ __forceinline__ int wide_table(const VxScalars *S, const int *start, const float4 me, long long row,
+                                          long long ocol, float R, long long dy0, int nr, int lane, DiffRow *wrow) {
     const long long nx = S->cnx, ny = S->cny;
     const double hyd = S->chy;
     const float hx = (float)S->ch, hy = (float)hyd;
@@ -587,25 +645,49 @@ __device__ __forceinline__ void wide_rows32(const VxScalars *S, const float4 *sr
     e.pre = inc - len;
     wrow[lane] = e;
     if (lane == 0) wrow[32].pre = total;
-    __syncwarp();
-    pairs += (unsigned long long)total;
+    return total;
+}
+
+// Sources [f0, f1) of a table's concatenation, the lanes 32 at a time (f1 - f0
+// at most 512: FP32 sums per lane over at most 16 sources), so rows of a
+// few sources (the window of an isolated vortex is mostly empty rows and short
+// ranges) do not idle the warp.
+constexpr int WIDE_RUN = 512;
+__device__ __forceinline__ void wide_run(const float4 *srt, const unsigned *skey, const float4 me, float hx, float R2,
+                                         float ndd, float thr2, int f0, int f1, int lane, const DiffRow *wrow,
+                                         double &I2x, double &I2y, double &I1) {
     float s2x = 0.f, s2y = 0.f, s1 = 0.f;
-    int rc = 0, cnt = 0;
-    for (int f = lane; f < total; f += 32) {
+    int rc = 0;
+    float4 qn = make_float4(0.f, 0.f, 0.f, 0.f);
+    unsigned kn = 0u;
+    const auto fetch = [&](int f) {
         while (wrow[rc + 1].pre <= f) ++rc;   // entry 32 (the total) stops it
+        const int j = wrow[rc].j0 + (f - wrow[rc].pre);
+        qn = srt[j];
+        kn = skey[j];
+    };
+    if (f0 + lane < f1) fetch(f0 + lane);
+    for (int f = f0 + lane; f < f1; f += 32) {
         const DiffRow r = wrow[rc];
-        const int j = r.j0 + (f - r.pre);
-        float4 q = srt[j];
-        q.x += (float)(int)(skey[j] - r.base) * hx;
+        float4 q = qn;
+        q.x += (float)(int)(kn - r.base) * hx;
         q.y += r.oy;
+        if (f + 32 < f1) fetch(f + 32);   // on its way while this source's pair runs
         diff_pair(me.x, me.y, R2, ndd, thr2, q, s2x, s2y, s1);
-        if (++cnt == 16) {
-            I2x += (double)s2x; I2y += (double)s2y; I1 += (double)s1;
-            s2x = s2y = s1 = 0.f;
-            cnt = 0;
-        }
     }
     I2x += (double)s2x; I2y += (double)s2y; I1 += (double)s1;
+}
+
+__device__ __forceinline__ void wide_rows32(const VxScalars *S, const float4 *srt, const unsigned *skey,
+                                            const int *start, const float4 me, long long row, long long ocol,
+                                            float R, float R2, float ndd, float thr2, long long dy0, int nr,
+                                            int lane, DiffRow *wrow, double &I2x, double &I2y, double &I1,
+                                            unsigned long long &pairs) {
+    const int total = wide_table(S, start, me, row, ocol, R, dy0, nr, lane, wrow);
+    __syncwarp();
+    pairs += (unsigned long long)total;
+    for (int f = 0; f < total; f += WIDE_RUN)
+        wide_run(srt, skey, me, (float)S->ch, R2, ndd, thr2, f, min(f + WIDE_RUN, total), lane, wrow, I2x, I2y, I1);
     __syncwarp();   // the table is rewritten by the next call
 }
 
@@ -619,43 +701,72 @@ __device__ __forceinline__ void wide_apply(const VxParams &p, VxView v, const in
     }
 }
 
+// W warps per target: they list 32 rows of the window each, then take the
+// listed sources in runs of 512 in turn.  An outlier of a Gaussian cloud
+// reaches thousands of sources in up to 129 rows, and where only a few
+// hundred targets are wide the longest of them, by one warp, was the kernel's
+// time; thousands of them (wall-layer targets far from their item's frame)
+// fill the GPU with a warp each.  W follows the body's own count of them, so
+// its results do not depend on the launch.  A Gaussian cloud of 20 000: 36 -> 21 us.
+constexpr int WIDE_NB = (2 * WIDE_ROWS + 1 + 31) / 32;   // batches of 32 rows of the widest window
 VX_DEVK void k_diff_wide_body(VxBlkB<CG_T, 0> vb, const VxParams &p, const VxView &v, VxScalars *S, const float4 *srt,
                               const unsigned *skey, const int *sorted, const int *start,
                               const int *wide, int *huge) {
-    __shared__ DiffRow stab[CG_T / 32][WIDE_TABLE];
-    const int lane = threadIdx.x & 31;
-    DiffRow *wrow = stab[threadIdx.x >> 5];
+    constexpr int NW = CG_T / 32;
+    __shared__ DiffRow stab[NW][WIDE_NB][WIDE_TABLE];
+    __shared__ int stot[NW][WIDE_NB];
+    __shared__ double ssum[NW][3];
+    const int nw = S->cnwide;
+    const int W = nw <= 512 ? NW : (nw <= 2048 ? 2 : 1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp % W, g = warp / W;
+    const auto barrier = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(32 * W) : "memory"); };
     const long long nx = S->cnx, ny = S->cny;
-    const float hy = (float)S->chy;
+    const float hx = (float)S->ch, hy = (float)S->chy;
     const unsigned unx = (unsigned)nx;
     const float cut = (float)p.diff_cutoff;
     const float thr2 = (float)(0.001 * p.eps) * (float)(0.001 * p.eps);
     const float log2e = 1.4426950408889634f;
-    const int nw = S->cnwide;
-    const int warps = (vb.n * blockDim.x) >> 5;
     unsigned long long pairs = 0;
-    for (int f = (vb.x * blockDim.x + threadIdx.x) >> 5; f < nw; f += warps) {
+    for (int f = vb.x * (NW / W) + g; f < nw; f += vb.n * (NW / W)) {
         const long long t = wide[f];
         const float4 me = srt[t];
         const long long ocol = (long long)(skey[t] % unx), row = (long long)(skey[t] / unx);
         const float R = cut * me.w, R2 = R * R, ndd = -log2e / me.w;
         const long long kk = min((long long)ceilf(R / hy), ny);
         if (kk > WIDE_ROWS) {
-            if (lane == 0) huge[atomicAdd(&S->cnhuge, 1)] = (int)t;
+            if (lane == 0 && part == 0) huge[atomicAdd(&S->cnhuge, 1)] = (int)t;
             continue;
         }
+        const int nb = (int)(2 * kk + 1 + 31) / 32;
+        for (int b = part; b < nb; b += W) {
+            const long long dy0 = -kk + 32 * b;
+            const int total = wide_table(S, start, me, row, ocol, R, dy0, (int)min(32LL, kk - dy0 + 1), lane, stab[g][b]);
+            if (lane == 0) stot[g][b] = total;
+        }
+        barrier();
         double I2x = 0.0, I2y = 0.0, I1 = 0.0;
-        for (long long dy0 = -kk; dy0 <= kk; dy0 += 32)
-            wide_rows32(S, srt, skey, start, me, row, ocol, R, R2, ndd, thr2, dy0, (int)min(32LL, kk - dy0 + 1),
-                        lane, wrow, I2x, I2y, I1, pairs);
+        int u = 0;   // runs so far
+        for (int b = 0; b < nb; ++b) {
+            const int total = stot[g][b];
+            for (int f0 = 0; f0 < total; f0 += WIDE_RUN, ++u)
+                if (u % W == part)
+                    wide_run(srt, skey, me, hx, R2, ndd, thr2, f0, min(f0 + WIDE_RUN, total), lane, stab[g][b], I2x,
+                             I2y, I1);
+            if (part == 0) pairs += (unsigned long long)total;
+        }
         for (int o = 16; o > 0; o >>= 1) {
             I2x += __shfl_xor_sync(0xffffffffu, I2x, o);
             I2y += __shfl_xor_sync(0xffffffffu, I2y, o);
             I1 += __shfl_xor_sync(0xffffffffu, I1, o);
         }
-        if (lane == 0) wide_apply(p, v, sorted, t, me.w, I2x, I2y, I1);
+        if (lane == 0) { ssum[warp][0] = I2x; ssum[warp][1] = I2y; ssum[warp][2] = I1; }
+        barrier();   // also: the tables are used up
+        if (part == 0 && lane == 0) {
+            for (int w = 1; w < W; ++w) { I2x += ssum[warp + w][0]; I2y += ssum[warp + w][1]; I1 += ssum[warp + w][2]; }
+            wide_apply(p, v, sorted, t, me.w, I2x, I2y, I1);
+        }
     }
-    if (lane == 0 && pairs) atomicAdd(&S->pairs_diff, pairs);   // every lane counted the same pairs
+    if (lane == 0 && pairs) atomicAdd(&S->pairs_diff, pairs);
 }
 __global__ void __launch_bounds__(CG_T) k_diff_wide(VxParams p, VxView v, VxScalars *S, const float4 *srt,
                                                     const unsigned *skey, const int *sorted, const int *start,
@@ -741,9 +852,11 @@ cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, cons
     vx_launch<k_cg_items, k_cg_items_body>(L, grid, VX_SCAN_T, 0, S, w.cg_start, w.items, w.items_cap, w.scan_tiles);
 
     VX_EV(L, 2);
-    vx_launch<k_diff_cells, k_diff_cells_body>(L, L.num_sms * 8, CG_T, 0, p, v, S, w.srt, skey, sorted, w.cg_start, w.items, w.cg_wide);
+    // blocks: one per item of a body whose items are split over 8 warps (64 a
+    // 2048 vortices); in a batch the other members' blocks fill the GPU too
+    vx_launch<k_diff_cells, k_diff_cells_body>(L, std::min(vx_full_sms(L) * 8, L.num_sms * (L.rec ? 16 : 64)), CG_T, 0, p, v, S, w.srt, skey, sorted, w.cg_start, w.items, w.cg_wide);
 
-    vx_launch<k_diff_wide, k_diff_wide_body>(L, L.num_sms * 4, CG_T, 0, p, v, S, w.srt, skey, sorted, w.cg_start, w.cg_wide, w.cg_huge);
+    vx_launch<k_diff_wide, k_diff_wide_body>(L, std::min(vx_full_sms(L) * 4, L.num_sms * (L.rec ? 4 : 16)), CG_T, 0, p, v, S, w.srt, skey, sorted, w.cg_start, w.cg_wide, w.cg_huge);
 
     vx_launch<k_diff_huge, k_diff_huge_body>(L, L.num_sms * 2, WIDE_T, 0, p, v, S, w.srt, skey, sorted, w.cg_start, w.cg_huge);
 

@@ -29,7 +29,7 @@
 // direct FP32 with the core smoothing; the 3 nearest come from there and are
 // exact when the third distance is below the leaf side (nothing outside the
 // 3x3 block can be closer); the few targets that fail the test are redone by
-// a ring search over the leaves.
+// a search over squares of leaves.
 #include <algorithm>
 
 #include "vx_internal.cuh"
@@ -896,7 +896,7 @@ __global__ void __launch_bounds__(FMM_T, VX_NEAR_MINB) k_fmm_near(VxParams p, Vx
 // sorted sources; coordinates relative to the target's leaf centre,
 // computed as the near field computes them).  Exact when the third distance
 // is below the quarter's side (every source outside the 3 x 3 block is
-// farther); the others go to the ring search over leaves (k_fmm_nn3_fix).
+// farther); the others go to the search over squares of leaves (k_fmm_nn3_fix).
 VX_DEVK void k_fmm_nn3_sub_body(VxBlkB<FMM_T, 0> vb, const VxView &v, VxScalars *S, const float4 *srt, const unsigned *skey,
                                 const int *sorted, const int *substart, int *flag_list) {
     const long long s = S->fs, n = S->n;
@@ -960,31 +960,27 @@ __global__ void __launch_bounds__(FMM_T) k_fmm_nn3_sub(VxView v, VxScalars *S, c
     k_fmm_nn3_sub_body(VxBlkB<FMM_T, 0>{blockIdx.x, gridDim.x}, v, S, srt, skey, sorted, substart, flag_list);
 }
 
-// Targets whose third-nearest distance reached the leaf side: exact 3
-// nearest by a ring search over the leaves (one warp per target).  Ring k
-// holds the 8k leaves at Chebyshev distance k from the target's leaf; every
-// source outside rings 0..k lies at least k*h from the target (a source
-// clamped into an edge leaf lies farther out than that leaf), so the search
-// stops once the third distance is below (k h)^2 or the rings cover the grid.
-// Coordinates are relative to the target's leaf centre, as in the near field.
-// The search stops after NN3_RINGS rings: an isolated vortex (one flung out
-// of the wake) would need rings over much of the grid, which one warp walks
-// for a millisecond or more; such targets go to k_fmm_nn3_brute instead, a
-// block scanning every source.
-constexpr int NN3_RINGS = 6;
-__device__ __forceinline__ void fmm_ring_cell(int k, int q, int &dx, int &dy) {
-    if (k == 0) { dx = dy = 0; return; }
-    const int w = 2 * k + 1;
-    if (q < w) { dx = q - k; dy = -k; return; }
-    q -= w;
-    if (q < w) { dx = q - k; dy = k; return; }
-    q -= w;
-    if (q < w - 2) { dx = -k; dy = q - k + 1; return; }
-    q -= w - 2;
-    dx = k; dy = q - k + 1;
-}
+// Targets whose third-nearest distance reached the quarter's side: exact 3
+// nearest by a search over the leaves (one warp per target) in the squares of
+// leaves within 1, 3 and 6 of the target's.  Every source outside the square
+// of half-width k lies at least k h from the target (a source clamped into an
+// edge leaf lies farther out than that leaf), so the search stops once the
+// third distance is below (k h)^2 or the square covers the grid.  A square's
+// rows are contiguous runs of the leaf-sorted sources; the lanes take the
+// concatenated runs 32 sources at a time (a lane per leaf, each walking its
+// own leaf's sources, left a dense cloud's edge to a few lanes: 48 us in a
+// batch of 16 bodies).  Coordinates are relative to the target's leaf
+// centre, as in the near field.  An isolated vortex (one flung out of the
+// wake) would need rows over much of the grid; it is left to the last block's
+// scan of every source.
+constexpr int NN3_HALF = 6;                      // half-width of the largest square
+constexpr int NN3_ROWS = 2 * NN3_HALF + 1;
+struct Nn3Row {
+    int j0, pre;   // first source of the row's run, sources of the rows before it
+    float oy;      // row offset
+};
 
-// The targets the ring search left over, by one block: each scans every
+// The targets that search left over, by one block: each scans every
 // source slot (FP64 differences, as the direct pass).
 __device__ void fmm_nn3_brute_block(VxView v, VxScalars *S, const int *brute_list) {
     __shared__ float sd[3][FMM_T / 32];
@@ -1022,72 +1018,80 @@ __device__ void fmm_nn3_brute_block(VxView v, VxScalars *S, const int *brute_lis
     }
 }
 
-VX_DEVK void k_fmm_nn3_fix_body(VxBlkB<0, 0> vb, const VxView &v, VxScalars *S, const float4 *srt, const int *sorted,
+VX_DEVK void k_fmm_nn3_fix_body(VxBlkB<FMM_T, 0> vb, const VxView &v, VxScalars *S, const float4 *srt, const int *sorted,
                                 const int *start, const int *flag_list, int *brute_list) {
+    __shared__ Nn3Row stab[FMM_T / 32][NN3_ROWS + 1];
     const int nf = S->fnflag;
     const long long m = 1LL << S->fL;
     const double h = S->fside / (double)m;
     const int lane = threadIdx.x & 31;
+    Nn3Row *rows = stab[threadIdx.x >> 5];
     const int warps = (vb.n * blockDim.x) >> 5;
     for (int f = (vb.x * blockDim.x + threadIdx.x) >> 5; f < nf; f += warps) {
         const long long t = flag_list[f];
         const long long i = sorted[t];
         const long long leaf = fmm_leaf(S, v.x[i * v.ps], v.y[i * v.ps]);
-        const long long cx = leaf % m, cy = leaf / m;
+        const int cx = (int)(leaf % m), cy = (int)(leaf / m);
         const float4 me = srt[t];
-        const long long kmax = max(max(cx, m - 1 - cx), max(cy, m - 1 - cy));
+        const int kmax = max(max(cx, (int)m - 1 - cx), max(cy, (int)m - 1 - cy));
         float d1 = 1e5f, d2 = 1e5f, d3 = 1e5f;
         bool found = false;
-        for (long long k = 0; k <= min(kmax, (long long)NN3_RINGS); ++k) {
-            const int ncell = k == 0 ? 1 : (int)(8 * k);
-            for (int q = lane; q < ncell; q += 32) {
-                int dx, dy;
-                fmm_ring_cell((int)k, q, dx, dy);
-                const long long X = cx + dx, Y = cy + dy;
-                if (X < 0 || X >= m || Y < 0 || Y >= m) continue;
-                const float ox = (float)((double)dx * h), oy = (float)((double)dy * h);
-                const long long c = Y * m + X;
-                for (long long j = start[c]; j < start[c + 1]; ++j) {
-                    if (j == t) continue;
-                    const float4 s = srt[j];
-                    const float ddx = me.x - (s.x + ox), ddy = me.y - (s.y + oy);
-                    vx_nn3_insert<float>(d1, d2, d3, fmaf(ddx, ddx, ddy * ddy));
-                }
+        for (int k = 1; k <= NN3_HALF; k = k == 1 ? 3 : (k == 3 ? NN3_HALF : NN3_HALF + 1)) {
+            const int c0 = max(cx - k, 0), c1 = min(cx + k, (int)m - 1), nr = 2 * k + 1;
+            int j0 = 0, len = 0;
+            const int rr = cy - k + lane;
+            if (lane < nr && rr >= 0 && rr < m) {
+                j0 = start[rr * m + c0];
+                len = start[rr * m + c1 + 1] - j0;
             }
+            int inc = len;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += u;
+            }
+            const int total = __shfl_sync(0xffffffffu, inc, 31);
+            if (lane < nr) rows[lane] = Nn3Row{j0, inc - len, (float)((double)(lane - k) * h)};
+            if (lane == 0) rows[nr].pre = total;
+            __syncwarp();
+            d1 = d2 = d3 = 1e5f;
+            int rc = 0;
+            for (int e = lane; e < total; e += 32) {
+                while (rows[rc + 1].pre <= e) ++rc;   // the entry after the last row (the total) stops it
+                const Nn3Row r = rows[rc];
+                const int j = r.j0 + (e - r.pre);
+                if (j == t) continue;
+                const float4 q = srt[j];
+                // the source's column less the target's, times h
+                const float ox = (float)((double)(q.w - (float)cx) * h);
+                const float dx = me.x - (q.x + ox), dy = me.y - (q.y + r.oy);
+                vx_nn3_insert_bf(d1, d2, d3, fmaf(dx, dx, dy * dy));
+            }
+            __syncwarp();   // the rows are rewritten by the next square
             for (int o = 16; o > 0; o >>= 1) {
                 const float e1 = __shfl_xor_sync(0xffffffffu, d1, o);
                 const float e2 = __shfl_xor_sync(0xffffffffu, d2, o);
                 const float e3 = __shfl_xor_sync(0xffffffffu, d3, o);
-                vx_nn3_insert<float>(d1, d2, d3, e1);
-                vx_nn3_insert<float>(d1, d2, d3, e2);
-                vx_nn3_insert<float>(d1, d2, d3, e3);
+                vx_nn3_insert_bf(d1, d2, d3, e1);
+                vx_nn3_insert_bf(d1, d2, d3, e2);
+                vx_nn3_insert_bf(d1, d2, d3, e3);
             }
-            // every lane holds the merged three; keep them in lane 0 only so
-            // that the next ring merges disjoint sets
             const float kh = (float)((double)k * h);
-            const bool done = d3 < kh * kh || k == kmax;
-            if (lane != 0) d1 = d2 = d3 = 1e5f;
-            if (done) { found = true; break; }
+            if (d3 < kh * kh || k >= kmax) { found = true; break; }
         }
         if (lane == 0) {
             if (found) v.d[i] = (double)((sqrtf(d1) + sqrtf(d2) + sqrtf(d3)) / 3);
             else brute_list[atomicAdd(&S->fnbrute, 1)] = (int)i;
         }
     }
-    // the rare targets no ring settled: the block that finishes last scans
+    // the rare targets no square settled: the block that finishes last scans
     // every source for them
     if (vx_last_block(&S->sync_ctr, vb.n)) fmm_nn3_brute_block(v, S, brute_list);
 }
-__global__ void k_fmm_nn3_fix(VxView v, VxScalars *S, const float4 *srt, const int *sorted,
+__global__ void __launch_bounds__(FMM_T) k_fmm_nn3_fix(VxView v, VxScalars *S, const float4 *srt, const int *sorted,
                               const int *start, const int *flag_list, int *brute_list) {
     VX_PDL_WAIT();
-    k_fmm_nn3_fix_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, srt, sorted, start, flag_list, brute_list);
+    k_fmm_nn3_fix_body(VxBlkB<FMM_T, 0>{blockIdx.x, gridDim.x}, v, S, srt, sorted, start, flag_list, brute_list);
 }
-
-// The 3 nearest of the targets the ring search left (original indices in
-// brute_list) over every source slot [0, fs): one block per target, each
-// thread keeping the three smallest of its stride, merged over the warp and
-// the block (the same set of sources as the ring search, so the same three).
 
 // Near-field work items: every leaf's targets in chunks of FMM_W, leaves in
 // index order (row-major), as (leaf, first target slot); one-pass scan of
