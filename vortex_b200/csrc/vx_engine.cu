@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <map>
+#include <mutex>
 #include <string>
 #include <cstddef>
 #include <vector>
@@ -48,12 +49,70 @@ void vx_keep_pool(int device) {
 }
 
 // A destroyed handle's stream-ordered memory goes back to the driver (the
-// pool keeps it otherwise, out of reach of plain cudaMalloc callers).
+// pool keeps it otherwise, out of reach of plain cudaMalloc callers), but for
+// a small body's worth: mapping it afresh for the next body and unmapping it
+// took 1 to 2 ms of a creation and a destruction each.
+constexpr size_t POOL_KEEP = 64 << 20;
 void vx_trim_pool(int device) {
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess) { cudaGetLastError(); return; }
-    if (cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
+    if (cudaMemPoolTrimTo(pool, POOL_KEEP) != cudaSuccess) cudaGetLastError();
 }
+
+// Pinned mirrors of the device scalars: slots of a pinned block shared by the
+// handles (a cudaMallocHost and cudaFreeHost of its own took 1.5 to 3 ms a
+// handle).  Blocks of 64 slots; a block none of whose slots is taken is given
+// back, but for one.  Any thread may take and return slots; the memory is
+// portable, so handles of every device share it.
+namespace {
+class PinnedScalars {
+public:
+    VxScalars *take() {
+        std::lock_guard<std::mutex> lock(mu_);
+        for (Block &b : blocks_)
+            if (b.used != ~0ull) return slot(b);
+        void *m = nullptr;
+        if (cudaHostAlloc(&m, 64 * STRIDE, cudaHostAllocPortable) != cudaSuccess) return nullptr;
+        blocks_.push_back(Block{static_cast<char *>(m), 0});
+        return slot(blocks_.back());
+    }
+    void give(VxScalars *p) {
+        std::lock_guard<std::mutex> lock(mu_);
+        const char *c = reinterpret_cast<char *>(p);
+        int empty = 0;
+        for (Block &b : blocks_) {
+            if (c >= b.base && c < b.base + 64 * STRIDE) b.used &= ~(1ull << ((c - b.base) / STRIDE));
+            empty += b.used == 0;
+        }
+        for (size_t k = 0; k < blocks_.size() && empty > 1;)
+            if (blocks_[k].used == 0) {
+                cudaFreeHost(blocks_[k].base);
+                blocks_.erase(blocks_.begin() + (long)k);
+                --empty;
+            } else {
+                ++k;
+            }
+    }
+
+private:
+    struct Block {
+        char *base;
+        unsigned long long used;
+    };
+    static constexpr size_t STRIDE = (sizeof(VxScalars) + 255) / 256 * 256;
+    static VxScalars *slot(Block &b) {
+        const int k = __builtin_ctzll(~b.used);
+        b.used |= 1ull << k;
+        return reinterpret_cast<VxScalars *>(b.base + (size_t)k * STRIDE);
+    }
+    std::mutex mu_;
+    std::vector<Block> blocks_;
+};
+PinnedScalars &pinned_scalars() {
+    static PinnedScalars *p = new PinnedScalars();   // never destroyed: handles may outlive static destructors
+    return *p;
+}
+}  // namespace
 
 extern "C" const char *vx_status_str(vx_status s) {
     switch (s) {
@@ -414,15 +473,17 @@ int vx_sim_rhs_chunks(vx_sim *s) { return rhs_chunks_for(s); }
 // Wall panel lists: cells of side 5 L_max (1 % margin) over the birth-point
 // box grown by 5 L_max; each panel is listed in the 3 x 3 cells around its
 // birth point, in ascending panel order.
-static vx_status build_wall_lists(vx_sim *s, const vx_panel *pan, int P) {
-    VxParams &p = s->prm;
+struct PanelLists {
+    std::vector<int> start, idx;   // per cell; empty: no lists
+};
+static void build_wall_lists(VxParams &p, const vx_panel *pan, int P, PanelLists &out) {
     double lmax = 0.0;
     for (int i = 0; i < P; ++i) lmax = std::max(lmax, pan[i].length);
-    if (P <= 0 || !(lmax > 0.0)) { p.wall_nx = p.wall_ny = 0; return VX_OK; }
+    if (P <= 0 || !(lmax > 0.0)) { p.wall_nx = p.wall_ny = 0; return; }
     const double h = 5.0 * lmax * 1.01;
     const long long nx = std::max(1LL, (long long)std::ceil((p.wall_x1 - p.wall_x0) / h));
     const long long ny = std::max(1LL, (long long)std::ceil((p.wall_y1 - p.wall_y0) / h));
-    if (nx * ny > (1LL << 24)) { p.wall_nx = p.wall_ny = 0; return VX_OK; }   // degenerate: test all
+    if (nx * ny > (1LL << 24)) { p.wall_nx = p.wall_ny = 0; return; }   // degenerate: test all
     std::vector<std::vector<int>> cells((size_t)(nx * ny));
     for (int f = 0; f < P; ++f) {
         const long long cx = std::min(std::max((long long)std::floor((pan[f].birth[0] - p.wall_x0) / h), 0LL), nx - 1);
@@ -438,23 +499,17 @@ static vx_status build_wall_lists(vx_sim *s, const vx_panel *pan, int P) {
     }
     start[cells.size()] = (int)idx.size();
     if (idx.empty()) idx.push_back(0);
-    s->wall_bytes = (long long)sizeof(int) * (long long)(start.size() + idx.size());
-    if (cudaMalloc(&s->d_wstart, sizeof(int) * start.size()) != cudaSuccess) return VX_ERR_NOMEM;
-    if (cudaMalloc(&s->d_widx, sizeof(int) * idx.size()) != cudaSuccess) return VX_ERR_NOMEM;
-    if (cudaMemcpy(s->d_wstart, start.data(), sizeof(int) * start.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(s->d_widx, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-        return VX_ERR_CUDA;
+    out.start.swap(start);
+    out.idx.swap(idx);
     p.wall_h = h;
     p.wall_nx = (int)nx;
     p.wall_ny = (int)ny;
-    return VX_OK;
 }
 
 // Hitting-test panel lists: a grid over the bounding box of all panel
 // endpoints (cells of side 4 L_max, at most 512 per side); each panel is
 // listed, in ascending order, in every cell its own bounding box touches.
-static vx_status build_hit_lists(vx_sim *s, const vx_panel *pan, int P) {
-    VxParams &p = s->prm;
+static void build_hit_lists(VxParams &p, const vx_panel *pan, int P, PanelLists &out) {
     p.hit_nx = p.hit_ny = 0;
     double x0 = 1e300, x1 = -1e300, y0 = 1e300, y1 = -1e300, lmax = 0.0;
     for (int i = 0; i < P; ++i) {
@@ -464,7 +519,7 @@ static vx_status build_hit_lists(vx_sim *s, const vx_panel *pan, int P) {
         }
         lmax = std::max(lmax, pan[i].length);
     }
-    if (P <= 0 || !(lmax > 0.0)) return VX_OK;
+    if (P <= 0 || !(lmax > 0.0)) return;
     double h = 4.0 * lmax;
     h = std::max(h, std::max(x1 - x0, y1 - y0) / 512.0);
     const double pad = 1e-9 * std::max(1.0, std::max(fabs(x0), fabs(x1)) + std::max(fabs(y0), fabs(y1)));
@@ -489,18 +544,13 @@ static vx_status build_hit_lists(vx_sim *s, const vx_panel *pan, int P) {
     }
     start[cells.size()] = (int)idx.size();
     if (idx.empty()) idx.push_back(0);
-    s->wall_bytes += (long long)sizeof(int) * (long long)(start.size() + idx.size());
-    if (cudaMalloc(&s->d_hstart, sizeof(int) * start.size()) != cudaSuccess) return VX_ERR_NOMEM;
-    if (cudaMalloc(&s->d_hidx, sizeof(int) * idx.size()) != cudaSuccess) return VX_ERR_NOMEM;
-    if (cudaMemcpy(s->d_hstart, start.data(), sizeof(int) * start.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(s->d_hidx, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-        return VX_ERR_CUDA;
+    out.start.swap(start);
+    out.idx.swap(idx);
     p.hit_x0 = x0;
     p.hit_y0 = y0;
     p.hit_h = h;
     p.hit_nx = (int)nx;
     p.hit_ny = (int)ny;
-    return VX_OK;
 }
 
 extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t P, int device,
@@ -529,14 +579,11 @@ extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t
     cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(VX_ERR_CUDA);
     vx_params_from_conf(conf, pan, (int)P, &s->prm);
-    std::vector<vx_panel> hp(s->P32);
-    memset(hp.data(), 0, sizeof(vx_panel) * s->P32);
-    memcpy(hp.data(), pan, sizeof(vx_panel) * P);
-    if (cudaMalloc(&s->d_pan, sizeof(vx_panel) * s->P32) != cudaSuccess) return fail(VX_ERR_NOMEM);
-    if (cudaMemcpy(s->d_pan, hp.data(), sizeof(vx_panel) * s->P32, cudaMemcpyHostToDevice) != cudaSuccess)
-        return fail(VX_ERR_CUDA);
-    if (cudaMalloc(&s->d_S, sizeof(VxScalars)) != cudaSuccess) return fail(VX_ERR_NOMEM);
-    if (cudaMallocHost(&s->h_S, sizeof(VxScalars)) != cudaSuccess) return fail(VX_ERR_NOMEM);
+    PanelLists wall, hit;
+    build_wall_lists(s->prm, pan, (int)P, wall);
+    build_hit_lists(s->prm, pan, (int)P, hit);
+    s->h_S = pinned_scalars().take();
+    if (!s->h_S) { vx_set_error("vx_create: no pinned memory"); return fail(VX_ERR_NOMEM); }
     memset(s->h_S, 0, sizeof(VxScalars));
     // V_inf ramp (src/main.c:585-592): with a ramp the flow starts at rest
     s->h_S->incr_steps = conf->v_inf_incr_steps;
@@ -547,17 +594,48 @@ extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t
         s->h_S->vinf[0] = conf->v_inf_x;
         s->h_S->vinf[1] = conf->v_inf_y;
     }
-    if (cudaMemcpy(s->d_S, s->h_S, sizeof(VxScalars), cudaMemcpyHostToDevice) != cudaSuccess)
-        return fail(VX_ERR_CUDA);
-    if (build_wall_lists(s, pan, (int)P) != VX_OK) return fail(VX_ERR_NOMEM);
-    if (build_hit_lists(s, pan, (int)P) != VX_OK) return fail(VX_ERR_NOMEM);
-    // panel system on the device
+    // the body's fixed data in one stream-ordered allocation: the panels
+    // (padded), the scalars and the panel lists, filled by one copy, then the
+    // inverted panel system
     const long long S1 = P + 1;
-    if (cudaMalloc(&s->d_minv, sizeof(double) * S1 * S1) != cudaSuccess) return fail(VX_ERR_NOMEM);
-    double *work = nullptr;
-    int *flag = nullptr;
-    if (cudaMalloc(&work, sizeof(double) * vx_matrix_work((int)P)) != cudaSuccess) return fail(VX_ERR_NOMEM);
-    if (cudaMalloc(&flag, sizeof(int)) != cudaSuccess) { cudaFree(work); return fail(VX_ERR_NOMEM); }
+    size_t at = 0;
+    const auto place = [&at](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) / 256 * 256;
+        return o;
+    };
+    const std::vector<int> *lists[4] = {&wall.start, &wall.idx, &hit.start, &hit.idx};
+    const size_t o_pan = place(sizeof(vx_panel) * (size_t)s->P32), o_S = place(sizeof(VxScalars));
+    size_t o_list[4];
+    for (int k = 0; k < 4; ++k) {
+        o_list[k] = place(sizeof(int) * lists[k]->size());
+        s->wall_bytes += (long long)(sizeof(int) * lists[k]->size());
+    }
+    std::vector<char> host(at, 0);
+    memcpy(host.data() + o_pan, pan, sizeof(vx_panel) * (size_t)P);
+    memcpy(host.data() + o_S, s->h_S, sizeof(VxScalars));
+    for (int k = 0; k < 4; ++k)
+        if (!lists[k]->empty()) memcpy(host.data() + o_list[k], lists[k]->data(), sizeof(int) * lists[k]->size());
+    const size_t o_minv = place(sizeof(double) * (size_t)(S1 * S1));
+    if (cudaMallocAsync(&s->d_fixed, at, s->stream) != cudaSuccess) {
+        vx_set_error("vx_create: %zu device bytes", at);
+        return fail(VX_ERR_NOMEM);
+    }
+    char *base = static_cast<char *>(s->d_fixed);
+    s->d_pan = reinterpret_cast<vx_panel *>(base + o_pan);
+    s->d_S = reinterpret_cast<VxScalars *>(base + o_S);
+    int **dlist[4] = {&s->d_wstart, &s->d_widx, &s->d_hstart, &s->d_hidx};
+    for (int k = 0; k < 4; ++k)
+        if (!lists[k]->empty()) *dlist[k] = reinterpret_cast<int *>(base + o_list[k]);
+    s->d_minv = reinterpret_cast<double *>(base + o_minv);
+    if (cudaMemcpyAsync(base, host.data(), host.size(), cudaMemcpyHostToDevice, s->stream) != cudaSuccess)
+        return fail(VX_ERR_CUDA);
+    // panel system on the device
+    const size_t work_bytes = (sizeof(double) * (size_t)vx_matrix_work((int)P) + 255) / 256 * 256;
+    void *wk = nullptr;
+    if (cudaMallocAsync(&wk, work_bytes + 256, s->stream) != cudaSuccess) return fail(VX_ERR_NOMEM);
+    double *work = static_cast<double *>(wk);
+    int *flag = reinterpret_cast<int *>(static_cast<char *>(wk) + work_bytes);
     VxLaunch L = launch_of(s);
     const int mode = conf->gj_pivot == 1 ? 1 : (conf->gj_pivot == 3 ? 3 : 0);
     cudaError_t e = vx_build_matrix(L, s->d_pan, (int)P, s->d_minv, work, flag, nullptr, mode);
@@ -569,8 +647,7 @@ extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t
         if (e == cudaSuccess) e = cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     }
-    cudaFree(work);
-    cudaFree(flag);
+    cudaFreeAsync(wk, s->stream);
     if (e != cudaSuccess) { vx_set_error("panel system: %s", cudaGetErrorString(e)); return fail(VX_ERR_CUDA); }
     if (hflag) { vx_set_error("panel system is singular (pivot < 1e-12)"); return fail(VX_ERR_SINGULAR); }
     vx_status st = grow(s, std::max<long long>(need_for(s, 0), conf->inc_step > 0 ? conf->inc_step : 8192));
@@ -587,15 +664,9 @@ extern "C" vx_status vx_destroy(vx_sim *s) {
     free_work(s);   // stream-ordered, as allocated
     double *arr[6] = {s->x, s->y, s->g, s->vx, s->vy, s->d};
     for (double *a : arr) if (a) cudaFreeAsync(a, s->stream);
+    if (s->d_fixed) cudaFreeAsync(s->d_fixed, s->stream);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    if (s->d_pan) cudaFree(s->d_pan);
-    if (s->d_minv) cudaFree(s->d_minv);
-    if (s->d_wstart) cudaFree(s->d_wstart);
-    if (s->d_widx) cudaFree(s->d_widx);
-    if (s->d_hstart) cudaFree(s->d_hstart);
-    if (s->d_hidx) cudaFree(s->d_hidx);
-    if (s->d_S) cudaFree(s->d_S);
-    if (s->h_S) cudaFreeHost(s->h_S);
+    if (s->h_S) pinned_scalars().give(s->h_S);
     if (s->d_probe) cudaFree(s->d_probe);
     if (s->d_pts) cudaFree(s->d_pts);
     if (s->d_St) cudaFree(s->d_St);

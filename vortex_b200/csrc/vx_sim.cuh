@@ -11,6 +11,7 @@ struct vx_sim {
     cudaStream_t stream = nullptr;
     int P = 0, P32 = 0;
     VxParams prm;
+    void *d_fixed = nullptr;     // one allocation: the panels, scalars, panel lists and inverse below
     vx_panel *d_pan = nullptr;
     double *d_minv = nullptr;
     int *d_wstart = nullptr, *d_widx = nullptr;   // wall panel lists per wall cell
