@@ -66,3 +66,27 @@ def test_plain_pair_sums(n, odd):
         scale = np.hypot(su, sv)[near].max()
         assert np.abs(a - su)[near].max() <= 1e-12 * scale and np.abs(b - sv)[near].max() <= 1e-12 * scale
     sim.close()
+
+
+@pytest.mark.parametrize("points", [1, 33, 511, 512, 513, 1024, 1025, 5000])
+@pytest.mark.parametrize("n", [1, 300, 20000])
+def test_probe_points(points, n):
+    """Probe velocities at the sizes where the tiles and the two-target form
+    end: plain form against the sums in numpy within 1e-12 of the largest, bulk
+    form within 2e-5 of it (the bulk form's stated velocity bound)."""
+    rng = np.random.default_rng(points + n)
+    x, y, g = rng.uniform(1.0, 3.0, n), rng.uniform(-1.0, 1.0, n), rng.normal(0.0, 1e-3, n)
+    px, py = rng.uniform(0.0, 4.0, points), rng.uniform(-2.0, 2.0, points)
+    ck = conf_kwargs(200)
+    ref = np.zeros((2, points))
+    for a in range(0, points, 500):
+        dx, dy = px[a:a + 500, None] - x, py[a:a + 500, None] - y
+        w = g / np.maximum(dx * dx + dy * dy, ck["ve_size"] ** 2)
+        ref[:, a:a + 500] = 1.0 - (w * dy).sum(1) / (2 * math.pi), (w * dx).sum(1) / (2 * math.pi)
+    scale = np.abs(ref).max()
+    for form, tol in ((N.PREC_FP64, 1e-12), (N.PREC_FP32, 2e-5)):
+        sim = N.Sim(N.default_conf(**dict(ck, precision=form)), profiles.circle(200))
+        sim.set_particles(x, y, g)
+        u, v = sim.probe(px, py)
+        sim.close()
+        assert np.abs(u - ref[0]).max() <= tol * scale and np.abs(v - ref[1]).max() <= tol * scale

@@ -23,7 +23,7 @@ constexpr int PT = 256;       // threads per block = sources per shared tile
 // Resident blocks per SM the pair kernels are compiled for (at most 128
 // registers a thread; the FP32 sum without the 3 nearest needs fewer).
 constexpr int PAIR_MINB = 2;
-constexpr int PROBE32_MINB = 3;
+constexpr int PROBE32_MINB = 4;
 
 // Source split of the pair kernels: K source chunks; the partial sums of
 // target i and chunk sc sit at part[(sc nout + q) tstride + i], tstride =
@@ -225,7 +225,7 @@ __device__ __forceinline__ float vx_rcp_approx(float x) {
 
 constexpr int BS32_TPT = 4;
 
-template <bool NN3, bool CHECK_SELF>
+template <bool CHECK_SELF>
 __device__ __forceinline__ void bs32_tile(const float4 *sm, int cnt, int jbase, const int *ti,
                                           const float *ax, const float *ay, float eps2, float *sx,
                                           float *sy, float *d1, float *d2, float *d3) {
@@ -236,12 +236,10 @@ __device__ __forceinline__ void bs32_tile(const float4 *sm, int cnt, int jbase, 
         for (int k = 0; k < BS32_TPT; ++k) {
             const float dx = ax[k] - s.x, dy = ay[k] - s.y;
             const float r2 = fmaf(dx, dx, dy * dy);
-            if (NN3) {
-                if (r2 < d3[k] && (!CHECK_SELF || jbase + q != ti[k])) {
-                    d3[k] = r2;
-                    float t = fminf(d3[k], d2[k]); d3[k] = fmaxf(d3[k], d2[k]); d2[k] = t;
-                    t = fminf(d1[k], d2[k]); d2[k] = fmaxf(d1[k], d2[k]); d1[k] = t;
-                }
+            if (r2 < d3[k] && (!CHECK_SELF || jbase + q != ti[k])) {
+                d3[k] = r2;
+                float t = fminf(d3[k], d2[k]); d3[k] = fmaxf(d3[k], d2[k]); d2[k] = t;
+                t = fminf(d1[k], d2[k]); d2[k] = fmaxf(d1[k], d2[k]); d1[k] = t;
             }
             const float m = s.z * vx_rcp_approx(fmaxf(r2, eps2));
             sy[k] = fmaf(m, dx, sy[k]);
@@ -250,26 +248,22 @@ __device__ __forceinline__ void bs32_tile(const float4 *sm, int cnt, int jbase, 
     }
 }
 
-template <bool NN3>
-VX_DEVK void k_bs32_partial_body(VxBlkB<PT, NN3 ? PAIR_MINB : PROBE32_MINB> vb, const VxParams &p, const VxScalars *S, const float4 *src32,
-                                 const double *tx, const double *ty, long long tstr,
-                                 long long nt_in, double *part, VxSplit sp) {
+VX_DEVK void k_bs32_partial_body(VxBlkB<PT, PAIR_MINB> vb, const VxParams &p, const VxScalars *S, const float4 *src32,
+                                 const double *tx, const double *ty, long long tstr, double *part, VxSplit sp) {
     int K;
     long long tstride;
     vx_split_of(S, sp, K, tstride);
-    constexpr int NOUT = NN3 ? 5 : 2;
     __shared__ float4 sm[PT];
     const long long n = S->n;
-    const long long nt = nt_in < 0 ? n : nt_in;
-    const long long srange = NN3 ? vx_round32(n) : n;
+    const long long srange = vx_round32(n);
     const long long tile = (long long)PT * BS32_TPT;
-    const long long tiles = vx_ceil_div(nt, tile);
+    const long long tiles = vx_ceil_div(n, tile);
     const long long cs = vx_split_chunk(srange, K);
     const long long items = tiles * K;
     const float eps2 = (float)p.eps2;
     for (long long it = vb.x; it < items; it += vb.n) {
         const long long tt = it % tiles, sc = it / tiles;
-        const long long tlo = tt * tile, thi = min(nt, tlo + tile);
+        const long long tlo = tt * tile, thi = min(n, tlo + tile);
         float ax[BS32_TPT], ay[BS32_TPT], d1[BS32_TPT], d2[BS32_TPT], d3[BS32_TPT];
         int ti[BS32_TPT];
         double vxa[BS32_TPT], vya[BS32_TPT];
@@ -277,7 +271,7 @@ VX_DEVK void k_bs32_partial_body(VxBlkB<PT, NN3 ? PAIR_MINB : PROBE32_MINB> vb, 
         for (int k = 0; k < BS32_TPT; ++k) {
             const long long t = tlo + (long long)k * PT + threadIdx.x;
             ti[k] = (int)t;
-            const long long i = t < nt ? t : 0;
+            const long long i = t < n ? t : 0;
             ax[k] = (float)tx[i * tstr];
             ay[k] = (float)ty[i * tstr];
             vxa[k] = 0.0; vya[k] = 0.0;
@@ -286,45 +280,130 @@ VX_DEVK void k_bs32_partial_body(VxBlkB<PT, NN3 ? PAIR_MINB : PROBE32_MINB> vb, 
         const long long j0 = min(sc * cs, srange), j1 = min(srange, j0 + cs);
         for (long long jt = j0; jt < j1; jt += PT) {
             __syncthreads();
-            if (jt + threadIdx.x < j1) {
-                float4 q = src32[jt + threadIdx.x];
-                if (!NN3 && jt + threadIdx.x >= n) q.z = 0.0f;
-                sm[threadIdx.x] = q;
-            }
+            if (jt + threadIdx.x < j1) sm[threadIdx.x] = src32[jt + threadIdx.x];
             __syncthreads();
             const int cnt = (int)min((long long)PT, j1 - jt);
             float sx[BS32_TPT], sy[BS32_TPT];
 #pragma unroll
             for (int k = 0; k < BS32_TPT; ++k) { sx[k] = 0.0f; sy[k] = 0.0f; }
-            const bool self = NN3 && jt < thi && jt + cnt > tlo;   // uniform per block
+            const bool self = jt < thi && jt + cnt > tlo;   // uniform per block
             if (self)
-                bs32_tile<NN3, true>(sm, cnt, (int)jt, ti, ax, ay, eps2, sx, sy, d1, d2, d3);
+                bs32_tile<true>(sm, cnt, (int)jt, ti, ax, ay, eps2, sx, sy, d1, d2, d3);
             else
-                bs32_tile<NN3, false>(sm, cnt, (int)jt, ti, ax, ay, eps2, sx, sy, d1, d2, d3);
+                bs32_tile<false>(sm, cnt, (int)jt, ti, ax, ay, eps2, sx, sy, d1, d2, d3);
 #pragma unroll
             for (int k = 0; k < BS32_TPT; ++k) { vxa[k] += (double)sx[k]; vya[k] += (double)sy[k]; }
         }
 #pragma unroll
         for (int k = 0; k < BS32_TPT; ++k) {
-            if (ti[k] < nt) {
-                double *o = part + (long long)sc * NOUT * tstride + ti[k];
+            if (ti[k] < n) {
+                double *o = part + (long long)sc * 5 * tstride + ti[k];
                 o[0] = vxa[k];
                 o[tstride] = vya[k];
-                if (NN3) {
-                    o[2 * tstride] = (double)d1[k];
-                    o[3 * tstride] = (double)d2[k];
-                    o[4 * tstride] = (double)d3[k];
-                }
+                o[2 * tstride] = (double)d1[k];
+                o[3 * tstride] = (double)d2[k];
+                o[4 * tstride] = (double)d3[k];
             }
         }
     }
 }
-template <bool NN3>
-__global__ void __launch_bounds__(PT, NN3 ? PAIR_MINB : PROBE32_MINB) k_bs32_partial(VxParams p, const VxScalars *S, const float4 *src32,
-                                                     const double *tx, const double *ty, long long tstr,
-                                                     long long nt_in, double *part, VxSplit sp) {
+__global__ void __launch_bounds__(PT, PAIR_MINB) k_bs32_partial(VxParams p, const VxScalars *S, const float4 *src32,
+                                                                const double *tx, const double *ty, long long tstr,
+                                                                double *part, VxSplit sp) {
     VX_PDL_WAIT();
-    k_bs32_partial_body<NN3>(VxBlkB<PT, NN3 ? PAIR_MINB : PROBE32_MINB>{blockIdx.x, gridDim.x}, p, S, src32, tx, ty, tstr, nt_in, part, sp);
+    k_bs32_partial_body(VxBlkB<PT, PAIR_MINB>{blockIdx.x, gridDim.x}, p, S, src32, tx, ty, tstr, part, sp);
+}
+
+// Bulk-form probe points: the same sums without the 3 nearest, two targets in
+// one packed FP32 operation (sources staged as pairs of equal values), so the
+// special-function pipe's reciprocal a pair is what bounds it (16 a clock and
+// SM) and not issue.  A probe call of 4096 points over 1e6 vortices: 1.50 ms
+// with one target an operation -> 1.30.  Four targets a thread, two where all
+// points fit a tile of 512.
+template <int PROBE_TPT>
+VX_DEVK void k_probe32_partial_body(VxBlkB<PT, PROBE32_MINB> vb, const VxParams &p, const VxScalars *S,
+                                    const float4 *src32, const double *tx, const double *ty, long long tstr,
+                                    long long nt, double *part, VxSplit sp) {
+    int K;
+    long long tstride;
+    vx_split_of(S, sp, K, tstride);
+    __shared__ ulonglong2 sxy[PT];   // (x, x), (y, y)
+    __shared__ f2 sg[PT];            // (G, G)
+    const long long n = S->n;
+    const long long tile = (long long)PT * PROBE_TPT;
+    const long long tiles = vx_ceil_div(nt, tile);
+    const long long cs = vx_split_chunk(n, K);
+    const long long items = tiles * K;
+    const float eps2 = (float)p.eps2;
+    for (long long it = vb.x; it < items; it += vb.n) {
+        const long long tt = it % tiles, sc = it / tiles;
+        f2 ax[PROBE_TPT / 2], ay[PROBE_TPT / 2];
+        double vxa[PROBE_TPT], vya[PROBE_TPT];
+#pragma unroll
+        for (int k = 0; k < PROBE_TPT; k += 2) {
+            float x[2], y[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const long long t = tt * tile + (long long)(k + h) * PT + threadIdx.x, i = t < nt ? t : 0;
+                x[h] = (float)tx[i * tstr];
+                y[h] = (float)ty[i * tstr];
+                vxa[k + h] = vya[k + h] = 0.0;
+            }
+            ax[k / 2] = f2_pack(x[0], x[1]);
+            ay[k / 2] = f2_pack(y[0], y[1]);
+        }
+        const long long j0 = min(sc * cs, n), j1 = min(n, j0 + cs);
+        for (long long jt = j0; jt < j1; jt += PT) {
+            __syncthreads();
+            if (jt + threadIdx.x < j1) {
+                const float4 q = src32[jt + threadIdx.x];
+                sxy[threadIdx.x] = make_ulonglong2(f2_pack(q.x, q.x), f2_pack(q.y, q.y));
+                sg[threadIdx.x] = f2_pack(q.z, q.z);
+            }
+            __syncthreads();
+            const int cnt = (int)min((long long)PT, j1 - jt);
+            f2 sx[PROBE_TPT / 2], sy[PROBE_TPT / 2];
+#pragma unroll
+            for (int k = 0; k < PROBE_TPT / 2; ++k) sx[k] = sy[k] = 0ull;   // +0.0f in both halves
+#pragma unroll 4
+            for (int q = 0; q < cnt; ++q) {
+                const ulonglong2 c = sxy[q];
+                const f2 g = sg[q];
+#pragma unroll
+                for (int k = 0; k < PROBE_TPT / 2; ++k) {
+                    const f2 dx = f2_sub(ax[k], c.x), dy = f2_sub(ay[k], c.y);
+                    float ra, rb;
+                    f2_unpack(f2_fma(dx, dx, f2_mul(dy, dy)), ra, rb);
+                    const f2 m = f2_mul(g, f2_pack(vx_rcp_approx(fmaxf(ra, eps2)), vx_rcp_approx(fmaxf(rb, eps2))));
+                    sy[k] = f2_fma(m, dx, sy[k]);
+                    sx[k] = f2_fma(m, dy, sx[k]);   // sum of +m dy: negated below
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < PROBE_TPT / 2; ++k) {
+                float a, b;
+                f2_unpack(sx[k], a, b); vxa[2 * k] -= (double)a; vxa[2 * k + 1] -= (double)b;
+                f2_unpack(sy[k], a, b); vya[2 * k] += (double)a; vya[2 * k + 1] += (double)b;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < PROBE_TPT; ++k) {
+            const long long t = tt * tile + (long long)k * PT + threadIdx.x;
+            if (t < nt) {
+                double *o = part + (long long)sc * 2 * tstride + t;
+                o[0] = vxa[k];
+                o[tstride] = vya[k];
+            }
+        }
+    }
+}
+template <int TPT>
+__global__ void __launch_bounds__(PT, PROBE32_MINB) k_probe32_partial(VxParams p, const VxScalars *S,
+                                                                      const float4 *src32, const double *tx,
+                                                                      const double *ty, long long tstr, long long nt,
+                                                                      double *part, VxSplit sp) {
+    VX_PDL_WAIT();
+    k_probe32_partial_body<TPT>(VxBlkB<PT, PROBE32_MINB>{blockIdx.x, gridDim.x}, p, S, src32, tx, ty, tstr, nt, part, sp);
 }
 
 // Combine: V = sum/(2 pi) + V_inf, d = mean of the 3 nearest distances.  A
@@ -683,7 +762,7 @@ cudaError_t vx_launch_velocity(const VxLaunch &L, const VxParams &p, const VxVie
     if (maybe_pack(L, p, v, S, w) != cudaSuccess) return cudaGetLastError();
     if (p.prec == VX_PREC_FP32) {
         VX_EV(L, 0);
-        vx_launch<k_bs32_partial<true>, k_bs32_partial_body<true>>(L, grid, PT, 0, p, S, w.src32, v.x, v.y, v.ps, -1, w.part, sp);
+        vx_launch<k_bs32_partial, k_bs32_partial_body>(L, grid, PT, 0, p, S, w.src32, v.x, v.y, v.ps, w.part, sp);
         VX_EV(L, 1);
 
         vx_launch<k_bs_combine<true>, k_bs_combine_body<true>>(L, L.num_sms * 16, CMB_T * CMB_S, 0, v, S, w.part, sp);
@@ -722,12 +801,16 @@ cudaError_t vx_launch_diffusion(const VxLaunch &L, const VxParams &p, const VxVi
 cudaError_t vx_launch_probe(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                             VxWork &w, const double *px, const double *py, long long pstride,
                             long long np, double *ovx, double *ovy, long long ostride) {
-    const VxSplit sp = pair_split(L, p, w, 2, vx_pair_split(np, 1LL << 30, pair_tile(p), pair_slots(L, p, true), 1));
+    const bool few = p.prec == VX_PREC_FP32 && np <= 2 * PT;   // two targets a thread
+    const int tile = few ? 2 * PT : pair_tile(p);
+    const VxSplit sp = pair_split(L, p, w, 2, vx_pair_split(np, 1LL << 30, tile, pair_slots(L, p, true), 1));
     const int grid = pair_slots(L, p, true);
     if (w.part_cap / (2LL * sp.K) < np) return cudaErrorInvalidValue;
     if (maybe_pack(L, p, v, S, w) != cudaSuccess) return cudaGetLastError();
-    if (p.prec == VX_PREC_FP32)
-        vx_launch<k_bs32_partial<false>, k_bs32_partial_body<false>>(L, grid, PT, 0, p, S, w.src32, px, py, pstride, np, w.part, sp);
+    if (few)
+        vx_launch<k_probe32_partial<2>, k_probe32_partial_body<2>>(L, grid, PT, 0, p, S, w.src32, px, py, pstride, np, w.part, sp);
+    else if (p.prec == VX_PREC_FP32)
+        vx_launch<k_probe32_partial<4>, k_probe32_partial_body<4>>(L, grid, PT, 0, p, S, w.src32, px, py, pstride, np, w.part, sp);
     else
         vx_launch<k_bs64_partial<false>, k_bs64_partial_body<false>>(L, grid, PT, 0, p, v, S, px, py, pstride, np, w.part, sp);
 
