@@ -481,16 +481,29 @@ __global__ void __launch_bounds__(32 * TOP_W) k_fmm_up_top(VxScalars *S, int *cn
 // 4 x 4 tile of target cells (two parents wide); the interaction lists of the
 // tile draw on the 8 x 8 source cells around it (children of the parents'
 // neighbours), whose multipoles are staged once in shared memory.  The
-// Hankel entries H_j = j! t^-(j+1) of the 40 integer offsets t are tabulated
-// per block.  Thread (cell, coefficient group cg, part pt) sums the G
-// coefficients G cg .. G cg + G - 1 (G = 8 where it divides the order, else
-// 4) over the interactions u = pt, pt + 4, ... of the cell's list, with a
-// sliding window over the Hankel entries: per term one shared load of the
-// source coefficient and one of the window's new entry serve 4 G FP64 FMAs
-// (with G = 4 the two shared loads per 16 FMAs bound the loop).  The four
-// parts (adjacent lanes) are then reduce-scattered in a fixed tree, so part
-// pt ends with coefficients G cg + (G / 4) pt onwards; every coefficient is
-// the same sum, in the same order, whatever G.
+// Hankel entries H_j = j! t^-(j+1) of the integer offsets t are tabulated
+// per block.
+//
+// H_j(-t) = (-1)^(j+1) H_j(t) and H_j(conj t) = conj H_j(t), so the sources B1
+// .. B4 of a cell at t, -t, conj t and -conj t share one Hankel product: with
+// sigma = (-1)^(k+l+1), U = B1 + sigma B2 and W = B3 + sigma B4,
+//   Re: (U.r + W.r) h.r - (U.i - W.i) h.i,
+//   Im: (U.r - W.r) h.i + (U.i + W.i) h.r
+// are the four sources' term of (k, l): 4 FP64 FMAs for four sources (and 16
+// additions a k for both signs, shared by the l) instead of 16.  The 27
+// sources of an interaction list, offsets [-2, 3]^2 (mirrored by the cell's
+// place in its parent) without [-1, 1]^2, fall into 12 such sets:
+//   (2,1) (1,2) (2,2) with all four; (3,1) (3,2) with their conjugates;
+//   (1,3) (2,3) with their negative conjugates; (2,0) (0,2) with their
+//   negatives; (3,0) (0,3) (3,3) alone.
+// Thread (cell, coefficient group cg, part pt) sums the G coefficients G cg ..
+// G cg + G - 1 (G = 8 where it divides the order, else 4) over three of them,
+// one of each kind of code (a missing source is a row of zeros), so that the
+// parts of a warp run together.  A ring of G Hankel entries stays in
+// registers.  The four parts (adjacent lanes) are then reduce-scattered in a
+// fixed tree, so part pt ends with coefficients G cg + (G / 4) pt onwards.
+// All levels at 1e6 vortices (event times) 171 -> 130 us, at 3e6 521 -> 364, against
+// a product per source with unpadded rows (4-way bank conflicts).
 //
 // The levels up to M2L_SMALL have few cells each: their M2L parts are
 // independent of one another and run in one launch over all their tiles
@@ -507,9 +520,11 @@ template <int P> __host__ __device__ constexpr int m2l_threads() { return M2L_TI
 
 template <int P>
 struct M2LShared {
-    cplx sh[49][2 * P - 1];   // offset (dx, dy) in [-3, 3]^2 at (dy+3)*7 + dx+3
+    // rows of 16 (odd) bytes, so that the rows of a warp's lanes fall into
+    // different banks
+    cplx sh[49][2 * P + 1];   // offset (dx, dy) in [-3, 3]^2 at (dy+3)*7 + dx+3
     cplx se[4][P];
-    cplx sm[M2L_SRC * M2L_SRC][P];
+    cplx sm[M2L_SRC * M2L_SRC + 1][P + 1];   // the last row: zeros
     int sc[M2L_SRC * M2L_SRC];
 };
 
@@ -526,6 +541,61 @@ __device__ void m2l_tables(M2LShared<P> &T) {
             T.sh[q][j] = cscale(tp, fact);
             tp = cmul(tp, ti);
             fact *= (double)(j + 1);
+        }
+        T.sh[q][2 * P - 1] = T.sh[q][2 * P] = cplx{0.0, 0.0};   // loaded ahead, not used
+    }
+    for (int k = threadIdx.x; k <= P; k += blockDim.x) T.sm[M2L_SRC * M2L_SRC][k] = cplx{0.0, 0.0};
+}
+
+// One set of sources (b2, b3, b4 at the negative, the conjugate, the negative
+// conjugate of b1's offset; MASK bits 2, 4, 8: which of them the code has)
+// into the G coefficients of v.  H: the offset's entries from G cg on.
+template <int P, int MASK>
+__device__ __forceinline__ void m2l_set(double (&v)[2 * m2l_group<P>()], const cplx *H, const cplx *b1, const cplx *b2,
+                                        const cplx *b3, const cplx *b4) {
+    constexpr int G = m2l_group<P>();
+    cplx h[G];   // H_{k + j} at (k + j) % G
+#pragma unroll
+    for (int j = 0; j < G; ++j) h[j] = H[j];
+#pragma unroll 1
+    for (int k0 = 0; k0 < P; k0 += G) {
+#pragma unroll
+        for (int kk = 0; kk < G; ++kk) {
+            const int k = k0 + kk;
+            // [0]: k + l even (sigma -1), [1]: odd (sigma +1)
+            cplx U[2], W[2];
+            U[0] = U[1] = b1[k];
+            W[0] = W[1] = cplx{0.0, 0.0};
+            if (MASK & 2) {
+                const cplx c = b2[k];
+                U[0] = cplx{U[0].r - c.r, U[0].i - c.i};
+                U[1] = cplx{U[1].r + c.r, U[1].i + c.i};
+            }
+            if (MASK & 4) W[0] = W[1] = b3[k];
+            if (MASK & 8) {
+                const cplx c = b4[k];
+                W[0] = cplx{W[0].r - c.r, W[0].i - c.i};
+                W[1] = cplx{W[1].r + c.r, W[1].i + c.i};
+            }
+            double pr[2], qi[2], ri[2], sr[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (MASK & 12) {
+                    pr[e] = U[e].r + W[e].r; qi[e] = U[e].i - W[e].i;
+                    ri[e] = U[e].r - W[e].r; sr[e] = U[e].i + W[e].i;
+                } else {
+                    pr[e] = ri[e] = U[e].r;
+                    qi[e] = sr[e] = U[e].i;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                const cplx t = h[(kk + j) % G];
+                const int e = (kk + j) & 1;
+                v[2 * j] = fma(pr[e], t.r, fma(-qi[e], t.i, v[2 * j]));
+                v[2 * j + 1] = fma(ri[e], t.i, fma(sr[e], t.r, v[2 * j + 1]));
+            }
+            h[kk] = H[k + G];
         }
     }
 }
@@ -568,36 +638,38 @@ __device__ bool m2l_tile(const VxScalars *S, const int *cnt, const cplx *M, int 
     }
     __syncthreads();
     busy = live && cl[c] > 0;
-    const long long px = ix >> 1, py = iy >> 1;
     double v[2 * G];   // (re, im) of coefficients G cg + j
 #pragma unroll
     for (int j = 0; j < 2 * G; ++j) v[j] = 0.0;
-    if (busy) {
-        for (int u = pt; u < 36; u += 4) {
-            const long long qy = 2 * (py - 1) + u / 6, qx = 2 * (px - 1) + u % 6;
-            if (qx < 0 || qx >= m || qy < 0 || qy >= m) continue;
-            if (llabs(qx - ix) <= 1 && llabs(qy - iy) <= 1) continue;   // neighbours: near field
-            const int q = (int)((qy - sy0) * M2L_SRC + (qx - sx0));
-            if (T.sc[q] == 0) continue;
-            const cplx *H = T.sh[(int)(iy - qy + 3) * 7 + (int)(ix - qx + 3)] + G * cg;   // H_{k + G cg + j}
-            const cplx *B = T.sm[q];
-            cplx h[G];
-#pragma unroll
-            for (int j = 0; j < G; ++j) h[j] = H[j];
-#pragma unroll
-            for (int k = 0; k < P; ++k) {
-                const cplx b = B[k];
-#pragma unroll
-                for (int j = 0; j < G; ++j) {
-                    v[2 * j] = fma(b.r, h[j].r, fma(-b.i, h[j].i, v[2 * j]));
-                    v[2 * j + 1] = fma(b.r, h[j].i, fma(b.i, h[j].r, v[2 * j + 1]));
-                }
-                if (k + 1 < P) {
-#pragma unroll
-                    for (int j = 0; j + 1 < G; ++j) h[j] = h[j + 1];
-                    h[G - 1] = H[k + G];
-                }
-            }
+    if (__any_sync(0xffffffffu, busy)) {
+        constexpr int NONE = M2L_SRC * M2L_SRC;
+        // the source fa right and fb up of the cell, mirrored by its place in
+        // its parent: its row of sm, the row of zeros if it is empty or not
+        // wanted (all lie in the staged region)
+        const int fx = (ix & 1) ? -1 : 1, fy = (iy & 1) ? -1 : 1;
+        const int here = (int)(iy - sy0) * M2L_SRC + (int)(ix - sx0);
+        const auto at = [&](int fa, int fb, bool want = true) {
+            const int q = here + fy * fb * M2L_SRC + fx * fa;
+            return want && T.sc[q] > 0 ? q : NONE;
+        };
+        const auto hank = [&](int fa, int fb) { return T.sh[(3 - fy * fb) * 7 + 3 - fx * fa] + G * cg; };
+        {   // (2,1) (1,2) (2,2) with all four, (2,0) with its negative
+            const int fa = pt == 1 ? 1 : 2, fb = pt == 0 ? 1 : (pt == 3 ? 0 : 2);
+            const int q1 = at(fa, fb), q2 = at(-fa, -fb), q3 = at(fa, -fb, pt != 3), q4 = at(-fa, fb, pt != 3);
+            if (__any_sync(0xffffffffu, min(min(q1, q2), min(q3, q4)) < NONE))
+                m2l_set<P, 15>(v, hank(fa, fb), T.sm[q1], T.sm[q2], T.sm[q3], T.sm[q4]);
+        }
+        {   // (3,1) (3,2) with their conjugates, (1,3) (2,3) with their negative conjugates
+            const int fa = pt < 2 ? 3 : pt - 1, fb = pt < 2 ? pt + 1 : 3;
+            const int q1 = at(fa, fb), q3 = at(fa, pt < 2 ? -fb : fb, pt < 2), q4 = at(pt < 2 ? fa : -fa, fb, pt >= 2);
+            if (__any_sync(0xffffffffu, min(q1, min(q3, q4)) < NONE))
+                m2l_set<P, 13>(v, hank(fa, fb), T.sm[q1], nullptr, T.sm[q3], T.sm[q4]);
+        }
+        {   // (3,0) (0,3) (3,3) alone, (0,2) with its negative
+            const int fa = pt == 0 || pt == 2 ? 3 : 0, fb = pt == 0 ? 0 : (pt == 3 ? 2 : 3);
+            const int q1 = at(fa, fb), q2 = at(0, pt == 3 ? -2 : 0, pt == 3);
+            if (__any_sync(0xffffffffu, min(q1, q2) < NONE))
+                m2l_set<P, 3>(v, hank(fa, fb), T.sm[q1], T.sm[q2], nullptr, nullptr);
         }
     }
     // reduce-scatter over the four parts (all lanes take part): first with
