@@ -54,6 +54,21 @@ constexpr int CG_KMAX = 3 * CG_DIV_Y;    // widest window of a work item, in row
 #define VX_DIFF_FRAME_D 64.0f          // farthest a target may sit from its item's frame, in units of its d
 #endif
 
+// Sum of a block's sd[] (complete after a barrier the caller passed) in the
+// tree that halves the block: sd[t] + sd[t + 128], + 64, ..., the last five
+// steps inside the first warp.  Valid in thread 0.
+__device__ __forceinline__ double cg_tree(double *sd) {
+    for (int o = CG_T / 2; o >= 32; o >>= 1) {
+        if (threadIdx.x < o) sd[threadIdx.x] += sd[threadIdx.x + o];
+        __syncthreads();
+    }
+    double t = threadIdx.x < 32 ? sd[threadIdx.x] : 0.0;
+    if (threadIdx.x < 32)
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    __syncthreads();
+    return t;
+}
+
 // Start of the diffusion stage, one launch: per partition the bounding-box
 // keys (into box[]) and the sum of d (into red[]); the block that finishes
 // last combines them, resets the stage's counters and sizes the grid.  The
@@ -64,7 +79,6 @@ constexpr int CG_KMAX = 3 * CG_DIV_Y;    // widest window of a work item, in row
 // c * mean(d) / CG_DIV_Y, both grown until the grid fits cells_cap.
 VX_DEVK void k_cg_prep_body(VxBlkB<CG_T, 0> vb, const VxView &v, VxScalars *S, double *red, unsigned long long *box,
                             int sms, double cutoff, long long cells_cap) {
-    __shared__ unsigned long long sk[4][CG_T];
     __shared__ double sd[CG_T];
     const long long n = S->n;
     const int nparts = vx_body_parts(n, sms, VX_RED_BLOCKS);
@@ -84,19 +98,13 @@ VX_DEVK void k_cg_prep_body(VxBlkB<CG_T, 0> vb, const VxView &v, VxScalars *S, d
             k[3] = min(k[3], vx_dkey(-y));
             dsum += v.d[i];
         }
-        for (int q = 0; q < 4; ++q) sk[q][threadIdx.x] = k[q];
         sd[threadIdx.x] = dsum;
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o) {
-                for (int q = 0; q < 4; ++q) sk[q][threadIdx.x] = min(sk[q][threadIdx.x], sk[q][threadIdx.x + o]);
-                sd[threadIdx.x] += sd[threadIdx.x + o];
-            }
-            __syncthreads();
+        vx_block_min4<CG_T / 32>(k);
+        dsum = cg_tree(sd);
+        if (threadIdx.x == 0) {
+            for (int q = 0; q < 4; ++q) box[4 * part + q] = k[q];
+            red[part] = dsum;
         }
-        if (threadIdx.x < 4) box[4 * part + threadIdx.x] = sk[threadIdx.x][0];
-        if (threadIdx.x == 0) red[part] = sd[0];
-        __syncthreads();
     }
     if (!vx_last_block(&S->sync_ctr, vb.n)) return;
     unsigned long long k[4] = {~0ull, ~0ull, ~0ull, ~0ull};
@@ -106,25 +114,17 @@ VX_DEVK void k_cg_prep_body(VxBlkB<CG_T, 0> vb, const VxView &v, VxScalars *S, d
         if ((long long)b * CG_T < n)
             for (int q = 0; q < 4; ++q) k[q] = min(k[q], __ldcg(&box[4 * b + q]));
     }
-    for (int q = 0; q < 4; ++q) sk[q][threadIdx.x] = k[q];
     sd[threadIdx.x] = dpart;
-    __syncthreads();
-    for (int o = CG_T / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            for (int q = 0; q < 4; ++q) sk[q][threadIdx.x] = min(sk[q][threadIdx.x], sk[q][threadIdx.x + o]);
-            sd[threadIdx.x] += sd[threadIdx.x + o];
-        }
-        __syncthreads();
-    }
+    vx_block_min4<CG_T / 32>(k);
+    const double dsum = cg_tree(sd);
     if (threadIdx.x != 0) return;
     S->cnwide = 0;
     S->cnhuge = 0;
     S->bk_nmid = S->bk_nbig = 0;
     S->cnitems = 0;
     if (n == 0) { S->cncells = 0; S->cnx = S->cny = 0; return; }
-    const double dsum = sd[0];
-    const double x0 = vx_dunkey(sk[0][0]), x1 = -vx_dunkey(sk[1][0]);
-    const double y0 = vx_dunkey(sk[2][0]), y1 = -vx_dunkey(sk[3][0]);
+    const double x0 = vx_dunkey(k[0]), x1 = -vx_dunkey(k[1]);
+    const double y0 = vx_dunkey(k[2]), y1 = -vx_dunkey(k[3]);
     double hy = cutoff * (dsum / (double)n) / (double)CG_DIV_Y;
     if (!(hy > 0.0)) hy = 1e-3;
     double hx = hy * ((double)CG_DIV_Y / (double)CG_DIV_X);
@@ -153,41 +153,34 @@ __device__ __forceinline__ long long cg_cell(const VxScalars *S, double x, doubl
     return cy * S->cnx + cx;
 }
 
-// Cell of every particle, counted per cell (the counts are zero between
-// steps: the bucket order leaves them at zero once the order is built).
-VX_DEVK void k_cg_cellid_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalars *S, unsigned *key, int *val, int *cnt) {
+// Cell of every particle and its rank in it, counted per cell (the counts are
+// zero between steps: the scan zeroes them behind it).
+VX_DEVK void k_cg_cellid_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalars *S, unsigned *key, int *rank, int *cnt) {
     const long long n = S->n;
     if (S->cncells == 0) return;
     for (long long i = vb.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)vb.n * blockDim.x) {
         const long long c = cg_cell(S, v.x[i * v.ps], v.y[i * v.ps]);
         key[i] = (unsigned)c;
-        val[i] = (int)i;
-        atomicAdd(&cnt[c], 1);
+        rank[i] = atomicAdd(&cnt[c], 1);
     }
 }
-__global__ void k_cg_cellid(VxView v, const VxScalars *S, unsigned *key, int *val, int *cnt) {
+__global__ void k_cg_cellid(VxView v, const VxScalars *S, unsigned *key, int *rank, int *cnt) {
     VX_PDL_WAIT();
-    k_cg_cellid_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, key, val, cnt);
+    k_cg_cellid_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, key, rank, cnt);
 }
 
 // Cell starts: one-pass scan of the counts, start[cncells] = n.
-VX_DEVK void k_cg_scan_body(VxBlkB<VX_SCAN_T, 0> vb, VxScalars *S, const int *cnt, int *start,
-                            unsigned long long *tiles) {
+constexpr int CG_SCAN_PER = 16;
+VX_DEVK void k_cg_scan_body(VxBlkB<VX_SCAN_T, 0> vb, VxScalars *S, int *cnt, int *start, unsigned long long *tiles) {
     const long long nc = S->cncells;
-    vx_scan_lookback<VX_CHUNK / VX_SCAN_T>(
-        vb.n, nc, S, tiles, [&](long long i) { return cnt[i]; },
-        [&](long long i0, const unsigned *val, long long run) {
-#pragma unroll
-            for (int q = 0; q < VX_CHUNK / VX_SCAN_T; ++q) {
-                if (i0 + q < nc) start[i0 + q] = (int)run;
-                run += val[q];
-            }
-        },
+    vx_scan_lookback<CG_SCAN_PER>(
+        vb.n, nc, S, tiles,
+        [&](long long i0, unsigned (&val)[CG_SCAN_PER]) { vx_scan_load<true>(cnt, i0, nc, val); },
+        [&](long long i0, const unsigned (&val)[CG_SCAN_PER], long long run) { vx_scan_store(start, i0, nc, val, run); },
         [&](long long) { start[nc] = (int)S->n; });
 }
-__global__ void __launch_bounds__(VX_SCAN_T) k_cg_scan(VxScalars *S, const int *cnt, int *start,
-                                                       unsigned long long *tiles) {
+__global__ void __launch_bounds__(VX_SCAN_T) k_cg_scan(VxScalars *S, int *cnt, int *start, unsigned long long *tiles) {
     VX_PDL_WAIT();
     k_cg_scan_body(VxBlkB<VX_SCAN_T, 0>{blockIdx.x, gridDim.x}, S, cnt, start, tiles);
 }
@@ -197,15 +190,25 @@ __global__ void __launch_bounds__(VX_SCAN_T) k_cg_scan(VxScalars *S, const int *
 // per thread.
 VX_DEVK void k_cg_items_body(VxBlkB<VX_SCAN_T, 0> vb, VxScalars *S, const int *start, int2 *items, long long items_cap,
                              unsigned long long *tiles) {
+    __shared__ int3 row_of[VX_SCAN_T];   // items, first item, first target of a row
     const long long ny = S->cny, nx = S->cnx;
     vx_scan_lookback<1>(
         vb.n, ny, S, tiles,
-        [&](long long r) { return (start[(r + 1) * nx] - start[r * nx] + CG_W - 1) / CG_W; },
-        [&](long long r, const unsigned *val, long long run) {
-            if (r >= ny) return;
-            const int s0 = start[r * nx];
-            for (unsigned q = 0; q < val[0]; ++q)
-                if (run + q < items_cap) items[run + q] = make_int2((int)r, s0 + (int)q * CG_W);
+        [&](long long r, unsigned (&val)[1]) {
+            val[0] = r < ny ? (unsigned)(start[(r + 1) * nx] - start[r * nx] + CG_W - 1) / CG_W : 0u;
+        },
+        [&](long long r, const unsigned (&val)[1], long long run) {
+            // the block's rows, a warp to a row (a thread walking its own row
+            // wrote some hundred items one after the other: 26 -> 15 us at
+            // 1e6 vortices, 52 -> 20 at 3e6)
+            row_of[threadIdx.x] = make_int3((int)val[0], (int)run, r < ny ? start[r * nx] : 0);
+            __syncthreads();
+            const long long first = r - threadIdx.x;
+            for (int t = threadIdx.x >> 5; t < VX_SCAN_T; t += VX_SCAN_T / 32) {
+                const int3 e = row_of[t];
+                for (int q = threadIdx.x & 31; q < e.x; q += 32)
+                    if (e.y + q < items_cap) items[e.y + q] = make_int2((int)(first + t), e.z + q * CG_W);
+            }
         },
         [&](long long tot) {
             S->cnitems = tot <= items_cap ? tot : 0;
@@ -837,15 +840,13 @@ cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, cons
     vx_launch<k_cg_scan, k_cg_scan_body>(L, grid, VX_SCAN_T, 0, S, w.cg_cnt, w.cg_start, w.scan_tiles);
 
     // cell order: each cell's vortices in index order (a stable sort by cell),
-    // the FP32 sources gathered at their slots on the way; the cell counts
-    // are left at zero for the next step's count
+    // the FP32 sources gathered at their slots on the way
     VxGather gt;
     gt.mode = 2;
-    gt.zero_counts = 1;
     gt.v = v;
     gt.S = S;
     gt.srt = w.srt;
-    vx_bucket_order(L, S, &S->n, &S->cncells, w.key0, w.cg_start, w.cg_cnt, nullptr, w.key1, w.val1, w.bk_mid, w.bk_big,
+    vx_bucket_order(L, S, &S->n, &S->cncells, w.key0, w.val0, w.cg_start, w.key1, w.val1, w.bk_mid, w.bk_big,
                     w.val0, gt);
     const unsigned *skey = w.key1;
     const int *sorted = w.val1;

@@ -17,10 +17,26 @@
 //    pointing at j; later ones merge with (0, 1e10) as the serial loop does,
 //    which re-rounds their position.
 //  * Compaction then runs as after convection.
-// A round is six launches before the compaction: prep (box, bookkeeping and
-// grid in one, the last block finishing), count, a one-pass scan of the cell
-// counts, scatter, query, and settle (resolution, merge and write-back in
-// one block).
+// The first round is six launches before the compaction: prep (box,
+// bookkeeping and grid in one, the last block finishing), count, a one-pass
+// scan of the cell counts, scatter, query, and settle (resolution, merge and
+// write-back in one block).
+//
+// The second round takes the first one's grid.  A pair that qualifies in it
+// holds a vortex the first round moved (two unmoved ones that qualify would
+// have made the first of them a candidate, and every candidate is merged or
+// consumed), so only the moved ones look for partners (k_col_query_moved).
+// The settle keeps the cell-sorted copy in step: a merged vortex's slot gets
+// its new place, a consumed one's strength 0, and the compaction renames the
+// ones it moves into holes.  A merged vortex lies between the two it came
+// from, closer than a cell side, so its slot is at most one cell off and
+// the query looks two cells around.  Second round's kernels before its
+// compaction at 1e6 / 3e6 vortices, each timed by itself: 150 / 406 us ->
+// 23 / 31.  A third round and later ones build their grid again.
+//
+// col, in_cnt, has_app and first_app are all zero between rounds: the settle
+// clears the entries its candidates used.  col holds INT_MAX - j, first_app
+// INT_MAX - i (atomicMax keeps the smallest index, 0 is none).
 #include <limits.h>
 
 #include "vx_internal.cuh"
@@ -28,17 +44,12 @@
 // Start of a round: the bounding box (per-block keys into part[], combined
 // by the last block), the round's bookkeeping and the cell grid.  A round
 // after one that removed nothing (or after a failed one) does nothing: the
-// pass has converged.  Cell side h = r (1 + 1e-6): any pair closer than r is
+// pass has converged (col_done, set by the compaction that removed nothing).  Cell side h = r (1 + 1e-6): any pair closer than r is
 // in neighbouring cells; when the box would need more than cells_cap cells,
 // h grows.
 VX_DEVK void k_col_prep_body(VxBlkB<VX_THREADS, 0> vb, const VxView &v, VxScalars *S, int reset, double r2,
                              long long cells_cap, unsigned long long *part) {
-    const bool done = reset ? false : (S->col_done || S->n == S->col_n_before);
-    if (done) {
-        if (vb.x == 0 && threadIdx.x == 0) S->col_done = 1;
-        return;
-    }
-    __shared__ unsigned long long sh[4][VX_THREADS];
+    if (!reset && S->col_done) return;
     const long long n = S->n;
     unsigned long long k[4] = {~0ull, ~0ull, ~0ull, ~0ull};
     for (long long i = vb.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -49,32 +60,21 @@ VX_DEVK void k_col_prep_body(VxBlkB<VX_THREADS, 0> vb, const VxView &v, VxScalar
         k[2] = min(k[2], vx_dkey(y));
         k[3] = min(k[3], vx_dkey(-y));
     }
-    for (int q = 0; q < 4; ++q) sh[q][threadIdx.x] = k[q];
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int q = 0; q < 4; ++q) sh[q][threadIdx.x] = min(sh[q][threadIdx.x], sh[q][threadIdx.x + o]);
-        __syncthreads();
-    }
-    if (threadIdx.x < 4) part[4 * vb.x + threadIdx.x] = sh[threadIdx.x][0];
+    vx_block_min4<VX_THREADS / 32>(k);
+    if (threadIdx.x == 0)
+        for (int q = 0; q < 4; ++q) part[4 * vb.x + q] = k[q];
     if (!vx_last_block(&S->sync_ctr, vb.n)) return;
     for (int q = 0; q < 4; ++q) k[q] = ~0ull;
     for (unsigned b = threadIdx.x; b < vb.n; b += blockDim.x)
         for (int q = 0; q < 4; ++q) k[q] = min(k[q], __ldcg(&part[4 * b + q]));
-    for (int q = 0; q < 4; ++q) sh[q][threadIdx.x] = k[q];
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int q = 0; q < 4; ++q) sh[q][threadIdx.x] = min(sh[q][threadIdx.x], sh[q][threadIdx.x + o]);
-        __syncthreads();
-    }
+    vx_block_min4<VX_THREADS / 32>(k);
     if (threadIdx.x != 0) return;
     S->col_done = 0;
-    S->col_n_before = n;
     S->ncand = 0;
+    S->nmoved = 0;
     if (n == 0) { S->gncells = 0; S->gnx = S->gny = 0; return; }
-    const double x0 = vx_dunkey(sh[0][0]), x1 = -vx_dunkey(sh[1][0]);
-    const double y0 = vx_dunkey(sh[2][0]), y1 = -vx_dunkey(sh[3][0]);
+    const double x0 = vx_dunkey(k[0]), x1 = -vx_dunkey(k[1]);
+    const double y0 = vx_dunkey(k[2]), y1 = -vx_dunkey(k[3]);
     // side = the collapse radius: the 3 x 3 search is exact and sees the
     // fewest candidates (a side at the mean spacing, with a quarter of the
     // cells to count and scan, was measured slower: the query dominates)
@@ -103,46 +103,35 @@ __device__ __forceinline__ void vx_cell_of(const VxScalars *S, double x, double 
     cy = cy < 0 ? 0 : (cy >= S->gny ? S->gny - 1 : cy);
 }
 
-VX_DEVK void k_col_count_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalars *S, int *cellid, int *cnt, int *in_cnt,
-                              int *has_app, int *first_app) {
+// Counts per cell (zero between rounds: the scan zeroes them behind it) and
+// each vortex's rank in its cell.
+VX_DEVK void k_col_count_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalars *S, int *rank, int *cnt) {
     if (S->col_done) return;
     const long long n = S->n;
     for (long long i = vb.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)vb.n * blockDim.x) {
         long long cx, cy;
         vx_cell_of(S, v.x[i * v.ps], v.y[i * v.ps], cx, cy);
-        const long long c = cy * S->gnx + cx;
-        cellid[i] = (int)c;
-        atomicAdd(&cnt[c], 1);
-        in_cnt[i] = 0;
-        has_app[i] = 0;
-        first_app[i] = INT_MAX;
+        rank[i] = atomicAdd(&cnt[cy * S->gnx + cx], 1);
     }
 }
-__global__ void k_col_count(VxView v, const VxScalars *S, int *cellid, int *cnt, int *in_cnt,
-                            int *has_app, int *first_app) {
+__global__ void k_col_count(VxView v, const VxScalars *S, int *rank, int *cnt) {
     VX_PDL_WAIT();
-    k_col_count_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, cellid, cnt, in_cnt, has_app, first_app);
+    k_col_count_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, rank, cnt);
 }
 
 // Cell starts: exclusive scan of the counts in one pass, start[gncells] = n.
-VX_DEVK void k_col_scan_body(VxBlkB<VX_SCAN_T, 0> vb, VxScalars *S, const int *cnt, int *start,
-                             unsigned long long *tiles) {
+constexpr int COL_SCAN_PER = 16;
+VX_DEVK void k_col_scan_body(VxBlkB<VX_SCAN_T, 0> vb, VxScalars *S, int *cnt, int *start, unsigned long long *tiles) {
     if (S->col_done) return;
     const long long nc = S->gncells;
-    vx_scan_lookback<VX_CHUNK / VX_SCAN_T>(
-        vb.n, nc, S, tiles, [&](long long i) { return cnt[i]; },
-        [&](long long i0, const unsigned *val, long long run) {
-#pragma unroll
-            for (int q = 0; q < VX_CHUNK / VX_SCAN_T; ++q) {
-                if (i0 + q < nc) start[i0 + q] = (int)run;
-                run += val[q];
-            }
-        },
+    vx_scan_lookback<COL_SCAN_PER>(
+        vb.n, nc, S, tiles,
+        [&](long long i0, unsigned (&val)[COL_SCAN_PER]) { vx_scan_load<true>(cnt, i0, nc, val); },
+        [&](long long i0, const unsigned (&val)[COL_SCAN_PER], long long run) { vx_scan_store(start, i0, nc, val, run); },
         [&](long long tot) { start[nc] = (int)tot; });
 }
-__global__ void __launch_bounds__(VX_SCAN_T) k_col_scan(VxScalars *S, const int *cnt, int *start,
-                                                        unsigned long long *tiles) {
+__global__ void __launch_bounds__(VX_SCAN_T) k_col_scan(VxScalars *S, int *cnt, int *start, unsigned long long *tiles) {
     VX_PDL_WAIT();
     k_col_scan_body(VxBlkB<VX_SCAN_T, 0>{blockIdx.x, gridDim.x}, S, cnt, start, tiles);
 }
@@ -154,26 +143,38 @@ struct __align__(32) ColRec {
     long long i;
 };
 
-// Each cell's slots from its start, counting its count back down to zero
-// (the zero the next pass's count starts from); the slot gets a copy of the
-// vortex (ColRec), so that the query reads its candidates as contiguous runs.
-VX_DEVK void k_col_scatter_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalars *S, const int *cellid, const int *start,
-                                int *cnt, ColRec *rec) {
+// Each vortex's slot from its cell's start and its rank (which becomes its
+// slot); the slot gets a copy of the vortex (ColRec), so that the query reads
+// its candidates as contiguous runs.
+VX_DEVK void k_col_scatter_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalars *S, const int *start, int *slot,
+                                ColRec *rec) {
     if (S->col_done) return;
     const long long n = S->n;
     for (long long i = vb.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)vb.n * blockDim.x) {
-        const int c = cellid[i];
-        const int k = start[c] + atomicSub(&cnt[c], 1) - 1;
+        const double x = v.x[i * v.ps], y = v.y[i * v.ps];
+        long long cx, cy;
+        vx_cell_of(S, x, y, cx, cy);
+        const int k = start[cy * S->gnx + cx] + slot[i];
+        slot[i] = k;
         double2 *r = reinterpret_cast<double2 *>(rec + k);
-        r[0] = make_double2(v.x[i * v.ps], v.y[i * v.ps]);
+        r[0] = make_double2(x, y);
         r[1] = make_double2(v.g[i * v.ps], __longlong_as_double(i));
     }
 }
-__global__ void k_col_scatter(VxView v, const VxScalars *S, const int *cellid, const int *start, int *cnt,
-                              ColRec *rec) {
+__global__ void k_col_scatter(VxView v, const VxScalars *S, const int *start, int *slot, ColRec *rec) {
     VX_PDL_WAIT();
-    k_col_scatter_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, cellid, start, cnt, rec);
+    k_col_scatter_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, start, slot, rec);
+}
+
+// Whether a pair qualifies in a pass.
+template <int PASS>
+__device__ __forceinline__ bool vx_col_pair(const VxParams &p, double xi, double yi, double gi, double xj, double yj,
+                                            double gj) {
+    const double dx = xi - xj, dy = yi - yj;
+    const double r2 = fma(dx, dx, dy * dy);
+    if (PASS == 1) return (gi * gj < 0) && (r2 < p.r_diff2);
+    return (gi * gj > 0) && (r2 < p.r_same2) && (fabs(gi + gj) < p.max_ve_g);
 }
 
 // COL[i] = smallest j > i in the 3x3 cell neighbourhood that qualifies.  The
@@ -184,11 +185,10 @@ __global__ void k_col_scatter(VxView v, const VxScalars *S, const int *cellid, c
 // position by the count's expression.
 template <int PASS>
 VX_DEVK void k_col_query_body(VxBlkB<VX_THREADS, 4> vb, const VxParams &p, VxScalars *S, const int *start, const ColRec *rec,
-                              int *col, int *in_cnt, int *cand) {
+                              int *col, int *cand) {
     if (S->col_done) return;
     const long long n = S->n;
     const long long gnx = S->gnx, gny = S->gny;
-    const double rd2 = p.r_diff2, rs2 = p.r_same2, mvg = p.max_ve_g;
     for (long long k0 = vb.x * (long long)blockDim.x + threadIdx.x; k0 < n;
          k0 += (long long)vb.n * blockDim.x) {
         const double2 m0 = reinterpret_cast<const double2 *>(rec + k0)[0];
@@ -206,30 +206,58 @@ VX_DEVK void k_col_query_body(VxBlkB<VX_THREADS, 4> vb, const VxParams &p, VxSca
                 const int j = (int)__double_as_longlong(q1.y);
                 if (j <= i || j >= best) continue;
                 const double2 q0 = reinterpret_cast<const double2 *>(rec + k)[0];
-                const double gj = q1.x;
-                const double dx = xi - q0.x, dy = yi - q0.y;
-                const double r2 = fma(dx, dx, dy * dy);
-                bool ok;
-                if (PASS == 1) ok = (gi * gj < 0) && (r2 < rd2);
-                else ok = (gi * gj > 0) && (r2 < rs2) && (fabs(gi + gj) < mvg);
-                if (ok) best = j;
+                if (vx_col_pair<PASS>(p, xi, yi, gi, q0.x, q0.y, q1.x)) best = j;
             }
         }
         if (best != INT_MAX) {
-            col[i] = best;
-            atomicAdd(&in_cnt[best], 1);
-            const int slot = atomicAdd(&S->ncand, 1);
-            cand[slot] = (int)i;
-        } else {
-            col[i] = -1;
+            col[i] = INT_MAX - best;
+            cand[atomicAdd(&S->ncand, 1)] = (int)i;
         }
     }
 }
 template <int PASS>
-__global__ void k_col_query(VxParams p, VxScalars *S, const int *start, const ColRec *rec, int *col, int *in_cnt,
-                            int *cand) {
+__global__ void k_col_query(VxParams p, VxScalars *S, const int *start, const ColRec *rec, int *col, int *cand) {
     VX_PDL_WAIT();
-    k_col_query_body<PASS>(VxBlkB<VX_THREADS, 4>{blockIdx.x, gridDim.x}, p, S, start, rec, col, in_cnt, cand);
+    k_col_query_body<PASS>(VxBlkB<VX_THREADS, 4>{blockIdx.x, gridDim.x}, p, S, start, rec, col, cand);
+}
+
+// Second round: the partners of the vortices the first one moved (their slots
+// in moved[]), a lane per row of cells, eight lanes a vortex; a pair of two
+// moved ones is met from both sides.
+template <int PASS>
+VX_DEVK void k_col_query_moved_body(VxBlkB<VX_THREADS, 0> vb, const VxParams &p, VxScalars *S, const int *start,
+                                    const ColRec *rec, const int *moved, int *col, int *cand) {
+    if (S->col_done) return;
+    const int nm = S->nmoved;
+    const long long gnx = S->gnx, gny = S->gny;
+    const int row = (threadIdx.x & 7) - 2;
+    if (row > 2) return;
+    for (int e = (vb.x * blockDim.x + threadIdx.x) >> 3; e < nm; e += (vb.n * blockDim.x) >> 3) {
+        const int k0 = moved[e];
+        const double2 m0 = reinterpret_cast<const double2 *>(rec + k0)[0];
+        const double2 m1 = reinterpret_cast<const double2 *>(rec + k0)[1];
+        const int i = (int)__double_as_longlong(m1.y);
+        long long cx, cy;
+        vx_cell_of(S, m0.x, m0.y, cx, cy);
+        if (cy + row < 0 || cy + row >= gny) continue;
+        const long long r0 = (cy + row) * gnx;
+        const int k1 = start[r0 + min(cx + 2, gnx - 1) + 1];
+        for (int k = start[r0 + max(cx - 2, 0LL)]; k < k1; ++k) {
+            if (k == k0) continue;
+            const double2 q0 = reinterpret_cast<const double2 *>(rec + k)[0];
+            const double2 q1 = reinterpret_cast<const double2 *>(rec + k)[1];
+            if (!vx_col_pair<PASS>(p, m0.x, m0.y, m1.x, q0.x, q0.y, q1.x)) continue;
+            const int j = (int)__double_as_longlong(q1.y), lo = min(i, j);
+            if (atomicMax(&col[lo], INT_MAX - max(i, j)) == 0) cand[atomicAdd(&S->ncand, 1)] = lo;
+        }
+    }
+}
+template <int PASS>
+__global__ void __launch_bounds__(VX_THREADS) k_col_query_moved(VxParams p, VxScalars *S, const int *start,
+                                                                const ColRec *rec, const int *moved, int *col,
+                                                                int *cand) {
+    VX_PDL_WAIT();
+    k_col_query_moved_body<PASS>(VxBlkB<VX_THREADS, 0>{blockIdx.x, gridDim.x}, p, S, start, rec, moved, col, cand);
 }
 
 // Settles the candidates in one block: rounds over the candidate list decide
@@ -237,14 +265,20 @@ __global__ void k_col_query(VxParams p, VxScalars *S, const int *start, const Co
 // every applied candidate's merged vortex is computed from the positions as
 // they were, then written (after a barrier: a merge may read a partner that
 // another merge removes).
+// track: the cell-sorted copy is kept in step for the second round, and the
+// slots of the moved vortices are listed (in cdec, done with by then).
 template <int PASS>
-VX_DEVK void k_col_settle_body(VxBlkB<1024, 0> vb, const VxView &v, VxScalars *S, const int *cand, const int *col,
+VX_DEVK void k_col_settle_body(VxBlkB<1024, 0> vb, const VxView &v, VxScalars *S, const int *cand, int *col,
                                int *in_cnt, int *has_app, int *first_app, int *cstate, int *cdec, double *mx,
-                               double *my, double *mg) {
+                               double *my, double *mg, const int *slot, ColRec *rec, double drop_eps, int track) {
     if (S->col_done) return;
-    __shared__ int undecided;
+    __shared__ int undecided, listed;
     const int nc = S->ncand;
-    for (int k = threadIdx.x; k < nc; k += blockDim.x) cstate[k] = 0;
+    if (threadIdx.x == 0) listed = 0;
+    for (int k = threadIdx.x; k < nc; k += blockDim.x) {
+        cstate[k] = 0;
+        atomicAdd(&in_cnt[INT_MAX - col[cand[k]]], 1);
+    }
     __syncthreads();
     const int max_rounds = nc + 2;
     int round = 0;
@@ -265,81 +299,104 @@ VX_DEVK void k_col_settle_body(VxBlkB<1024, 0> vb, const VxView &v, VxScalars *S
             const int d = cdec[k];
             if (d == 0) { atomicAdd(&undecided, 1); continue; }
             cstate[k] = d;
-            const int i = cand[k], j = col[i];
+            const int i = cand[k], j = INT_MAX - col[i];
             atomicSub(&in_cnt[j], 1);
             if (d == 1) {
                 has_app[j] = 1;
-                atomicMin(&first_app[j], i);
+                atomicMax(&first_app[j], INT_MAX - i);
             }
         }
         __syncthreads();
         if (undecided == 0) break;
         __syncthreads();
     }
-    if (round >= max_rounds) {
-        if (threadIdx.x == 0) {
+    const bool failed = round >= max_rounds;
+    if (!failed)
+        for (int k = threadIdx.x; k < nc; k += blockDim.x) {
+            if (cstate[k] != 1) continue;
+            const long long i = cand[k], j = INT_MAX - col[i];
+            const double xi = v.x[i * v.ps], yi = v.y[i * v.ps], gi = v.g[i * v.ps];
+            double xj = 1e10, yj = 1e10, gj = 0.0;
+            if (first_app[j] == (int)(INT_MAX - i)) { xj = v.x[j * v.ps]; yj = v.y[j * v.ps]; gj = v.g[j * v.ps]; }
+            if (PASS == 1) {
+                const double ai = fabs(gi), aj = fabs(gj);
+                const double mn = ai + aj;
+                mx[k] = (xi * ai + xj * aj) / fabs(mn);
+                my[k] = (yi * ai + yj * aj) / fabs(mn);
+                mg[k] = gi + gj;
+            } else {
+                const double ng = gi + gj;
+                mx[k] = (xi * gi + xj * gj) / ng;
+                my[k] = (yi * gi + yj * gj) / ng;
+                mg[k] = ng;
+            }
+        }
+    __syncthreads();
+    for (int k = threadIdx.x; k < nc; k += blockDim.x) {
+        const long long i = cand[k], j = INT_MAX - col[i];
+        if (!failed && cstate[k] == 1) {
+            v.x[i * v.ps] = mx[k]; v.y[i * v.ps] = my[k]; v.g[i * v.ps] = mg[k];
+            v.x[j * v.ps] = 1e10; v.y[j * v.ps] = 1e10; v.g[j * v.ps] = 0.0;
+            if (track) {
+                const bool left = fabs(mg[k]) >= drop_eps;   // else the compaction removes it
+                ColRec *r = rec + slot[i];
+                r->x = mx[k]; r->y = my[k]; r->g = left ? mg[k] : 0.0;
+                rec[slot[j]].g = 0.0;
+                if (left) cdec[atomicAdd(&listed, 1)] = slot[i];
+            }
+        }
+        col[i] = 0;   // the next round finds the entries clear
+        in_cnt[j] = 0; has_app[j] = 0; first_app[j] = 0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        S->ncand = 0;
+        S->nmoved = listed;
+        if (failed) {
             S->err |= VX_DERR_RESOLVE;
             S->col_done = 1;
         }
-        return;
-    }
-    for (int k = threadIdx.x; k < nc; k += blockDim.x) {
-        if (cstate[k] != 1) continue;
-        const long long i = cand[k], j = col[i];
-        const double xi = v.x[i * v.ps], yi = v.y[i * v.ps], gi = v.g[i * v.ps];
-        double xj = 1e10, yj = 1e10, gj = 0.0;
-        if (first_app[j] == i) { xj = v.x[j * v.ps]; yj = v.y[j * v.ps]; gj = v.g[j * v.ps]; }
-        if (PASS == 1) {
-            const double ai = fabs(gi), aj = fabs(gj);
-            const double mn = ai + aj;
-            mx[k] = (xi * ai + xj * aj) / fabs(mn);
-            my[k] = (yi * ai + yj * aj) / fabs(mn);
-            mg[k] = gi + gj;
-        } else {
-            const double ng = gi + gj;
-            mx[k] = (xi * gi + xj * gj) / ng;
-            my[k] = (yi * gi + yj * gj) / ng;
-            mg[k] = ng;
-        }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < nc; k += blockDim.x) {
-        if (cstate[k] != 1) continue;
-        const long long i = cand[k], j = col[i];
-        v.x[i * v.ps] = mx[k]; v.y[i * v.ps] = my[k]; v.g[i * v.ps] = mg[k];
-        v.x[j * v.ps] = 1e10; v.y[j * v.ps] = 1e10; v.g[j * v.ps] = 0.0;
     }
 }
 template <int PASS>
-__global__ void __launch_bounds__(1024) k_col_settle(VxView v, VxScalars *S, const int *cand, const int *col,
+__global__ void __launch_bounds__(1024) k_col_settle(VxView v, VxScalars *S, const int *cand, int *col,
                                                      int *in_cnt, int *has_app, int *first_app, int *cstate,
-                                                     int *cdec, double *mx, double *my, double *mg) {
+                                                     int *cdec, double *mx, double *my, double *mg, const int *slot,
+                                                     ColRec *rec, double drop_eps, int track) {
     VX_PDL_WAIT();
     k_col_settle_body<PASS>(VxBlkB<1024, 0>{blockIdx.x, gridDim.x}, v, S, cand, col, in_cnt, has_app, first_app,
-                            cstate, cdec, mx, my, mg);
+                            cstate, cdec, mx, my, mg, slot, rec, drop_eps, track);
+}
+
+template <int PASS>
+static cudaError_t collapse_pass(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
+                                 int n_col) {
+    const double r2 = PASS == 1 ? p.r_diff2 : p.r_same2;
+    const int grid = std::min(L.num_sms * 4, VX_RED_BLOCKS);   // 4 box keys per block
+    // the cell-sorted copy (32 bytes a vortex) lives in the pair kernels'
+    // partial-sum buffer, unused by collapse (at least 5 doubles a slot)
+    ColRec *rec = reinterpret_cast<ColRec *>(w.part);
+    for (int cc = 0; cc < n_col; ++cc) {
+        const int track = cc == 0 && n_col > 1;
+        if (cc == 1) {
+            vx_launch<k_col_query_moved<PASS>, k_col_query_moved_body<PASS>>(L, grid, VX_THREADS, 0, p, S, w.cell_start, (const ColRec *)rec, (const int *)w.cdec, w.col, w.cand);
+        } else {
+            vx_launch<k_col_prep, k_col_prep_body>(L, grid, VX_THREADS, 0, v, S, cc == 0, r2, w.cells_cap, w.box);
+            vx_launch<k_col_count, k_col_count_body>(L, grid, VX_THREADS, 0, v, S, w.cellid, w.cell_cnt);
+            vx_launch<k_col_scan, k_col_scan_body>(L, grid, VX_SCAN_T, 0, S, w.cell_cnt, w.cell_start, w.scan_tiles);
+            vx_launch<k_col_scatter, k_col_scatter_body>(L, grid, VX_THREADS, 0, v, S, w.cell_start, w.cellid, rec);
+            vx_launch<k_col_query<PASS>, k_col_query_body<PASS>>(L, grid, VX_THREADS, 0, p, S, w.cell_start, (const ColRec *)rec, w.col, w.cand);
+        }
+        vx_launch<k_col_settle<PASS>, k_col_settle_body<PASS>>(L, 1, 1024, 0, v, S, w.cand, w.col, w.in_cnt, w.has_app, w.first_app, w.cstate, w.cdec, w.mx, w.my, w.mg, w.cellid, rec, p.drop_eps, track);
+        // the compaction renames, in the copy, the vortices it moves
+        vx_launch_compact_round(L, p, v, S, w, w.cellid, track ? &rec[0].i : nullptr);
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t vx_launch_collapse(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                                VxWork &w, int pass, int n_col) {
     const double r2 = pass == 1 ? p.r_diff2 : p.r_same2;
     if (!(r2 > 0.0) || n_col <= 0) return cudaSuccess;   // no pair can qualify
-    const int grid = std::min(L.num_sms * 4, VX_RED_BLOCKS);   // 4 box keys per block
-    // the cell-sorted copy (32 bytes a vortex) lives in the pair kernels'
-    // partial-sum buffer, unused by collapse (at least 5 doubles a slot)
-    ColRec *rec = reinterpret_cast<ColRec *>(w.part);
-    for (int cc = 0; cc < n_col; ++cc) {
-        vx_launch<k_col_prep, k_col_prep_body>(L, grid, VX_THREADS, 0, v, S, cc == 0, r2, w.cells_cap, w.box);
-        vx_launch<k_col_count, k_col_count_body>(L, grid, VX_THREADS, 0, v, S, w.cellid, w.cell_cnt, w.in_cnt, w.has_app, w.first_app);
-        vx_launch<k_col_scan, k_col_scan_body>(L, grid, VX_SCAN_T, 0, S, w.cell_cnt, w.cell_start, w.scan_tiles);
-        vx_launch<k_col_scatter, k_col_scatter_body>(L, grid, VX_THREADS, 0, v, S, w.cellid, w.cell_start, w.cell_cnt, rec);
-        if (pass == 1) {
-            vx_launch<k_col_query<1>, k_col_query_body<1>>(L, grid, VX_THREADS, 0, p, S, w.cell_start, (const ColRec *)rec, w.col, w.in_cnt, w.cand);
-            vx_launch<k_col_settle<1>, k_col_settle_body<1>>(L, 1, 1024, 0, v, S, w.cand, w.col, w.in_cnt, w.has_app, w.first_app, w.cstate, w.cdec, w.mx, w.my, w.mg);
-        } else {
-            vx_launch<k_col_query<2>, k_col_query_body<2>>(L, grid, VX_THREADS, 0, p, S, w.cell_start, (const ColRec *)rec, w.col, w.in_cnt, w.cand);
-            vx_launch<k_col_settle<2>, k_col_settle_body<2>>(L, 1, 1024, 0, v, S, w.cand, w.col, w.in_cnt, w.has_app, w.first_app, w.cstate, w.cdec, w.mx, w.my, w.mg);
-        }
-        vx_launch_compact_skip(L, p, v, S, w, &S->col_done);
-    }
-    return cudaGetLastError();
+    return pass == 1 ? collapse_pass<1>(L, p, v, S, w, n_col) : collapse_pass<2>(L, p, v, S, w, n_col);
 }

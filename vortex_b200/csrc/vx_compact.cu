@@ -28,57 +28,47 @@ __device__ __forceinline__ bool vx_live(const VxView &v, long long p, double eps
 VX_DEVK void k_cmp_count_body(VxBlkB<VX_THREADS, 0> vb, const VxView &v, VxScalars *S, double eps, int *cnt,
                               long long *off, const int *skip) {
     if (skip && *skip) return;
-    __shared__ long long sh[VX_THREADS];
+    constexpr int NW = VX_THREADS / 32, PER = VX_CHUNK / VX_THREADS;
     const long long n0 = S->n;
     const long long nch = vx_ceil_div(n0, VX_CHUNK);
     for (long long c = vb.x; c < nch; c += vb.n) {
         int k = 0;
-        const long long b = c * VX_CHUNK, e = min(n0, b + VX_CHUNK);
-        for (long long p = b + threadIdx.x; p < e; p += blockDim.x) k += vx_live(v, p, eps);
-        sh[threadIdx.x] = k;
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-            __syncthreads();
+        const long long b = c * VX_CHUNK + threadIdx.x;
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const long long p = b + q * VX_THREADS;
+            k += p < n0 && vx_live(v, p, eps);
         }
-        if (threadIdx.x == 0) cnt[c] = (int)sh[0];
-        __syncthreads();
+        k = vx_block_add<NW>(k);
+        if (threadIdx.x == 0) cnt[c] = k;
     }
     if (!vx_last_block(&S->sync_ctr, vb.n)) return;
-    // exclusive scan of the chunk counts, VX_THREADS at a time
-    __shared__ long long carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (long long base = 0; base < nch; base += blockDim.x) {
-        const long long c = base + threadIdx.x;
-        const long long val = c < nch ? __ldcg(&cnt[c]) : 0;
-        sh[threadIdx.x] = val;
-        __syncthreads();
-        for (int o = 1; o < (int)blockDim.x; o <<= 1) {       // inclusive Hillis-Steele
-            const long long t = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-            __syncthreads();
-            sh[threadIdx.x] += t;
-            __syncthreads();
+    // exclusive scan of the chunk counts, eight a thread
+    long long m = 0;
+    for (long long base = 0; base < nch; base += VX_THREADS * 8) {
+        const long long c0 = base + threadIdx.x * 8LL;
+        int val[8], loc = 0, total;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            val[q] = c0 + q < nch ? __ldcg(&cnt[c0 + q]) : 0;
+            loc += val[q];
         }
-        if (c < nch) off[c] = carry + sh[threadIdx.x] - val;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry += sh[threadIdx.x];
-        __syncthreads();
+        long long run = m + vx_block_scan<NW>(loc, total);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if (c0 + q < nch) off[c0 + q] = run;
+            run += val[q];
+        }
+        m += total;
     }
-    const long long m = carry;
+    __syncthreads();   // off is read below
     // live elements in [0, m)
     long long scan_m = m;
     if (m < n0) {
         const long long cm = m / VX_CHUNK;
-        long long k = 0;
+        int k = 0;
         for (long long p = cm * VX_CHUNK + threadIdx.x; p < m; p += blockDim.x) k += vx_live(v, p, eps);
-        sh[threadIdx.x] = k;
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-            __syncthreads();
-        }
-        scan_m = off[cm] + sh[0];
+        scan_m = off[cm] + vx_block_add<NW>(k);
     }
     if (threadIdx.x == 0) {
         S->c_n0 = n0;
@@ -101,7 +91,6 @@ VX_DEVK void k_cmp_classify_body(VxBlkB<VX_THREADS, 0> vb, const VxView &v, cons
                                  const int *skip) {
     if (skip && *skip) return;
     constexpr int PER = VX_CHUNK / VX_THREADS;
-    __shared__ int sh[VX_THREADS];
     const long long n0 = S->c_n0, m = S->c_m, H = S->c_H, scan_m = S->c_scan_m;
     if (m == n0) return;
     const long long nch = vx_ceil_div(n0, VX_CHUNK);
@@ -115,16 +104,8 @@ VX_DEVK void k_cmp_classify_body(VxBlkB<VX_THREADS, 0> vb, const VxView &v, cons
             lv[q] = p < n0 && vx_live(v, p, eps);
             loc += lv[q];
         }
-        sh[threadIdx.x] = loc;
-        __syncthreads();
-        for (int o = 1; o < VX_THREADS; o <<= 1) {
-            int t = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-            __syncthreads();
-            sh[threadIdx.x] += t;
-            __syncthreads();
-        }
-        long long scan = off[c] + sh[threadIdx.x] - loc;   // live before b
-        __syncthreads();
+        int total;
+        long long scan = off[c] + vx_block_scan<VX_THREADS / 32>(loc, total);   // live before b
 #pragma unroll
         for (int q = 0; q < PER; ++q) {
             const long long p = b + q;
@@ -184,10 +165,15 @@ __global__ void k_cmp_gather(VxView v, const VxScalars *S, const int *hole_pos, 
 }
 
 // count_step: this compaction closes a whole step, which it counts (no
-// kernel after it in the step reads the step index).
-VX_DEVK void k_cmp_scatter_body(VxBlkB<0, 0> vb, const VxView &v, VxScalars *S, const int *hole_pos, const double *hx,
-                                const double *hy, const double *hg, const double *tx, const double *ty,
-                                const int *skip, int count_step) {
+// kernel after it in the step reads the step index).  done: set if nothing
+// was removed (a collapse round's flag, which skip points to as well).  With
+// rec_i, a vortex moved into a hole gets its new index in the collapse's
+// cell-sorted copy (rec_i: the copy's index fields, 4 apart; slot: each
+// vortex's slot, by its index before).
+VX_DEVK void k_cmp_scatter_body(VxBlkB<0, 0> vb, const VxView &v, VxScalars *S, const int *hole_pos,
+                                const int *hole_src, const double *hx, const double *hy, const double *hg,
+                                const double *tx, const double *ty, const int *skip, int count_step, int *done,
+                                const int *slot, long long *rec_i) {
     if (count_step && vb.x == 0 && threadIdx.x == 0) S->step += 1;
     if (skip && *skip) return;
     const long long n0 = S->c_n0, m = S->c_m, H = S->c_H;
@@ -198,6 +184,7 @@ VX_DEVK void k_cmp_scatter_body(VxBlkB<0, 0> vb, const VxView &v, VxScalars *S, 
             if (k < H) {
                 const long long d = (long long)hole_pos[k] * v.ps;
                 v.x[d] = hx[k]; v.y[d] = hy[k]; v.g[d] = hg[k];
+                if (rec_i) rec_i[4LL * slot[hole_src[k]]] = hole_pos[k];
             } else {
                 const long long e = k - H;
                 const long long d = (m + e) * v.ps;
@@ -205,27 +192,35 @@ VX_DEVK void k_cmp_scatter_body(VxBlkB<0, 0> vb, const VxView &v, VxScalars *S, 
             }
         }
     }
-    if (vb.x == 0 && threadIdx.x == 0) S->n = m;
+    if (vb.x == 0 && threadIdx.x == 0) {
+        S->n = m;
+        if (done && m == n0) *done = 1;
+    }
 }
-__global__ void k_cmp_scatter(VxView v, VxScalars *S, const int *hole_pos, const double *hx,
+__global__ void k_cmp_scatter(VxView v, VxScalars *S, const int *hole_pos, const int *hole_src, const double *hx,
                               const double *hy, const double *hg, const double *tx, const double *ty,
-                              const int *skip, int count_step) {
+                              const int *skip, int count_step, int *done, const int *slot, long long *rec_i) {
     VX_PDL_WAIT();
-    k_cmp_scatter_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, hole_pos, hx, hy, hg, tx, ty, skip, count_step);
+    k_cmp_scatter_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, hole_pos, hole_src, hx, hy, hg, tx, ty, skip,
+                       count_step, done, slot, rec_i);
 }
 
-cudaError_t vx_launch_compact_skip(const VxLaunch &L, const VxParams &p, const VxView &v,
-                                   VxScalars *S, VxWork &w, const int *skip, bool count_step) {
+static cudaError_t compact_impl(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
+                                int *skip, bool count_step, const int *slot, long long *rec_i) {
     const int grid = L.num_sms * 4;
     vx_launch<k_cmp_count, k_cmp_count_body>(L, grid, VX_THREADS, 0, v, S, p.drop_eps, w.cmp_cnt, w.cmp_off, skip);
     vx_launch<k_cmp_classify, k_cmp_classify_body>(L, grid, VX_THREADS, 0, v, S, p.drop_eps, w.cmp_off, w.hole_pos, w.hole_src, w.tail_src, skip);
     vx_launch<k_cmp_gather, k_cmp_gather_body>(L, grid, VX_THREADS, 0, v, S, w.hole_pos, w.hole_src, w.tail_src, w.hx, w.hy, w.hg, w.tx, w.ty, skip);
-    vx_launch<k_cmp_scatter, k_cmp_scatter_body>(L, grid, VX_THREADS, 0, v, S, w.hole_pos, w.hx, w.hy, w.hg, w.tx, w.ty, skip, count_step ? 1 : 0);
-
+    vx_launch<k_cmp_scatter, k_cmp_scatter_body>(L, grid, VX_THREADS, 0, v, S, w.hole_pos, w.hole_src, w.hx, w.hy, w.hg, w.tx, w.ty, skip, count_step ? 1 : 0, skip, slot, rec_i);
     return cudaGetLastError();
 }
 
 cudaError_t vx_launch_compact(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                               VxWork &w, bool count_step) {
-    return vx_launch_compact_skip(L, p, v, S, w, nullptr, count_step);
+    return compact_impl(L, p, v, S, w, nullptr, count_step, nullptr, nullptr);
+}
+
+cudaError_t vx_launch_compact_round(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
+                                    const int *slot, long long *rec_i) {
+    return compact_impl(L, p, v, S, w, &S->col_done, false, slot, rec_i);
 }

@@ -308,10 +308,12 @@ static vx_status work_alloc_impl(VxWork &w, std::vector<void *> *allocs, long lo
     A(w.hx, cap); A(w.hy, cap); A(w.hg, cap); A(w.tx, cap); A(w.ty, cap);
     w.cells_cap = std::max(4 * cap, 65536LL);
     A(w.cellid, cap); A(w.cell_start, w.cells_cap + 1); A(w.sorted, cap);
-    // the collapse grid's cell counts are zero between passes (the scatter
-    // that consumes them counts them back down), so they start at zero
+    // the collapse grid's cell counts are zero between rounds (the scan that
+    // reads them zeroes them), and so are the per-candidate arrays, so they
+    // start at zero
     if ((st = dalloc_zero(allocs, &w.bytes, &w.cell_cnt, w.cells_cap, stream, cv)) != VX_OK) return st;
-    A(w.col, cap); A(w.in_cnt, cap); A(w.has_app, cap); A(w.first_app, cap);
+    if ((st = dalloc_zero(allocs, &w.bytes, &w.col, 4 * cap, stream, cv)) != VX_OK) return st;
+    if (w.col) { w.in_cnt = w.col + cap; w.has_app = w.in_cnt + cap; w.first_app = w.has_app + cap; }
     A(w.cand, cap); A(w.cstate, cap); A(w.cdec, cap);
     A(w.mx, cap); A(w.my, cap); A(w.mg, cap);
     // pair partials: K * n <= num_sms*8*tile + n for the split K the launchers pick
@@ -327,8 +329,8 @@ static vx_status work_alloc_impl(VxWork &w, std::vector<void *> *allocs, long lo
     // neighbour-list grid of the bulk form
     A(w.key0, cap); A(w.key1, cap); A(w.val0, cap); A(w.val1, cap);
     A(w.cg_start, w.cells_cap + 1);
-    // the diffusion grid's cell counts are zero between steps (its bucket
-    // order leaves them so), so they start at zero
+    // the diffusion grid's cell counts are zero between steps (the scan that
+    // reads them zeroes them), so they start at zero
     if ((st = dalloc_zero(allocs, &w.bytes, &w.cg_cnt, w.cells_cap, stream, cv)) != VX_OK) return st;
     A(w.srt, cap);
     w.items_cap = cap / 32 + w.cells_cap + 2;

@@ -77,7 +77,6 @@ extern __shared__ __align__(16) unsigned char vx_fmm_dyn[];
 // 3-nearest pass left more than 0.5 % of its targets to the exact search.
 VX_DEVK void k_fmm_prep_body(VxBlkB<FMM_T, 0> vb, const VxView &v, VxScalars *S, double eps, int Lmax, int leaf, int *cnt,
                              long long ncnt, int *subcnt, long long nsub, unsigned long long *part) {
-    __shared__ unsigned long long sk[4][FMM_T];
     const long long n = S->n;
     for (long long c = vb.x * (long long)blockDim.x + threadIdx.x; c < ncnt + nsub;
          c += (long long)vb.n * blockDim.x) {
@@ -91,25 +90,14 @@ VX_DEVK void k_fmm_prep_body(VxBlkB<FMM_T, 0> vb, const VxView &v, VxScalars *S,
         k[0] = min(k[0], vx_dkey(x)); k[1] = min(k[1], vx_dkey(-x));
         k[2] = min(k[2], vx_dkey(y)); k[3] = min(k[3], vx_dkey(-y));
     }
-    for (int q = 0; q < 4; ++q) sk[q][threadIdx.x] = k[q];
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int q = 0; q < 4; ++q) sk[q][threadIdx.x] = min(sk[q][threadIdx.x], sk[q][threadIdx.x + o]);
-        __syncthreads();
-    }
-    if (threadIdx.x < 4) part[4 * vb.x + threadIdx.x] = sk[threadIdx.x][0];
+    vx_block_min4<FMM_T / 32>(k);
+    if (threadIdx.x == 0)
+        for (int q = 0; q < 4; ++q) part[4 * vb.x + q] = k[q];
     if (!vx_last_block(&S->sync_ctr, vb.n)) return;
     for (int q = 0; q < 4; ++q) k[q] = ~0ull;
     for (unsigned b = threadIdx.x; b < vb.n; b += blockDim.x)
         for (int q = 0; q < 4; ++q) k[q] = min(k[q], __ldcg(&part[4 * b + q]));
-    for (int q = 0; q < 4; ++q) sk[q][threadIdx.x] = k[q];
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int q = 0; q < 4; ++q) sk[q][threadIdx.x] = min(sk[q][threadIdx.x], sk[q][threadIdx.x + o]);
-        __syncthreads();
-    }
+    vx_block_min4<FMM_T / 32>(k);
     if (threadIdx.x != 0) return;
     // the last build's quarter-cell occupancy, sources, box, depth and the
     // targets its 3-nearest pass left to the exact search
@@ -122,8 +110,8 @@ VX_DEVK void k_fmm_prep_body(VxBlkB<FMM_T, 0> vb, const VxView &v, VxScalars *S,
     S->fnflag = 0;
     S->fnbrute = 0;
     S->bk_nmid = S->bk_nbig = 0;
-    const double x0 = vx_dunkey(sk[0][0]), x1 = -vx_dunkey(sk[1][0]);
-    const double y0 = vx_dunkey(sk[2][0]), y1 = -vx_dunkey(sk[3][0]);
+    const double x0 = vx_dunkey(k[0]), x1 = -vx_dunkey(k[1]);
+    const double y0 = vx_dunkey(k[2]), y1 = -vx_dunkey(k[3]);
     double side = fmax(x1 - x0, y1 - y0);
     side = side * (1.0 + 1e-9) + 1e-12;
     // the depth's ceiling follows the count, not the store's capacity (the
@@ -195,46 +183,46 @@ __device__ __forceinline__ unsigned fmm_subkey(const VxScalars *S, double x, dou
 
 // The sum of count^2 over the cells (the next build's depth rule) comes from
 // the same increments: a cell's count going from c to c + 1 adds 2 c + 1.
-VX_DEVK void k_fmm_leafid_body(VxBlkB<0, 0> vb, const VxView &v, VxScalars *S, unsigned *key, int *val, int *subcnt) {
+VX_DEVK void k_fmm_leafid_body(VxBlkB<0, 0> vb, const VxView &v, VxScalars *S, unsigned *key, int *rank, int *subcnt) {
     const long long s = S->fs;
     unsigned long long sq = 0;
     for (long long j = vb.x * (long long)blockDim.x + threadIdx.x; j < s;
          j += (long long)vb.n * blockDim.x) {
         const unsigned k = fmm_subkey(S, v.x[j * v.ps], v.y[j * v.ps]);
+        const int r = atomicAdd(&subcnt[k], 1);
         key[j] = k;
-        val[j] = (int)j;
-        sq += 2ull * (unsigned)atomicAdd(&subcnt[k], 1) + 1ull;
+        rank[j] = r;
+        sq += 2ull * (unsigned)r + 1ull;
     }
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
     if ((threadIdx.x & 31) == 0 && sq) atomicAdd(&S->fsq, sq);
 }
-__global__ void k_fmm_leafid(VxView v, VxScalars *S, unsigned *key, int *val, int *subcnt) {
+__global__ void k_fmm_leafid(VxView v, VxScalars *S, unsigned *key, int *rank, int *subcnt) {
     VX_PDL_WAIT();
-    k_fmm_leafid_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, key, val, subcnt);
+    k_fmm_leafid_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, key, rank, subcnt);
 }
 
+constexpr int FMM_SCAN_PER = 8;
 // Starts of the quarters (one-pass scan of their counts), and with them the
 // leaf counts (the tree's leaf level: the sum of a leaf's four quarters) and
 // the leaf starts (its first quarter's); both end with the sources' total.
-VX_DEVK void k_fmm_scan_body(VxBlkB<VX_SCAN_T, 0> vb, VxScalars *S, const int *subcnt, int *substart, int *cnt,
+VX_DEVK void k_fmm_scan_body(VxBlkB<VX_SCAN_T, 0> vb, VxScalars *S, int *subcnt, int *substart, int *cnt,
                              int *start, unsigned long long *tiles) {
-    constexpr int PER = VX_CHUNK / VX_SCAN_T;   // a multiple of 4: a thread holds whole leaves
+    constexpr int PER = FMM_SCAN_PER;   // a multiple of 4: a thread holds whole leaves
     const long long len = S->fnsub, nl = S->fnleaves;
     int *leafcnt = cnt + fmm_level_off(S->fL);
     vx_scan_lookback<PER>(
-        vb.n, len, S, tiles, [&](long long i) { return subcnt[i]; },
-        [&](long long i0, const unsigned *val, long long run) {
+        vb.n, len, S, tiles, [&](long long i0, unsigned (&val)[PER]) { vx_scan_load<false>(subcnt, i0, len, val); },
+        [&](long long i0, const unsigned (&val)[PER], long long run) {
+            vx_scan_store(substart, i0, len, val, run);
 #pragma unroll
             for (int q = 0; q < PER; q += 4) {
                 if (i0 + q >= len) break;
                 const long long leaf = (i0 + q) >> 2;
-                leafcnt[leaf] = (int)(val[q] + val[q + 1] + val[q + 2] + val[q + 3]);
+                const int c = (int)(val[q] + val[q + 1] + val[q + 2] + val[q + 3]);
+                leafcnt[leaf] = c;
                 start[leaf] = (int)run;
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    substart[i0 + q + e] = (int)run;
-                    run += val[q + e];
-                }
+                run += c;
             }
         },
         [&](long long) {
@@ -242,8 +230,8 @@ VX_DEVK void k_fmm_scan_body(VxBlkB<VX_SCAN_T, 0> vb, VxScalars *S, const int *s
             start[nl] = (int)S->fs;
         });
 }
-__global__ void __launch_bounds__(VX_SCAN_T) k_fmm_scan(VxScalars *S, const int *subcnt, int *substart, int *cnt,
-                                                        int *start, unsigned long long *tiles) {
+__global__ void __launch_bounds__(VX_SCAN_T) k_fmm_scan(VxScalars *S, int *subcnt, int *substart, int *cnt, int *start,
+                                                        unsigned long long *tiles) {
     VX_PDL_WAIT();
     k_fmm_scan_body(VxBlkB<VX_SCAN_T, 0>{blockIdx.x, gridDim.x}, S, subcnt, substart, cnt, start, tiles);
 }
@@ -1173,8 +1161,13 @@ VX_DEVK void k_fmm_items_body(VxBlkB<VX_SCAN_T, 0> vb, VxScalars *S, const int *
     constexpr int PER = 4;
     const long long nl = S->fnleaves;
     vx_scan_lookback<PER>(
-        vb.n, nl, S, tiles, [&](long long c) { return (start[c + 1] - start[c] + FMM_W - 1) / FMM_W; },
-        [&](long long c0, const unsigned *val, long long run) {
+        vb.n, nl, S, tiles,
+        [&](long long c0, unsigned (&val)[PER]) {
+#pragma unroll
+            for (int q = 0; q < PER; ++q)
+                val[q] = c0 + q < nl ? (unsigned)(start[c0 + q + 1] - start[c0 + q] + FMM_W - 1) / FMM_W : 0u;
+        },
+        [&](long long c0, const unsigned (&val)[PER], long long run) {
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
                 const long long c = c0 + q;
@@ -1225,7 +1218,7 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
                                            w.fmm_cnt, vx_fmm_cells(Lmax), w.fmm_sub_cnt, 1LL << (2 * (Lmax + 1)),
                                            w.box);
     vx_launch<k_fmm_leafid, k_fmm_leafid_body>(L, grid, FMM_T, 0, v, S, w.key0, w.val0, w.fmm_sub_cnt);
-    vx_launch<k_fmm_scan, k_fmm_scan_body>(L, grid, VX_SCAN_T, 0, S, (const int *)w.fmm_sub_cnt, w.fmm_sub_start,
+    vx_launch<k_fmm_scan, k_fmm_scan_body>(L, grid, VX_SCAN_T, 0, S, w.fmm_sub_cnt, w.fmm_sub_start,
                                            w.fmm_cnt, w.fmm_start, w.scan_tiles);
     // source order: by quarter-leaf, each quarter's sources in index order
     // (a stable sort by the key 4 leaf + child; each leaf stays contiguous),
@@ -1235,7 +1228,7 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
     gt.v = v;
     gt.S = S;
     gt.srt = w.srt;
-    vx_bucket_order(L, S, &S->fs, &S->fnsub, w.key0, w.fmm_sub_start, w.fmm_sub_cnt, nullptr, w.key1, w.val1,
+    vx_bucket_order(L, S, &S->fs, &S->fnsub, w.key0, w.val0, w.fmm_sub_start, w.key1, w.val1,
                     w.bk_mid, w.bk_big, w.val0, gt);
     const unsigned *skey = w.key1;
     const int *sorted = w.val1;

@@ -79,9 +79,9 @@ struct VxScalars {
     // compaction
     long long c_n0, c_m, c_H, c_scan_m;
     // collapse
-    long long col_n_before;
     int col_done;
     int ncand;
+    int nmoved;            // vortices the running round's merges moved
     double gx0, gy0, gh;
     long long gnx, gny, gncells;
     int err;
@@ -295,6 +295,66 @@ __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
     return r;
 }
 
+// Smallest of a warp's unsigned 64-bit keys, in every lane.
+__device__ __forceinline__ unsigned long long vx_warp_min(unsigned long long k) {
+    const unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32));
+    const unsigned lo = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : 0xffffffffu);
+    return ((unsigned long long)hi << 32) | lo;
+}
+// Smallest of a block's keys k[0..3] (NW warps), in k[0..3] of every thread.
+template <int NW>
+__device__ __forceinline__ void vx_block_min4(unsigned long long (&k)[4]) {
+    __shared__ unsigned long long sh[NW][4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) k[q] = vx_warp_min(k[q]);
+    if (lane < 4) sh[warp][lane] = lane == 0 ? k[0] : (lane == 1 ? k[1] : (lane == 2 ? k[2] : k[3]));
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        k[q] = sh[0][q];
+#pragma unroll
+        for (int w = 1; w < NW; ++w) k[q] = min(k[q], sh[w][q]);
+    }
+    __syncthreads();   // sh may be used again
+}
+// Sum of a block's non-negative ints (NW warps), in every thread.
+template <int NW>
+__device__ __forceinline__ int vx_block_add(int v) {
+    __shared__ int sh[NW];
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    int t = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) t += sh[w];
+    __syncthreads();
+    return t;
+}
+// Exclusive scan of a block's ints (NW warps); total: their sum.
+template <int NW>
+__device__ __forceinline__ int vx_block_scan(int v, int &total) {
+    __shared__ int sh[NW];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    if (lane == 31) sh[warp] = inc;
+    __syncthreads();
+    int before = 0;
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        before += w < warp ? sh[w] : 0;
+        total += sh[w];
+    }
+    __syncthreads();
+    return before + inc - v;
+}
+
 // Monotonic unsigned key of a double (for atomicMin on signed values).
 __device__ __forceinline__ unsigned long long vx_dkey(double v) {
     unsigned long long b = (unsigned long long)__double_as_longlong(v);
@@ -342,8 +402,8 @@ __device__ __forceinline__ bool vx_last_block(unsigned *ctr, unsigned nblk) {
 //   counts, nor does zeroed memory.
 // A wait is bounded: after VX_SCAN_SPIN polls the scan sets VX_DERR_SCAN and
 // takes the missing sums as 0 (the step then reports the flag).
-// load(i) gives count i; store(i0, val, run) gets a thread's PER counts from
-// i0 (PER-aligned; entries at or past `count` are 0) and the scan value at i0;
+// load(i0, val) fills a thread's PER counts from i0 (PER-aligned; entries at
+// or past `count` as 0); store(i0, val, run) gets them and the scan value at i0;
 // total(sum) is called once, by one thread, with the sum of all counts.
 // The block must have VX_SCAN_T threads.  Totals below 2^32.
 constexpr int VX_SCAN_T = 256;
@@ -358,6 +418,51 @@ __device__ __forceinline__ unsigned long long vx_scan_peek(const unsigned long l
     unsigned long long w;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
     return w;
+}
+
+// A thread's counts of an array by 16-byte loads (the array 16-byte aligned;
+// zeroed behind them if ZERO), and their scan values by 16-byte stores: one
+// count at a time, a warp's loads and stores touch a sector a lane.  With 8 /
+// 16 / 32 counts a thread the collapse grid's scan takes 9.9 / 12.4 / 15.9 us at
+// 2e4 vortices, 43 / 31.5 / 30 at 1e6, 108 / 72 / 56 at 3e6 (one at a time, the
+// zeroing elsewhere: 40 and 85), the diffusion grid's 20 / 17 / 20 at 1e6,
+// the quadtree's 14 / 16 / 19: 16 in the first two, 8 in the last.
+template <bool ZERO, int PER>
+__device__ __forceinline__ void vx_scan_load(int *cnt, long long i0, long long count, unsigned (&val)[PER]) {
+    if (i0 + PER <= count) {
+        int4 *c = reinterpret_cast<int4 *>(cnt + i0);
+        int4 a[PER / 4];
+#pragma unroll
+        for (int q = 0; q < PER / 4; ++q) a[q] = c[q];
+#pragma unroll
+        for (int q = 0; q < PER / 4; ++q) {
+            if (ZERO) c[q] = make_int4(0, 0, 0, 0);
+            val[4 * q] = a[q].x; val[4 * q + 1] = a[q].y; val[4 * q + 2] = a[q].z; val[4 * q + 3] = a[q].w;
+        }
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        val[q] = i0 + q < count ? (unsigned)cnt[i0 + q] : 0u;
+        if (ZERO && i0 + q < count) cnt[i0 + q] = 0;
+    }
+}
+template <int PER>
+__device__ __forceinline__ void vx_scan_store(int *start, long long i0, long long count,
+                                              const unsigned (&val)[PER], long long run) {
+    int o[PER];
+    unsigned r = (unsigned)run;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) { o[q] = (int)r; r += val[q]; }
+    if (i0 + PER <= count) {
+        int4 *c = reinterpret_cast<int4 *>(start + i0);
+#pragma unroll
+        for (int q = 0; q < PER / 4; ++q) c[q] = make_int4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < PER; ++q)
+        if (i0 + q < count) start[i0 + q] = o[q];
 }
 
 template <int PER, typename Load, typename Store, typename Total>
@@ -380,11 +485,9 @@ __device__ void vx_scan_lookback(unsigned nblk, long long count, VxScalars *S, u
         const long long i0 = t * TILE + (long long)threadIdx.x * PER;
         unsigned val[PER];
         unsigned loc = 0;
+        load(i0, val);
 #pragma unroll
-        for (int q = 0; q < PER; ++q) {
-            val[q] = i0 + q < count ? (unsigned)load(i0 + q) : 0u;
-            loc += val[q];
-        }
+        for (int q = 0; q < PER; ++q) loc += val[q];
         unsigned inc = loc;   // inclusive scan over the warp
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -737,8 +840,10 @@ cudaError_t vx_invert_gj(const VxLaunch &L, double *A, double *Inv, long long S,
 // overwritten, piv holds n ints; *flag set on a pivot below 1e-12.
 cudaError_t vx_invert_lu(const VxLaunch &L, double *A, double *Inv, long long n, int *piv, int *flag);
 cudaError_t vx_launch_step_end(const VxLaunch &L, VxScalars *S);
-cudaError_t vx_launch_compact_skip(const VxLaunch &L, const VxParams &p, const VxView &v,
-                                   VxScalars *S, VxWork &w, const int *skip, bool count_step = false);
+// The compaction of a collapse round: skipped when S->col_done, which it sets
+// if it removed nothing; slot, rec_i: see k_cmp_scatter (vx_compact.cu).
+cudaError_t vx_launch_compact_round(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
+                                    const int *slot, long long *rec_i);
 void vx_params_from_conf(const vx_conf *c, const vx_panel *pan, int P, VxParams *p);
 void vx_set_error(const char *fmt, ...);
 void vx_keep_pool(int device);
@@ -750,11 +855,9 @@ long long vx_work_bytes(long long cap, int P32, int num_sms, int fmm_p = VX_FMM_
 // j, bucket key b): nothing (mode 0), the quadtree's FP32 source (mode 1:
 // position relative to the centre of leaf b / 4, G masked beyond n, the
 // leaf's column), or the diffusion grid's (mode 2: position relative to the
-// centre of cell b, G, d).  zero_counts: the bucket counts are left at zero
-// instead of restored.
+// centre of cell b, G, d).
 struct VxGather {
     int mode = 0;
-    int zero_counts = 0;
     VxView v = {};
     const VxScalars *S = nullptr;
     float4 *srt = nullptr;
@@ -776,14 +879,14 @@ __device__ __forceinline__ void vx_gather_slot(const VxGather &gt, long long k, 
                                 (float)v.d[j]);
     }
 }
-// Stable order by bucket from bucket counts (used up, then restored or
-// zeroed) and starts: (okey, oval) = keys and element indices in bucket
-// order, elements of a bucket in index order, and the gather of gt at each
-// element's final slot (vx_sort.cu).
+// Stable order by bucket from each element's bucket, its rank in it (any order:
+// what counting the buckets returned) and the buckets' starts: (okey, oval)
+// = keys and element indices in bucket order, elements of a bucket in index
+// order, and the gather of gt at each element's final slot (vx_sort.cu).
+// scratch: n ints (rank may be used).
 cudaError_t vx_bucket_order(const VxLaunch &L, VxScalars *S, const long long *d_n, const long long *d_nbuckets,
-                            const unsigned *key, const int *start, int *cnt, const long long *d_cnt_off,
-                            unsigned *okey, int *oval, int *mid, int *big, int *scratch,
-                            const VxGather &gt = VxGather());
+                            const unsigned *key, const int *rank, const int *start, unsigned *okey, int *oval,
+                            int *mid, int *big, int *scratch, const VxGather &gt = VxGather());
 int vx_fmm_max_level(long long cap);
 long long vx_fmm_cells(int lmax);         // cells of all levels 0..lmax
 constexpr int VX_BF_P = 48;          // terms of the birth far-field expansion

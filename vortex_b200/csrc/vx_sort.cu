@@ -9,47 +9,42 @@
 
 #include "vx_internal.cuh"
 
-// Stable order by bucket, for keys whose buckets already have counts and
-// starts (an exclusive scan of the counts): every element
-// takes a slot of its bucket (its start plus an atomic rank, in no fixed
-// order), then each bucket's slots are put back in element-index order, the
-// order a stable sort by bucket gives (rank of an element = the number of
-// the bucket's elements with a lower index).  A bucket of up to 16 elements
-// takes one thread, one of up to 128 a warp, a larger one a block (the warps
-// and blocks in one launch after the threads').  The
-// counts are used up by the placement and written back by the ordering.
-VX_DEVK void k_bk_place_body(VxBlkB<0, 0> vb, const long long *d_n, const unsigned *key, const int *start, int *cnt0,
-                             const long long *d_off, unsigned *okey, int *oval) {
+// Stable order by bucket, for keys whose buckets have starts (an exclusive
+// scan of their counts) and whose elements have ranks (what counting them
+// returned, in no fixed order): every element takes its slot, then each
+// bucket's slots are put back in element-index order, the order a stable sort
+// by bucket gives (rank of an element = the number of the bucket's elements
+// with a lower index).  A bucket of up to 16 elements takes one thread, one of
+// up to 128 a warp, a larger one a block (the warps and blocks in one launch
+// after the threads').
+VX_DEVK void k_bk_place_body(VxBlkB<0, 0> vb, const long long *d_n, const unsigned *key, const int *rank,
+                             const int *start, unsigned *okey, int *oval) {
     const long long n = *d_n;
-    int *cnt = cnt0 + (d_off ? *d_off : 0);
     for (long long i = vb.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)vb.n * blockDim.x) {
         const unsigned c = key[i];
-        const int pos = start[c] + atomicSub(&cnt[c], 1) - 1;
+        const int pos = start[c] + rank[i];
         okey[pos] = c;
         oval[pos] = (int)i;
     }
 }
-__global__ void k_bk_place(const long long *d_n, const unsigned *key, const int *start, int *cnt0,
-                           const long long *d_off, unsigned *okey, int *oval) {
+__global__ void k_bk_place(const long long *d_n, const unsigned *key, const int *rank, const int *start,
+                           unsigned *okey, int *oval) {
     VX_PDL_WAIT();
-    k_bk_place_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, d_n, key, start, cnt0, d_off, okey, oval);
+    k_bk_place_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, d_n, key, rank, start, okey, oval);
 }
 
 constexpr int BK_S = 16;  // a thread orders buckets of up to BK_S elements
 constexpr int BK_E = 4;   // elements per lane: a warp orders buckets of up to 32 * BK_E
 
-// One thread per bucket: writes the count back, orders a bucket of up to
-// BK_S elements itself (ranks by counting, in registers) and lists larger
+// One thread per bucket: orders a bucket of up to BK_S elements itself (ranks by counting, in registers) and lists larger
 // ones for a warp (mid) or a block (big).
-VX_DEVK void k_bk_order_body(VxBlkB<256, 3> vb, VxScalars *S, const long long *d_nb, const int *start, int *cnt0, const long long *d_off,
+VX_DEVK void k_bk_order_body(VxBlkB<256, 3> vb, VxScalars *S, const long long *d_nb, const int *start,
                              int *oval, int *mid, int *big, VxGather gt) {
     const long long nb = *d_nb;
-    int *cnt = cnt0 + (d_off ? *d_off : 0);
     for (long long b = vb.x * (long long)blockDim.x + threadIdx.x; b < nb;
          b += (long long)vb.n * blockDim.x) {
         const int a = start[b], m = start[b + 1] - a;
-        cnt[b] = gt.zero_counts ? 0 : m;
         if (m <= 1) {
             if (m == 1 && gt.mode) vx_gather_slot(gt, a, oval[a], (unsigned)b);
             continue;
@@ -74,10 +69,9 @@ VX_DEVK void k_bk_order_body(VxBlkB<256, 3> vb, VxScalars *S, const long long *d
         }
     }
 }
-__global__ void k_bk_order(VxScalars *S, const long long *d_nb, const int *start, int *cnt0, const long long *d_off,
-                           int *oval, int *mid, int *big, VxGather gt) {
+__global__ void k_bk_order(VxScalars *S, const long long *d_nb, const int *start, int *oval, int *mid, int *big, VxGather gt) {
     VX_PDL_WAIT();
-    k_bk_order_body(VxBlkB<256, 3>{blockIdx.x, gridDim.x}, S, d_nb, start, cnt0, d_off, oval, mid, big, gt);
+    k_bk_order_body(VxBlkB<256, 3>{blockIdx.x, gridDim.x}, S, d_nb, start, oval, mid, big, gt);
 }
 
 // The listed buckets, one launch: a block per bucket of more than 32 BK_E
@@ -145,11 +139,11 @@ __global__ void __launch_bounds__(BK_T) k_bk_order_rest(const VxScalars *S, cons
 }
 
 cudaError_t vx_bucket_order(const VxLaunch &L, VxScalars *S, const long long *d_n, const long long *d_nbuckets,
-                            const unsigned *key, const int *start, int *cnt, const long long *d_cnt_off,
-                            unsigned *okey, int *oval, int *mid, int *big, int *scratch, const VxGather &gt) {
-    vx_launch<k_bk_place, k_bk_place_body>(L, L.num_sms * 4, 256, 0, d_n, key, start, cnt, d_cnt_off, okey, oval);
+                            const unsigned *key, const int *rank, const int *start, unsigned *okey, int *oval,
+                            int *mid, int *big, int *scratch, const VxGather &gt) {
+    vx_launch<k_bk_place, k_bk_place_body>(L, L.num_sms * 4, 256, 0, d_n, key, rank, start, okey, oval);
 
-    vx_launch<k_bk_order, k_bk_order_body>(L, L.num_sms * 4, 256, 0, S, d_nbuckets, start, cnt, d_cnt_off, oval, mid, big, gt);
+    vx_launch<k_bk_order, k_bk_order_body>(L, L.num_sms * 4, 256, 0, S, d_nbuckets, start, oval, mid, big, gt);
 
     vx_launch<k_bk_order_rest, k_bk_order_rest_body>(L, L.num_sms * 4, BK_T, 0, S, start, mid, big, oval, scratch, gt);
 
@@ -157,8 +151,8 @@ cudaError_t vx_bucket_order(const VxLaunch &L, VxScalars *S, const long long *d_
 }
 
 // Validation hook: the bucket order of n keys (device array, each below nb)
-// into `order` (device array of n element indices), with counts and starts
-// computed on the host.  Allocates its own scratch; not for the step path.
+// into `order` (device array of n element indices), with starts and ranks
+// computed on the host (the ranks against index order).  Allocates its own scratch; not for the step path.
 extern "C" vx_status vx_eval_bucket_order(const unsigned *key, int64_t n, int64_t nb, int *order) {
     if (n < 0 || nb < 1 || n > INT_MAX || (n > 0 && (!key || !order))) return VX_ERR_ARG;
     if (n == 0) return VX_OK;
@@ -170,11 +164,13 @@ extern "C" vx_status vx_eval_bucket_order(const unsigned *key, int64_t n, int64_
         ++cnt[k];
     }
     for (int64_t b = 0; b < nb; ++b) start[b + 1] = start[b] + cnt[b];
+    std::vector<int> rank((size_t)n), left(cnt);
+    for (int64_t i = 0; i < n; ++i) rank[i] = --left[hk[i]];
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     void *mem[8] = {};
-    const size_t sz[8] = {sizeof(VxScalars), 2 * sizeof(long long), sizeof(int) * (nb + 1), sizeof(int) * nb,
+    const size_t sz[8] = {sizeof(VxScalars), 2 * sizeof(long long), sizeof(int) * (nb + 1), sizeof(int) * n,
                           sizeof(unsigned) * n, sizeof(int) * (n / 16 + 2), sizeof(int) * (n / 128 + 2),
                           sizeof(int) * n};
     vx_status st = VX_OK;
@@ -184,23 +180,20 @@ extern "C" vx_status vx_eval_bucket_order(const unsigned *key, int64_t n, int64_
         VxScalars *S = (VxScalars *)mem[0];
         long long *dn = (long long *)mem[1];
         const long long hn[2] = {(long long)n, (long long)nb};
-        int *dstart = (int *)mem[2], *dcnt = (int *)mem[3];
+        int *dstart = (int *)mem[2], *drank = (int *)mem[3];
         bool ok = cudaMemset(S, 0, sizeof(VxScalars)) == cudaSuccess &&
                   cudaMemcpy(dn, hn, sizeof(hn), cudaMemcpyHostToDevice) == cudaSuccess &&
                   cudaMemcpy(dstart, start.data(), sizeof(int) * (nb + 1), cudaMemcpyHostToDevice) == cudaSuccess &&
-                  cudaMemcpy(dcnt, cnt.data(), sizeof(int) * nb, cudaMemcpyHostToDevice) == cudaSuccess;
+                  cudaMemcpy(drank, rank.data(), sizeof(int) * n, cudaMemcpyHostToDevice) == cudaSuccess;
         if (ok) {
             VxLaunch L;
             L.stream = 0;
             L.launches = nullptr;
             L.num_sms = sms;
-            ok = vx_bucket_order(L, S, dn, dn + 1, key, dstart, dcnt, nullptr, (unsigned *)mem[4], order,
-                                 (int *)mem[5], (int *)mem[6], (int *)mem[7]) == cudaSuccess &&
+            ok = vx_bucket_order(L, S, dn, dn + 1, key, drank, dstart, (unsigned *)mem[4], order, (int *)mem[5],
+                                 (int *)mem[6], (int *)mem[7]) == cudaSuccess &&
                  cudaDeviceSynchronize() == cudaSuccess;
         }
-        std::vector<int> back((size_t)nb);
-        if (ok) ok = cudaMemcpy(back.data(), dcnt, sizeof(int) * nb, cudaMemcpyDeviceToHost) == cudaSuccess;
-        if (ok && back != cnt) st = VX_ERR_DEVICE;   // the counts must come back as they went in
         if (!ok) st = VX_ERR_CUDA;
     }
     for (void *p : mem) if (p) cudaFree(p);
