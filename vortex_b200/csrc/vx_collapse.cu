@@ -17,10 +17,10 @@
 //    pointing at j; later ones merge with (0, 1e10) as the serial loop does,
 //    which re-rounds their position.
 //  * Compaction then runs as after convection.
-// The first round is six launches before the compaction: prep (box,
-// bookkeeping and grid in one, the last block finishing), count, a one-pass
-// scan of the cell counts, scatter, query, and settle (resolution, merge and
-// write-back in one block).
+// The first round is six launches: prep (box, bookkeeping and grid in one, the
+// last block finishing), count, a one-pass scan of the cell counts, scatter,
+// query, and settle (resolution, merge, write-back and compaction in one
+// block: the settle knows which vortices its merges removed).
 //
 // The second round takes the first one's grid.  A pair that qualifies in it
 // holds a vortex the first round moved (two unmoved ones that qualify would
@@ -39,7 +39,7 @@
 // INT_MAX - i (atomicMax keeps the smallest index, 0 is none).
 #include <limits.h>
 
-#include "vx_internal.cuh"
+#include "vx_compact.cuh"
 
 // Start of a round: the bounding box (per-block keys into part[], combined
 // by the last block), the round's bookkeeping and the cell grid.  A round
@@ -145,9 +145,10 @@ struct __align__(32) ColRec {
 
 // Each vortex's slot from its cell's start and its rank (which becomes its
 // slot); the slot gets a copy of the vortex (ColRec), so that the query reads
-// its candidates as contiguous runs.
+// its candidates as contiguous runs.  A vortex too weak to stay (there is none
+// after a compaction) is marked for the round's own.
 VX_DEVK void k_col_scatter_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalars *S, const int *start, int *slot,
-                                ColRec *rec) {
+                                ColRec *rec, double drop_eps, unsigned *dead) {
     if (S->col_done) return;
     const long long n = S->n;
     for (long long i = vb.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -159,12 +160,15 @@ VX_DEVK void k_col_scatter_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalar
         slot[i] = k;
         double2 *r = reinterpret_cast<double2 *>(rec + k);
         r[0] = make_double2(x, y);
-        r[1] = make_double2(v.g[i * v.ps], __longlong_as_double(i));
+        const double g = v.g[i * v.ps];
+        r[1] = make_double2(g, __longlong_as_double(i));
+        if (!(fabs(g) >= drop_eps)) vx_set_dead(dead, i);
     }
 }
-__global__ void k_col_scatter(VxView v, const VxScalars *S, const int *start, int *slot, ColRec *rec) {
+__global__ void k_col_scatter(VxView v, const VxScalars *S, const int *start, int *slot, ColRec *rec, double drop_eps,
+                              unsigned *dead) {
     VX_PDL_WAIT();
-    k_col_scatter_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, start, slot, rec);
+    k_col_scatter_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, start, slot, rec, drop_eps, dead);
 }
 
 // Whether a pair qualifies in a pass.
@@ -246,6 +250,7 @@ VX_DEVK void k_col_query_moved_body(VxBlkB<VX_THREADS, 0> vb, const VxParams &p,
             if (k == k0) continue;
             const double2 q0 = reinterpret_cast<const double2 *>(rec + k)[0];
             const double2 q1 = reinterpret_cast<const double2 *>(rec + k)[1];
+            if (!(fabs(q1.x) >= p.drop_eps)) continue;   // removed after the first round
             if (!vx_col_pair<PASS>(p, m0.x, m0.y, m1.x, q0.x, q0.y, q1.x)) continue;
             const int j = (int)__double_as_longlong(q1.y), lo = min(i, j);
             if (atomicMax(&col[lo], INT_MAX - max(i, j)) == 0) cand[atomicAdd(&S->ncand, 1)] = lo;
@@ -267,10 +272,15 @@ __global__ void __launch_bounds__(VX_THREADS) k_col_query_moved(VxParams p, VxSc
 // another merge removes).
 // track: the cell-sorted copy is kept in step for the second round, and the
 // slots of the moved vortices are listed (in cdec, done with by then).
+// The round's compaction follows in the same block (vx_cmp_block): what the
+// merges removed is marked as they are written.  It adds 8 / 16 / 20 us at
+// 2e4 / 1e6 / 3e6 vortices; as four launches over all of them (count,
+// classify, gather, scatter) it took 32 / 39 / 50.
 template <int PASS>
 VX_DEVK void k_col_settle_body(VxBlkB<1024, 0> vb, const VxView &v, VxScalars *S, const int *cand, int *col,
                                int *in_cnt, int *has_app, int *first_app, int *cstate, int *cdec, double *mx,
-                               double *my, double *mg, const int *slot, ColRec *rec, double drop_eps, int track) {
+                               double *my, double *mg, const int *slot, ColRec *rec, double drop_eps, int track,
+                               const VxCompact &cmp) {
     if (S->col_done) return;
     __shared__ int undecided, listed;
     const int nc = S->ncand;
@@ -335,10 +345,14 @@ VX_DEVK void k_col_settle_body(VxBlkB<1024, 0> vb, const VxView &v, VxScalars *S
     for (int k = threadIdx.x; k < nc; k += blockDim.x) {
         const long long i = cand[k], j = INT_MAX - col[i];
         if (!failed && cstate[k] == 1) {
+            const bool weak = !(fabs(v.g[i * v.ps]) >= drop_eps);
             v.x[i * v.ps] = mx[k]; v.y[i * v.ps] = my[k]; v.g[i * v.ps] = mg[k];
             v.x[j * v.ps] = 1e10; v.y[j * v.ps] = 1e10; v.g[j * v.ps] = 0.0;
+            const bool left = fabs(mg[k]) >= drop_eps;   // else the compaction removes it
+            if (!(0.0 >= drop_eps)) vx_set_dead(cmp.bits, j);
+            if (!left) vx_set_dead(cmp.bits, i);
+            else if (weak) atomicAnd(&cmp.bits[i >> 5], ~(1u << (i & 31)));   // marked by the scatter
             if (track) {
-                const bool left = fabs(mg[k]) >= drop_eps;   // else the compaction removes it
                 ColRec *r = rec + slot[i];
                 r->x = mx[k]; r->y = my[k]; r->g = left ? mg[k] : 0.0;
                 rec[slot[j]].g = 0.0;
@@ -349,23 +363,25 @@ VX_DEVK void k_col_settle_body(VxBlkB<1024, 0> vb, const VxView &v, VxScalars *S
         in_cnt[j] = 0; has_app[j] = 0; first_app[j] = 0;
     }
     __syncthreads();
+    // the round's compaction (none after a failed one); one that removes
+    // nothing ends the pass
+    const long long n0 = S->n;
+    const long long removed = vx_cmp_block<1024>(v, S, cmp, n0, n0, !failed, slot, track ? &rec[0].i : nullptr);
     if (threadIdx.x == 0) {
         S->ncand = 0;
         S->nmoved = listed;
-        if (failed) {
-            S->err |= VX_DERR_RESOLVE;
-            S->col_done = 1;
-        }
+        if (failed) S->err |= VX_DERR_RESOLVE;
+        if (failed || removed == 0) S->col_done = 1;
     }
 }
 template <int PASS>
 __global__ void __launch_bounds__(1024) k_col_settle(VxView v, VxScalars *S, const int *cand, int *col,
                                                      int *in_cnt, int *has_app, int *first_app, int *cstate,
                                                      int *cdec, double *mx, double *my, double *mg, const int *slot,
-                                                     ColRec *rec, double drop_eps, int track) {
+                                                     ColRec *rec, double drop_eps, int track, VxCompact cmp) {
     VX_PDL_WAIT();
     k_col_settle_body<PASS>(VxBlkB<1024, 0>{blockIdx.x, gridDim.x}, v, S, cand, col, in_cnt, has_app, first_app,
-                            cstate, cdec, mx, my, mg, slot, rec, drop_eps, track);
+                            cstate, cdec, mx, my, mg, slot, rec, drop_eps, track, cmp);
 }
 
 template <int PASS>
@@ -384,12 +400,10 @@ static cudaError_t collapse_pass(const VxLaunch &L, const VxParams &p, const VxV
             vx_launch<k_col_prep, k_col_prep_body>(L, grid, VX_THREADS, 0, v, S, cc == 0, r2, w.cells_cap, w.box);
             vx_launch<k_col_count, k_col_count_body>(L, grid, VX_THREADS, 0, v, S, w.cellid, w.cell_cnt);
             vx_launch<k_col_scan, k_col_scan_body>(L, grid, VX_SCAN_T, 0, S, w.cell_cnt, w.cell_start, w.scan_tiles);
-            vx_launch<k_col_scatter, k_col_scatter_body>(L, grid, VX_THREADS, 0, v, S, w.cell_start, w.cellid, rec);
+            vx_launch<k_col_scatter, k_col_scatter_body>(L, grid, VX_THREADS, 0, v, S, w.cell_start, w.cellid, rec, p.drop_eps, w.cmp.bits);
             vx_launch<k_col_query<PASS>, k_col_query_body<PASS>>(L, grid, VX_THREADS, 0, p, S, w.cell_start, (const ColRec *)rec, w.col, w.cand);
         }
-        vx_launch<k_col_settle<PASS>, k_col_settle_body<PASS>>(L, 1, 1024, 0, v, S, w.cand, w.col, w.in_cnt, w.has_app, w.first_app, w.cstate, w.cdec, w.mx, w.my, w.mg, w.cellid, rec, p.drop_eps, track);
-        // the compaction renames, in the copy, the vortices it moves
-        vx_launch_compact_round(L, p, v, S, w, w.cellid, track ? &rec[0].i : nullptr);
+        vx_launch<k_col_settle<PASS>, k_col_settle_body<PASS>>(L, 1, 1024, 0, v, S, w.cand, w.col, w.in_cnt, w.has_app, w.first_app, w.cstate, w.cdec, w.mx, w.my, w.mg, w.cellid, rec, p.drop_eps, track, w.cmp);
     }
     return cudaGetLastError();
 }

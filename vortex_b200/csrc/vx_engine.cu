@@ -300,12 +300,11 @@ static vx_status work_alloc_impl(VxWork &w, std::vector<void *> *allocs, long lo
     w.cap = cap;
     w.fmm_p = fmm_p;
     w.bytes = 0;
-    const long long nch = cap / VX_CHUNK + 2;
     vx_status st;
 #define A(ptr, n) if ((st = dalloc(allocs, &w.bytes, &(ptr), (n), stream, cv)) != VX_OK) return st
-    A(w.cmp_cnt, nch); A(w.cmp_off, nch);
-    A(w.hole_pos, cap); A(w.hole_src, cap); A(w.tail_src, cap);
-    A(w.hx, cap); A(w.hy, cap); A(w.hg, cap); A(w.tx, cap); A(w.ty, cap);
+    if ((st = dalloc_zero(allocs, &w.bytes, &w.cmp.bits, cap / 32 + 8, stream, cv)) != VX_OK) return st;
+    A(w.cmp.hole_pos, cap); A(w.cmp.hole_src, cap); A(w.cmp.tail_src, cap);
+    A(w.cmp.hx, cap); A(w.cmp.hy, cap); A(w.cmp.hg, cap); A(w.cmp.tx, cap); A(w.cmp.ty, cap);
     w.cells_cap = std::max(4 * cap, 65536LL);
     A(w.cellid, cap); A(w.cell_start, w.cells_cap + 1); A(w.sorted, cap);
     // the collapse grid's cell counts are zero between rounds (the scan that

@@ -77,7 +77,7 @@ struct VxScalars {
     double fx, fy, m;      // force and moment of the last step
     double raw[4];         // unscaled sums of dg, Fx, Fy, M of the last convection
     // compaction
-    long long c_n0, c_m, c_H, c_scan_m;
+    long long c_n0, c_m, c_H;
     // collapse
     int col_done;
     int ncand;
@@ -118,15 +118,21 @@ enum {
     VX_DERR_SCAN = 4,        // a look-back scan gave up waiting on a predecessor tile
 };
 
+// Scratch of a compaction: the dead vortices' bits (zero between compactions,
+// a word past the last vortex's), the lists of holes, of what fills them and
+// of the tail's sources (a source below zero: the position of hole
+// -(value + 1)), and the moved values.
+struct VxCompact {
+    unsigned *bits;
+    int *hole_pos, *hole_src, *tail_src;
+    double *hx, *hy, *hg, *tx, *ty;
+};
+
 // Device scratch of one body.  Sizes are in elements.
 struct VxWork {
     long long cap;           // particle capacity the arrays below were sized for
     long long bytes;         // device bytes the arrays below take
-    // compaction
-    int *cmp_cnt;
-    long long *cmp_off;
-    int *hole_pos, *hole_src, *tail_src;
-    double *hx, *hy, *hg, *tx, *ty;
+    VxCompact cmp;
     // collapse
     long long cells_cap;
     int *cellid, *cell_cnt, *cell_start, *sorted;
@@ -174,8 +180,6 @@ struct VxWork {
 constexpr int VX_FMM_P = 16;              // default expansion terms of the quadtree FMM (vx_fmm.cu)
 inline bool vx_fmm_order_ok(int p) { return p == 8 || p == 12 || p == 16 || p == 20; }
 
-// Compaction chunk size (elements per scan chunk).
-constexpr int VX_CHUNK = 2048;
 constexpr int VX_RED_BLOCKS = 592;   // 4 x 148 SMs: fixed, so sums are deterministic
 constexpr int VX_THREADS = 256;
 
@@ -840,10 +844,6 @@ cudaError_t vx_invert_gj(const VxLaunch &L, double *A, double *Inv, long long S,
 // overwritten, piv holds n ints; *flag set on a pivot below 1e-12.
 cudaError_t vx_invert_lu(const VxLaunch &L, double *A, double *Inv, long long n, int *piv, int *flag);
 cudaError_t vx_launch_step_end(const VxLaunch &L, VxScalars *S);
-// The compaction of a collapse round: skipped when S->col_done, which it sets
-// if it removed nothing; slot, rec_i: see k_cmp_scatter (vx_compact.cu).
-cudaError_t vx_launch_compact_round(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
-                                    const int *slot, long long *rec_i);
 void vx_params_from_conf(const vx_conf *c, const vx_panel *pan, int P, VxParams *p);
 void vx_set_error(const char *fmt, ...);
 void vx_keep_pool(int device);
