@@ -827,15 +827,93 @@ __device__ __forceinline__ void near_pair2(f2 SX, f2 SYs, f2 G, f2 TX, f2 TY, fl
 #ifndef VX_NEAR_MINB
 #define VX_NEAR_MINB 2   // minimum resident blocks per SM requested for k_fmm_near (at most 128 registers)
 #endif
+// The sources of an item: the 3 x 3 leaves around its own are three
+// contiguous runs (rows row-1..row+1 of columns c0..c1), walked as one stream
+// in chunks of 32 sources, so only the stream's last chunk is padded.
+struct NearRows {
+    int j0[3], pre[4];
+    float oy[3];   // y offset of the run's row
+};
+constexpr int NEAR_STRIDE = 36;   // floats a staged chunk: the groups' chunks lie on different banks
+
+// Velocity sums of a warp's targets over the stream.  GF groups of 32 / GF
+// lanes hold the same targets and take every GF-th chunk; their sums, FP64
+// between chunks, are added at the end (in every lane).  wx, wy, wg: the
+// warp's staging rows, a chunk's x, y, G each in NEAR_STRIDE floats, so that
+// one 16-byte shared load brings four sources' x (or y, or G).
+template <int GF>
+__device__ __forceinline__ void near_stream(const float4 *srt, const NearRows &r, f2 TX, f2 TY, float eps2, float hf,
+                                            float colf, float *wx, float *wy, float *wg, int lane, double &ax,
+                                            double &ay) {
+    const int total = r.pre[3];
+    // source f of the stream: its slot in the leaf-sorted array and the
+    // y offset of its row; the x offset of its column, (column - col) h
+    // with the difference -1, 0 or 1, is exact in FP32
+    auto src_of = [&](int f, float &oy) {
+        const bool in0 = f < r.pre[1], in1 = f < r.pre[2];
+        oy = in0 ? r.oy[0] : (in1 ? r.oy[1] : r.oy[2]);
+        return in0 ? r.j0[0] + f : (in1 ? r.j0[1] + (f - r.pre[1]) : r.j0[2] + (f - r.pre[2]));
+    };
+    const int own = GF == 1 ? 0 : lane / (32 / GF) * (NEAR_STRIDE / 4);
+    const float4 *cx = reinterpret_cast<const float4 *>(wx) + own, *cy = reinterpret_cast<const float4 *>(wy) + own,
+                 *cg = reinterpret_cast<const float4 *>(wg) + own;
+    // the next chunks' sources are loaded before the current ones' pairs run
+    float4 qn[GF];
+    float oyn[GF];
+#pragma unroll
+    for (int k = 0; k < GF; ++k)
+        if (32 * k + lane < total) qn[k] = srt[src_of(32 * k + lane, oyn[k])];
+    for (int jt = 0; jt < total; jt += 32 * GF) {
+#pragma unroll
+        for (int k = 0; k < GF; ++k) {
+            // padding: G = 0 sources far away add exactly 0
+            const int f = jt + 32 * k + lane;
+            float x = 1e12f, y = 1e12f, g = 0.f;
+            if (f < total) {
+                x = qn[k].x + (qn[k].w - colf) * hf;
+                y = qn[k].y + oyn[k];
+                g = qn[k].z;
+            }
+            if (f + 32 * GF < total) qn[k] = srt[src_of(f + 32 * GF, oyn[k])];
+            wx[k * NEAR_STRIDE + lane] = x;
+            wy[k * NEAR_STRIDE + lane] = y;
+            wg[k * NEAR_STRIDE + lane] = g;
+        }
+        __syncwarp();
+        f2 SY = 0ull, SXN = 0ull;   // +0.0f in both halves
+#pragma unroll
+        for (int q4 = 0; q4 < 8; ++q4) {   // sources 2q, 2q + 1 a pair step, in index order
+            const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(cx + q4);
+            const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(cy + q4);
+            const ulonglong2 G = *reinterpret_cast<const ulonglong2 *>(cg + q4);
+            near_pair2(X.x, Y.x, G.x, TX, TY, eps2, SY, SXN);
+            near_pair2(X.y, Y.y, G.y, TX, TY, eps2, SY, SXN);
+        }
+        __syncwarp();
+        float a, b;   // the two halves are added in FP32, then carried in FP64
+        f2_unpack(SXN, a, b); ax -= (double)(a + b);
+        f2_unpack(SY, a, b); ay += (double)(a + b);
+    }
+#pragma unroll
+    for (int o = 32 / GF; o < 32; o <<= 1) {
+        ax += __shfl_xor_sync(0xffffffffu, ax, o);
+        ay += __shfl_xor_sync(0xffffffffu, ay, o);
+    }
+}
+
+// Near field and the far field's evaluation, one warp per item (up to 32
+// targets of one leaf).  Bound: the FMA pipe's nine packed instructions per
+// two pairs, and the lanes without a target: a leaf's last item holds any
+// number of them, so with at most 16 (8) the warp's halves (quarters) take
+// the same targets and every second (fourth) chunk of sources.
+// A warp of up to 32 lanes for each item: 262 us at 1e6 vortices, 840 at 3e6; so
+// 252 and 667.
 template <int P>
 VX_DEVK void k_fmm_near_body(VxBlkB<FMM_T, VX_NEAR_MINB> vb, const VxParams &p, const VxView &v, VxScalars *S, const float4 *srt,
                              const int *sorted, const int *start, const int2 *items, const cplx *Loc) {
-    // per warp 32 staged sources as x[32], y[32], G[32]: one 16-byte shared
-    // load brings four sources' x (or y, or G)
-    __shared__ float4 sx[FMM_T / 4], sy[FMM_T / 4], sg[FMM_T / 4];
+    __shared__ __align__(16) float stage[FMM_T / 32][3][4 * NEAR_STRIDE];
     const int lane = threadIdx.x & 31;
-    float4 *wx = sx + ((threadIdx.x & ~31) >> 2), *wy = sy + ((threadIdx.x & ~31) >> 2),
-           *wg = sg + ((threadIdx.x & ~31) >> 2);
+    float *wx = stage[threadIdx.x >> 5][0], *wy = stage[threadIdx.x >> 5][1], *wg = stage[threadIdx.x >> 5][2];
     const long long n = S->n;
     const int L = S->fL;
     const long long m = 1LL << L;
@@ -848,82 +926,39 @@ VX_DEVK void k_fmm_near_body(VxBlkB<FMM_T, VX_NEAR_MINB> vb, const VxParams &p, 
         const int2 item = items[it];
         const long long leaf = item.x;
         const long long row = leaf / m, col = leaf % m;
-        const long long last = min((long long)item.y + FMM_W, (long long)start[leaf + 1]);
-        const long long t = item.y + lane;
-        const bool valid = t < last;
+        const int nt = min(FMM_W, start[leaf + 1] - item.y);   // targets
+        const int GF = nt > 16 ? 1 : (nt > 8 ? 2 : 4);
+        const int slot = lane & (32 / GF - 1);
+        const long long t = item.y + slot;
+        const bool valid = slot < nt;
         const float4 me = valid ? srt[t] : make_float4(0.f, 0.f, 0.f, 0.f);   // relative to the leaf centre
-        const long long j_self = valid ? sorted[t] : -1;
+        const long long j_self = valid && slot == lane ? sorted[t] : n;
         const long long c0 = max(col - 1, 0LL), c1 = min(col + 1, m - 1);
         const f2 TX = f2_pack(me.x, me.x), TY = f2_pack(me.y, me.y);
         double ax = 0.0, ay = 0.0;
-        // the 3 x 3 leaves are three contiguous runs (rows row-1..row+1 of
-        // columns c0..c1), walked as one stream in chunks of 32 sources, so
-        // only the stream's last chunk is padded
         const long long r_lo = max(row - 1, 0LL), r_hi = min(row + 1, m - 1);
-        int rj0[3], rpre[4];
-        float roy[3];
-        rpre[0] = 0;
+        NearRows rows;
+        rows.pre[0] = 0;
+#pragma unroll
         for (int r = 0; r < 3; ++r) {
             const long long rr = r_lo + r;
             int len = 0;
-            rj0[r] = 0;
-            roy[r] = 0.f;
+            rows.j0[r] = 0;
+            rows.oy[r] = 0.f;
             if (rr <= r_hi) {
-                rj0[r] = start[rr * m + c0];
-                len = start[rr * m + c1 + 1] - rj0[r];
-                roy[r] = (float)((double)(rr - row) * h);
+                rows.j0[r] = start[rr * m + c0];
+                len = start[rr * m + c1 + 1] - rows.j0[r];
+                rows.oy[r] = (float)((double)(rr - row) * h);
             }
-            rpre[r + 1] = rpre[r] + len;
+            rows.pre[r + 1] = rows.pre[r] + len;
         }
-        const int total = rpre[3];
-        // source f of the stream: its slot in the leaf-sorted array and the
-        // y offset of its row; the x offset of its column, (column - col) h
-        // with the difference -1, 0 or 1, is exact in FP32
         const float hf = (float)h, colf = (float)col;
-        auto src_of = [&](int f, float &oy) {
-            const bool in0 = f < rpre[1], in1 = f < rpre[2];
-            oy = in0 ? roy[0] : (in1 ? roy[1] : roy[2]);
-            return in0 ? rj0[0] + f : (in1 ? rj0[1] + (f - rpre[1]) : rj0[2] + (f - rpre[2]));
-        };
-        // the next chunk's source is loaded before the current chunk's pairs run
-        float4 qn = make_float4(1e12f, 1e12f, 0.f, colf);
-        float oyn = 0.f;
-        if (lane < total) qn = srt[src_of(lane, oyn)];
-        for (int jt = 0; jt < total; jt += 32) {
-            // padding: G = 0 sources far away add exactly 0
-            const float4 q = qn;
-            const float oy = oyn;
-            const int fnext = jt + 32 + lane;
-            if (fnext < total) qn = srt[src_of(fnext, oyn)];
-            float x = 1e12f, y = 1e12f, g = 0.f;
-            if (jt + lane < total) {
-                x = q.x + (q.w - colf) * hf;
-                y = q.y + oy;
-                g = q.z;
-            }
-            reinterpret_cast<float *>(wx)[lane] = x;
-            reinterpret_cast<float *>(wy)[lane] = y;
-            reinterpret_cast<float *>(wg)[lane] = g;
-            __syncwarp();
-            f2 SY = 0ull, SXN = 0ull;   // +0.0f in both halves
-#pragma unroll
-            for (int q4 = 0; q4 < 8; ++q4) {   // sources 2q, 2q + 1 a pair step, in index order
-                const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(wx + q4);
-                const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(wy + q4);
-                const ulonglong2 G = *reinterpret_cast<const ulonglong2 *>(wg + q4);
-                near_pair2(X.x, Y.x, G.x, TX, TY, eps2, SY, SXN);
-                near_pair2(X.y, Y.y, G.y, TX, TY, eps2, SY, SXN);
-            }
-            __syncwarp();
-            float a, b;   // the two halves are added in FP32, then carried in FP64
-            f2_unpack(SXN, a, b); ax -= (double)(a + b);
-            f2_unpack(SY, a, b); ay += (double)(a + b);
-        }
-        {   // executed near-field pairs: every target of the item sees the same 3x3 leaves
-            const unsigned long long nv = __popc(__ballot_sync(0xffffffffu, valid));
-            if (lane == 0) atomicAdd(&S->pairs_bs, (unsigned long long)total * nv);
-        }
-        if (valid && j_self < n) {
+        if (GF == 1) near_stream<1>(srt, rows, TX, TY, eps2, hf, colf, wx, wy, wg, lane, ax, ay);
+        else if (GF == 2) near_stream<2>(srt, rows, TX, TY, eps2, hf, colf, wx, wy, wg, lane, ax, ay);
+        else near_stream<4>(srt, rows, TX, TY, eps2, hf, colf, wx, wy, wg, lane, ax, ay);
+        // executed near-field pairs: every target of the item sees the same 3x3 leaves
+        if (lane == 0) atomicAdd(&S->pairs_bs, (unsigned long long)rows.pre[3] * (unsigned long long)nt);
+        if (j_self < n) {
             // far field: f(z) = sum a_l u^l at the target's leaf (none below depth 2)
             cplx f = {0.0, 0.0};
             if (L >= 2) {
@@ -951,62 +986,114 @@ __global__ void __launch_bounds__(FMM_T, VX_NEAR_MINB) k_fmm_near(VxParams p, Vx
 
 // The 3 nearest sources of every live target (the reference's padded
 // launch: sources include the round-32 slots after the live ones; the
-// target itself excluded), one thread per target, over the 3 x 3 quarter
-// leaves around its own quarter (each quarter a contiguous run of the
-// sorted sources; coordinates relative to the target's leaf centre,
-// computed as the near field computes them).  Exact when the third distance
-// is below the quarter's side (every source outside the 3 x 3 block is
-// farther); the others go to the search over squares of leaves (k_fmm_nn3_fix).
+// target itself excluded) over the 3 x 3 quarter leaves around its own
+// quarter (each quarter a contiguous run of the sorted sources; coordinates
+// relative to the target's leaf centre, computed as the near field computes
+// them).  Exact when the third distance is below the quarter's side (every
+// source outside the 3 x 3 block is farther); the others go to the search over
+// squares of leaves (k_fmm_nn3_fix).
+//
+// Bound: issue slots.  A lane takes its target's own quarter first, which
+// usually settles the three.  A quarter around it whose box lies farther than
+// the third distance found so far (with a margin over FP32 rounding) cannot
+// hold one of them; a target needs about one of the four edge neighbours
+// still, few a corner.  Walked by each lane for its own target, these
+// left 12 of 32 lanes active; so the warp lists the (target, quarter) pairs
+// that are left, edges, then corners, and deals them out, a pair a lane.  The
+// three smallest of several lists do not depend on the order.  2e4 / 1e6 / 3e6
+// vortices: 29 -> 15, 144 -> 83, 349 -> 203 us.
 VX_DEVK void k_fmm_nn3_sub_body(VxBlkB<FMM_T, 0> vb, const VxView &v, VxScalars *S, const float4 *srt, const unsigned *skey,
                                 const int *sorted, const int *substart, int *flag_list) {
+    __shared__ unsigned char pair_of[FMM_T / 32][4 * 32];   // lane | neighbour << 5
     const long long s = S->fs, n = S->n;
-    const int m = 1 << S->fL, m2 = 2 * m;
+    const int L = S->fL, m = 1 << L;
+    const int lane = threadIdx.x & 31;
+    const unsigned before = (1u << lane) - 1u;
+    unsigned char *pairs = pair_of[threadIdx.x >> 5];
     const double h = S->fside / (double)m;
     const float sq2 = (float)(0.25 * h * h);   // (quarter side)^2
-    for (long long t = vb.x * (long long)blockDim.x + threadIdx.x; t < s; t += (long long)vb.n * blockDim.x) {
-        const int j = sorted[t];
-        if (j >= n) continue;
-        const unsigned key = skey[t];
-        const int leaf = (int)(key >> 2), col = leaf % m, row = leaf / m;
-        const int ix2 = 2 * col + (int)(key & 1), iy2 = 2 * row + (int)((key >> 1) & 1);
-        const float4 me = srt[t];
+    // a source's offset to the target's leaf centre: (its leaf's column -
+    // col) h and (its leaf's row - row) h, differences of -1, 0 or 1, so
+    // exact in FP32 and the same for every source of a quarter
+    const float hf = (float)h, hq = 0.5f * hf;
+    for (long long t0 = vb.x * (long long)blockDim.x + (threadIdx.x & ~31); t0 < s; t0 += (long long)vb.n * blockDim.x) {
+        const long long t = t0 + lane;
+        const int j = t < s ? sorted[t] : INT_MAX;
+        const bool valid = j < n;
+        const unsigned key = valid ? skey[t] : 0u;
+        const float4 me = valid ? srt[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+        // the quarter's column and row inside its leaf's row of quarters are
+        // 2 col + bit 0 and 2 row + bit 1 of the key
+        const int col = (int)(key >> 2) & (m - 1), row = (int)(key >> 2) >> L;
         float d1 = 1e5f, d2 = 1e5f, d3 = 1e5f;
-        const int y0 = max(iy2 - 1, 0), y1 = min(iy2 + 1, m2 - 1);
-        const int x0 = max(ix2 - 1, 0), x1 = min(ix2 + 1, m2 - 1);
-        // a source's offset to the target's leaf centre: (its leaf's column -
-        // col) h and (its leaf's row - row) h, differences of -1, 0 or 1, so
-        // exact in FP32 and the same for every source of a quarter
-        const float hf = (float)h, hq = 0.5f * hf;
-        // the target's own quarter first, then its four edge neighbours, then
-        // the corners; a quarter whose box lies farther than the third
-        // distance found so far (with a margin over FP32 rounding) cannot
-        // hold one of the 3 nearest and is not read: in a dense region the
-        // own quarter alone usually settles them.  (A quarter X2 spans
-        // [(X2 - 2 col - 1) hq, (X2 - 2 col) hq] in the leaf frame.)
-#pragma unroll 1
-        for (int o = 0; o < 9; ++o) {
-            const int ddx = (o == 1 || o == 5 || o == 7) ? -1 : ((o == 2 || o == 6 || o == 8) ? 1 : 0);
-            const int ddy = (o == 3 || o == 5 || o == 6) ? -1 : ((o == 4 || o == 7 || o == 8) ? 1 : 0);
-            const int X2 = ix2 + ddx, Y2 = iy2 + ddy;
-            if (X2 < x0 || X2 > x1 || Y2 < y0 || Y2 > y1) continue;
-            if (o > 0) {
-                const float qx = (float)(X2 - 2 * col), qy = (float)(Y2 - 2 * row);
-                const float gx = fmaxf(fmaxf((qx - 1.0f) * hq - me.x, me.x - qx * hq), 0.0f);
-                const float gy = fmaxf(fmaxf((qy - 1.0f) * hq - me.y, me.y - qy * hq), 0.0f);
-                if (fmaf(gx, gx, gy * gy) > 1.0001f * d3) continue;
-            }
-            const int lr = Y2 >> 1;
-            const float oy = (float)(lr - row) * hf;
-            const float ox = (float)((X2 >> 1) - col) * hf;
-            const int k = 4 * (lr * m + (X2 >> 1)) + 2 * (Y2 & 1) + (X2 & 1);
-            const int q1 = substart[k + 1];
-            for (int qq = substart[k]; qq < q1; ++qq) {
-                if (qq == t) continue;
+        if (valid) {
+            const int q1 = substart[key + 1];
+#pragma unroll 2
+            for (int qq = substart[key]; qq < q1; ++qq) {
                 const float2 q = *reinterpret_cast<const float2 *>(srt + qq);   // x, y of the source
-                const float dx = me.x - (q.x + ox), dy = me.y - (q.y + oy);
-                vx_nn3_insert_bf(d1, d2, d3, fmaf(dx, dx, dy * dy));
+                const float dx = me.x - q.x, dy = me.y - q.y;
+                vx_nn3_insert_bf(d1, d2, d3, qq == t ? 1e5f : fmaf(dx, dx, dy * dy));
             }
         }
+#pragma unroll
+        for (int ring = 0; ring < 2; ++ring) {   // the edge neighbours, then the corners
+            unsigned want[4];
+            int off[4], count = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int ddx = ring ? (e & 1 ? 1 : -1) : (e == 0 ? -1 : (e == 1 ? 1 : 0));
+                const int ddy = ring ? (e & 2 ? 1 : -1) : (e == 2 ? -1 : (e == 3 ? 1 : 0));
+                // in quarters of the leaf frame: a quarter X of it spans
+                // [(X - 1) hq, X hq]
+                const int X = (int)(key & 1) + ddx, Y = (int)((key >> 1) & 1) + ddy;
+                const float gx = fmaxf(fmaxf((float)(X - 1) * hq - me.x, me.x - (float)X * hq), 0.0f);
+                const float gy = fmaxf(fmaxf((float)(Y - 1) * hq - me.y, me.y - (float)Y * hq), 0.0f);
+                const bool need = valid && 2 * col + X >= 0 && 2 * col + X < 2 * m && 2 * row + Y >= 0 &&
+                                  2 * row + Y < 2 * m && !(fmaf(gx, gx, gy * gy) > 1.0001f * d3);
+                want[e] = __ballot_sync(0xffffffffu, need);
+                off[e] = count + __popc(want[e] & before);
+                count += __popc(want[e]);
+                if (need) pairs[off[e]] = (unsigned char)(lane | e << 5);
+            }
+            __syncwarp();
+            for (int base = 0; base < count; base += 32) {
+                const bool mine = base + lane < count;
+                const int pr = mine ? pairs[base + lane] : 0, src = pr & 31, e = pr >> 5;
+                const float tx = __shfl_sync(0xffffffffu, me.x, src), ty = __shfl_sync(0xffffffffu, me.y, src);
+                const unsigned tk = __shfl_sync(0xffffffffu, key, src);
+                float f1 = 1e5f, f2 = 1e5f, f3 = 1e5f;
+                if (mine) {
+                    const int ddx = ring ? (e & 1 ? 1 : -1) : (e == 0 ? -1 : (e == 1 ? 1 : 0));
+                    const int ddy = ring ? (e & 2 ? 1 : -1) : (e == 2 ? -1 : (e == 3 ? 1 : 0));
+                    const int X = (int)(tk & 1) + ddx, Y = (int)((tk >> 1) & 1) + ddy;   // -1 .. 2
+                    const int lx = X >> 1, ly = Y >> 1;                                  // leaves off: -1, 0, 1
+                    const float ox = (float)lx * hf, oy = (float)ly * hf;
+                    const int k = 4 * ((int)(tk >> 2) + ly * m + lx) + 2 * (Y & 1) + (X & 1);
+                    const int q1 = substart[k + 1];
+#pragma unroll 2
+                    for (int qq = substart[k]; qq < q1; ++qq) {
+                        const float2 q = *reinterpret_cast<const float2 *>(srt + qq);
+                        const float dx = tx - (q.x + ox), dy = ty - (q.y + oy);
+                        vx_nn3_insert_bf(f1, f2, f3, fmaf(dx, dx, dy * dy));
+                    }
+                }
+#pragma unroll
+                for (int o = 0; o < 4; ++o) {
+                    if (want[o] == 0u) continue;
+                    const int from = off[o] - base;
+                    const float e1 = __shfl_sync(0xffffffffu, f1, from & 31);
+                    const float e2 = __shfl_sync(0xffffffffu, f2, from & 31);
+                    const float e3 = __shfl_sync(0xffffffffu, f3, from & 31);
+                    if ((want[o] >> lane & 1u) && from >= 0 && from < 32) {
+                        vx_nn3_insert_bf(d1, d2, d3, e1);
+                        vx_nn3_insert_bf(d1, d2, d3, e2);
+                        vx_nn3_insert_bf(d1, d2, d3, e3);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        if (!valid) continue;
         v.d[j] = (double)((sqrtf(d1) + sqrtf(d2) + sqrtf(d3)) / 3);
         if (!(d3 < sq2)) {   // a closer source could lie outside the 3x3 quarters
             const int slot = atomicAdd(&S->fnflag, 1);
@@ -1257,7 +1344,7 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
     vx_launch<k_fmm_near<P>, k_fmm_near_body<P>>(L, L.num_sms * 8, FMM_T, 0, p, v, S, w.srt, sorted, w.fmm_start,
                                                  w.items, (const cplx *)w.fmm_L);
     VX_EV(L, 1);
-    vx_launch<k_fmm_nn3_sub, k_fmm_nn3_sub_body>(L, grid, FMM_T, 0, v, S, w.srt, skey, sorted,
+    vx_launch<k_fmm_nn3_sub, k_fmm_nn3_sub_body>(L, grid * 2, FMM_T, 0, v, S, w.srt, skey, sorted,
                                                  (const int *)w.fmm_sub_start, w.fmm_flags);
 
     vx_launch<k_fmm_nn3_fix, k_fmm_nn3_fix_body>(L, grid, FMM_T, 0, v, S, w.srt, sorted, w.fmm_start, w.fmm_flags, w.fmm_brute);
