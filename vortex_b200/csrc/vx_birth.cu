@@ -674,19 +674,22 @@ __device__ __forceinline__ float vx_half_log_ratio(float r0, float r1, float num
     return 0.5f * logf(r1 / r0);
 }
 
-// Direct FP32 panel terms over the near list (chunked like k_rhs_partial).
-VX_DEVK void k_rhs_near_body(VxBlkB<RHS_T, 8> vb, const VxScalars *S, const vx_panel *pan, int P, int P32,
-                             const float4 *near, double *part, int sms) {
-    const int nchunks = vx_rhs_chunks(S->n0, P, sms, false);   // from the body's own count
-    __shared__ float4 sq4[RHS_T];   // (x, y, G, unused)
-    const long long nn = S->bf_nnear;
-    const long long cs = vx_ceil_div(vx_ceil_div(nn, nchunks), RHS_T) * RHS_T;
-    const int tiles = (P + RHS_T - 1) / RHS_T;
+// Direct FP32 panel terms over the near list (chunked like k_rhs_partial):
+// the sum over a chunk in source order for each panel, by LP lanes a panel.
+// They compute the terms of LP sources at a time and all add them up in
+// order (a shuffle and a product more per term), so the bits do not depend
+// on LP.
+template <int LP>
+__device__ __forceinline__ void rhs_near_items(VxBlkB<RHS_T, 8> vb, const vx_panel *pan, int P, int P32,
+                                               const float4 *near, double *part, long long nn, long long cs,
+                                               int nchunks, float4 *sq4) {
+    constexpr int TP = RHS_T / LP;   // panels of an item
+    const int tiles = (P + TP - 1) / TP, sub = threadIdx.x % LP;
     const long long items = (long long)tiles * nchunks;
     for (long long it = vb.x; it < items; it += vb.n) {
         const int pt = (int)(it % tiles);
         const long long sc = it / tiles;
-        const int i = pt * RHS_T + threadIdx.x;
+        const int i = pt * TP + threadIdx.x / LP;
         const bool valid = i < P;
         float al0 = 0, al1 = 0, d0 = 1, d1 = 0;
         if (valid) {
@@ -703,8 +706,8 @@ VX_DEVK void k_rhs_near_body(VxBlkB<RHS_T, 8> vb, const VxScalars *S, const vx_p
             if (j < j1) sq4[threadIdx.x] = near[j];
             __syncthreads();
             const int cnt = (int)min((long long)RHS_T, j1 - jt);
-            for (int q = 0; q < cnt; ++q) {
-                const float4 src = sq4[q];
+            for (int q = 0; q < cnt; q += LP) {
+                const float4 src = sq4[LP == 1 ? q : min(q + sub, cnt - 1)];
                 float s00 = al0 - src.x, s01 = al1 - src.y;
                 float s10 = s00 + d0, s11 = s01 + d1;
                 float A = fmaf(s00, d0, s01 * d1);
@@ -713,15 +716,44 @@ VX_DEVK void k_rhs_near_body(VxBlkB<RHS_T, 8> vb, const VxScalars *S, const vx_p
                 float alpha = vx_atan2_bulk(-dd2 * z, fmaf(z, z, A * B));
                 float r1 = fmaf(s10, s10, s11 * s11), r0 = fmaf(s00, s00, s01 * s01);
                 float beta = vx_half_log_ratio(r0, r1, fmaf(2.0f, A, dd2));
-                y0 = fmaf(src.z, fmaf(alpha, d0, beta * kd0), y0);
-                y1 = fmaf(src.z, fmaf(alpha, d1, beta * kd1), y1);
+                const float t0 = fmaf(alpha, d0, beta * kd0), t1 = fmaf(alpha, d1, beta * kd1);
+                if (LP == 1) {
+                    y0 = fmaf(src.z, t0, y0);
+                    y1 = fmaf(src.z, t1, y1);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < LP; ++u) {
+                        const float v0 = __shfl_sync(0xffffffffu, t0, u, LP), v1 = __shfl_sync(0xffffffffu, t1, u, LP);
+                        const float g = __shfl_sync(0xffffffffu, src.z, u, LP);
+                        if (q + u < cnt) {
+                            y0 = fmaf(g, v0, y0);
+                            y1 = fmaf(g, v1, y1);
+                        }
+                    }
+                }
             }
         }
-        if (valid) {
+        if (valid && sub == 0) {
             part[(sc * P32 + i) * 2 + 0] = (double)y0;
             part[(sc * P32 + i) * 2 + 1] = (double)y1;
         }
     }
+}
+// Bound: the terms' some 50 instructions where (panel tile, chunk) items fill
+// the GPU; with fewer, a thread's serial walk over its chunk (384 sources at
+// 2e4 vortices), so the panels are given more lanes as long as the grid has
+// blocks for them: 53 -> 16 us at 1000 vortices, 31 -> 13 at 2e4; 72 at 1e6,
+// where one lane a panel fills the GPU.
+VX_DEVK void k_rhs_near_body(VxBlkB<RHS_T, 8> vb, const VxScalars *S, const vx_panel *pan, int P, int P32,
+                             const float4 *near, double *part, int sms) {
+    __shared__ float4 sq4[RHS_T];   // (x, y, G, unused)
+    const int nchunks = vx_rhs_chunks(S->n0, P, sms, false);   // from the body's own count
+    const long long nn = S->bf_nnear;
+    const long long cs = vx_ceil_div(vx_ceil_div(nn, nchunks), RHS_T) * RHS_T;
+    const long long full = nn > 0 ? vx_ceil_div(nn, cs) * ((P + RHS_T - 1) / RHS_T) : 0;   // items with sources
+    if (8 * full <= vb.n) rhs_near_items<8>(vb, pan, P, P32, near, part, nn, cs, nchunks, sq4);
+    else if (4 * full <= vb.n) rhs_near_items<4>(vb, pan, P, P32, near, part, nn, cs, nchunks, sq4);
+    else rhs_near_items<1>(vb, pan, P, P32, near, part, nn, cs, nchunks, sq4);
 }
 __global__ void __launch_bounds__(RHS_T) k_rhs_near(const VxScalars *S, const vx_panel *pan, int P, int P32,
                                                     const float4 *near, double *part, int sms) {
@@ -855,7 +887,9 @@ cudaError_t vx_launch_birth(const VxLaunch &L, const VxParams &p, const VxView &
         const int gb = std::min(VX_BF_MAX_BLOCKS, 2 * L.num_sms);
         vx_launch<k_bf_far, k_bf_far_body>(L, gb, BF_T, 0, p, v, S, w.bf_part, w.bf_cnt, sms, w.bf_off, w.bf_coef);
         vx_launch<k_bf_scatter, k_bf_scatter_body>(L, gb, BF_T, 0, p, v, S, w.bf_off, w.bf_near, sms);
-        vx_launch<k_rhs_near, k_rhs_near_body>(L, grid, RHS_T, 0, S, pan, P, P32, w.bf_near, w.rhs_part, sms);
+        // up to 8 lanes a panel, where its own blocks leave room for them
+        const int gn = (int)std::min((long long)vx_ceil_div(P, RHS_T) * rhs_chunks * 8, 16LL * (L.rec ? L.num_sms : sms));
+        vx_launch<k_rhs_near, k_rhs_near_body>(L, gn, RHS_T, 0, S, pan, P, P32, w.bf_near, w.rhs_part, sms);
     } else if (p.prec == VX_PREC_FP32) {
         vx_launch<k_rhs_partial<float>, k_rhs_partial_body<float>>(L, grid, RHS_T, 0, v, S, pan, P, P32, w.rhs_part, sms);
     } else {
