@@ -120,7 +120,6 @@ VX_DEVK void k_cg_prep_body(VxBlkB<CG_T, 0> vb, const VxView &v, VxScalars *S, d
     if (threadIdx.x != 0) return;
     S->cnwide = 0;
     S->cnhuge = 0;
-    S->bk_nmid = S->bk_nbig = 0;
     S->cnitems = 0;
     if (n == 0) { S->cncells = 0; S->cnx = S->cny = 0; return; }
     const double x0 = vx_dunkey(k[0]), x1 = -vx_dunkey(k[1]);
@@ -846,8 +845,7 @@ cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, cons
     gt.v = v;
     gt.S = S;
     gt.srt = w.srt;
-    vx_bucket_order(L, S, &S->n, &S->cncells, w.key0, w.val0, w.cg_start, w.key1, w.val1, w.bk_mid, w.bk_big,
-                    w.val0, gt);
+    vx_bucket_order(L, &S->n, w.key0, w.val0, w.cg_start, w.key1, w.val1, vx_order_rec(w), gt);
     const unsigned *skey = w.key1;
     const int *sorted = w.val1;
     vx_launch<k_cg_items, k_cg_items_body>(L, grid, VX_SCAN_T, 0, S, w.cg_start, w.items, w.items_cap, w.scan_tiles);

@@ -306,7 +306,7 @@ static vx_status work_alloc_impl(VxWork &w, std::vector<void *> *allocs, long lo
     A(w.cmp.hole_pos, cap); A(w.cmp.hole_src, cap); A(w.cmp.tail_src, cap);
     A(w.cmp.hx, cap); A(w.cmp.hy, cap); A(w.cmp.hg, cap); A(w.cmp.tx, cap); A(w.cmp.ty, cap);
     w.cells_cap = std::max(4 * cap, 65536LL);
-    A(w.cellid, cap); A(w.cell_start, w.cells_cap + 1); A(w.sorted, cap);
+    A(w.cellid, cap); A(w.cell_start, w.cells_cap + 1);
     // the collapse grid's cell counts are zero between rounds (the scan that
     // reads them zeroes them), and so are the per-candidate arrays, so they
     // start at zero
@@ -334,7 +334,7 @@ static vx_status work_alloc_impl(VxWork &w, std::vector<void *> *allocs, long lo
     A(w.srt, cap);
     w.items_cap = cap / 32 + w.cells_cap + 2;
     A(w.items, w.items_cap);
-    A(w.cg_wide, cap); A(w.cg_huge, cap); A(w.bk_mid, cap / 16 + 2); A(w.bk_big, cap / 128 + 2);
+    A(w.cg_wide, cap); A(w.cg_huge, cap);
     // quadtree of the bulk-form Biot-Savart
     w.fmm_lmax = vx_fmm_max_level(cap);
     A(w.fmm_cnt, vx_fmm_cells(w.fmm_lmax));

@@ -109,7 +109,6 @@ VX_DEVK void k_fmm_prep_body(VxBlkB<FMM_T, 0> vb, const VxView &v, VxScalars *S,
     S->fsq = 0;
     S->fnflag = 0;
     S->fnbrute = 0;
-    S->bk_nmid = S->bk_nbig = 0;
     const double x0 = vx_dunkey(k[0]), x1 = -vx_dunkey(k[1]);
     const double y0 = vx_dunkey(k[2]), y1 = -vx_dunkey(k[3]);
     double side = fmax(x1 - x0, y1 - y0);
@@ -1315,8 +1314,7 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
     gt.v = v;
     gt.S = S;
     gt.srt = w.srt;
-    vx_bucket_order(L, S, &S->fs, &S->fnsub, w.key0, w.val0, w.fmm_sub_start, w.key1, w.val1,
-                    w.bk_mid, w.bk_big, w.val0, gt);
+    vx_bucket_order(L, &S->fs, w.key0, w.val0, w.fmm_sub_start, w.key1, w.val1, vx_order_rec(w), gt);
     const unsigned *skey = w.key1;
     const int *sorted = w.val1;
     // upward pass: P2M + M2M of the 2 levels above the leaves, then the

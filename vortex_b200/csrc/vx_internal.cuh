@@ -97,7 +97,6 @@ struct VxScalars {
     long long fnsub;       // cells of the level below the leaves (4 per leaf): the 3-nearest grid
     int fL, fnflag;
     int fnbrute;           // flagged targets left to the whole-set 3-nearest scan
-    int bk_nmid, bk_nbig;  // buckets of 17..128 / more elements in the running bucket order (vx_sort.cu)
     long long fcnt_off;    // offset of the leaf level in the quadtree's count array
     unsigned long long fsq;   // sum over the quarter-leaf cells of count^2 at the last tree build (depth rule)
     int fLcap;                // deepest level the depth rule may deepen to (0: none): set when a deepened tree
@@ -135,7 +134,7 @@ struct VxWork {
     VxCompact cmp;
     // collapse
     long long cells_cap;
-    int *cellid, *cell_cnt, *cell_start, *sorted;
+    int *cellid, *cell_cnt, *cell_start;
     int *col, *in_cnt, *has_app, *first_app, *cand, *cstate, *cdec;
     double *mx, *my, *mg;
     // pair partial sums
@@ -165,7 +164,6 @@ struct VxWork {
     long long items_cap;
     int *cg_wide;            // sorted slots of the diffusion targets summed one warp each
     int *cg_huge;            // sorted slots of those summed one block each
-    int *bk_mid, *bk_big;    // buckets of 17..128 / more than 128 elements (vx_bucket_order)
     // quadtree: counts and expansions of every level up to fmm_lmax
     int fmm_lmax;
     int *fmm_cnt, *fmm_start, *fmm_flags, *fmm_brute;
@@ -862,7 +860,7 @@ struct VxGather {
     const VxScalars *S = nullptr;
     float4 *srt = nullptr;
 };
-__device__ __forceinline__ void vx_gather_slot(const VxGather &gt, long long k, long long j, unsigned b) {
+__device__ __forceinline__ float4 vx_gather(const VxGather &gt, long long j, unsigned b) {
     const VxScalars *S = gt.S;
     const VxView &v = gt.v;
     if (gt.mode == 1) {
@@ -870,23 +868,31 @@ __device__ __forceinline__ void vx_gather_slot(const VxGather &gt, long long k, 
         const double h = S->fside / (double)m;
         const unsigned leaf = b >> 2, col = leaf % m, row = leaf / m;
         const double ccx = S->fx0 + ((double)col + 0.5) * h, ccy = S->fy0 + ((double)row + 0.5) * h;
-        gt.srt[k] = make_float4((float)(v.x[j * v.ps] - ccx), (float)(v.y[j * v.ps] - ccy),
-                                j < S->n ? (float)v.g[j * v.ps] : 0.0f, (float)col);
-    } else if (gt.mode == 2) {
-        const long long nx = S->cnx;
-        const double ccx = S->cx0 + ((double)(b % nx) + 0.5) * S->ch, ccy = S->cy0 + ((double)(b / nx) + 0.5) * S->chy;
-        gt.srt[k] = make_float4((float)(v.x[j * v.ps] - ccx), (float)(v.y[j * v.ps] - ccy), (float)v.g[j * v.ps],
-                                (float)v.d[j]);
+        return make_float4((float)(v.x[j * v.ps] - ccx), (float)(v.y[j * v.ps] - ccy),
+                           j < S->n ? (float)v.g[j * v.ps] : 0.0f, (float)col);
     }
+    const unsigned nx = (unsigned)S->cnx;
+    const double ccx = S->cx0 + ((double)(b % nx) + 0.5) * S->ch, ccy = S->cy0 + ((double)(b / nx) + 0.5) * S->chy;
+    return make_float4((float)(v.x[j * v.ps] - ccx), (float)(v.y[j * v.ps] - ccy), (float)v.g[j * v.ps],
+                       (float)v.d[j]);
 }
+// A slot's element, its bucket and what is kept of it, before the elements
+// of a bucket are in order (32 bytes, one DRAM sector, written by one thread).
+struct __align__(32) VxOrderRec {
+    float4 val;
+    unsigned key;
+    int idx, unused0, unused1;
+};
+// A body's records: the pair kernels' partial-sum buffer, which the bulk
+// grids leave unused (at least 5 doubles a slot).
+inline VxOrderRec *vx_order_rec(const VxWork &w) { return reinterpret_cast<VxOrderRec *>(w.part); }
 // Stable order by bucket from each element's bucket, its rank in it (any order:
 // what counting the buckets returned) and the buckets' starts: (okey, oval)
 // = keys and element indices in bucket order, elements of a bucket in index
-// order, and the gather of gt at each element's final slot (vx_sort.cu).
-// scratch: n ints (rank may be used).
-cudaError_t vx_bucket_order(const VxLaunch &L, VxScalars *S, const long long *d_n, const long long *d_nbuckets,
-                            const unsigned *key, const int *rank, const int *start, unsigned *okey, int *oval,
-                            int *mid, int *big, int *scratch, const VxGather &gt = VxGather());
+// order, and the gather of gt at each element's slot (vx_sort.cu).
+cudaError_t vx_bucket_order(const VxLaunch &L, const long long *d_n, const unsigned *key, const int *rank,
+                            const int *start, unsigned *okey, int *oval, VxOrderRec *rec,
+                            const VxGather &gt = VxGather());
 int vx_fmm_max_level(long long cap);
 long long vx_fmm_cells(int lmax);         // cells of all levels 0..lmax
 constexpr int VX_BF_P = 48;          // terms of the birth far-field expansion
