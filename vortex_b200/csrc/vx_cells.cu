@@ -106,7 +106,7 @@ VX_DEVK void k_cg_prep_body(VxBlkB<CG_T, 0> vb, const VxView &v, VxScalars *S, d
             red[part] = dsum;
         }
     }
-    if (!vx_last_block(&S->sync_ctr, vb.n)) return;
+    if (!vx_last_block(&S->sync_side, vb.n)) return;
     unsigned long long k[4] = {~0ull, ~0ull, ~0ull, ~0ull};
     double dpart = 0.0;
     for (int b = threadIdx.x; b < nparts; b += CG_T) {
@@ -831,12 +831,18 @@ __global__ void __launch_bounds__(WIDE_T) k_diff_huge(VxParams p, VxView v, VxSc
 cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                                       VxWork &w) {
     const int grid = L.num_sms * 4;
+    // the grid is built beside the near field of the same step (whose arrays it
+    // leaves alone: its order takes the places of the unordered keys, its
+    // sources those of the direct sums) where the body has a side stream
+    VxLaunch B = L;
+    if (L.side) B.stream = L.side;
+    float4 *srt = w.src32;
     // partitions of the mean spacing follow the body's count on the device
     // (vx_body_parts), the grid the SMs this launch is given
-    vx_launch<k_cg_prep, k_cg_prep_body>(L, std::min(VX_RED_BLOCKS, L.num_sms * 4), CG_T, 0, v, S, w.red, w.box,
+    vx_launch<k_cg_prep, k_cg_prep_body>(B, std::min(VX_RED_BLOCKS, L.num_sms * 4), CG_T, 0, v, S, w.red, w.box,
                                          vx_full_sms(L), p.diff_cutoff, w.cells_cap);
-    vx_launch<k_cg_cellid, k_cg_cellid_body>(L, grid, CG_T, 0, v, S, w.key0, w.val0, w.cg_cnt);
-    vx_launch<k_cg_scan, k_cg_scan_body>(L, grid, VX_SCAN_T, 0, S, w.cg_cnt, w.cg_start, w.scan_tiles);
+    vx_launch<k_cg_cellid, k_cg_cellid_body>(B, grid, CG_T, 0, v, S, w.key0, w.val0, w.cg_cnt);
+    vx_launch<k_cg_scan, k_cg_scan_body>(B, grid, VX_SCAN_T, 0, S, w.cg_cnt, w.cg_start, w.scan_tiles);
 
     // cell order: each cell's vortices in index order (a stable sort by cell),
     // the FP32 sources gathered at their slots on the way
@@ -844,20 +850,21 @@ cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, cons
     gt.mode = 2;
     gt.v = v;
     gt.S = S;
-    gt.srt = w.srt;
-    vx_bucket_order(L, &S->n, w.key0, w.val0, w.cg_start, w.key1, w.val1, vx_order_rec(w), gt);
-    const unsigned *skey = w.key1;
-    const int *sorted = w.val1;
-    vx_launch<k_cg_items, k_cg_items_body>(L, grid, VX_SCAN_T, 0, S, w.cg_start, w.items, w.items_cap, w.scan_tiles);
+    gt.srt = srt;
+    vx_bucket_order(B, &S->n, w.key0, w.val0, w.cg_start, w.key0, w.val0, vx_order_rec(w), gt);
+    const unsigned *skey = w.key0;
+    const int *sorted = w.val0;
+    vx_launch<k_cg_items, k_cg_items_body>(B, grid, VX_SCAN_T, 0, S, w.cg_start, w.items, w.items_cap, w.scan_tiles);
 
+    vx_join(L);
     VX_EV(L, 2);
     // blocks: one per item of a body whose items are split over 8 warps (64 a
     // 2048 vortices); in a batch the other members' blocks fill the GPU too
-    vx_launch<k_diff_cells, k_diff_cells_body>(L, std::min(vx_full_sms(L) * 8, L.num_sms * (L.rec ? 16 : 64)), CG_T, 0, p, v, S, w.srt, skey, sorted, w.cg_start, w.items, w.cg_wide);
+    vx_launch<k_diff_cells, k_diff_cells_body>(vx_full_dependency(L), std::min(vx_full_sms(L) * 8, L.num_sms * (L.rec ? 16 : 64)), CG_T, 0, p, v, S, srt, skey, sorted, w.cg_start, w.items, w.cg_wide);
 
-    vx_launch<k_diff_wide, k_diff_wide_body>(L, std::min(vx_full_sms(L) * 4, L.num_sms * (L.rec ? 4 : 16)), CG_T, 0, p, v, S, w.srt, skey, sorted, w.cg_start, w.cg_wide, w.cg_huge);
+    vx_launch<k_diff_wide, k_diff_wide_body>(L, std::min(vx_full_sms(L) * 4, L.num_sms * (L.rec ? 4 : 16)), CG_T, 0, p, v, S, srt, skey, sorted, w.cg_start, w.cg_wide, w.cg_huge);
 
-    vx_launch<k_diff_huge, k_diff_huge_body>(L, L.num_sms * 2, WIDE_T, 0, p, v, S, w.srt, skey, sorted, w.cg_start, w.cg_huge);
+    vx_launch<k_diff_huge, k_diff_huge_body>(L, L.num_sms * 2, WIDE_T, 0, p, v, S, srt, skey, sorted, w.cg_start, w.cg_huge);
 
     VX_EV(L, 3);
     return cudaGetLastError();

@@ -338,6 +338,8 @@ static vx_status work_alloc_impl(VxWork &w, std::vector<void *> *allocs, long lo
     // quadtree of the bulk-form Biot-Savart
     w.fmm_lmax = vx_fmm_max_level(cap);
     A(w.fmm_cnt, vx_fmm_cells(w.fmm_lmax));
+    w.fitems_cap = cap / 32 + (1LL << (2 * w.fmm_lmax)) + 2;
+    A(w.fitems, w.fitems_cap);
     A(w.fmm_start, (1LL << (2 * w.fmm_lmax)) + 1);
     A(w.fmm_flags, cap); A(w.fmm_brute, cap);
     A(w.fmm_sub_cnt, 1LL << (2 * (w.fmm_lmax + 1)));
@@ -580,6 +582,14 @@ extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t
     cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(VX_ERR_CUDA);
     vx_params_from_conf(conf, pan, (int)P, &s->prm);
+    if (s->prm.prec == VX_PREC_FP32 && s->conf.fmm) {
+        // the side work's launches go first where both have blocks waiting
+        int lo = 0, hi = 0;
+        cudaDeviceGetStreamPriorityRange(&lo, &hi);
+        if (cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, hi) != cudaSuccess) return fail(VX_ERR_CUDA);
+        for (auto &e : s->side_ev)
+            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(VX_ERR_CUDA);
+    }
     PanelLists wall, hit;
     build_wall_lists(s->prm, pan, (int)P, wall);
     build_hit_lists(s->prm, pan, (int)P, hit);
@@ -674,6 +684,9 @@ extern "C" vx_status vx_destroy(vx_sim *s) {
     if (s->d_pred) cudaFree(s->d_pred);
     for (auto &e : s->ev) if (e) cudaEventDestroy(e);
     for (auto &e : s->pev) if (e) cudaEventDestroy(e);
+    for (auto &e : s->side_ev)
+        if (e) cudaEventDestroy(e);
+    if (s->side) cudaStreamDestroy(s->side);
     if (s->stream) cudaStreamDestroy(s->stream);
     vx_trim_pool(s->device);
     delete s;
@@ -988,6 +1001,13 @@ static cudaError_t launch_stages(vx_sim *s, unsigned mask, bool whole_step, VxRe
     const bool timed = s->timing && !whole_step && !rec;
     if (timed)
         for (int k = 0; k < 4; ++k) L.pair_ev[k] = s->pev[k];
+    // stages or kernels that are timed one by one run one after the other
+    const bool bulk = p.prec == VX_PREC_FP32 && s->conf.fmm;
+    if (s->side && bulk && (mask & VX_STAGE_VELOCITY) && !rec && !timed && !s->kt) {
+        L.side = s->side;
+        L.ev_fork = s->side_ev[0];
+        L.ev_join = s->side_ev[1];
+    }
     auto ev = [&](int k) { if (timed) cudaEventRecord(s->ev[k], s->stream); };
     ev(0);
     if (mask & VX_STAGE_BIRTH) {
@@ -997,15 +1017,21 @@ static cudaError_t launch_stages(vx_sim *s, unsigned mask, bool whole_step, VxRe
     ev(1);
     if (mask & VX_STAGE_VELOCITY) {
         // bulk form: quadtree FMM (vx_fmm.cu); plain form: direct sum
-        if (p.prec == VX_PREC_FP32 && s->conf.fmm)
+        if (bulk)
             e = vx_launch_velocity_fmm(L, p, v, s->d_S, s->w);
         else
             e = vx_launch_velocity(L, p, v, s->d_S, s->w);
+        // joined by the bulk diffusion once its grid is built (vx_cells.cu)
+        if (!(mask & VX_STAGE_DIFFUSION) || !(p.diff_cutoff > 0.0) || e != cudaSuccess) {
+            vx_join(L);
+            L.side = nullptr;
+        }
         if (e != cudaSuccess) return e;
     }
     ev(2);
     if (mask & VX_STAGE_DIFFUSION)
         if ((e = vx_launch_diffusion(L, p, v, s->d_S, s->w)) != cudaSuccess) return e;
+    L.side = nullptr;
     ev(3);
     if (mask & VX_STAGE_WALL)
         if ((e = vx_launch_wall(L, p, v, s->d_S, s->d_pan, s->d_wstart, s->d_widx)) != cudaSuccess) return e;

@@ -109,6 +109,8 @@ struct VxScalars {
     // tile ticket, finished-block count and epoch (all at rest between
     // launches: the counters at zero, the epoch advanced once per scan)
     unsigned sync_ctr, scan_ticket, scan_done, scan_epoch;
+    unsigned sync_side;   // sync_ctr of the kernels that may run beside others of the body (VxLaunch::side)
+    long long fnitems;    // near-field work items
 };
 
 enum {
@@ -162,6 +164,8 @@ struct VxWork {
     float4 *srt;
     int2 *items;             // (row, first sorted slot) of each target segment
     long long items_cap;
+    int2 *fitems;            // (leaf, first sorted slot) of each near-field target segment
+    long long fitems_cap;
     int *cg_wide;            // sorted slots of the diffusion targets summed one warp each
     int *cg_huge;            // sorted slots of those summed one block each
     // quadtree: counts and expansions of every level up to fmm_lmax
@@ -733,11 +737,37 @@ struct VxLaunch {
     // optional events recorded around the Biot-Savart and diffusion pair
     // kernels: [0,1] Biot-Savart, [2,3] diffusion (null: not recorded)
     cudaEvent_t pair_ev[4] = {nullptr, nullptr, nullptr, nullptr};
+    // second stream of the body, for work beside the main one between
+    // vx_fork and vx_join (null: everything on `stream`)
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    bool pdl = true;       // false: a full dependency on the work before (the first launch after a fork or join)
     // recording instead of launching (multi-body steps), per-kernel timing
     VxRecorder *rec = nullptr;
     VxKernelTimer *kt = nullptr;
 };
 inline int vx_full_sms(const VxLaunch &L) { return L.full_sms > 0 ? L.full_sms : L.num_sms; }
+// The launch context of the side stream, which waits for what `stream` holds
+// so far (L itself without a side stream); and the main one's wait for it.
+inline VxLaunch vx_fork(const VxLaunch &L) {
+    VxLaunch B = L;
+    if (L.side) {
+        cudaEventRecord(L.ev_fork, L.stream);
+        cudaStreamWaitEvent(L.side, L.ev_fork, 0);
+        B.stream = L.side;
+    }
+    return B;
+}
+inline void vx_join(const VxLaunch &L) {
+    if (!L.side) return;
+    cudaEventRecord(L.ev_join, L.side);
+    cudaStreamWaitEvent(L.stream, L.ev_join, 0);
+}
+inline VxLaunch vx_full_dependency(const VxLaunch &L) {
+    VxLaunch F = L;
+    if (L.side) F.pdl = false;
+    return F;
+}
 #define VX_EV(L, k) do { if ((L).pair_ev[k] && !(L).rec) cudaEventRecord((L).pair_ev[k], (L).stream); } while (0)
 
 // Launch kernel K (the __global__ wrapper of body DEV) for one body: with
@@ -781,7 +811,7 @@ struct VxLauncher<K, DEV, void (*)(VxBlkB<MAXT, MINB>, A0...)> {
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = L.pdl ? 1 : 0;
         const cudaError_t e = cudaLaunchKernelEx(&cfg, K, static_cast<vx_arg_t<A0>>(args)...);
         if (L.kt) {
             cudaEventRecord(eb, L.stream);
