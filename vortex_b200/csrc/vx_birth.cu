@@ -270,21 +270,48 @@ cudaError_t vx_build_matrix(const VxLaunch &L, const vx_panel *d_pan, int P, dou
 }
 
 // ---------------------------------------------------------------------------
-// Step begin: V_inf ramp (src/main.c:654-659) and the pre-birth count.
-VX_DEVK void k_step_begin_body(VxBlkB<0, 0> vb, VxScalars *S) {
-    if (S->step < S->incr_steps) {
-        S->vinf[0] += S->dvinf[0];
-        S->vinf[1] += S->dvinf[1];
+// Place of panel q's new vortex (src/kernel.cu:862-872).
+__device__ __forceinline__ void vx_birth_place(const VxView &v, const vx_panel &q, int mode, long long slot) {
+    const double mx = (q.left[0] + q.right[0]) / 2, my = (q.left[1] + q.right[1]) / 2;
+    double bx, by;
+    if (mode == VX_BIRTH_FILE) {
+        bx = q.birth[0]; by = q.birth[1];
+    } else if (mode == VX_BIRTH_HALF_PANEL) {
+        const double h = 0.5 * q.length;
+        bx = mx + h * q.norm[0]; by = my + h * q.norm[1];
+    } else {
+        bx = mx + 1e-6 * q.norm[0]; by = my + 1e-6 * q.norm[1];
     }
-    S->n0 = S->n;
-}
-__global__ void k_step_begin(VxScalars *S) {
-    VX_PDL_WAIT();
-    k_step_begin_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, S);
+    v.x[slot * v.ps] = bx;
+    v.y[slot * v.ps] = by;
 }
 
-cudaError_t vx_launch_step_begin(const VxLaunch &L, VxScalars *S) {
-    vx_launch<k_step_begin, k_step_begin_body>(L, 1, 1, 0, S);
+// Step begin, one block: V_inf ramp (src/main.c:654-659), the pre-birth
+// count, and the new vortices' places, which follow from the panels alone (so
+// that the quadtree can be begun while their strengths are solved for).
+constexpr int BEGIN_T = 1024;
+VX_DEVK void k_step_begin_body(VxBlkB<BEGIN_T, 0> vb, const VxView &v, VxScalars *S, const vx_panel *pan, int P,
+                               int mode) {
+    const long long n0 = S->n;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (S->step < S->incr_steps) {
+            S->vinf[0] += S->dvinf[0];
+            S->vinf[1] += S->dvinf[1];
+        }
+        S->n0 = n0;
+        S->n = n0 + P;
+    }
+    for (int i = threadIdx.x; i < P; i += BEGIN_T) vx_birth_place(v, pan[i], mode, n0 + i);
+}
+__global__ void __launch_bounds__(BEGIN_T) k_step_begin(VxView v, VxScalars *S, const vx_panel *pan, int P, int mode) {
+    VX_PDL_WAIT();
+    k_step_begin_body(VxBlkB<BEGIN_T, 0>{blockIdx.x, gridDim.x}, v, S, pan, P, mode);
+}
+
+cudaError_t vx_launch_step_begin(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
+                                 const vx_panel *pan) {
+    vx_launch<k_step_begin, k_step_begin_body>(L, 1, BEGIN_T, 0, v, S, pan, p.P, p.birth_mode);
     return cudaGetLastError();
 }
 
@@ -765,12 +792,11 @@ __global__ void __launch_bounds__(RHS_T) k_rhs_near(const VxScalars *S, const vx
 // coef) adds Re[I_far (tau_x + i tau_y) / (2 pi i dz)] with dz = zb - za.
 // One warp per panel: its lanes sum the chunk partials, and two terms each of
 // the far field's series, (z - c)^(l + 1) by squaring, by fixed butterflies (one
-// lane's chain of 48 products and divisions: 1000 panels 22 -> 12 us).  The panel's new
-// vortex gets its place here (src/kernel.cu:862-872); its strength follows
-// from the gamma solve.
+// lane's chain of 48 products and divisions: 1000 panels 22 -> 12 us).  place: the
+// panel's new vortex gets its place here (no step began before).
 VX_DEVK void k_rhs_final_body(VxBlkB<128, 0> vb, const VxView &v, const VxScalars *S, const vx_panel *pan, int P,
                               int P32, const double *part, int sms, double *R, const VxParams &p,
-                              const double *coef) {
+                              const double *coef, int place) {
     const int nchunks = vx_rhs_chunks(S->n0, P, sms, p.prec == VX_PREC_FP64);   // from the body's own count
     const int i = (int)((vb.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (i >= P) return;
@@ -821,25 +847,13 @@ VX_DEVK void k_rhs_final_body(VxBlkB<128, 0> vb, const VxView &v, const VxScalar
         w -= (Ii * qr - Ir * qi) / qq;
     }
     R[i] = -((u + S->vinf[0]) * pan[i].tang[0] + (w + S->vinf[1]) * pan[i].tang[1]);
-    const double mx = (l0 + r0) / 2, my = (l1 + r1) / 2;
-    double bx, by;
-    if (p.birth_mode == VX_BIRTH_FILE) {
-        bx = pan[i].birth[0]; by = pan[i].birth[1];
-    } else if (p.birth_mode == VX_BIRTH_HALF_PANEL) {
-        const double h = 0.5 * pan[i].length;
-        bx = mx + h * pan[i].norm[0]; by = my + h * pan[i].norm[1];
-    } else {
-        bx = mx + 1e-6 * pan[i].norm[0]; by = my + 1e-6 * pan[i].norm[1];
-    }
-    const long long k = (S->n0 + i) * v.ps;
-    v.x[k] = bx;
-    v.y[k] = by;
+    if (place) vx_birth_place(v, pan[i], p.birth_mode, S->n0 + i);
 }
 __global__ void __launch_bounds__(128) k_rhs_final(VxView v, const VxScalars *S, const vx_panel *pan, int P, int P32,
                                                    const double *part, int sms, double *R, VxParams p,
-                                                   const double *coef) {
+                                                   const double *coef, int place) {
     VX_PDL_WAIT();
-    k_rhs_final_body(VxBlkB<128, 0>{blockIdx.x, gridDim.x}, v, S, pan, P, P32, part, sms, R, p, coef);
+    k_rhs_final_body(VxBlkB<128, 0>{blockIdx.x, gridDim.x}, v, S, pan, P, P32, part, sms, R, p, coef, place);
 }
 
 // gamma_i = sum_j M_ij R_j + M_iP dg: a warp per row (row stride ld), lanes
@@ -849,7 +863,7 @@ __global__ void __launch_bounds__(128) k_rhs_final(VxView v, const VxScalars *S,
 // neighbour too, so every gamma must be final).
 constexpr int GAM_T = 256;
 VX_DEVK void k_gamma_body(VxBlkB<GAM_T, 0> vb, const VxView &v, VxScalars *S, const vx_panel *pan, const double *M,
-                          long long ld, int P, const double *R, double *gamma) {
+                          long long ld, int P, const double *R, double *gamma, int place) {
     const int lane = threadIdx.x & 31;
     const int i = (vb.x * blockDim.x + threadIdx.x) >> 5;
     if (i < P) {
@@ -867,16 +881,16 @@ VX_DEVK void k_gamma_body(VxBlkB<GAM_T, 0> vb, const VxView &v, VxScalars *S, co
         const int in = (int)pan[q].n_of_rpanel;
         v.g[(n0 + q) * v.ps] = 0.5 * (__ldcg(&gamma[q]) * pan[q].length + __ldcg(&gamma[in]) * pan[in].length);
     }
-    if (threadIdx.x == 0) S->n = n0 + P;
+    if (place && threadIdx.x == 0) S->n = n0 + P;
 }
 __global__ void __launch_bounds__(GAM_T) k_gamma(VxView v, VxScalars *S, const vx_panel *pan, const double *M,
-                                                 long long ld, int P, const double *R, double *gamma) {
+                                                 long long ld, int P, const double *R, double *gamma, int place) {
     VX_PDL_WAIT();
-    k_gamma_body(VxBlkB<GAM_T, 0>{blockIdx.x, gridDim.x}, v, S, pan, M, ld, P, R, gamma);
+    k_gamma_body(VxBlkB<GAM_T, 0>{blockIdx.x, gridDim.x}, v, S, pan, M, ld, P, R, gamma, place);
 }
 
 cudaError_t vx_launch_birth(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
-                            const vx_panel *pan, const double *minv, long long ld, int rhs_chunks) {
+                            const vx_panel *pan, const double *minv, long long ld, int rhs_chunks, bool place) {
     const int P = p.P, P32 = (int)vx_round32(P);
     const int T = p.prec == VX_PREC_FP64 ? rhs_t<double>() : RHS_T;
     const int grid = (int)std::min((long long)((P + T - 1) / T) * rhs_chunks,
@@ -895,8 +909,8 @@ cudaError_t vx_launch_birth(const VxLaunch &L, const VxParams &p, const VxView &
     } else {
         vx_launch<k_rhs_partial<double>, k_rhs_partial_body<double>>(L, grid, T, 0, v, S, pan, P, P32, w.rhs_part, sms);
     }
-    vx_launch<k_rhs_final, k_rhs_final_body>(L, (P + 3) / 4, 128, 0, v, S, pan, P, P32, w.rhs_part, sms, w.R, p, far ? w.bf_coef : nullptr);
-    vx_launch<k_gamma, k_gamma_body>(L, (int)vx_ceil_div(P, GAM_T / 32), GAM_T, 0, v, S, pan, minv, ld, P, w.R, w.gamma);
+    vx_launch<k_rhs_final, k_rhs_final_body>(L, (P + 3) / 4, 128, 0, v, S, pan, P, P32, w.rhs_part, sms, w.R, p, far ? w.bf_coef : nullptr, place ? 1 : 0);
+    vx_launch<k_gamma, k_gamma_body>(L, (int)vx_ceil_div(P, GAM_T / 32), GAM_T, 0, v, S, pan, minv, ld, P, w.R, w.gamma, place ? 1 : 0);
     return cudaGetLastError();
 }
 

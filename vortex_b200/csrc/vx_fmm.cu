@@ -93,7 +93,7 @@ VX_DEVK void k_fmm_prep_body(VxBlkB<FMM_T, 0> vb, const VxView &v, VxScalars *S,
     vx_block_min4<FMM_T / 32>(k);
     if (threadIdx.x == 0)
         for (int q = 0; q < 4; ++q) part[4 * vb.x + q] = k[q];
-    if (!vx_last_block(&S->sync_ctr, vb.n)) return;
+    if (!vx_last_block(&S->sync_side, vb.n)) return;
     for (int q = 0; q < 4; ++q) k[q] = ~0ull;
     for (unsigned b = threadIdx.x; b < vb.n; b += blockDim.x)
         for (int q = 0; q < 4; ++q) k[q] = min(k[q], __ldcg(&part[4 * b + q]));
@@ -1283,8 +1283,22 @@ int vx_fmm_max_level(long long cap) {
     return L;
 }
 
+cudaError_t vx_launch_fmm_tree(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w) {
+    const int grid = L.num_sms * 4;
+    const int Lmax = w.fmm_lmax;
+    const int pgrid = std::min(grid, VX_RED_BLOCKS);   // 4 box keys per block
+    vx_launch<k_fmm_prep, k_fmm_prep_body>(vx_full_dependency(L), pgrid, FMM_T, 0, v, S, p.eps, Lmax, p.fmm_leaf > 0 ? p.fmm_leaf : 32,
+                                           w.fmm_cnt, vx_fmm_cells(Lmax), w.fmm_sub_cnt, 1LL << (2 * (Lmax + 1)),
+                                           w.box);
+    vx_launch<k_fmm_leafid, k_fmm_leafid_body>(L, grid, FMM_T, 0, v, S, w.key0, w.val0, w.fmm_sub_cnt);
+    vx_launch<k_fmm_scan, k_fmm_scan_body>(L, grid, VX_SCAN_T, 0, S, w.fmm_sub_cnt, w.fmm_sub_start,
+                                           w.fmm_cnt, w.fmm_start, w.scan_tiles);
+    return cudaGetLastError();
+}
+
 template <int P>
-static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w) {
+static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
+                                bool built) {
     constexpr int M2L_T = m2l_threads<P>();
     constexpr size_t M2L_SMEM = sizeof(M2LShared<P>);
     if (M2L_SMEM > 48 * 1024 && !L.rec) {   // opt in to more than 48 KB of shared memory (once per device)
@@ -1299,13 +1313,7 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
     }
     const int grid = L.num_sms * 4;
     const int Lmax = w.fmm_lmax;
-    const int pgrid = std::min(grid, VX_RED_BLOCKS);   // 4 box keys per block
-    vx_launch<k_fmm_prep, k_fmm_prep_body>(L, pgrid, FMM_T, 0, v, S, p.eps, Lmax, p.fmm_leaf > 0 ? p.fmm_leaf : 32,
-                                           w.fmm_cnt, vx_fmm_cells(Lmax), w.fmm_sub_cnt, 1LL << (2 * (Lmax + 1)),
-                                           w.box);
-    vx_launch<k_fmm_leafid, k_fmm_leafid_body>(L, grid, FMM_T, 0, v, S, w.key0, w.val0, w.fmm_sub_cnt);
-    vx_launch<k_fmm_scan, k_fmm_scan_body>(L, grid, VX_SCAN_T, 0, S, w.fmm_sub_cnt, w.fmm_sub_start,
-                                           w.fmm_cnt, w.fmm_start, w.scan_tiles);
+    if (!built) vx_launch_fmm_tree(L, p, v, S, w);
     // source order: by quarter-leaf, each quarter's sources in index order
     // (a stable sort by the key 4 leaf + child; each leaf stays contiguous),
     // the FP32 sources gathered at their slots on the way
@@ -1314,7 +1322,7 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
     gt.v = v;
     gt.S = S;
     gt.srt = w.srt;
-    vx_bucket_order(L, &S->fs, w.key0, w.val0, w.fmm_sub_start, w.key1, w.val1, vx_order_rec(w), gt);
+    vx_bucket_order(built ? vx_full_dependency(L) : L, &S->fs, w.key0, w.val0, w.fmm_sub_start, w.key1, w.val1, vx_order_rec(w), gt);
     const unsigned *skey = w.key1;
     const int *sorted = w.val1;
     vx_launch<k_fmm_items, k_fmm_items_body>(L, grid, VX_SCAN_T, 0, S, w.fmm_start, w.fitems, w.fitems_cap, w.scan_tiles);
@@ -1355,11 +1363,11 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
 }
 
 cudaError_t vx_launch_velocity_fmm(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
-                                   VxWork &w) {
+                                   VxWork &w, bool built) {
     switch (p.fmm_p) {
-    case 8: return velocity_fmm<8>(L, p, v, S, w);
-    case 12: return velocity_fmm<12>(L, p, v, S, w);
-    case 20: return velocity_fmm<20>(L, p, v, S, w);
-    default: return velocity_fmm<16>(L, p, v, S, w);
+    case 8: return velocity_fmm<8>(L, p, v, S, w, built);
+    case 12: return velocity_fmm<12>(L, p, v, S, w, built);
+    case 20: return velocity_fmm<20>(L, p, v, S, w, built);
+    default: return velocity_fmm<16>(L, p, v, S, w, built);
     }
 }

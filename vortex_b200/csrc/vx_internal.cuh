@@ -827,12 +827,14 @@ inline cudaError_t vx_launch(const VxLaunch &L, dim3 grid, dim3 block, size_t sm
 
 
 // Stage launchers (each returns the first CUDA error it saw).
-cudaError_t vx_launch_step_begin(const VxLaunch &L, VxScalars *S);
+cudaError_t vx_launch_step_begin(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
+                                 const vx_panel *pan);
 // minv: the inverted panel system, row stride ld; rhs_chunks: the source
 // chunks the host expects, for the grid only
+// place: the new vortices get their places and are counted here (else by the step's begin)
 cudaError_t vx_launch_birth(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                             VxWork &w, const vx_panel *pan, const double *minv, long long ld,
-                            int rhs_chunks);
+                            int rhs_chunks, bool place);
 cudaError_t vx_launch_velocity(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                                VxWork &w);
 cudaError_t vx_launch_diffusion(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
@@ -928,8 +930,11 @@ long long vx_fmm_cells(int lmax);         // cells of all levels 0..lmax
 constexpr int VX_BF_P = 48;          // terms of the birth far-field expansion
 constexpr double VX_BF_RHO = 1.5;    // far-field sources lie beyond VX_BF_RHO body radii of its centre
 constexpr int VX_BF_MAX_BLOCKS = 1024;
+// The quadtree from the positions alone (box, depth, quarter counts and
+// starts); velocity_fmm begins with it unless `built`.
+cudaError_t vx_launch_fmm_tree(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w);
 cudaError_t vx_launch_velocity_fmm(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
-                                   VxWork &w);
+                                   VxWork &w, bool built);
 cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                                       VxWork &w);
 void vx_work_free(VxWork &w, std::vector<void *> &allocs, cudaStream_t stream = nullptr);

@@ -71,7 +71,9 @@ cudaError_t vx_bucket_order(const VxLaunch &L, const long long *d_n, const unsig
                             const int *start, unsigned *okey, int *oval, VxOrderRec *rec, const VxGather &gt) {
     const int grid = L.num_sms * 8;
     vx_launch<k_bk_place, k_bk_place_body>(L, grid, 256, 0, d_n, key, rank, start, rec, gt);
-    vx_launch<k_bk_order, k_bk_order_body>(L, grid, 256, 0, d_n, (const VxOrderRec *)rec, start, okey, oval, gt.mode ? gt.srt : nullptr);
+    VxLaunch next = L;
+    next.pdl = true;
+    vx_launch<k_bk_order, k_bk_order_body>(next, grid, 256, 0, d_n, (const VxOrderRec *)rec, start, okey, oval, gt.mode ? gt.srt : nullptr);
     return cudaGetLastError();
 }
 

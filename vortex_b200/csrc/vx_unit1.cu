@@ -309,7 +309,7 @@ int vort_creation(vxu_vortex *pos, double (*V_infDev)[2], size_t n_of_birth, siz
     ++U.launches;
     const int chunks = vx_rhs_chunks((long long)n, (int)n_of_birth, U.num_sms, U.prm.prec == VX_PREC_FP64);
     CK(vx_launch_birth(launch0(), U.prm, aos_view(pos, nullptr, nullptr), U.d_S, U.w, panels, M_Dev,
-                          (long long)n_of_birth_BLOCK_S + 1, chunks));
+                          (long long)n_of_birth_BLOCK_S + 1, chunks, true));
     CK(cudaDeviceSynchronize());
     return 0;
 }
