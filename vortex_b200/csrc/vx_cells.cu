@@ -844,6 +844,7 @@ cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, cons
     vx_launch<k_cg_cellid, k_cg_cellid_body>(B, grid, CG_T, 0, v, S, w.key0, w.val0, w.cg_cnt);
     vx_launch<k_cg_scan, k_cg_scan_body>(B, grid, VX_SCAN_T, 0, S, w.cg_cnt, w.cg_start, w.scan_tiles);
 
+    vx_launch<k_cg_items, k_cg_items_body>(B, grid, VX_SCAN_T, 0, S, w.cg_start, w.items, w.items_cap, w.scan_tiles);
     // cell order: each cell's vortices in index order (a stable sort by cell),
     // the FP32 sources gathered at their slots on the way
     VxGather gt;
@@ -851,10 +852,10 @@ cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, cons
     gt.v = v;
     gt.S = S;
     gt.srt = srt;
-    vx_bucket_order(B, &S->n, w.key0, w.val0, w.cg_start, w.key0, w.val0, vx_order_rec(w), gt);
+    if (L.ev_born) cudaStreamWaitEvent(B.stream, L.ev_born, 0);   // strengths from here on
+    vx_bucket_order(L.ev_born ? vx_full_dependency(B) : B, &S->n, w.key0, w.val0, w.cg_start, w.key0, w.val0, vx_order_rec(w), gt);
     const unsigned *skey = w.key0;
     const int *sorted = w.val0;
-    vx_launch<k_cg_items, k_cg_items_body>(B, grid, VX_SCAN_T, 0, S, w.cg_start, w.items, w.items_cap, w.scan_tiles);
 
     vx_join(L);
     VX_EV(L, 2);

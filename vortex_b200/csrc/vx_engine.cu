@@ -340,6 +340,7 @@ static vx_status work_alloc_impl(VxWork &w, std::vector<void *> *allocs, long lo
     A(w.fmm_cnt, vx_fmm_cells(w.fmm_lmax));
     w.fitems_cap = cap / 32 + (1LL << (2 * w.fmm_lmax)) + 2;
     A(w.fitems, w.fitems_cap);
+    A(w.born, P32);
     A(w.fmm_start, (1LL << (2 * w.fmm_lmax)) + 1);
     A(w.fmm_flags, cap); A(w.fmm_brute, cap);
     A(w.fmm_sub_cnt, 1LL << (2 * (w.fmm_lmax + 1)));
@@ -583,10 +584,8 @@ extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(VX_ERR_CUDA);
     vx_params_from_conf(conf, pan, (int)P, &s->prm);
     if (s->prm.prec == VX_PREC_FP32 && s->conf.fmm) {
-        // the side work's launches go first where both have blocks waiting
-        int lo = 0, hi = 0;
-        cudaDeviceGetStreamPriorityRange(&lo, &hi);
-        if (cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, hi) != cudaSuccess) return fail(VX_ERR_CUDA);
+        // (a higher priority than the main stream's made no difference)
+        if (cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking) != cudaSuccess) return fail(VX_ERR_CUDA);
         for (auto &e : s->side_ev)
             if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(VX_ERR_CUDA);
     }
@@ -1012,20 +1011,32 @@ static cudaError_t launch_stages(vx_sim *s, unsigned mask, bool whole_step, VxRe
     ev(0);
     if (mask & VX_STAGE_BIRTH) {
         if ((e = vx_launch_step_begin(L, p, v, s->d_S, s->d_pan)) != cudaSuccess) return e;
-        // the quadtree needs the new vortices' places, not their strengths, so
-        // its start runs beside the birth's sums (a step of 2e4 vortices 257 ->
-        // 243 us, of 1e6 2215 -> 2198)
-        if (L.side) e = vx_launch_fmm_tree(vx_fork(L), p, v, s->d_S, s->w);
+        // the quadtree's order, the 3 nearest and the diffusion grid up to
+        // its sources need the new vortices' places, not their strengths, so
+        // they run beside the birth's sums (all side work together, a step and
+        // its share of the copies in and out of 8 / 4 / 2 steps at 2e4 / 1e6 /
+        // 3e6 vortices: 296 -> 236, 2260 -> 2190, 7390 -> 7210 us)
+        if (L.side) {
+            L.ev_tree = s->side_ev[2];
+            L.ev_born = s->side_ev[3];
+            const VxLaunch B = vx_fork(L);
+            e = vx_launch_fmm_tree(B, p, v, s->d_S, s->w, true);
+            cudaEventRecord(L.ev_tree, B.stream);
+            if (e == cudaSuccess) e = vx_launch_fmm_nn3(B, v, s->d_S, s->w);
+        }
         const cudaError_t eb = vx_launch_birth(L, p, v, s->d_S, s->w, s->d_pan, s->d_minv, (long long)s->P + 1, rhs_chunks_for(s), false);
-        vx_join(L);
+        if (L.side) cudaEventRecord(L.ev_born, L.stream);
         if (e == cudaSuccess) e = eb;
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            vx_join(L);
+            return e;
+        }
     }
     ev(1);
     if (mask & VX_STAGE_VELOCITY) {
         // bulk form: quadtree FMM (vx_fmm.cu); plain form: direct sum
         if (bulk)
-            e = vx_launch_velocity_fmm(L, p, v, s->d_S, s->w, L.side && (mask & VX_STAGE_BIRTH));
+            e = vx_launch_velocity_fmm(L, p, v, s->d_S, s->w, L.ev_tree != nullptr);
         else
             e = vx_launch_velocity(L, p, v, s->d_S, s->w);
         // joined by the bulk diffusion once its grid is built (vx_cells.cu)

@@ -1283,17 +1283,50 @@ int vx_fmm_max_level(long long cap) {
     return L;
 }
 
-cudaError_t vx_launch_fmm_tree(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w) {
+cudaError_t vx_launch_fmm_tree(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
+                               bool early) {
     const int grid = L.num_sms * 4;
     const int Lmax = w.fmm_lmax;
     const int pgrid = std::min(grid, VX_RED_BLOCKS);   // 4 box keys per block
-    vx_launch<k_fmm_prep, k_fmm_prep_body>(vx_full_dependency(L), pgrid, FMM_T, 0, v, S, p.eps, Lmax, p.fmm_leaf > 0 ? p.fmm_leaf : 32,
+    vx_launch<k_fmm_prep, k_fmm_prep_body>(early ? vx_full_dependency(L) : L, pgrid, FMM_T, 0, v, S, p.eps, Lmax, p.fmm_leaf > 0 ? p.fmm_leaf : 32,
                                            w.fmm_cnt, vx_fmm_cells(Lmax), w.fmm_sub_cnt, 1LL << (2 * (Lmax + 1)),
                                            w.box);
     vx_launch<k_fmm_leafid, k_fmm_leafid_body>(L, grid, FMM_T, 0, v, S, w.key0, w.val0, w.fmm_sub_cnt);
     vx_launch<k_fmm_scan, k_fmm_scan_body>(L, grid, VX_SCAN_T, 0, S, w.fmm_sub_cnt, w.fmm_sub_start,
                                            w.fmm_cnt, w.fmm_start, w.scan_tiles);
+    // source order: by quarter-leaf, each quarter's sources in index order
+    // (a stable sort by the key 4 leaf + child; each leaf stays contiguous),
+    // the FP32 sources gathered at their slots on the way
+    VxGather gt;
+    gt.mode = 1;
+    gt.v = v;
+    gt.S = S;
+    gt.srt = w.srt;
+    gt.born = early ? w.born : nullptr;
+    vx_bucket_order(L, &S->fs, w.key0, w.val0, w.fmm_sub_start, w.key1, w.val1, vx_order_rec(w), gt);
+    vx_launch<k_fmm_items, k_fmm_items_body>(L, grid, VX_SCAN_T, 0, S, w.fmm_start, w.fitems, w.fitems_cap, w.scan_tiles);
     return cudaGetLastError();
+}
+
+cudaError_t vx_launch_fmm_nn3(const VxLaunch &L, const VxView &v, VxScalars *S, VxWork &w) {
+    const int grid = L.num_sms * 4;
+    vx_launch<k_fmm_nn3_sub, k_fmm_nn3_sub_body>(L, grid * 2, FMM_T, 0, v, S, w.srt, w.key1, w.val1,
+                                                 (const int *)w.fmm_sub_start, w.fmm_flags);
+    VxLaunch next = L;
+    next.pdl = true;
+    vx_launch<k_fmm_nn3_fix, k_fmm_nn3_fix_body>(next, grid, FMM_T, 0, v, S, w.srt, w.val1, w.fmm_start, w.fmm_flags, w.fmm_brute);
+    return cudaGetLastError();
+}
+
+// The new vortices' strengths in the quadtree's order, once they are known.
+VX_DEVK void k_fmm_born_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalars *S, const int *born, float4 *srt) {
+    const long long n0 = S->n0, m = S->n - n0;
+    for (long long i = vb.x * (long long)blockDim.x + threadIdx.x; i < m; i += (long long)vb.n * blockDim.x)
+        srt[born[i]].z = (float)v.g[(n0 + i) * v.ps];
+}
+__global__ void k_fmm_born(VxView v, const VxScalars *S, const int *born, float4 *srt) {
+    VX_PDL_WAIT();
+    k_fmm_born_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, born, srt);
 }
 
 template <int P>
@@ -1313,29 +1346,21 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
     }
     const int grid = L.num_sms * 4;
     const int Lmax = w.fmm_lmax;
-    if (!built) vx_launch_fmm_tree(L, p, v, S, w);
-    // source order: by quarter-leaf, each quarter's sources in index order
-    // (a stable sort by the key 4 leaf + child; each leaf stays contiguous),
-    // the FP32 sources gathered at their slots on the way
-    VxGather gt;
-    gt.mode = 1;
-    gt.v = v;
-    gt.S = S;
-    gt.srt = w.srt;
-    vx_bucket_order(built ? vx_full_dependency(L) : L, &S->fs, w.key0, w.val0, w.fmm_sub_start, w.key1, w.val1, vx_order_rec(w), gt);
-    const unsigned *skey = w.key1;
     const int *sorted = w.val1;
-    vx_launch<k_fmm_items, k_fmm_items_body>(L, grid, VX_SCAN_T, 0, S, w.fmm_start, w.fitems, w.fitems_cap, w.scan_tiles);
     // The 3 nearest (and, in a step, the diffusion grid's build after them)
     // share nothing with the expansions and the near field but what is built
     // above, so they run beside them where the body has a side stream: they
     // are short launches, bound by latency, that fill what the others leave.
     // One after the other, velocity and diffusion of 1000 / 30 000 vortices
     // took 148 / 257 us, a step of 2e4 / 1e6 290 / 2260; so 127 / 229, 257 / 2215.
-    const VxLaunch B = vx_fork(L);
-    vx_launch<k_fmm_nn3_sub, k_fmm_nn3_sub_body>(vx_full_dependency(B), grid * 2, FMM_T, 0, v, S, w.srt, skey, sorted,
-                                                 (const int *)w.fmm_sub_start, w.fmm_flags);
-    vx_launch<k_fmm_nn3_fix, k_fmm_nn3_fix_body>(B, grid, FMM_T, 0, v, S, w.srt, sorted, w.fmm_start, w.fmm_flags, w.fmm_brute);
+    if (!built) {
+        vx_launch_fmm_tree(L, p, v, S, w, false);
+        const VxLaunch B = vx_fork(L);
+        vx_launch_fmm_nn3(vx_full_dependency(B), v, S, w);
+    } else {
+        cudaStreamWaitEvent(L.stream, L.ev_tree, 0);
+        vx_launch<k_fmm_born, k_fmm_born_body>(vx_full_dependency(L), (int)vx_ceil_div(p.P, 256), 256, 0, v, S, (const int *)w.born, w.srt);
+    }
     // upward pass: P2M + M2M of the 2 levels above the leaves, then the
     // levels above those (two launches whatever the depth)
     const int gup = (int)std::min<long long>(grid * 4, 1LL << (2 * std::max(Lmax - 2, 0)));

@@ -164,6 +164,7 @@ struct VxWork {
     float4 *srt;
     int2 *items;             // (row, first sorted slot) of each target segment
     long long items_cap;
+    int *born;               // slots of the step's new vortices in the quadtree order
     int2 *fitems;            // (leaf, first sorted slot) of each near-field target segment
     long long fitems_cap;
     int *cg_wide;            // sorted slots of the diffusion targets summed one warp each
@@ -741,6 +742,9 @@ struct VxLaunch {
     // vx_fork and vx_join (null: everything on `stream`)
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // set in a step whose quadtree is begun before its birth is done: the tree's
+    // order on the side stream, the new strengths on the main one
+    cudaEvent_t ev_tree = nullptr, ev_born = nullptr;
     bool pdl = true;       // false: a full dependency on the work before (the first launch after a fork or join)
     // recording instead of launching (multi-body steps), per-kernel timing
     VxRecorder *rec = nullptr;
@@ -885,9 +889,11 @@ long long vx_work_bytes(long long cap, int P32, int num_sms, int fmm_p = VX_FMM_
 // j, bucket key b): nothing (mode 0), the quadtree's FP32 source (mode 1:
 // position relative to the centre of leaf b / 4, G masked beyond n, the
 // leaf's column), or the diffusion grid's (mode 2: position relative to the
-// centre of cell b, G, d).
+// centre of cell b, G, d).  born: the slots of the step's new vortices are
+// kept, whose strengths are not known yet (0 until k_fmm_born).
 struct VxGather {
     int mode = 0;
+    int *born = nullptr;
     VxView v = {};
     const VxScalars *S = nullptr;
     float4 *srt = nullptr;
@@ -901,7 +907,7 @@ __device__ __forceinline__ float4 vx_gather(const VxGather &gt, long long j, uns
         const unsigned leaf = b >> 2, col = leaf % m, row = leaf / m;
         const double ccx = S->fx0 + ((double)col + 0.5) * h, ccy = S->fy0 + ((double)row + 0.5) * h;
         return make_float4((float)(v.x[j * v.ps] - ccx), (float)(v.y[j * v.ps] - ccy),
-                           j < S->n ? (float)v.g[j * v.ps] : 0.0f, (float)col);
+                           j < (gt.born ? S->n0 : S->n) ? (float)v.g[j * v.ps] : 0.0f, (float)col);
     }
     const unsigned nx = (unsigned)S->cnx;
     const double ccx = S->cx0 + ((double)(b % nx) + 0.5) * S->ch, ccy = S->cy0 + ((double)(b / nx) + 0.5) * S->chy;
@@ -930,9 +936,12 @@ long long vx_fmm_cells(int lmax);         // cells of all levels 0..lmax
 constexpr int VX_BF_P = 48;          // terms of the birth far-field expansion
 constexpr double VX_BF_RHO = 1.5;    // far-field sources lie beyond VX_BF_RHO body radii of its centre
 constexpr int VX_BF_MAX_BLOCKS = 1024;
-// The quadtree from the positions alone (box, depth, quarter counts and
-// starts); velocity_fmm begins with it unless `built`.
-cudaError_t vx_launch_fmm_tree(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w);
+// The quadtree's order and its near-field items, from the positions and
+// (unless `early`: those of the step's new vortices) strengths; the 3
+// nearest.  velocity_fmm begins with both unless they are `built` (early).
+cudaError_t vx_launch_fmm_tree(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S, VxWork &w,
+                               bool early);
+cudaError_t vx_launch_fmm_nn3(const VxLaunch &L, const VxView &v, VxScalars *S, VxWork &w);
 cudaError_t vx_launch_velocity_fmm(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                                    VxWork &w, bool built);
 cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,

@@ -10,7 +10,7 @@ struct vx_sim {
     int num_sms = 148;
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;             // bulk form: work beside the main stream (VxLaunch::side)
-    cudaEvent_t side_ev[2] = {nullptr, nullptr};
+    cudaEvent_t side_ev[4] = {nullptr, nullptr, nullptr, nullptr};
     int P = 0, P32 = 0;
     VxParams prm;
     void *d_fixed = nullptr;     // one allocation: the panels, scalars, panel lists and inverse below

@@ -44,8 +44,9 @@ __global__ void k_bk_place(const long long *d_n, const unsigned *key, const int 
 }
 
 VX_DEVK void k_bk_order_body(VxBlkB<0, 0> vb, const long long *d_n, const VxOrderRec *rec, const int *start,
-                             unsigned *okey, int *oval, float4 *srt) {
+                             unsigned *okey, int *oval, float4 *srt, const VxScalars *born_of, int *born) {
     const long long n = *d_n;
+    const long long b0 = born ? born_of->n0 : 0, b1 = born ? born_of->n : 0;
     for (long long p = vb.x * (long long)blockDim.x + threadIdx.x; p < n;
          p += (long long)vb.n * blockDim.x) {
         const int2 ki = *reinterpret_cast<const int2 *>(&rec[p].key);
@@ -59,12 +60,13 @@ VX_DEVK void k_bk_order_body(VxBlkB<0, 0> vb, const long long *d_n, const VxOrde
         okey[p] = c;
         oval[to] = i;
         if (srt) srt[to] = q;
+        if (i >= b0 && i < b1) born[i - b0] = to;
     }
 }
 __global__ void k_bk_order(const long long *d_n, const VxOrderRec *rec, const int *start, unsigned *okey, int *oval,
-                           float4 *srt) {
+                           float4 *srt, const VxScalars *born_of, int *born) {
     VX_PDL_WAIT();
-    k_bk_order_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, d_n, rec, start, okey, oval, srt);
+    k_bk_order_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, d_n, rec, start, okey, oval, srt, born_of, born);
 }
 
 cudaError_t vx_bucket_order(const VxLaunch &L, const long long *d_n, const unsigned *key, const int *rank,
@@ -73,7 +75,7 @@ cudaError_t vx_bucket_order(const VxLaunch &L, const long long *d_n, const unsig
     vx_launch<k_bk_place, k_bk_place_body>(L, grid, 256, 0, d_n, key, rank, start, rec, gt);
     VxLaunch next = L;
     next.pdl = true;
-    vx_launch<k_bk_order, k_bk_order_body>(next, grid, 256, 0, d_n, (const VxOrderRec *)rec, start, okey, oval, gt.mode ? gt.srt : nullptr);
+    vx_launch<k_bk_order, k_bk_order_body>(next, grid, 256, 0, d_n, (const VxOrderRec *)rec, start, okey, oval, gt.mode ? gt.srt : nullptr, gt.S, gt.born);
     return cudaGetLastError();
 }
 
