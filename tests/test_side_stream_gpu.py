@@ -58,3 +58,30 @@ def test_stages_in_one_call(n):
         same(state(a), state(b))
     a.close()
     b.close()
+
+
+def test_batch_of_all_forms():
+    """Bodies whose steps have two branches, one branch (direct sums) and the
+    plain form in one batch: each as stepped alone."""
+    kinds = [dict(precision=N.PREC_FP32), dict(precision=N.PREC_FP32, fmm=0), dict(precision=N.PREC_FP64),
+             dict(precision=N.PREC_FP32, fmm_p=8), dict(precision=N.PREC_FP32, diff_cutoff=0.0, fmm=0)]
+
+    def build():
+        out = []
+        for k, kw in enumerate(kinds * 2):
+            sim = N.Sim(N.default_conf(**conf_kwargs(60 + 40 * k, **kw)), profiles.circle(60 + 40 * k))
+            sim.set_particles(*wake_cloud(300 + 700 * k, seed=k))
+            out.append(sim)
+        return out
+
+    alone, members = build(), build()
+    batch = N.Batch(members)
+    for steps in (1, 4):
+        batch.step(steps)
+        for s in alone:
+            s.step(steps)
+    batch.close()
+    for a, m in zip(alone, members):
+        same(state(a), state(m))
+        a.close()
+        m.close()

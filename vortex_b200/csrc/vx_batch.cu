@@ -75,6 +75,8 @@ struct Slot {
     std::vector<int> launch;      // index of the launch in each body's recording
     long long total = 0;          // blocks of all bodies
     size_t pack = 0;              // bytes of one argument pack
+    bool beside = false;          // on the step's second branch
+    unsigned await = 0, mark = 0; // the events of its launches (VX_EVT_*)
 };
 
 // What the instantiated graph holds for a slot.
@@ -83,6 +85,8 @@ struct SlotSig {
     unsigned bx;
     size_t smem;
     long long bound;
+    bool beside;
+    unsigned await, mark;
 };
 
 // What a batched step leaves of each member, gathered into one array that
@@ -113,6 +117,8 @@ struct vx_batch {
     int device = 0;
     int num_sms = 148;
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;            // the step's second branch, in its graph
+    cudaEvent_t side_ev[VX_EVTS] = {};
     std::vector<Body> bodies;
     int share_div = 1;
     std::vector<Slot> slots;
@@ -178,7 +184,7 @@ static vx_status merge(vx_batch *b) {
     using Key = std::pair<const void *, unsigned>;
     auto key_at = [&](int i, size_t q) {
         const VxRecLaunch &r = b->bodies[(size_t)i].rec.launches[q];
-        return Key(r.key, r.block.x);
+        return Key(r.key, r.block.x | (r.beside ? 1u << 31 : 0u));   // the branches share no slot
     };
     // the merged sequence (each entry a slot key with a stable id) and, per
     // body, the slot id of each of its launches
@@ -250,6 +256,7 @@ static vx_status merge(vx_batch *b) {
                 sl.many = r.many;
                 sl.block = r.block;
                 sl.pack = r.size;
+                sl.beside = r.beside;
             } else if (r.size != sl.pack || r.many != sl.many) {
                 vx_set_error("batch: one kernel recorded with different argument packs");
                 return VX_ERR_ARG;
@@ -258,6 +265,8 @@ static vx_status merge(vx_batch *b) {
             sl.bodies.push_back(i);
             sl.launch.push_back((int)q);
             sl.total += r.grid.x;
+            sl.await |= r.await;
+            sl.mark |= r.mark;
         }
     }
     return VX_OK;
@@ -331,23 +340,44 @@ static vx_status build_graph(vx_batch *b) {
     cudaGraph_t graph;
     BCU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = cudaSuccess;
+    // The step's second branch (VxLaunch::split) runs on the second stream.  A
+    // slot waits for the last of its events' slots so far: each member's own is
+    // among them or before them on that stream.  16 bodies of 1000 to 20 000
+    // vortices: 1240 -> 1125 us a step, copies in and out included.
+    unsigned marked = 0;
+    bool split = false;
     for (size_t j = 0; j < b->slots.size() && e == cudaSuccess; ++j) {
         const Slot &sl = b->slots[j];
-        SlotSig g{sl.many, sl.block.x, sl.smem, std::max<long long>(1, pow2_at_least(sl.total))};
+        SlotSig g{sl.many, sl.block.x, sl.smem, std::max<long long>(1, pow2_at_least(sl.total)), sl.beside, sl.await, sl.mark};
+        const cudaStream_t stream = sl.beside ? b->side : b->stream;
+        split |= sl.beside;
+        for (int k = 0; k < VX_EVTS && e == cudaSuccess; ++k)
+            if (sl.await & marked & (1u << k)) e = cudaStreamWaitEvent(stream, b->side_ev[k], 0);
+        if (e != cudaSuccess) break;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)g.bound);
         cfg.blockDim = sl.block;
         cfg.dynamicSmemBytes = sl.smem;
-        cfg.stream = b->stream;
+        cfg.stream = stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = sl.await ? 0 : 1;
         const VxSlot *slot = reinterpret_cast<const VxSlot *>(b->d_arena) + j;
         void *args[1] = {&slot};
         e = cudaLaunchKernelExC(&cfg, sl.many, args);
         b->sig.push_back(g);
+        for (int k = 0; k < VX_EVTS && e == cudaSuccess; ++k)
+            if (sl.mark & (1u << k)) {
+                e = cudaEventRecord(b->side_ev[k], stream);
+                marked |= 1u << k;
+            }
+    }
+    if (split) {
+        const cudaError_t r = cudaEventRecord(b->side_ev[VX_EVT_JOIN], b->side);
+        const cudaError_t w = cudaStreamWaitEvent(b->stream, b->side_ev[VX_EVT_JOIN], 0);
+        if (e == cudaSuccess) e = r != cudaSuccess ? r : w;
     }
     if (e == cudaSuccess) {
         const int nb = (int)b->bodies.size();
@@ -383,7 +413,9 @@ static bool graph_fits(const vx_batch *b) {
     for (size_t j = 0; j < b->slots.size(); ++j) {
         const SlotSig &g = b->sig[j];
         const Slot &sl = b->slots[j];
-        if (g.many != sl.many || g.bx != sl.block.x || sl.smem > g.smem || sl.total > g.bound) return false;
+        if (g.many != sl.many || g.bx != sl.block.x || sl.smem > g.smem || sl.total > g.bound || g.beside != sl.beside ||
+            g.await != sl.await || g.mark != sl.mark)
+            return false;
     }
     return true;
 }
@@ -453,6 +485,7 @@ static vx_status refresh(vx_batch *b) {
         const BodyKey k = key_of(b, bd.s);
         if (bd.recorded && k == bd.key) continue;
         bd.rec.launches.clear();
+        bd.rec.pending[0] = bd.rec.pending[1] = 0;
         bd.rec.arena.clear();
         const cudaError_t e = vx_sim_launch_stages(bd.s, VX_STAGE_ALL, true, &bd.rec, k.share);
         if (e != cudaSuccess) {
@@ -563,6 +596,9 @@ static void release(vx_batch *b) {
     }
     for (void *h : b->retired) cudaFreeHost(h);
     b->retired.clear();
+    for (cudaEvent_t &e : b->side_ev)
+        if (e) cudaEventDestroy(e);
+    if (b->side) cudaStreamDestroy(b->side);
     if (b->stream) cudaStreamDestroy(b->stream);
 }
 
@@ -617,6 +653,9 @@ extern "C" vx_status vx_batch_new(int device, vx_batch **out) {
     vx_keep_pool(device);
     cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(VX_ERR_CUDA);
+    if (cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess) return fail(VX_ERR_CUDA);
+    for (cudaEvent_t &e : b->side_ev)
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(VX_ERR_CUDA);
     for (int k = 0; k < 2; ++k)
         if (cudaEventCreateWithFlags(&b->stage_ev[k], cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&b->cnt_ev[k], cudaEventDisableTiming) != cudaSuccess)

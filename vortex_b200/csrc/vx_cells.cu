@@ -834,8 +834,7 @@ cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, cons
     // the grid is built beside the near field of the same step (whose arrays it
     // leaves alone: its order takes the places of the unordered keys, its
     // sources those of the direct sums) where the body has a side stream
-    VxLaunch B = L;
-    if (L.side) B.stream = L.side;
+    const VxLaunch B = vx_beside(L);
     float4 *srt = w.src32;
     // partitions of the mean spacing follow the body's count on the device
     // (vx_body_parts), the grid the SMs this launch is given
@@ -852,8 +851,8 @@ cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, cons
     gt.v = v;
     gt.S = S;
     gt.srt = srt;
-    if (L.ev_born) cudaStreamWaitEvent(B.stream, L.ev_born, 0);   // strengths from here on
-    vx_bucket_order(L.ev_born ? vx_full_dependency(B) : B, &S->n, w.key0, w.val0, w.cg_start, w.key0, w.val0, vx_order_rec(w), gt);
+    if (L.early) vx_await(B, VX_EVT_BORN);   // strengths from here on
+    vx_bucket_order(L.early ? vx_full_dependency(B) : B, &S->n, w.key0, w.val0, w.cg_start, w.key0, w.val0, vx_order_rec(w), gt);
     const unsigned *skey = w.key0;
     const int *sorted = w.val0;
 

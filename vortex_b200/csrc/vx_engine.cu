@@ -1002,11 +1002,9 @@ static cudaError_t launch_stages(vx_sim *s, unsigned mask, bool whole_step, VxRe
         for (int k = 0; k < 4; ++k) L.pair_ev[k] = s->pev[k];
     // stages or kernels that are timed one by one run one after the other
     const bool bulk = p.prec == VX_PREC_FP32 && s->conf.fmm;
-    if (s->side && bulk && (mask & VX_STAGE_VELOCITY) && !rec && !timed && !s->kt) {
-        L.side = s->side;
-        L.ev_fork = s->side_ev[0];
-        L.ev_join = s->side_ev[1];
-    }
+    L.split = bulk && (mask & VX_STAGE_VELOCITY) && (rec || s->side) && !timed && !L.kt;
+    L.side = s->side;
+    L.evts = s->side_ev;
     auto ev = [&](int k) { if (timed) cudaEventRecord(s->ev[k], s->stream); };
     ev(0);
     if (mask & VX_STAGE_BIRTH) {
@@ -1016,16 +1014,15 @@ static cudaError_t launch_stages(vx_sim *s, unsigned mask, bool whole_step, VxRe
         // they run beside the birth's sums (all side work together, a step and
         // its share of the copies in and out of 8 / 4 / 2 steps at 2e4 / 1e6 /
         // 3e6 vortices: 296 -> 236, 2260 -> 2190, 7390 -> 7210 us)
-        if (L.side) {
-            L.ev_tree = s->side_ev[2];
-            L.ev_born = s->side_ev[3];
+        if (L.split) {
+            L.early = true;
             const VxLaunch B = vx_fork(L);
             e = vx_launch_fmm_tree(B, p, v, s->d_S, s->w, true);
-            cudaEventRecord(L.ev_tree, B.stream);
+            vx_mark(B, VX_EVT_TREE);
             if (e == cudaSuccess) e = vx_launch_fmm_nn3(B, v, s->d_S, s->w);
         }
         const cudaError_t eb = vx_launch_birth(L, p, v, s->d_S, s->w, s->d_pan, s->d_minv, (long long)s->P + 1, rhs_chunks_for(s), false);
-        if (L.side) cudaEventRecord(L.ev_born, L.stream);
+        if (L.split) vx_mark(L, VX_EVT_BORN);
         if (e == cudaSuccess) e = eb;
         if (e != cudaSuccess) {
             vx_join(L);
@@ -1036,20 +1033,20 @@ static cudaError_t launch_stages(vx_sim *s, unsigned mask, bool whole_step, VxRe
     if (mask & VX_STAGE_VELOCITY) {
         // bulk form: quadtree FMM (vx_fmm.cu); plain form: direct sum
         if (bulk)
-            e = vx_launch_velocity_fmm(L, p, v, s->d_S, s->w, L.ev_tree != nullptr);
+            e = vx_launch_velocity_fmm(L, p, v, s->d_S, s->w, L.early);
         else
             e = vx_launch_velocity(L, p, v, s->d_S, s->w);
         // joined by the bulk diffusion once its grid is built (vx_cells.cu)
         if (!(mask & VX_STAGE_DIFFUSION) || !(p.diff_cutoff > 0.0) || e != cudaSuccess) {
             vx_join(L);
-            L.side = nullptr;
+            L.split = false;
         }
         if (e != cudaSuccess) return e;
     }
     ev(2);
     if (mask & VX_STAGE_DIFFUSION)
         if ((e = vx_launch_diffusion(L, p, v, s->d_S, s->w)) != cudaSuccess) return e;
-    L.side = nullptr;
+    L.split = false;
     ev(3);
     if (mask & VX_STAGE_WALL)
         if ((e = vx_launch_wall(L, p, v, s->d_S, s->d_pan, s->d_wstart, s->d_widx)) != cudaSuccess) return e;

@@ -1358,7 +1358,7 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
         const VxLaunch B = vx_fork(L);
         vx_launch_fmm_nn3(vx_full_dependency(B), v, S, w);
     } else {
-        cudaStreamWaitEvent(L.stream, L.ev_tree, 0);
+        vx_await(L, VX_EVT_TREE);
         vx_launch<k_fmm_born, k_fmm_born_body>(vx_full_dependency(L), (int)vx_ceil_div(p.P, 256), 256, 0, v, S, (const int *)w.born, w.srt);
     }
     // upward pass: P2M + M2M of the 2 levels above the leaves, then the

@@ -109,7 +109,7 @@ struct VxScalars {
     // tile ticket, finished-block count and epoch (all at rest between
     // launches: the counters at zero, the epoch advanced once per scan)
     unsigned sync_ctr, scan_ticket, scan_done, scan_epoch;
-    unsigned sync_side;   // sync_ctr of the kernels that may run beside others of the body (VxLaunch::side)
+    unsigned sync_side;   // sync_ctr of the kernels that may run beside others of the body (VxLaunch::split)
     long long fnitems;    // near-field work items
 };
 
@@ -680,22 +680,35 @@ __global__ void __launch_bounds__(MAXT, MINB) k_many_tb(const VxSlot *sd) {
 // A launch recorded instead of issued (building a multi-body step): the
 // single-body kernel (identity), its multi-body kernel, the shape and the
 // argument pack (bytes in the recorder's arena).
+// Points where the two branches of a step meet (VxLaunch::split).
+enum { VX_EVT_FORK, VX_EVT_JOIN, VX_EVT_TREE, VX_EVT_BORN, VX_EVTS };
 struct VxRecLaunch {
     const void *key;
     const void *many;
     dim3 grid, block;
     size_t smem;
     size_t off, size;
+    bool beside;           // on the second branch
+    unsigned await, mark;  // bits: events it waits for, events that are it
 };
 struct VxRecorder {
     std::vector<VxRecLaunch> launches;
     std::vector<unsigned char> arena;
+    unsigned pending[2] = {0, 0};   // waits of each branch's next launch
     void add(const void *key, const void *many, dim3 grid, dim3 block, size_t smem, const void *pack,
-             size_t size) {
+             size_t size, bool beside) {
         const size_t off = (arena.size() + 15) / 16 * 16;
         arena.resize(off + size);
         memcpy(arena.data() + off, pack, size);
-        launches.push_back(VxRecLaunch{key, many, grid, block, smem, off, size});
+        launches.push_back(VxRecLaunch{key, many, grid, block, smem, off, size, beside, pending[beside], 0u});
+        pending[beside] = 0;
+    }
+    void mark(bool beside, int ev) {   // the branch's last launch
+        for (size_t q = launches.size(); q-- > 0;)
+            if (launches[q].beside == beside) {
+                launches[q].mark |= 1u << ev;
+                return;
+            }
     }
 };
 
@@ -738,38 +751,54 @@ struct VxLaunch {
     // optional events recorded around the Biot-Savart and diffusion pair
     // kernels: [0,1] Biot-Savart, [2,3] diffusion (null: not recorded)
     cudaEvent_t pair_ev[4] = {nullptr, nullptr, nullptr, nullptr};
-    // second stream of the body, for work beside the main one between
-    // vx_fork and vx_join (null: everything on `stream`)
+    // A step's work may be split over two branches between vx_fork and
+    // vx_join: `beside` are the launches of the second one (on the stream
+    // `side`; a recording keeps the branch and the events with each launch).
+    // early: the quadtree is begun before the birth is done.
+    bool split = false, beside = false, early = false;
     cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    // set in a step whose quadtree is begun before its birth is done: the tree's
-    // order on the side stream, the new strengths on the main one
-    cudaEvent_t ev_tree = nullptr, ev_born = nullptr;
+    const cudaEvent_t *evts = nullptr;   // VX_EVTS
     bool pdl = true;       // false: a full dependency on the work before (the first launch after a fork or join)
     // recording instead of launching (multi-body steps), per-kernel timing
     VxRecorder *rec = nullptr;
     VxKernelTimer *kt = nullptr;
 };
 inline int vx_full_sms(const VxLaunch &L) { return L.full_sms > 0 ? L.full_sms : L.num_sms; }
-// The launch context of the side stream, which waits for what `stream` holds
-// so far (L itself without a side stream); and the main one's wait for it.
-inline VxLaunch vx_fork(const VxLaunch &L) {
+// An event after the branch's last launch; a wait for it before its next.
+inline void vx_mark(const VxLaunch &L, int ev) {
+    if (L.rec) L.rec->mark(L.beside, ev);
+    else cudaEventRecord(L.evts[ev], L.stream);
+}
+inline void vx_await(const VxLaunch &L, int ev) {
+    if (L.rec) L.rec->pending[L.beside] |= 1u << ev;
+    else cudaStreamWaitEvent(L.stream, L.evts[ev], 0);
+}
+// The second branch's launch context (L itself without one).
+inline VxLaunch vx_beside(const VxLaunch &L) {
     VxLaunch B = L;
-    if (L.side) {
-        cudaEventRecord(L.ev_fork, L.stream);
-        cudaStreamWaitEvent(L.side, L.ev_fork, 0);
+    if (L.split) {
+        B.beside = true;
         B.stream = L.side;
     }
     return B;
 }
+// The same after what L's branch holds so far; L's wait for the second one.
+inline VxLaunch vx_fork(const VxLaunch &L) {
+    const VxLaunch B = vx_beside(L);
+    if (L.split) {
+        vx_mark(L, VX_EVT_FORK);
+        vx_await(B, VX_EVT_FORK);
+    }
+    return B;
+}
 inline void vx_join(const VxLaunch &L) {
-    if (!L.side) return;
-    cudaEventRecord(L.ev_join, L.side);
-    cudaStreamWaitEvent(L.stream, L.ev_join, 0);
+    if (!L.split) return;
+    vx_mark(vx_beside(L), VX_EVT_JOIN);
+    vx_await(L, VX_EVT_JOIN);
 }
 inline VxLaunch vx_full_dependency(const VxLaunch &L) {
     VxLaunch F = L;
-    if (L.side) F.pdl = false;
+    if (L.split) F.pdl = false;
     return F;
 }
 #define VX_EV(L, k) do { if ((L).pair_ev[k] && !(L).rec) cudaEventRecord((L).pair_ev[k], (L).stream); } while (0)
@@ -797,7 +826,7 @@ struct VxLauncher<K, DEV, void (*)(VxBlkB<MAXT, MINB>, A0...)> {
         if (L.launches) ++*L.launches;
         if (L.rec) {
             const VxPack<vx_arg_t<A0>...> p = VxPackMake<vx_arg_t<A0>...>::make(static_cast<vx_arg_t<A0>>(args)...);
-            L.rec->add((const void *)K, many(), grid, block, smem, &p, sizeof(p));
+            L.rec->add((const void *)K, many(), grid, block, smem, &p, sizeof(p), L.beside);
             return cudaSuccess;
         }
         cudaEvent_t ea = nullptr, eb = nullptr;

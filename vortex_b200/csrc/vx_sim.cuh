@@ -9,8 +9,8 @@ struct vx_sim {
     int device = 0;
     int num_sms = 148;
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;             // bulk form: work beside the main stream (VxLaunch::side)
-    cudaEvent_t side_ev[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaStream_t side = nullptr;             // bulk form: work beside the main stream (VxLaunch::split)
+    cudaEvent_t side_ev[VX_EVTS] = {};
     int P = 0, P32 = 0;
     VxParams prm;
     void *d_fixed = nullptr;     // one allocation: the panels, scalars, panel lists and inverse below
