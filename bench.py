@@ -123,17 +123,14 @@ HBM_BYTES = {
     "k_fmm_leafid": (24, "read x, y; write leaf key and index"),
     "k_cg_prep": (24, "read x, y, d"),
     "k_cg_cellid": (24, "read x, y; write cell key and index"),
-    "k_bk_place": (12, "read key; write key and index at the bucket slot"),
-    "k_bk_order": (8, "read and write the bucket's indices"),
-    "k_fmm_gather": (48, "read order index and key, x, y, G; write float4"),
-    "k_cg_gather": (56, "read order index and key, x, y, G, d; write float4"),
+    "k_bk_place": (64, "read key, rank, x, y, G; write the 32-byte record at the bucket slot"),
+    "k_bk_order": (56, "read the record; write key, index and float4"),
     "k_col_prep": (16, "read x, y"),
     "k_col_count": (32, "read x, y; write cell id, in-count and the two merge flags"),
     "k_col_scatter": (64, "read cell id, cell start, x, y, G; write the 32-byte cell-sorted record"),
     "k_col_query<2>": (36, "read the cell-sorted record (x, y, G, index); write COL"),
     "k_col_query<1>": (36, "read the cell-sorted record (x, y, G, index); write COL"),
-    "k_cmp_count": (8, "read G"),
-    "k_cmp_classify": (8, "read G"),
+    "k_cmp_mark": (8, "read G"),
 }
 
 
