@@ -62,3 +62,29 @@ def test_collapse_of_weak(pas, n_col):
         xs, ys, gs, n = O.collapse(p, pas, xs, ys, gs, n)
         same(sim, xs, ys, gs, n)
     sim.close()
+
+
+@pytest.mark.parametrize("n_col", [1, 2, 3])
+@pytest.mark.parametrize("pas", [1, 2])
+def test_collapse_of_many(pas, n_col):
+    """In a store of more than 65536 slots a round with more than 1024 dead
+    leaves the moves to further launches, the second round's renaming too."""
+    rng = np.random.default_rng(7 + pas)
+    n, groups = 20000, 1500
+    cx, cy, k = rng.uniform(0.6, 3.0, groups), rng.normal(0, 0.4, groups), rng.integers(0, groups, n)
+    x, y = cx[k] + rng.normal(0, 0.004, n), cy[k] + rng.normal(0, 0.004, n)
+    g = rng.choice([1e-3, 2e-3, -1e-3], n)
+    ck = conf_kwargs(200, r_col_diff_sign=0.3, r_col_same_sign=0.25, max_ve_g=6e-3, n_col=n_col)
+    pan = profiles.circle(200)
+    sim = N.Sim(N.default_conf(**ck), pan)
+    p = oracle_params(pan, ck)
+    sim.set_particles(rng.uniform(1, 3, 70001), rng.uniform(-1, 1, 70001), np.full(70001, 1e-3))
+    xs, ys, gs = with_tail(x, y, g, extra=32)
+    sim.set_slots(xs, ys, gs, n)
+    for _ in range(2):
+        sim.stage("collapse1" if pas == 1 else "collapse2")
+        before = n
+        xs, ys, gs, n = O.collapse(p, pas, xs, ys, gs, n)
+        same(sim, xs, ys, gs, n)
+        assert _ == 1 or before - n > 2048
+    sim.close()

@@ -280,7 +280,8 @@ template <int PASS>
 VX_DEVK void k_col_settle_body(VxBlkB<1024, 0> vb, const VxView &v, VxScalars *S, const int *cand, int *col,
                                int *in_cnt, int *has_app, int *first_app, int *cstate, int *cdec, double *mx,
                                double *my, double *mg, const int *slot, ColRec *rec, double drop_eps, int track,
-                               const VxCompact &cmp) {
+                               const VxCompact &cmp, long long limit) {
+    if (threadIdx.x == 0) S->cmp_many = 0;
     if (S->col_done) return;
     __shared__ int undecided, listed;
     const int nc = S->ncand;
@@ -366,7 +367,7 @@ VX_DEVK void k_col_settle_body(VxBlkB<1024, 0> vb, const VxView &v, VxScalars *S
     // the round's compaction (none after a failed one); one that removes
     // nothing ends the pass
     const long long n0 = S->n;
-    const long long removed = vx_cmp_block<1024>(v, S, cmp, n0, n0, !failed, slot, track ? &rec[0].i : nullptr);
+    const long long removed = vx_cmp_block<1024>(v, S, cmp, n0, limit, !failed, slot, track ? &rec[0].i : nullptr);
     if (threadIdx.x == 0) {
         S->ncand = 0;
         S->nmoved = listed;
@@ -378,10 +379,11 @@ template <int PASS>
 __global__ void __launch_bounds__(1024) k_col_settle(VxView v, VxScalars *S, const int *cand, int *col,
                                                      int *in_cnt, int *has_app, int *first_app, int *cstate,
                                                      int *cdec, double *mx, double *my, double *mg, const int *slot,
-                                                     ColRec *rec, double drop_eps, int track, VxCompact cmp) {
+                                                     ColRec *rec, double drop_eps, int track, VxCompact cmp,
+                                                     long long limit) {
     VX_PDL_WAIT();
     k_col_settle_body<PASS>(VxBlkB<1024, 0>{blockIdx.x, gridDim.x}, v, S, cand, col, in_cnt, has_app, first_app,
-                            cstate, cdec, mx, my, mg, slot, rec, drop_eps, track, cmp);
+                            cstate, cdec, mx, my, mg, slot, rec, drop_eps, track, cmp, limit);
 }
 
 template <int PASS>
@@ -392,6 +394,7 @@ static cudaError_t collapse_pass(const VxLaunch &L, const VxParams &p, const VxV
     // the cell-sorted copy (32 bytes a vortex) lives in the pair kernels'
     // partial-sum buffer, unused by collapse (at least 5 doubles a slot)
     ColRec *rec = reinterpret_cast<ColRec *>(w.part);
+    const bool small = w.cap <= VX_CMP_SMALL;
     for (int cc = 0; cc < n_col; ++cc) {
         const int track = cc == 0 && n_col > 1;
         if (cc == 1) {
@@ -403,7 +406,8 @@ static cudaError_t collapse_pass(const VxLaunch &L, const VxParams &p, const VxV
             vx_launch<k_col_scatter, k_col_scatter_body>(L, grid, VX_THREADS, 0, v, S, w.cell_start, w.cellid, rec, p.drop_eps, w.cmp.bits);
             vx_launch<k_col_query<PASS>, k_col_query_body<PASS>>(L, grid, VX_THREADS, 0, p, S, w.cell_start, (const ColRec *)rec, w.col, w.cand);
         }
-        vx_launch<k_col_settle<PASS>, k_col_settle_body<PASS>>(L, 1, 1024, 0, v, S, w.cand, w.col, w.in_cnt, w.has_app, w.first_app, w.cstate, w.cdec, w.mx, w.my, w.mg, w.cellid, rec, p.drop_eps, track, w.cmp);
+        vx_launch<k_col_settle<PASS>, k_col_settle_body<PASS>>(L, 1, 1024, 0, v, S, w.cand, w.col, w.in_cnt, w.has_app, w.first_app, w.cstate, w.cdec, w.mx, w.my, w.mg, w.cellid, rec, p.drop_eps, track, w.cmp, small ? w.cap : VX_CMP_FEW);
+        if (!small) vx_launch_moves(L, v, S, w, w.cellid, track ? &rec[0].i : nullptr);
     }
     return cudaGetLastError();
 }

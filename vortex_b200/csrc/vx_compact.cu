@@ -18,13 +18,11 @@
 //
 // The dead ones are marked in a bitmap, from which one block finds all places
 // (vx_cmp_block).  Where few are dead, as after a step's convection, that
-// block makes the moves too, and the two launches after it (gather into
-// scratch, scatter back) return at once.
+// block makes the moves too; else the three launches after it (lists, gather
+// into scratch, scatter back) do, which return at once otherwise.
 #include "vx_compact.cuh"
 
 constexpr int CMP_T = 1024;
-// Most dead vortices the marking kernel's last block removes by itself.
-constexpr long long CMP_FEW = 8192;
 
 // Marks the dead; the block that finishes last goes on (vx_cmp_block).  A
 // warp takes whole words of the bitmap, four at a time, and writes those that
@@ -57,20 +55,58 @@ VX_DEVK void k_cmp_mark_body(VxBlkB<CMP_T, 0> vb, const VxView &v, VxScalars *S,
     if (!vx_last_block(&S->sync_ctr, vb.n)) return;
     if (threadIdx.x == 0) {
         if (count_step) S->step += 1;
-        S->c_n0 = S->c_m = n0;   // nothing left for the next two launches
-        S->c_H = 0;
+        S->cmp_many = 0;
     }
     __syncthreads();
-    vx_cmp_block<CMP_T>(v, S, c, n0, CMP_FEW, true, nullptr, nullptr);
+    vx_cmp_block<CMP_T>(v, S, c, n0, VX_CMP_FEW, true, nullptr, nullptr);
 }
 __global__ void __launch_bounds__(CMP_T) k_cmp_mark(VxView v, VxScalars *S, double eps, VxCompact c, int count_step) {
     VX_PDL_WAIT();
     k_cmp_mark_body(VxBlkB<CMP_T, 0>{blockIdx.x, gridDim.x}, v, S, eps, c, count_step);
 }
 
+// Lists of the holes, of what fills them and of the tail's sources, a warp to
+// 128 vortices; then the moves.  All bits stay until the last launch.
+VX_DEVK void k_cmp_list_body(VxBlkB<0, 0> vb, VxScalars *S, const VxCompact &c) {
+    if (!S->cmp_many) return;
+    const long long n0 = S->c_n0, m = S->c_m, n4 = (n0 + 127) / 128, m4 = m >> 7;
+    const int lane = threadIdx.x & 31;
+    int below = c.pre[m4];   // dead below m: the holes
+    for (int u = 0; u < 4; ++u) {
+        const long long w = m4 * 4 + u;
+        if (w * 32 + 32 <= m) below += __popc(c.bits[w]);
+        else if (w * 32 < m) below += __popc(c.bits[w] & ((1u << (m & 31)) - 1u));
+    }
+    const int H = below;
+    if (vb.x == 0 && threadIdx.x == 0) S->c_H = H;
+    for (long long q = (vb.x * (long long)blockDim.x + threadIdx.x) >> 5; q < n4; q += ((long long)vb.n * blockDim.x) >> 5) {
+        int before = c.pre[q];   // dead before the word
+        for (int u = 0; u < 4; ++u) {
+            const long long w = q * 4 + u, p = w * 32 + lane;
+            const unsigned dead = c.bits[w], next = c.bits[w + 1];
+            const int k = before + __popc(dead & ((1u << lane) - 1u));
+            const bool dd = dead >> lane & 1;
+            if (p < m) {
+                if (dd) c.hole_pos[k] = (int)p;
+            } else if (p < n0) {
+                const int r = (int)(p - m) - (k - H);   // live ones in [m, p)
+                if (!dd) c.hole_src[H - 1 - r] = (int)p;
+                const bool next_live = p + 1 < n0 && !((lane < 31 ? dead >> (lane + 1) : next) & 1u);
+                const int grp = H - r - (dd ? 0 : 1);   // live ones in (p, n0)
+                c.tail_src[p - m] = p == n0 - 1 || next_live ? (grp < H ? -(grp + 1) : (int)m) : (int)(p + 1);
+            }
+            before += __popc(dead);
+        }
+    }
+}
+__global__ void k_cmp_list(VxScalars *S, VxCompact c) {
+    VX_PDL_WAIT();
+    k_cmp_list_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, S, c);
+}
+
 VX_DEVK void k_cmp_gather_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalars *S, const VxCompact &c) {
+    if (!S->cmp_many) return;
     const long long n0 = S->c_n0, m = S->c_m, H = S->c_H;
-    if (m == n0) return;
     vx_cmp_gather<1>(v, c, H, H + n0 - m, vb.x * (long long)blockDim.x + threadIdx.x, (long long)vb.n * blockDim.x);
 }
 __global__ void k_cmp_gather(VxView v, const VxScalars *S, VxCompact c) {
@@ -78,22 +114,31 @@ __global__ void k_cmp_gather(VxView v, const VxScalars *S, VxCompact c) {
     k_cmp_gather_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, c);
 }
 
-VX_DEVK void k_cmp_scatter_body(VxBlkB<0, 0> vb, const VxView &v, VxScalars *S, const VxCompact &c) {
+VX_DEVK void k_cmp_scatter_body(VxBlkB<0, 0> vb, const VxView &v, VxScalars *S, const VxCompact &c, const int *slot,
+                                long long *rec_i) {
+    if (!S->cmp_many) return;
     const long long n0 = S->c_n0, m = S->c_m, H = S->c_H;
-    if (m == n0) return;
-    vx_cmp_scatter<1>(v, c, m, H, H + n0 - m, vb.x * (long long)blockDim.x + threadIdx.x,
-                      (long long)vb.n * blockDim.x, nullptr, nullptr);
-    if (vb.x == 0 && threadIdx.x == 0) S->n = m;
+    const long long first = vb.x * (long long)blockDim.x + threadIdx.x, stride = (long long)vb.n * blockDim.x;
+    vx_cmp_scatter<1>(v, c, m, H, H + n0 - m, first, stride, slot, rec_i);
+    for (long long w = first; w < (n0 + 31) / 32; w += stride) c.bits[w] = 0;
+    if (first == 0) S->n = m;
 }
-__global__ void k_cmp_scatter(VxView v, VxScalars *S, VxCompact c) {
+__global__ void k_cmp_scatter(VxView v, VxScalars *S, VxCompact c, const int *slot, long long *rec_i) {
     VX_PDL_WAIT();
-    k_cmp_scatter_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, c);
+    k_cmp_scatter_body(VxBlkB<0, 0>{blockIdx.x, gridDim.x}, v, S, c, slot, rec_i);
+}
+
+// The moves of a compaction that found more dead than one block should make.
+cudaError_t vx_launch_moves(const VxLaunch &L, const VxView &v, VxScalars *S, VxWork &w, const int *slot,
+                            long long *rec_i) {
+    vx_launch<k_cmp_list, k_cmp_list_body>(L, L.num_sms * 4, VX_THREADS, 0, S, w.cmp);
+    vx_launch<k_cmp_gather, k_cmp_gather_body>(L, L.num_sms * 4, VX_THREADS, 0, v, S, w.cmp);
+    vx_launch<k_cmp_scatter, k_cmp_scatter_body>(L, L.num_sms * 4, VX_THREADS, 0, v, S, w.cmp, slot, rec_i);
+    return cudaGetLastError();
 }
 
 cudaError_t vx_launch_compact(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                               VxWork &w, bool count_step) {
     vx_launch<k_cmp_mark, k_cmp_mark_body>(L, L.num_sms * 2, CMP_T, 0, v, S, p.drop_eps, w.cmp, count_step ? 1 : 0);
-    vx_launch<k_cmp_gather, k_cmp_gather_body>(L, L.num_sms * 4, VX_THREADS, 0, v, S, w.cmp);
-    vx_launch<k_cmp_scatter, k_cmp_scatter_body>(L, L.num_sms * 4, VX_THREADS, 0, v, S, w.cmp);
-    return cudaGetLastError();
+    return vx_launch_moves(L, v, S, w, nullptr, nullptr);
 }

@@ -78,8 +78,9 @@ __device__ __forceinline__ void vx_cmp_scatter(const VxView &v, const VxCompact 
 // Compaction of [0, n0) from the dead bits, by one block of T threads, which
 // leaves the bits at zero.  Returns the dead vortices found.  With up to
 // `limit` of them the moves are made and the count S->n set here; with more,
-// the lists and S->c_* are left for k_cmp_gather and k_cmp_scatter.  apply =
-// false: only the bits are cleared.
+// S->cmp_many is set and the bits, the dead before each 16 bytes of them
+// (c.pre) and S->c_* are left for the three launches of vx_launch_moves.
+// apply = false: only the bits are cleared.
 //
 // Bound: the latency of a few dependent passes.  The bits are read twice (31
 // KB each 250,000 vortices), a run of them to a warp and four 16-byte loads a
@@ -116,14 +117,19 @@ __device__ long long vx_cmp_block(const VxView &v, VxScalars *S, const VxCompact
     if (!apply) {
         for (long long q = a + lane; q < b; q += 32) b4[q] = make_int4(0, 0, 0, 0);
     } else {
-        if (__any_sync(0xffffffffu, mine != 0))
+        const bool many = total > limit;
+        if (many || __any_sync(0xffffffffu, mine != 0))
             for (long long q = a; q < b; q += 128) {
                 int4 w4[4];
                 load(w4, q);
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int k = dead_in(w4[u]);
-                    if (!__any_sync(0xffffffffu, k != 0)) continue;
+                    const long long q4 = q + u * 32 + lane;
+                    if (!__any_sync(0xffffffffu, k != 0)) {
+                        if (many && q4 < b) c.pre[q4] = rank;
+                        continue;
+                    }
                     int inc = k;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
@@ -132,15 +138,27 @@ __device__ long long vx_cmp_block(const VxView &v, VxScalars *S, const VxCompact
                     }
                     int h = rank + inc - k;
                     rank += __shfl_sync(0xffffffffu, inc, 31);
+                    if (many) {
+                        if (q4 < b) c.pre[q4] = h;
+                        continue;
+                    }
                     const unsigned w[4] = {(unsigned)w4[u].x, (unsigned)w4[u].y, (unsigned)w4[u].z, (unsigned)w4[u].w};
 #pragma unroll
                     for (int s = 0; s < 4; ++s)
                         for (unsigned x = w[s]; x; x &= x - 1) {
-                            const long long p = (q + u * 32 + lane) * 128 + s * 32 + __ffs(x) - 1;
+                            const long long p = q4 * 128 + s * 32 + __ffs(x) - 1;
                             if (p < m) c.hole_pos[h++] = (int)p;
                         }
                 }
             }
+        if (many) {
+            if (tid == 0) {
+                S->cmp_many = 1;
+                S->c_n0 = n0;
+                S->c_m = m;
+            }
+            return total;
+        }
         // the tail [m, n0): live ones fill the holes, from the top
         const long long w0 = m >> 5, nt = ((n0 - 1) >> 5) - w0 + 1, per = (nt + NW - 1) / NW;
         const long long wa = w0 + min(nt, warp * per), wb = w0 + min(nt, (warp + 1) * per);
@@ -172,16 +190,10 @@ __device__ long long vx_cmp_block(const VxView &v, VxScalars *S, const VxCompact
         for (int e = tid; e < H; e += T) c.bits[c.hole_pos[e] >> 5] = 0;
         for (long long w = w0 + tid; w < w0 + nt; w += T) c.bits[w] = 0;
         const long long moves = H + (long long)total;
-        if (total <= limit) {
-            vx_cmp_gather<4>(v, c, H, moves, tid, T);
-            __syncthreads();
-            vx_cmp_scatter<4>(v, c, m, H, moves, tid, T, slot, rec_i);
-            if (tid == 0) S->n = m;
-        } else if (tid == 0) {
-            S->c_n0 = n0;
-            S->c_m = m;
-            S->c_H = H;
-        }
+        vx_cmp_gather<4>(v, c, H, moves, tid, T);
+        __syncthreads();
+        vx_cmp_scatter<4>(v, c, m, H, moves, tid, T, slot, rec_i);
+        if (tid == 0) S->n = m;
     }
     return total;
 }

@@ -303,7 +303,7 @@ static vx_status work_alloc_impl(VxWork &w, std::vector<void *> *allocs, long lo
     vx_status st;
 #define A(ptr, n) if ((st = dalloc(allocs, &w.bytes, &(ptr), (n), stream, cv)) != VX_OK) return st
     if ((st = dalloc_zero(allocs, &w.bytes, &w.cmp.bits, cap / 32 + 8, stream, cv)) != VX_OK) return st;
-    A(w.cmp.hole_pos, cap); A(w.cmp.hole_src, cap); A(w.cmp.tail_src, cap);
+    A(w.cmp.pre, cap / 128 + 4); A(w.cmp.hole_pos, cap); A(w.cmp.hole_src, cap); A(w.cmp.tail_src, cap);
     A(w.cmp.hx, cap); A(w.cmp.hy, cap); A(w.cmp.hg, cap); A(w.cmp.tx, cap); A(w.cmp.ty, cap);
     w.cells_cap = std::max(4 * cap, 65536LL);
     A(w.cellid, cap); A(w.cell_start, w.cells_cap + 1);

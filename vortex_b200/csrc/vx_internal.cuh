@@ -78,6 +78,7 @@ struct VxScalars {
     double raw[4];         // unscaled sums of dg, Fx, Fy, M of the last convection
     // compaction
     long long c_n0, c_m, c_H;
+    int cmp_many;          // the running compaction's moves are left to vx_launch_moves
     // collapse
     int col_done;
     int ncand;
@@ -125,9 +126,20 @@ enum {
 // -(value + 1)), and the moved values.
 struct VxCompact {
     unsigned *bits;
+    int *pre;              // dead before each 16 bytes of bits (many dead only)
     int *hole_pos, *hole_src, *tail_src;
     double *hx, *hy, *hg, *tx, *ty;
 };
+
+// Most dead vortices one block removes by itself.  The whole compaction at
+// 2e4 / 1e6 / 3e6 vortices by one block: 200 dead 38 / 48 / 64 us, 2000 dead 41 /
+// 63 / 86, 128,000 dead 626 / 733 at the last two; by the further launches
+// 2000 dead 39 / 50 / 73, 128,000 dead 52 / 79.
+constexpr long long VX_CMP_FEW = 1024;
+// Collapse rounds of bodies whose store holds at most this many leave none to
+// further launches, which would cost every step more than a rare state with
+// thousands of merges gains.
+constexpr long long VX_CMP_SMALL = 65536;
 
 // Device scratch of one body.  Sizes are in elements.
 struct VxWork {
@@ -882,6 +894,8 @@ cudaError_t vx_launch_advect(const VxLaunch &L, const VxParams &p, const VxView 
 // count_step: the compaction of a whole step also advances the step index.
 cudaError_t vx_launch_compact(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                               VxWork &w, bool count_step = false);
+cudaError_t vx_launch_moves(const VxLaunch &L, const VxView &v, VxScalars *S, VxWork &w, const int *slot,
+                            long long *rec_i);
 cudaError_t vx_launch_collapse(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                                VxWork &w, int pass, int n_col);
 cudaError_t vx_launch_probe(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
