@@ -76,7 +76,11 @@ __device__ __forceinline__ double cg_tree(double *sd) {
 // partition past the last particle adds 0) and the partition sums are added
 // in a fixed tree, so the mean spacing, and the grid built from it, do not
 // depend on the launch's grid.  Cell width c * mean(d) / CG_DIV_X, height
-// c * mean(d) / CG_DIV_Y, both grown until the grid fits cells_cap.
+// c * mean(d) / CG_DIV_Y, both grown until the grid fits cells_cap.  A box
+// that cannot be gridded (a position out of all range, or not finite) sets
+// VX_DERR_GRID and leaves a grid of no cells, rows and elements: the stage's
+// other kernels find nothing to do, and none reads keys or starts that an
+// earlier grid, or the quadtree, left behind.
 VX_DEVK void k_cg_prep_body(VxBlkB<CG_T, 0> vb, const VxView &v, VxScalars *S, double *red, unsigned long long *box,
                             int sms, double cutoff, long long cells_cap) {
     __shared__ double sd[CG_T];
@@ -121,7 +125,8 @@ VX_DEVK void k_cg_prep_body(VxBlkB<CG_T, 0> vb, const VxView &v, VxScalars *S, d
     S->cnwide = 0;
     S->cnhuge = 0;
     S->cnitems = 0;
-    if (n == 0) { S->cncells = 0; S->cnx = S->cny = 0; return; }
+    S->cncells = S->cnx = S->cny = S->cnsort = 0;
+    if (n == 0) return;
     const double x0 = vx_dunkey(k[0]), x1 = -vx_dunkey(k[1]);
     const double y0 = vx_dunkey(k[2]), y1 = -vx_dunkey(k[3]);
     double hy = cutoff * (dsum / (double)n) / (double)CG_DIV_Y;
@@ -134,9 +139,10 @@ VX_DEVK void k_cg_prep_body(VxBlkB<CG_T, 0> vb, const VxView &v, VxScalars *S, d
         hx *= 1.25;
         hy *= 1.25;
     }
-    if (nx < 0) { S->err |= VX_DERR_GRID; S->cncells = 0; return; }
+    if (nx < 0) { S->err |= VX_DERR_GRID; return; }
     S->cx0 = x0; S->cy0 = y0; S->ch = hx; S->chy = hy;
     S->cnx = nx; S->cny = ny; S->cncells = nx * ny;
+    S->cnsort = n;
 }
 __global__ void __launch_bounds__(CG_T) k_cg_prep(VxView v, VxScalars *S, double *red, unsigned long long *box,
                                                   int sms, double cutoff, long long cells_cap) {
@@ -155,8 +161,7 @@ __device__ __forceinline__ long long cg_cell(const VxScalars *S, double x, doubl
 // Cell of every particle and its rank in it, counted per cell (the counts are
 // zero between steps: the scan zeroes them behind it).
 VX_DEVK void k_cg_cellid_body(VxBlkB<0, 0> vb, const VxView &v, const VxScalars *S, unsigned *key, int *rank, int *cnt) {
-    const long long n = S->n;
-    if (S->cncells == 0) return;
+    const long long n = S->cnsort;
     for (long long i = vb.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)vb.n * blockDim.x) {
         const long long c = cg_cell(S, v.x[i * v.ps], v.y[i * v.ps]);
@@ -177,7 +182,7 @@ VX_DEVK void k_cg_scan_body(VxBlkB<VX_SCAN_T, 0> vb, VxScalars *S, int *cnt, int
         vb.n, nc, S, tiles,
         [&](long long i0, unsigned (&val)[CG_SCAN_PER]) { vx_scan_load<true>(cnt, i0, nc, val); },
         [&](long long i0, const unsigned (&val)[CG_SCAN_PER], long long run) { vx_scan_store(start, i0, nc, val, run); },
-        [&](long long) { start[nc] = (int)S->n; });
+        [&](long long) { start[nc] = (int)S->cnsort; });
 }
 __global__ void __launch_bounds__(VX_SCAN_T) k_cg_scan(VxScalars *S, int *cnt, int *start, unsigned long long *tiles) {
     VX_PDL_WAIT();
@@ -852,7 +857,7 @@ cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, cons
     gt.S = S;
     gt.srt = srt;
     if (L.early) vx_await(B, VX_EVT_BORN);   // strengths from here on
-    vx_bucket_order(L.early ? vx_full_dependency(B) : B, &S->n, w.key0, w.val0, w.cg_start, w.key0, w.val0, vx_order_rec(w), gt);
+    vx_bucket_order(L.early ? vx_full_dependency(B) : B, &S->cnsort, w.key0, w.val0, w.cg_start, w.key0, w.val0, vx_order_rec(w), gt);
     const unsigned *skey = w.key0;
     const int *sorted = w.val0;
 

@@ -92,6 +92,7 @@ struct VxScalars {
     // neighbour-list grid of the bulk form (vortex diffusion)
     double cx0, cy0, ch, chy;   // origin, cell width and cell height
     long long cnx, cny, cncells, cnitems;
+    long long cnsort;      // vortices put in cell order: n, or 0 where no grid could be made
     // quadtree of the bulk-form Biot-Savart (vx_fmm.cu)
     double fx0, fy0, fside;
     long long fnleaves, fs;
@@ -116,7 +117,7 @@ struct VxScalars {
 
 enum {
     VX_DERR_RESOLVE = 1,     // collapse resolution did not converge
-    VX_DERR_GRID = 2,        // collapse grid did not fit its cell capacity
+    VX_DERR_GRID = 2,        // a collapse or diffusion grid did not fit its cell capacity
     VX_DERR_SCAN = 4,        // a look-back scan gave up waiting on a predecessor tile
 };
 
