@@ -1045,7 +1045,7 @@ static cudaError_t launch_stages(vx_sim *s, unsigned mask, bool whole_step, VxRe
     }
     ev(2);
     if (mask & VX_STAGE_DIFFUSION)
-        if ((e = vx_launch_diffusion(L, p, v, s->d_S, s->w)) != cudaSuccess) return e;
+        if ((e = vx_launch_diffusion(L, p, v, s->d_S, s->w, (mask & VX_STAGE_VELOCITY) && !bulk)) != cudaSuccess) return e;
     L.split = false;
     ev(3);
     if (mask & VX_STAGE_WALL)

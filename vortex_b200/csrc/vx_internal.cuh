@@ -883,8 +883,10 @@ cudaError_t vx_launch_birth(const VxLaunch &L, const VxParams &p, const VxView &
                             int rhs_chunks, bool place);
 cudaError_t vx_launch_velocity(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                                VxWork &w);
+// packed: the direct velocity sums came before it in the same call (they pack
+// the vortices as they are into w.src32, which an all-pairs FP32 diffusion reads)
 cudaError_t vx_launch_diffusion(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
-                                VxWork &w);
+                                VxWork &w, bool packed);
 // wstart/widx: per wall cell, the panels that can act on a particle in the
 // cell (CSR, ascending panel index); null: every panel is tested
 cudaError_t vx_launch_wall(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,

@@ -778,9 +778,10 @@ cudaError_t vx_launch_velocity(const VxLaunch &L, const VxParams &p, const VxVie
 }
 
 cudaError_t vx_launch_diffusion(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
-                                VxWork &w) {
+                                VxWork &w, bool packed) {
     // bulk form: neighbour lists within diff_cutoff * d_i (vx_cells.cu)
     if (p.prec == VX_PREC_FP32 && p.diff_cutoff > 0.0) return vx_launch_diffusion_cells(L, p, v, S, w);
+    if (!packed && maybe_pack(L, p, v, S, w) != cudaSuccess) return cudaGetLastError();
     const VxSplit sp = pair_split(L, p, w, 3, 0);
     const int grid = pair_slots(L, p);
     VX_EV(L, 2);

@@ -343,7 +343,7 @@ int Speed(vxu_vortex *pos, double (*v_inf)[2], size_t s, vxu_velocity *v, double
     const VxLaunch L = launch0();
     const VxView vw = aos_view(pos, v, d);
     CK(vx_launch_velocity(L, U.prm, vw, U.d_S, U.w));
-    CK(vx_launch_diffusion(L, U.prm, vw, U.d_S, U.w));
+    CK(vx_launch_diffusion(L, U.prm, vw, U.d_S, U.w, true));
     CK(vx_launch_wall(L, U.prm, vw, U.d_S, panels));
     CK(cudaDeviceSynchronize());
     return 0;
