@@ -1037,22 +1037,29 @@ static cudaError_t launch_stages(vx_sim *s, unsigned mask, bool whole_step, VxRe
         else
             e = vx_launch_velocity(L, p, v, s->d_S, s->w);
         // joined by the bulk diffusion once its grid is built (vx_cells.cu)
-        if (!(mask & VX_STAGE_DIFFUSION) || !(p.diff_cutoff > 0.0) || e != cudaSuccess) {
+        if (L.split && (!(mask & VX_STAGE_DIFFUSION) || !(p.diff_cutoff > 0.0) || e != cudaSuccess)) {
             vx_join(L);
             L.split = false;
+            L.pdl = false;   // until the stage that comes next is launched
         }
         if (e != cudaSuccess) return e;
     }
     ev(2);
-    if (mask & VX_STAGE_DIFFUSION)
+    if (mask & VX_STAGE_DIFFUSION) {
         if ((e = vx_launch_diffusion(L, p, v, s->d_S, s->w, (mask & VX_STAGE_VELOCITY) && !bulk)) != cudaSuccess) return e;
+        L.pdl = true;
+    }
     L.split = false;
     ev(3);
-    if (mask & VX_STAGE_WALL)
+    if (mask & VX_STAGE_WALL) {
         if ((e = vx_launch_wall(L, p, v, s->d_S, s->d_pan, s->d_wstart, s->d_widx)) != cudaSuccess) return e;
+        L.pdl = true;
+    }
     ev(4);
-    if (mask & VX_STAGE_ADVECT)
+    if (mask & VX_STAGE_ADVECT) {
         if ((e = vx_launch_advect(L, p, v, s->d_S, s->w, s->d_pan, s->d_hstart, s->d_hidx)) != cudaSuccess) return e;
+        L.pdl = true;
+    }
     if (mask & VX_STAGE_COMPACT)
         if ((e = vx_launch_compact(L, p, v, s->d_S, s->w, whole_step)) != cudaSuccess) return e;
     if (mask & VX_STAGE_COLLAPSE1)
