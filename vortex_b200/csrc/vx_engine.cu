@@ -19,6 +19,7 @@
 #include <mutex>
 #include <string>
 #include <cstddef>
+#include <cstdlib>
 #include <vector>
 
 #include "vx_sim.cuh"
@@ -59,47 +60,57 @@ void vx_trim_pool(int device) {
     if (cudaMemPoolTrimTo(pool, POOL_KEEP) != cudaSuccess) cudaGetLastError();
 }
 
-// Pinned mirrors of the device scalars: slots of a pinned block shared by the
-// handles (a cudaMallocHost and cudaFreeHost of its own took 1.5 to 3 ms a
-// handle).  Blocks of 64 slots; a block none of whose slots is taken is given
-// back, but for one.  Any thread may take and return slots; the memory is
-// portable, so handles of every device share it.
+// What the bodies of one device share, for as long as there is one: host memory
+// for the copies of their scalars (page-locked: a copy from the device takes 10.5
+// us, 12.9 into pageable memory), given back with the last of them.  Each
+// handle's own cudaMallocHost took 2 ms where no other page-locked memory was;
+// a block is registered in 0.5.
+//
+// The blocks are the process's own memory, registered with one device: should
+// a caller reset that device, its bodies are lost with it, but the scalars of
+// the others stay where they are, and a slot taken from a block that is not
+// registered any more is ordinary memory.  Any thread may take and give slots.
 namespace {
-class PinnedScalars {
+class BodyShare {
 public:
-    VxScalars *take() {
+    VxScalars *take(int device) {
         std::lock_guard<std::mutex> lock(mu_);
         for (Block &b : blocks_)
-            if (b.used != ~0ull) return slot(b);
-        void *m = nullptr;
-        if (cudaHostAlloc(&m, 64 * STRIDE, cudaHostAllocPortable) != cudaSuccess) return nullptr;
-        blocks_.push_back(Block{static_cast<char *>(m), 0});
+            if (b.device == device && b.used != ~0ull) return slot(b);
+        void *m = std::aligned_alloc(4096, BYTES);
+        if (!m) return nullptr;
+        if (cudaHostRegister(m, BYTES, cudaHostRegisterDefault) != cudaSuccess) {
+            cudaGetLastError();
+            std::free(m);
+            return nullptr;
+        }
+        blocks_.push_back(Block{static_cast<char *>(m), device, 0});
         return slot(blocks_.back());
     }
-    void give(VxScalars *p) {
+    void give(VxScalars *p) {   // the slot's device is the current one
         std::lock_guard<std::mutex> lock(mu_);
         const char *c = reinterpret_cast<char *>(p);
-        int empty = 0;
-        for (Block &b : blocks_) {
-            if (c >= b.base && c < b.base + 64 * STRIDE) b.used &= ~(1ull << ((c - b.base) / STRIDE));
-            empty += b.used == 0;
-        }
-        for (size_t k = 0; k < blocks_.size() && empty > 1;)
-            if (blocks_[k].used == 0) {
-                cudaFreeHost(blocks_[k].base);
+        for (size_t k = 0; k < blocks_.size(); ++k) {
+            Block &b = blocks_[k];
+            if (c < b.base || c >= b.base + BYTES) continue;
+            b.used &= ~(1ull << ((c - b.base) / STRIDE));
+            if (b.used == 0) {
+                if (cudaHostUnregister(b.base) != cudaSuccess) cudaGetLastError();
+                std::free(b.base);
                 blocks_.erase(blocks_.begin() + (long)k);
-                --empty;
-            } else {
-                ++k;
             }
+            return;
+        }
     }
 
 private:
     struct Block {
         char *base;
-        unsigned long long used;
+        int device;
+        unsigned long long used;   // a bit per slot; a block without any is given back
     };
     static constexpr size_t STRIDE = (sizeof(VxScalars) + 255) / 256 * 256;
+    static constexpr size_t BYTES = (64 * STRIDE + 4095) / 4096 * 4096;
     static VxScalars *slot(Block &b) {
         const int k = __builtin_ctzll(~b.used);
         b.used |= 1ull << k;
@@ -108,8 +119,8 @@ private:
     std::mutex mu_;
     std::vector<Block> blocks_;
 };
-PinnedScalars &pinned_scalars() {
-    static PinnedScalars *p = new PinnedScalars();   // never destroyed: handles may outlive static destructors
+BodyShare &body_share() {
+    static BodyShare *p = new BodyShare();   // never destroyed: handles may outlive static destructors
     return *p;
 }
 }  // namespace
@@ -592,7 +603,7 @@ extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t
     PanelLists wall, hit;
     build_wall_lists(s->prm, pan, (int)P, wall);
     build_hit_lists(s->prm, pan, (int)P, hit);
-    s->h_S = pinned_scalars().take();
+    s->h_S = body_share().take(device);
     if (!s->h_S) { vx_set_error("vx_create: no pinned memory"); return fail(VX_ERR_NOMEM); }
     memset(s->h_S, 0, sizeof(VxScalars));
     // V_inf ramp (src/main.c:585-592): with a ramp the flow starts at rest
@@ -676,7 +687,7 @@ extern "C" vx_status vx_destroy(vx_sim *s) {
     for (double *a : arr) if (a) cudaFreeAsync(a, s->stream);
     if (s->d_fixed) cudaFreeAsync(s->d_fixed, s->stream);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    if (s->h_S) pinned_scalars().give(s->h_S);
+    if (s->h_S) body_share().give(s->h_S);
     if (s->d_probe) cudaFree(s->d_probe);
     if (s->d_pts) cudaFree(s->d_pts);
     if (s->d_St) cudaFree(s->d_St);

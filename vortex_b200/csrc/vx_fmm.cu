@@ -1334,15 +1334,11 @@ static cudaError_t velocity_fmm(const VxLaunch &L, const VxParams &p, const VxVi
                                 bool built) {
     constexpr int M2L_T = m2l_threads<P>();
     constexpr size_t M2L_SMEM = sizeof(M2LShared<P>);
-    if (M2L_SMEM > 48 * 1024 && !L.rec) {   // opt in to more than 48 KB of shared memory (once per device)
-        static bool done[64] = {};
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev >= 0 && dev < 64 && !done[dev]) {
-            cudaFuncSetAttribute(k_fmm_m2l_l2l<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M2L_SMEM);
-            cudaFuncSetAttribute(k_fmm_m2l_small<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M2L_SMEM);
-            done[dev] = true;
-        }
+    // over 48 KB of shared memory (P = 20); asked for each time, as a device
+    // that was reset has forgotten it
+    if (M2L_SMEM > 48 * 1024 && !L.rec) {
+        cudaFuncSetAttribute(k_fmm_m2l_l2l<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M2L_SMEM);
+        cudaFuncSetAttribute(k_fmm_m2l_small<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M2L_SMEM);
     }
     const int grid = L.num_sms * 4;
     const int Lmax = w.fmm_lmax;

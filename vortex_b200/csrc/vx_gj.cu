@@ -35,7 +35,6 @@
 // the diagonal, where those steps read them.
 #include <algorithm>
 #include <climits>
-#include <mutex>
 
 #include <cooperative_groups.h>
 
@@ -336,19 +335,13 @@ __global__ void k_gj_finish(const double *A, const double *W, long long ld, int 
 static int gj_blocks(long long S) { return (int)vx_ceil_div(S, GJ_B); }
 static long long gj_ld(long long S) { return vx_ceil_div(S, GJ_STRIP) * GJ_STRIP; }
 
-static cudaError_t gj_shared(int nt) {   // over 48 KB of shared memory from 362 rows a block
-    static std::mutex mu;
-    static bool done[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess || dev < 0 || dev >= 64) return e;
-    std::lock_guard<std::mutex> lock(mu);
-    if (done[dev]) return cudaSuccess;
-    const int most = (int)sizeof(double) * (GJ_B + 1) * GJ_T;
-    e = cudaFuncSetAttribute(k_gj_panel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gj_panel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    done[dev] = e == cudaSuccess;
-    return e;
+// Over 48 KB of shared memory from 362 rows a block on.  Asked for each time (a
+// device that was reset has forgotten it), always for the most a block takes
+// (bodies may be created from several threads).
+static cudaError_t gj_shared(int robust) {
+    constexpr int most = (int)sizeof(double) * (GJ_B + 1) * GJ_T;
+    return robust ? cudaFuncSetAttribute(k_gj_panel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most)
+                  : cudaFuncSetAttribute(k_gj_panel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
 }
 
 bool vx_gj_fits(long long S) { return S <= (long long)GJ_MAXC * GJ_T; }
@@ -374,7 +367,7 @@ cudaError_t vx_invert_gj(const VxLaunch &L, double *A, double *Inv, long long S,
     const unsigned nt = (unsigned)vx_round32(vx_ceil_div(S, (long long)nc));
     VX_COUNT(L);
     cudaError_t e = vx_launch_pdl(k_gj_begin, (unsigned)vx_ceil_div(S, 256LL), 256, 0, L.stream, orig, n, nmoved, nblk);
-    if (e == cudaSuccess) e = gj_shared((int)nt);
+    if (e == cudaSuccess) e = gj_shared(robust);
     for (int k0 = 0; k0 < n - 1 && e == cudaSuccess; k0 += GJ_B) {
         const int kb = std::min(GJ_B, n - 1 - k0), b = k0 / GJ_B;
         cudaLaunchConfig_t cfg = {};
