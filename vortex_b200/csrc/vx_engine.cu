@@ -49,27 +49,21 @@ void vx_keep_pool(int device) {
     if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
 }
 
-// A destroyed handle's stream-ordered memory goes back to the driver (the
-// pool keeps it otherwise, out of reach of plain cudaMalloc callers), but for
-// a small body's worth: mapping it afresh for the next body and unmapping it
-// took 1 to 2 ms of a creation and a destruction each.
-constexpr size_t POOL_KEEP = 64 << 20;
-void vx_trim_pool(int device) {
-    cudaMemPool_t pool;
-    if (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess) { cudaGetLastError(); return; }
-    if (cudaMemPoolTrimTo(pool, POOL_KEEP) != cudaSuccess) cudaGetLastError();
-}
-
 // What the bodies of one device share, for as long as there is one: host memory
 // for the copies of their scalars (page-locked: a copy from the device takes 10.5
-// us, 12.9 into pageable memory), given back with the last of them.  Each
-// handle's own cudaMallocHost took 2 ms where no other page-locked memory was;
-// a block is registered in 0.5.
+// us, 12.9 into pageable memory), and up to 64 MB of freed memory left in the
+// device's pool, about one small body's worth, so that a body that follows
+// another one does not map it afresh.  The last body to be closed gives both
+// back, as a pool that no body uses is only lost to others: a body created and
+// closed beside another takes 1.5 ms at 200 panels and 3.8 at 1000, by itself 2.1 and
+// 4.8 (0.75 and 3.4 with both kept for good).  Each handle's own cudaMallocHost took
+// 2 ms where no other page-locked memory was.
 //
 // The blocks are the process's own memory, registered with one device: should
 // a caller reset that device, its bodies are lost with it, but the scalars of
 // the others stay where they are, and a slot taken from a block that is not
 // registered any more is ordinary memory.  Any thread may take and give slots.
+constexpr size_t POOL_KEEP = 64 << 20;
 namespace {
 class BodyShare {
 public:
@@ -102,6 +96,12 @@ public:
             return;
         }
     }
+    bool live(int device) {
+        std::lock_guard<std::mutex> lock(mu_);
+        for (const Block &b : blocks_)
+            if (b.device == device) return true;
+        return false;
+    }
 
 private:
     struct Block {
@@ -124,6 +124,14 @@ BodyShare &body_share() {
     return *p;
 }
 }  // namespace
+
+// Freed memory of the pool back to the driver, out of reach of plain cudaMalloc
+// callers until then.
+void vx_trim_pool(int device) {
+    cudaMemPool_t pool;
+    if (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess) { cudaGetLastError(); return; }
+    if (cudaMemPoolTrimTo(pool, body_share().live(device) ? POOL_KEEP : 0) != cudaSuccess) cudaGetLastError();
+}
 
 extern "C" const char *vx_status_str(vx_status s) {
     switch (s) {
