@@ -321,6 +321,11 @@ vx_status vx_eval_bulk_atan2(const float *y, const float *x, float *out, int64_t
  * Allocates its own scratch. */
 vx_status vx_eval_bucket_order(const unsigned *key, int64_t n, int64_t nb, int *order);
 
+/* Validation hook (no counterpart in the reference): a function of the plain
+ * form's pair sums at n points x (device arrays): which = 0 1/x, 1 1/sqrt(x),
+ * 2 2^(x/32) for -32672 <= x <= 0. */
+vx_status vx_eval_fp64(int which, const double *x, double *out, int64_t n);
+
 /* Number of kernels this handle has launched since creation. */
 vx_status vx_get_launch_count(vx_sim *sim, int64_t *count);
 

@@ -819,3 +819,20 @@ cudaError_t vx_launch_probe(const VxLaunch &L, const VxParams &p, const VxView &
 
     return cudaGetLastError();
 }
+
+// Validation hook: one of the plain sums' own FP64 functions at n points.
+__global__ void __launch_bounds__(PT) k_eval_fp64(int which, const double *x, double *out, long long n) {
+    const double tab = c_exp_table[threadIdx.x & 31];
+    for (long long b = blockIdx.x * (long long)PT; b < n; b += (long long)gridDim.x * PT) {   // whole warps
+        const long long i = b + threadIdx.x;
+        const double v = i < n ? x[i] : 0.0;
+        const double r = which == 0 ? vx_rcp64(v) : (which == 1 ? vx_rsqrt64(v) : vx_exp2_32(v, tab));
+        if (i < n) out[i] = r;
+    }
+}
+extern "C" vx_status vx_eval_fp64(int which, const double *x, double *out, int64_t n) {
+    if (which < 0 || which > 2 || n < 0 || (n > 0 && (!x || !out))) return VX_ERR_ARG;
+    if (n == 0) return VX_OK;
+    k_eval_fp64<<<(unsigned)std::min<long long>(vx_ceil_div(n, (long long)PT), 1024), PT>>>(which, x, out, n);
+    return cudaDeviceSynchronize() == cudaSuccess ? VX_OK : VX_ERR_CUDA;
+}
