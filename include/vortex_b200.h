@@ -326,6 +326,13 @@ vx_status vx_eval_bucket_order(const unsigned *key, int64_t n, int64_t nb, int *
  * 2 2^(x/32) for -32672 <= x <= 0. */
 vx_status vx_eval_fp64(int which, const double *x, double *out, int64_t n);
 
+/* Validation hook (no counterpart in the reference): the inverted panel system
+ * of P panels (host arrays, (P+1)^2 row-major) by the reference's pivot rule
+ * (robust = 0) or partial pivoting (1), in the blocks of columns that bodies
+ * are made with (columns = 0) or column by column (1).  Allocates its own
+ * scratch. */
+vx_status vx_eval_inverse(const vx_panel *panels, int64_t P, int robust, int columns, double *minv);
+
 /* Number of kernels this handle has launched since creation. */
 vx_status vx_get_launch_count(vx_sim *sim, int64_t *count);
 

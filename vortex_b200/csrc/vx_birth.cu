@@ -243,12 +243,12 @@ long long vx_matrix_work(int P) {
 // systems whose rows fit the threads of a cluster, 4095 panels; a larger
 // one column by column, two launches each.
 cudaError_t vx_build_matrix(const VxLaunch &L, const vx_panel *d_pan, int P, double *d_minv,
-                            double *d_work, int *d_flag, double *d_L_out, int robust) {
+                            double *d_work, int *d_flag, double *d_L_out, int robust, bool columns) {
     const long long S = P + 1;
     double *A = d_work;
     double *c = d_work + S * S;
     const int grid = L.num_sms * 4;
-    const bool blocked = robust != 3 && vx_gj_fits(S);
+    const bool blocked = robust != 3 && !columns && vx_gj_fits(S);
     const long long ld = blocked ? vx_gj_stride(S) : S;
     cudaMemsetAsync(d_flag, 0, sizeof(int), L.stream);
     vx_launch<k_panel_influence, k_panel_influence_body>(L, grid, 256, 0, d_pan, P, A, ld);
@@ -267,6 +267,37 @@ cudaError_t vx_build_matrix(const VxLaunch &L, const vx_panel *d_pan, int P, dou
     vx_launch<k_gj_last_elim, k_gj_last_elim_body>(L, grid, 256, 0, d_minv, S, c, d_flag);
     vx_launch<k_gj_scale, k_gj_scale_body>(L, grid, 256, 0, A, d_minv, S, d_flag);
     return cudaGetLastError();
+}
+
+// Validation hook: the panel system's inverse, in blocks of columns or column
+// by column.
+extern "C" vx_status vx_eval_inverse(const vx_panel *pan, int64_t P, int robust, int columns, double *minv) {
+    if (!pan || !minv || P < 2 || (robust != 0 && robust != 1)) return VX_ERR_ARG;
+    const long long S = P + 1;
+    int dev = 0, hflag = 0;
+    VxLaunch L;
+    L.stream = 0;
+    L.launches = nullptr;
+    L.num_sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&L.num_sms, cudaDevAttrMultiProcessorCount, dev);
+    void *mem[4] = {};
+    const size_t sz[4] = {sizeof(vx_panel) * (size_t)P, sizeof(double) * (size_t)(S * S),
+                          sizeof(double) * (size_t)vx_matrix_work((int)P), sizeof(int)};
+    vx_status st = VX_OK;
+    for (int q = 0; q < 4 && st == VX_OK; ++q)
+        if (cudaMalloc(&mem[q], sz[q]) != cudaSuccess) st = VX_ERR_NOMEM;
+    if (st == VX_OK) {
+        const bool ok = cudaMemcpy(mem[0], pan, sz[0], cudaMemcpyHostToDevice) == cudaSuccess &&
+                        vx_build_matrix(L, (const vx_panel *)mem[0], (int)P, (double *)mem[1], (double *)mem[2],
+                                        (int *)mem[3], nullptr, robust, columns != 0) == cudaSuccess &&
+                        cudaMemcpy(&hflag, mem[3], sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess &&
+                        cudaMemcpy(minv, mem[1], sz[1], cudaMemcpyDeviceToHost) == cudaSuccess;
+        st = !ok ? VX_ERR_CUDA : (hflag ? VX_ERR_SINGULAR : VX_OK);
+    }
+    for (void *q : mem)
+        if (q) cudaFree(q);
+    return st;
 }
 
 // ---------------------------------------------------------------------------

@@ -908,9 +908,10 @@ cudaError_t vx_launch_probe(const VxLaunch &L, const VxParams &p, const VxView &
 // d_L_out (nullable) receives a copy of the influence matrix before elimination.
 cudaError_t vx_build_matrix(const VxLaunch &L, const vx_panel *d_pan, int P, double *d_minv,
                             double *d_work, int *d_flag, double *d_L_out,
-                            int robust = 0);
+                            int robust = 0, bool columns = false);
 // robust: 0 the reference's pivot rule, 1 Gauss-Jordan with partial
-// pivoting, 3 blocked LU with partial pivoting (vx_invert_lu).  d_work:
+// pivoting, 3 blocked LU with partial pivoting (vx_invert_lu).  columns: column
+// by column whatever the size (what the blocks are checked against).  d_work:
 // vx_matrix_work(P) doubles.
 long long vx_matrix_work(int P);
 // The Gauss-Jordan inverse in blocks of columns (vx_gj.cu): systems it takes,
