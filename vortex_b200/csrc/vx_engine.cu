@@ -576,6 +576,17 @@ static void build_hit_lists(VxParams &p, const vx_panel *pan, int P, PanelLists 
     p.hit_ny = (int)ny;
 }
 
+// The stream and events of the bulk form's second branch (VxLaunch::split), if
+// the body has none yet; the stream last, as a body that has it has all.  (A
+// higher priority than the main stream's made no difference.)
+static vx_status make_side(vx_sim *s) {
+    if (s->side || s->prm.prec != VX_PREC_FP32) return VX_OK;
+    for (auto &e : s->side_ev)
+        if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    CU(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
+    return VX_OK;
+}
+
 extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t P, int device,
                                vx_sim **out) {
     if (!conf || !pan || P < 2 || !out) { vx_set_error("vx_create: bad arguments"); return VX_ERR_ARG; }
@@ -602,12 +613,7 @@ extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t
     cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(VX_ERR_CUDA);
     vx_params_from_conf(conf, pan, (int)P, &s->prm);
-    if (s->prm.prec == VX_PREC_FP32 && s->conf.fmm) {
-        // (a higher priority than the main stream's made no difference)
-        if (cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking) != cudaSuccess) return fail(VX_ERR_CUDA);
-        for (auto &e : s->side_ev)
-            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(VX_ERR_CUDA);
-    }
+    if (s->conf.fmm && make_side(s) != VX_OK) return fail(VX_ERR_CUDA);
     PanelLists wall, hit;
     build_wall_lists(s->prm, pan, (int)P, wall);
     build_hit_lists(s->prm, pan, (int)P, hit);
@@ -1306,6 +1312,10 @@ extern "C" vx_status vx_set_fmm(vx_sim *s, int fmm, int leaf) {
     if (!s || leaf < 1) return VX_ERR_ARG;
     CU(cudaSetDevice(s->device));
     CU(cudaStreamSynchronize(s->stream));
+    if (fmm) {
+        const vx_status st = make_side(s);
+        if (st != VX_OK) return st;
+    }
     s->conf.fmm = fmm != 0;
     s->conf.fmm_leaf = leaf;
     s->prm.fmm_leaf = leaf;
