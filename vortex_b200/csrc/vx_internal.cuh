@@ -338,19 +338,6 @@ __device__ __forceinline__ void vx_block_min4(unsigned long long (&k)[4]) {
     }
     __syncthreads();   // sh may be used again
 }
-// Sum of a block's non-negative ints (NW warps), in every thread.
-template <int NW>
-__device__ __forceinline__ int vx_block_add(int v) {
-    __shared__ int sh[NW];
-    v = __reduce_add_sync(0xffffffffu, v);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    int t = 0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) t += sh[w];
-    __syncthreads();
-    return t;
-}
 // Exclusive scan of a block's ints (NW warps); total: their sum.
 template <int NW>
 __device__ __forceinline__ int vx_block_scan(int v, int &total) {
@@ -994,5 +981,3 @@ cudaError_t vx_launch_velocity_fmm(const VxLaunch &L, const VxParams &p, const V
 cudaError_t vx_launch_diffusion_cells(const VxLaunch &L, const VxParams &p, const VxView &v, VxScalars *S,
                                       VxWork &w);
 void vx_work_free(VxWork &w, std::vector<void *> &allocs, cudaStream_t stream = nullptr);
-
-// Split factor so that (target tiles x source chunks) fills the GPU.
