@@ -34,8 +34,8 @@
 // compaction at 1e6 / 3e6 vortices, each timed by itself: 150 / 406 us ->
 // 23 / 31.  A third round and later ones build their grid again.
 //
-// col, in_cnt, has_app and first_app are all zero between rounds: the settle
-// clears the entries its candidates used.  col holds INT_MAX - j, first_app
+// col, in_cnt and first_app are all zero between rounds: the settle clears the
+// entries its candidates used.  col holds INT_MAX - j, first_app
 // INT_MAX - i (atomicMax keeps the smallest index, 0 is none).
 #include <limits.h>
 
@@ -189,7 +189,7 @@ __device__ __forceinline__ bool vx_col_pair(const VxParams &p, double xi, double
 // position by the count's expression.
 template <int PASS>
 VX_DEVK void k_col_query_body(VxBlkB<VX_THREADS, 4> vb, const VxParams &p, VxScalars *S, const int *start, const ColRec *rec,
-                              int *col, int *cand) {
+                              int *col, int *cand, int *cstate, int *in_cnt) {
     if (S->col_done) return;
     const long long n = S->n;
     const long long gnx = S->gnx, gny = S->gny;
@@ -214,15 +214,19 @@ VX_DEVK void k_col_query_body(VxBlkB<VX_THREADS, 4> vb, const VxParams &p, VxSca
             }
         }
         if (best != INT_MAX) {
+            const int c = atomicAdd(&S->ncand, 1);
             col[i] = INT_MAX - best;
-            cand[atomicAdd(&S->ncand, 1)] = (int)i;
+            cand[c] = (int)i;
+            cstate[c] = 0;
+            atomicAdd(&in_cnt[best], 1);
         }
     }
 }
 template <int PASS>
-__global__ void k_col_query(VxParams p, VxScalars *S, const int *start, const ColRec *rec, int *col, int *cand) {
+__global__ void k_col_query(VxParams p, VxScalars *S, const int *start, const ColRec *rec, int *col, int *cand,
+                            int *cstate, int *in_cnt) {
     VX_PDL_WAIT();
-    k_col_query_body<PASS>(VxBlkB<VX_THREADS, 4>{blockIdx.x, gridDim.x}, p, S, start, rec, col, cand);
+    k_col_query_body<PASS>(VxBlkB<VX_THREADS, 4>{blockIdx.x, gridDim.x}, p, S, start, rec, col, cand, cstate, in_cnt);
 }
 
 // Second round: the partners of the vortices the first one moved (their slots
@@ -230,7 +234,7 @@ __global__ void k_col_query(VxParams p, VxScalars *S, const int *start, const Co
 // moved ones is met from both sides.
 template <int PASS>
 VX_DEVK void k_col_query_moved_body(VxBlkB<VX_THREADS, 0> vb, const VxParams &p, VxScalars *S, const int *start,
-                                    const ColRec *rec, const int *moved, int *col, int *cand) {
+                                    const ColRec *rec, const int *moved, int *col, int *cand, int *cstate) {
     if (S->col_done) return;
     const int nm = S->nmoved;
     const long long gnx = S->gnx, gny = S->gny;
@@ -253,115 +257,155 @@ VX_DEVK void k_col_query_moved_body(VxBlkB<VX_THREADS, 0> vb, const VxParams &p,
             if (!(fabs(q1.x) >= p.drop_eps)) continue;   // removed after the first round
             if (!vx_col_pair<PASS>(p, m0.x, m0.y, m1.x, q0.x, q0.y, q1.x)) continue;
             const int j = (int)__double_as_longlong(q1.y), lo = min(i, j);
-            if (atomicMax(&col[lo], INT_MAX - max(i, j)) == 0) cand[atomicAdd(&S->ncand, 1)] = lo;
+            if (atomicMax(&col[lo], INT_MAX - max(i, j)) == 0) {
+                const int c = atomicAdd(&S->ncand, 1);
+                cand[c] = lo;
+                cstate[c] = 0;
+            }
         }
     }
 }
 template <int PASS>
 __global__ void __launch_bounds__(VX_THREADS) k_col_query_moved(VxParams p, VxScalars *S, const int *start,
                                                                 const ColRec *rec, const int *moved, int *col,
-                                                                int *cand) {
+                                                                int *cand, int *cstate) {
     VX_PDL_WAIT();
-    k_col_query_moved_body<PASS>(VxBlkB<VX_THREADS, 0>{blockIdx.x, gridDim.x}, p, S, start, rec, moved, col, cand);
+    k_col_query_moved_body<PASS>(VxBlkB<VX_THREADS, 0>{blockIdx.x, gridDim.x}, p, S, start, rec, moved, col, cand, cstate);
+}
+
+// One round over the candidate list, by one block: those whose turn it is are
+// decided.  U candidates of a thread at a time, all loads of a kind before the
+// next: the time of a long list is their latency.
+template <int U>
+__device__ __forceinline__ void col_decide(int nc, const int *cand, const int *col, int *in_cnt, int *first_app,
+                                           int *cstate, int *cdec, int &undecided) {
+    const int T = blockDim.x;
+    for (int k0 = threadIdx.x; k0 < nc; k0 += U * T) {
+        int i[U], taken[U], before[U];
+        bool open[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) open[u] = k0 + u * T < nc && cstate[k0 + u * T] == 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) i[u] = open[u] ? cand[k0 + u * T] : 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            taken[u] = open[u] ? first_app[i[u]] : 0;   // by an applied candidate before it
+            before[u] = open[u] ? in_cnt[i[u]] : 0;     // undecided ones before it
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (open[u]) cdec[k0 + u * T] = taken[u] ? 2 : (before[u] == 0 ? 1 : 0);
+    }
+    if (threadIdx.x == 0) undecided = 0;
+    __syncthreads();
+    for (int k0 = threadIdx.x; k0 < nc; k0 += U * T) {
+        int i[U], j[U], d[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) d[u] = k0 + u * T < nc && cstate[k0 + u * T] == 0 ? cdec[k0 + u * T] : -1;
+#pragma unroll
+        for (int u = 0; u < U; ++u) i[u] = d[u] > 0 ? cand[k0 + u * T] : 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) j[u] = d[u] > 0 ? INT_MAX - col[i[u]] : 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (d[u] == 0) undecided = 1;
+            if (d[u] <= 0) continue;
+            cstate[k0 + u * T] = d[u];
+            atomicSub(&in_cnt[j[u]], 1);
+            if (d[u] == 1) atomicMax(&first_app[j[u]], INT_MAX - i[u]);
+        }
+    }
 }
 
 // Settles the candidates in one block: rounds over the candidate list decide
 // each one (cstate: 0 undecided, 1 applied, 2 consumed before its turn), then
-// every applied candidate's merged vortex is computed from the positions as
-// they were, then written (after a barrier: a merge may read a partner that
-// another merge removes).
+// every applied candidate's merged vortex is written.  An applied candidate is
+// nobody's partner, and of those that share a partner the first alone reads
+// it and removes it, so no merge reads what another writes.
+// counted: in_cnt holds the candidates that point at each vortex (the second
+// round's partners are settled only when its query is done).
 // track: the cell-sorted copy is kept in step for the second round, and the
 // slots of the moved vortices are listed (in cdec, done with by then).
 // The round's compaction follows in the same block (vx_cmp_block): what the
 // merges removed is marked as they are written.  It adds 8 / 16 / 20 us at
 // 2e4 / 1e6 / 3e6 vortices; as four launches over all of them (count,
 // classify, gather, scatter) it took 32 / 39 / 50.
+// A whole pass of two rounds (vx_stage) with 460 / 44,000 / 406,000 merges of 1e6
+// vortices takes 188 / 965 / 9560 us, with 630 / 5300 of 2e4 90 / 200.  With the merged
+// values kept between two passes over the list, a second flag per vortex and
+// four entries of each candidate cleared, 190 / 1250 / 13,300 and 94 / 236.
 template <int PASS>
 VX_DEVK void k_col_settle_body(VxBlkB<1024, 0> vb, const VxView &v, VxScalars *S, const int *cand, int *col,
-                               int *in_cnt, int *has_app, int *first_app, int *cstate, int *cdec, double *mx,
-                               double *my, double *mg, const int *slot, ColRec *rec, double drop_eps, int track,
-                               const VxCompact &cmp, long long limit) {
+                               int *in_cnt, int *first_app, int *cstate, int *cdec, const int *slot, ColRec *rec,
+                               double drop_eps, int track, int counted, const VxCompact &cmp, long long limit) {
     if (threadIdx.x == 0) S->cmp_many = 0;
     if (S->col_done) return;
     __shared__ int undecided, listed;
     const int nc = S->ncand;
     if (threadIdx.x == 0) listed = 0;
-    for (int k = threadIdx.x; k < nc; k += blockDim.x) {
-        cstate[k] = 0;
-        atomicAdd(&in_cnt[INT_MAX - col[cand[k]]], 1);
-    }
+    if (!counted)
+        for (int k = threadIdx.x; k < nc; k += blockDim.x) atomicAdd(&in_cnt[INT_MAX - col[cand[k]]], 1);
     __syncthreads();
     const int max_rounds = nc + 2;
     int round = 0;
     for (; round < max_rounds; ++round) {
-        for (int k = threadIdx.x; k < nc; k += blockDim.x) {
-            int d = 0;
-            if (cstate[k] == 0) {
-                const int i = cand[k];
-                if (has_app[i]) d = 2;
-                else if (in_cnt[i] == 0) d = 1;
-            }
-            cdec[k] = d;
-        }
-        if (threadIdx.x == 0) undecided = 0;
-        __syncthreads();
-        for (int k = threadIdx.x; k < nc; k += blockDim.x) {
-            if (cstate[k] != 0) continue;
-            const int d = cdec[k];
-            if (d == 0) { atomicAdd(&undecided, 1); continue; }
-            cstate[k] = d;
-            const int i = cand[k], j = INT_MAX - col[i];
-            atomicSub(&in_cnt[j], 1);
-            if (d == 1) {
-                has_app[j] = 1;
-                atomicMax(&first_app[j], INT_MAX - i);
-            }
-        }
+        if (nc > (int)blockDim.x) col_decide<4>(nc, cand, col, in_cnt, first_app, cstate, cdec, undecided);
+        else col_decide<1>(nc, cand, col, in_cnt, first_app, cstate, cdec, undecided);
         __syncthreads();
         if (undecided == 0) break;
         __syncthreads();
     }
     const bool failed = round >= max_rounds;
-    if (!failed)
-        for (int k = threadIdx.x; k < nc; k += blockDim.x) {
-            if (cstate[k] != 1) continue;
+    for (int k0 = 0; k0 < nc; k0 += blockDim.x) {
+        const int k = k0 + threadIdx.x;
+        int moved = -1;   // slot of a vortex the second round starts from
+        if (k < nc) {
             const long long i = cand[k], j = INT_MAX - col[i];
-            const double xi = v.x[i * v.ps], yi = v.y[i * v.ps], gi = v.g[i * v.ps];
-            double xj = 1e10, yj = 1e10, gj = 0.0;
-            if (first_app[j] == (int)(INT_MAX - i)) { xj = v.x[j * v.ps]; yj = v.y[j * v.ps]; gj = v.g[j * v.ps]; }
-            if (PASS == 1) {
-                const double ai = fabs(gi), aj = fabs(gj);
-                const double mn = ai + aj;
-                mx[k] = (xi * ai + xj * aj) / fabs(mn);
-                my[k] = (yi * ai + yj * aj) / fabs(mn);
-                mg[k] = gi + gj;
-            } else {
-                const double ng = gi + gj;
-                mx[k] = (xi * gi + xj * gj) / ng;
-                my[k] = (yi * gi + yj * gj) / ng;
-                mg[k] = ng;
+            if (!failed && cstate[k] == 1) {
+                const double xi = v.x[i * v.ps], yi = v.y[i * v.ps], gi = v.g[i * v.ps];
+                const bool first = first_app[j] == (int)(INT_MAX - i);
+                double xj = 1e10, yj = 1e10, gj = 0.0, x, y, g;
+                if (first) { xj = v.x[j * v.ps]; yj = v.y[j * v.ps]; gj = v.g[j * v.ps]; }
+                if (PASS == 1) {
+                    const double ai = fabs(gi), aj = fabs(gj);
+                    const double mn = ai + aj;
+                    x = (xi * ai + xj * aj) / fabs(mn);
+                    y = (yi * ai + yj * aj) / fabs(mn);
+                    g = gi + gj;
+                } else {
+                    g = gi + gj;
+                    x = (xi * gi + xj * gj) / g;
+                    y = (yi * gi + yj * gj) / g;
+                }
+                v.x[i * v.ps] = x; v.y[i * v.ps] = y; v.g[i * v.ps] = g;
+                const bool left = fabs(g) >= drop_eps;   // else the compaction removes it
+                if (!left) vx_set_dead(cmp.bits, i);
+                else if (!(fabs(gi) >= drop_eps)) atomicAnd(&cmp.bits[i >> 5], ~(1u << (i & 31)));   // marked by the scatter
+                if (track) {
+                    const int si = slot[i];
+                    ColRec *r = rec + si;
+                    r->x = x; r->y = y; r->g = left ? g : 0.0;
+                    if (left) moved = si;
+                }
+                if (first) {
+                    v.x[j * v.ps] = 1e10; v.y[j * v.ps] = 1e10; v.g[j * v.ps] = 0.0;
+                    if (!(0.0 >= drop_eps)) vx_set_dead(cmp.bits, j);
+                    if (track) rec[slot[j]].g = 0.0;
+                    first_app[j] = 0;
+                }
             }
+            // the next round finds the entries clear (every decision took its
+            // candidate off in_cnt)
+            col[i] = 0;
+            if (failed) in_cnt[j] = first_app[j] = 0;
         }
-    __syncthreads();
-    for (int k = threadIdx.x; k < nc; k += blockDim.x) {
-        const long long i = cand[k], j = INT_MAX - col[i];
-        if (!failed && cstate[k] == 1) {
-            const bool weak = !(fabs(v.g[i * v.ps]) >= drop_eps);
-            v.x[i * v.ps] = mx[k]; v.y[i * v.ps] = my[k]; v.g[i * v.ps] = mg[k];
-            v.x[j * v.ps] = 1e10; v.y[j * v.ps] = 1e10; v.g[j * v.ps] = 0.0;
-            const bool left = fabs(mg[k]) >= drop_eps;   // else the compaction removes it
-            if (!(0.0 >= drop_eps)) vx_set_dead(cmp.bits, j);
-            if (!left) vx_set_dead(cmp.bits, i);
-            else if (weak) atomicAnd(&cmp.bits[i >> 5], ~(1u << (i & 31)));   // marked by the scatter
-            if (track) {
-                ColRec *r = rec + slot[i];
-                r->x = mx[k]; r->y = my[k]; r->g = left ? mg[k] : 0.0;
-                rec[slot[j]].g = 0.0;
-                if (left) cdec[atomicAdd(&listed, 1)] = slot[i];
-            }
+        if (track) {
+            const unsigned w = __ballot_sync(0xffffffffu, moved >= 0);
+            int at = 0;
+            if ((threadIdx.x & 31) == 0 && w) at = atomicAdd(&listed, __popc(w));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(w & ((1u << (threadIdx.x & 31)) - 1u));
+            if (moved >= 0) cdec[at] = moved;
         }
-        col[i] = 0;   // the next round finds the entries clear
-        in_cnt[j] = 0; has_app[j] = 0; first_app[j] = 0;
     }
     __syncthreads();
     // the round's compaction (none after a failed one); one that removes
@@ -377,13 +421,12 @@ VX_DEVK void k_col_settle_body(VxBlkB<1024, 0> vb, const VxView &v, VxScalars *S
 }
 template <int PASS>
 __global__ void __launch_bounds__(1024) k_col_settle(VxView v, VxScalars *S, const int *cand, int *col,
-                                                     int *in_cnt, int *has_app, int *first_app, int *cstate,
-                                                     int *cdec, double *mx, double *my, double *mg, const int *slot,
-                                                     ColRec *rec, double drop_eps, int track, VxCompact cmp,
-                                                     long long limit) {
+                                                     int *in_cnt, int *first_app, int *cstate, int *cdec,
+                                                     const int *slot, ColRec *rec, double drop_eps, int track,
+                                                     int counted, VxCompact cmp, long long limit) {
     VX_PDL_WAIT();
-    k_col_settle_body<PASS>(VxBlkB<1024, 0>{blockIdx.x, gridDim.x}, v, S, cand, col, in_cnt, has_app, first_app,
-                            cstate, cdec, mx, my, mg, slot, rec, drop_eps, track, cmp, limit);
+    k_col_settle_body<PASS>(VxBlkB<1024, 0>{blockIdx.x, gridDim.x}, v, S, cand, col, in_cnt, first_app,
+                            cstate, cdec, slot, rec, drop_eps, track, counted, cmp, limit);
 }
 
 template <int PASS>
@@ -398,15 +441,15 @@ static cudaError_t collapse_pass(const VxLaunch &L, const VxParams &p, const VxV
     for (int cc = 0; cc < n_col; ++cc) {
         const int track = cc == 0 && n_col > 1;
         if (cc == 1) {
-            vx_launch<k_col_query_moved<PASS>, k_col_query_moved_body<PASS>>(L, grid, VX_THREADS, 0, p, S, w.cell_start, (const ColRec *)rec, (const int *)w.cdec, w.col, w.cand);
+            vx_launch<k_col_query_moved<PASS>, k_col_query_moved_body<PASS>>(L, grid, VX_THREADS, 0, p, S, w.cell_start, (const ColRec *)rec, (const int *)w.cdec, w.col, w.cand, w.cstate);
         } else {
             vx_launch<k_col_prep, k_col_prep_body>(L, grid, VX_THREADS, 0, v, S, cc == 0, r2, w.cells_cap, w.box);
             vx_launch<k_col_count, k_col_count_body>(L, grid, VX_THREADS, 0, v, S, w.cellid, w.cell_cnt);
             vx_launch<k_col_scan, k_col_scan_body>(L, grid, VX_SCAN_T, 0, S, w.cell_cnt, w.cell_start, w.scan_tiles);
             vx_launch<k_col_scatter, k_col_scatter_body>(L, grid, VX_THREADS, 0, v, S, w.cell_start, w.cellid, rec, p.drop_eps, w.cmp.bits);
-            vx_launch<k_col_query<PASS>, k_col_query_body<PASS>>(L, grid, VX_THREADS, 0, p, S, w.cell_start, (const ColRec *)rec, w.col, w.cand);
+            vx_launch<k_col_query<PASS>, k_col_query_body<PASS>>(L, grid, VX_THREADS, 0, p, S, w.cell_start, (const ColRec *)rec, w.col, w.cand, w.cstate, w.in_cnt);
         }
-        vx_launch<k_col_settle<PASS>, k_col_settle_body<PASS>>(L, 1, 1024, 0, v, S, w.cand, w.col, w.in_cnt, w.has_app, w.first_app, w.cstate, w.cdec, w.mx, w.my, w.mg, w.cellid, rec, p.drop_eps, track, w.cmp, small ? w.cap : VX_CMP_FEW);
+        vx_launch<k_col_settle<PASS>, k_col_settle_body<PASS>>(L, 1, 1024, 0, v, S, w.cand, w.col, w.in_cnt, w.first_app, w.cstate, w.cdec, w.cellid, rec, p.drop_eps, track, cc != 1, w.cmp, small ? w.cap : VX_CMP_FEW);
         if (!small) vx_launch_moves(L, v, S, w, w.cellid, track ? &rec[0].i : nullptr);
     }
     return cudaGetLastError();

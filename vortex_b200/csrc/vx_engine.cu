@@ -330,10 +330,9 @@ static vx_status work_alloc_impl(VxWork &w, std::vector<void *> *allocs, long lo
     // reads them zeroes them), and so are the per-candidate arrays, so they
     // start at zero
     if ((st = dalloc_zero(allocs, &w.bytes, &w.cell_cnt, w.cells_cap, stream, cv)) != VX_OK) return st;
-    if ((st = dalloc_zero(allocs, &w.bytes, &w.col, 4 * cap, stream, cv)) != VX_OK) return st;
-    if (w.col) { w.in_cnt = w.col + cap; w.has_app = w.in_cnt + cap; w.first_app = w.has_app + cap; }
+    if ((st = dalloc_zero(allocs, &w.bytes, &w.col, 3 * cap, stream, cv)) != VX_OK) return st;
+    if (w.col) { w.in_cnt = w.col + cap; w.first_app = w.in_cnt + cap; }
     A(w.cand, cap); A(w.cstate, cap); A(w.cdec, cap);
-    A(w.mx, cap); A(w.my, cap); A(w.mg, cap);
     // pair partials: K * n <= num_sms*8*tile + n for the split K the launchers pick
     w.part_cap = 5LL * ((long long)num_sms * 8 * 1024 + cap + 1024);
     A(w.part, w.part_cap);

@@ -150,8 +150,7 @@ struct VxWork {
     // collapse
     long long cells_cap;
     int *cellid, *cell_cnt, *cell_start;
-    int *col, *in_cnt, *has_app, *first_app, *cand, *cstate, *cdec;
-    double *mx, *my, *mg;
+    int *col, *in_cnt, *first_app, *cand, *cstate, *cdec;
     // pair partial sums
     double *part;
     long long part_cap;      // doubles
