@@ -49,46 +49,48 @@ void vx_keep_pool(int device) {
     if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
 }
 
-// What the bodies of one device share, for as long as there is one: host memory
-// for the copies of their scalars (page-locked: a copy from the device takes 10.5
-// us, 12.9 into pageable memory), and up to 64 MB of freed memory left in the
-// device's pool, about one small body's worth, so that a body that follows
-// another one does not map it afresh.  The last body to be closed gives both
-// back, as a pool that no body uses is only lost to others: a body created and
-// closed beside another takes 1.5 ms at 200 panels and 3.8 at 1000, by itself 2.1 and
-// 4.8 (0.75 and 3.4 with both kept for good).  Each handle's own cudaMallocHost took
-// 2 ms where no other page-locked memory was.
+// What the bodies of one device share: host memory for the copies of their
+// scalars (page-locked: a copy from the device takes 10.5 us, 12.9 into pageable
+// memory), and, for as long as there is one, up to 64 MB of freed memory left in
+// the device's pool, about one small body's worth, so that a body that follows
+// another one does not map it afresh.  The last body to be closed gives the pool's
+// memory back, as it is only lost to others then, and all blocks of host memory but
+// one (36 KB).  A body created and closed by itself takes 1.55 ms at 200 panels and
+// 4.25 at 1000, beside another 1.5 and 3.8.  Each handle's own cudaMallocHost took 2
+// ms where no other page-locked memory was, a block registered anew 0.5.
 //
 // The blocks are the process's own memory, registered with one device: should
 // a caller reset that device, its bodies are lost with it, but the scalars of
-// the others stay where they are, and a slot taken from a block that is not
-// registered any more is ordinary memory.  Any thread may take and give slots.
+// the others stay where they are.  A block that the reset has unregistered is
+// registered again when the next body takes its first slot; a slot taken beside
+// bodies that were lost is ordinary memory.  Any thread may take and give slots.
 constexpr size_t POOL_KEEP = 64 << 20;
 namespace {
 class BodyShare {
 public:
-    VxScalars *take(int device) {
+    VxScalars *take(int device) {   // the current device
         std::lock_guard<std::mutex> lock(mu_);
         for (Block &b : blocks_)
-            if (b.device == device && b.used != ~0ull) return slot(b);
-        void *m = std::aligned_alloc(4096, BYTES);
+            if (b.device == device && b.used != ~0ull) return b.used || lock_pages(b.base) ? slot(b) : nullptr;
+        char *m = static_cast<char *>(std::aligned_alloc(4096, BYTES));
         if (!m) return nullptr;
-        if (cudaHostRegister(m, BYTES, cudaHostRegisterDefault) != cudaSuccess) {
-            cudaGetLastError();
+        if (!lock_pages(m)) {
             std::free(m);
             return nullptr;
         }
-        blocks_.push_back(Block{static_cast<char *>(m), device, 0});
+        blocks_.push_back(Block{m, device, 0});
         return slot(blocks_.back());
     }
-    void give(VxScalars *p) {   // the slot's device is the current one
+    void give(VxScalars *p) {   // of the current device
         std::lock_guard<std::mutex> lock(mu_);
         const char *c = reinterpret_cast<char *>(p);
         for (size_t k = 0; k < blocks_.size(); ++k) {
             Block &b = blocks_[k];
             if (c < b.base || c >= b.base + BYTES) continue;
             b.used &= ~(1ull << ((c - b.base) / STRIDE));
-            if (b.used == 0) {
+            int same = 0;
+            for (const Block &o : blocks_) same += o.device == b.device;
+            if (b.used == 0 && same > 1) {
                 if (cudaHostUnregister(b.base) != cudaSuccess) cudaGetLastError();
                 std::free(b.base);
                 blocks_.erase(blocks_.begin() + (long)k);
@@ -99,7 +101,7 @@ public:
     bool live(int device) {
         std::lock_guard<std::mutex> lock(mu_);
         for (const Block &b : blocks_)
-            if (b.device == device) return true;
+            if (b.device == device && b.used) return true;
         return false;
     }
 
@@ -107,10 +109,17 @@ private:
     struct Block {
         char *base;
         int device;
-        unsigned long long used;   // a bit per slot; a block without any is given back
+        unsigned long long used;   // a bit per slot
     };
     static constexpr size_t STRIDE = (sizeof(VxScalars) + 255) / 256 * 256;
     static constexpr size_t BYTES = (64 * STRIDE + 4095) / 4096 * 4096;
+    static bool lock_pages(char *m) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, m) == cudaSuccess && a.type == cudaMemoryTypeHost) return true;
+        if (cudaHostRegister(m, BYTES, cudaHostRegisterDefault) == cudaSuccess) return true;
+        cudaGetLastError();
+        return false;
+    }
     static VxScalars *slot(Block &b) {
         const int k = __builtin_ctzll(~b.used);
         b.used |= 1ull << k;
