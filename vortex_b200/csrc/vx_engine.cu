@@ -49,24 +49,29 @@ void vx_keep_pool(int device) {
     if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
 }
 
-// What the bodies of one device share: host memory for the copies of their
-// scalars (page-locked: a copy from the device takes 10.5 us, 12.9 into pageable
-// memory), and, for as long as there is one, up to 64 MB of freed memory left in
-// the device's pool, about one small body's worth, so that a body that follows
-// another one does not map it afresh.  The last body to be closed gives the pool's
-// memory back, as it is only lost to others then, and all blocks of host memory but
-// one (36 KB).  A body created and closed by itself takes 1.55 ms at 200 panels and
-// 4.25 at 1000, beside another 1.5 and 3.8.  Each handle's own cudaMallocHost took 2
-// ms where no other page-locked memory was, a block registered anew 0.5.
+// A destroyed handle's stream-ordered memory goes back to the driver (the
+// pool keeps it otherwise, out of reach of plain cudaMalloc callers).  64 MB left
+// in the pool would save a body created and closed by itself 0.8 ms (200 panels
+// 1.55, 1000 panels 4.25), and beside another body, which uses as much, nothing.
+void vx_trim_pool(int device) {
+    cudaMemPool_t pool;
+    if (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess) { cudaGetLastError(); return; }
+    if (cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
+}
+
+// Host memory for the copies of the bodies' scalars, page-locked (a copy from the
+// device takes 10.5 us, 12.9 into pageable memory): blocks of slots that a device's
+// bodies share.  All blocks without a body but one a device (32 KB) are given
+// back.  Each handle's own cudaMallocHost took 2 ms where no other page-locked
+// memory was, a block registered anew takes 0.5.
 //
 // The blocks are the process's own memory, registered with one device: should
 // a caller reset that device, its bodies are lost with it, but the scalars of
 // the others stay where they are.  A block that the reset has unregistered is
 // registered again when the next body takes its first slot; a slot taken beside
 // bodies that were lost is ordinary memory.  Any thread may take and give slots.
-constexpr size_t POOL_KEEP = 64 << 20;
 namespace {
-class BodyShare {
+class ScalarSlots {
 public:
     VxScalars *take(int device) {   // the current device
         std::lock_guard<std::mutex> lock(mu_);
@@ -98,12 +103,6 @@ public:
             return;
         }
     }
-    bool live(int device) {
-        std::lock_guard<std::mutex> lock(mu_);
-        for (const Block &b : blocks_)
-            if (b.device == device && b.used) return true;
-        return false;
-    }
 
 private:
     struct Block {
@@ -128,19 +127,11 @@ private:
     std::mutex mu_;
     std::vector<Block> blocks_;
 };
-BodyShare &body_share() {
-    static BodyShare *p = new BodyShare();   // never destroyed: handles may outlive static destructors
+ScalarSlots &scalar_slots() {
+    static ScalarSlots *p = new ScalarSlots();   // never destroyed: handles may outlive static destructors
     return *p;
 }
 }  // namespace
-
-// Freed memory of the pool back to the driver, out of reach of plain cudaMalloc
-// callers until then.
-void vx_trim_pool(int device) {
-    cudaMemPool_t pool;
-    if (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess) { cudaGetLastError(); return; }
-    if (cudaMemPoolTrimTo(pool, body_share().live(device) ? POOL_KEEP : 0) != cudaSuccess) cudaGetLastError();
-}
 
 extern "C" const char *vx_status_str(vx_status s) {
     switch (s) {
@@ -625,7 +616,7 @@ extern "C" vx_status vx_create(const vx_conf *conf, const vx_panel *pan, int64_t
     PanelLists wall, hit;
     build_wall_lists(s->prm, pan, (int)P, wall);
     build_hit_lists(s->prm, pan, (int)P, hit);
-    s->h_S = body_share().take(device);
+    s->h_S = scalar_slots().take(device);
     if (!s->h_S) { vx_set_error("vx_create: no pinned memory"); return fail(VX_ERR_NOMEM); }
     memset(s->h_S, 0, sizeof(VxScalars));
     // V_inf ramp (src/main.c:585-592): with a ramp the flow starts at rest
@@ -709,7 +700,7 @@ extern "C" vx_status vx_destroy(vx_sim *s) {
     for (double *a : arr) if (a) cudaFreeAsync(a, s->stream);
     if (s->d_fixed) cudaFreeAsync(s->d_fixed, s->stream);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    if (s->h_S) body_share().give(s->h_S);
+    if (s->h_S) scalar_slots().give(s->h_S);
     if (s->d_probe) cudaFree(s->d_probe);
     if (s->d_pts) cudaFree(s->d_pts);
     if (s->d_St) cudaFree(s->d_St);
