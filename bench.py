@@ -120,16 +120,16 @@ def workload_config(args, world: int) -> dict:
 HBM_BYTES = {
     "k_advect": (64, "read x, y, G, Vx, Vy; write x, y, G"),
     "k_fmm_prep": (16, "read x, y"),
-    "k_fmm_leafid": (24, "read x, y; write leaf key and index"),
+    "k_fmm_leafid": (24, "read x, y; write leaf key and rank in it"),
     "k_cg_prep": (24, "read x, y, d"),
-    "k_cg_cellid": (24, "read x, y; write cell key and index"),
+    "k_cg_cellid": (24, "read x, y; write cell key and rank in it"),
     "k_bk_place": (64, "read key, rank, x, y, G; write the 32-byte record at the bucket slot"),
     "k_bk_order": (56, "read the record; write key, index and float4"),
     "k_col_prep": (16, "read x, y"),
-    "k_col_count": (32, "read x, y; write cell id, in-count and the two merge flags"),
-    "k_col_scatter": (64, "read cell id, cell start, x, y, G; write the 32-byte cell-sorted record"),
-    "k_col_query<2>": (36, "read the cell-sorted record (x, y, G, index); write COL"),
-    "k_col_query<1>": (36, "read the cell-sorted record (x, y, G, index); write COL"),
+    "k_col_count": (20, "read x, y; write the rank in the cell"),
+    "k_col_scatter": (64, "read rank, x, y, G; write slot and the 32-byte cell-sorted record"),
+    "k_col_query<2>": (32, "read the cell-sorted record (x, y, G, index)"),
+    "k_col_query<1>": (32, "read the cell-sorted record (x, y, G, index)"),
     "k_cmp_mark": (8, "read G"),
 }
 
