@@ -336,8 +336,8 @@ def run_ours(args, rank, world, device):
     value = world * 1e3 * K / total_ms
     mp = measured_peaks()
     hbm_peak = float(mp.get("hbm_gbs") or 6650.0)
-    hbm_src = "MEASURED_PEAKS.json hbm_gbs (copy bandwidth measured on this pool)" if mp.get("hbm_gbs") else \
-        "fallback 6.65 TB/s (earlier measurement on this pool)"
+    hbm_src = "MEASURED_PEAKS.json hbm_gbs (copy bandwidth measured on a B200)" if mp.get("hbm_gbs") else \
+        "fallback 6.65 TB/s (earlier measurement on a B200)"
     eff = float(np.mean([n * ((n + 31) // 32 * 32) for n in nvec]))
     achieved = kflop * kpairs / (kms * 1e-3) / 1e12
     traffic = None
